@@ -35,9 +35,10 @@ WORKLOAD = dict(name="bist_stream_480x854_T30", H=480, W=854, T=30, nseeds=400, 
                 sigma2_app=0.009 ** 2, alpha=math.log(0.5), split_alpha=0.0)
 # Algorithmic bytes of one BASS pass (the scope's measurement rules): 4 sweeps x (label
 # read 4 + image read 12 + label write 4) + the statistics of the new labels 16 = 96 B/px.
-# The 4 sweep launches of an update do the whole pass: they keep the statistics current
-# by moving those of every relabelled pixel (incremental statistics), so no separate
-# statistics pass runs between two updates: 24 B/px per sweep launch on average.
+# The sweeps of an update do the whole pass: they keep the statistics current by moving
+# those of every relabelled pixel (incremental statistics), so no separate statistics pass
+# runs between two updates: 24 B/px per sweep, and a launch runs all 4 sweeps of an update
+# (one or two with --sweep-schedule / --sweep-tile / --sweep-queue).
 SWEEP_BYTES_PER_PX = 24
 # DRAM bytes (read + write) per sweep launch from one ncu capture of the same workload
 # (a batch of 8 frames, mean of a full and an active-set sweep); a constant of that
@@ -753,7 +754,7 @@ def run_precision(args, world, rank):
         res["superpixels"] = int(live.sum())
         per_frame.append(res)
     # per-kernel bandwidth of the int64 run at 4K (CUDA events)
-    bytes_per_px = {"kb_sweep_t32": 20, "kb_sweep_t64": 20, "kb_accumulate": 16}
+    bytes_per_px = {"kb_sweep4_m": 80, "kb_sweep4_l": 80, "kb_accumulate": 16}
     gbs = {}
     for k, (nl, ms) in kern.items():
         if k in bytes_per_px and ms > 0:
@@ -806,11 +807,10 @@ def main():
     ap.add_argument("--fps", type=float, default=30.0, help="serve: mean frame rate per stream")
     ap.add_argument("--frames", type=int, default=30, help="serve: frames per stream")
     ap.add_argument("--sweep-schedule", type=int, default=0, choices=[0, 1, 2],
-                    help="stream: boundary sweeps per launch (0 autotuned, 1 one, 2 two); "
+                    help="stream: boundary sweeps per launch (0 four, 1 one, 2 two); "
                          "the labels are the same")
     ap.add_argument("--sweep-tile", type=int, default=0, choices=[0, 16, 32, 64],
-                    help="stream: single-sweep tile width (0 autotuned); profiler runs pin "
-                         "the width the autotuner picks without the profiler")
+                    help="stream: single-sweep tile width (0: the default four-sweep launches)")
     ap.add_argument("--sweep-queue", type=int, default=0, choices=[0, 1],
                     help="stream: 1 runs single sweeps as the persistent work-queue kernel")
     ap.add_argument("--no-group-sizes", action="store_true",
@@ -1123,10 +1123,12 @@ def main():
     npix = w["H"] * w["W"]
     B0 = len(lanes[0])
     fam = max(prof, key=lambda k: prof[k][1])
-    nsweep = prof["sweep"][0]       # one fused launch per sweep, over the lane's batch
+    nsweep = prof["sweep"][0]       # launches over the lane's batch
+    per_sweeps = (2 if args.sweep_schedule == 2 else
+                  1 if args.sweep_schedule or args.sweep_tile or args.sweep_queue else 4)
     sweep_ms = prof["sweep"][1]
     peak, peak_kind = read_peaks()
-    per_launch = SWEEP_BYTES_PER_PX * npix * B0
+    per_launch = SWEEP_BYTES_PER_PX * per_sweeps * npix * B0
     achieved = per_launch * nsweep / (sweep_ms / 1000.0) / 1e9 if sweep_ms else 0
     passes_per_video = w["niters"] + (T - 1) * w["prop_niters"]
     mpix_pass = world * S * args.steps * passes_per_video * npix / elapsed / 1e6
@@ -1164,7 +1166,7 @@ def main():
         "plain_per_frame_fps": plain_fps,
         "plain_vs_batched_label_agreement": agree,
         "mpix_per_s_per_pass": mpix_pass,
-        "roofline": {"bound": "hbm", "kernel": "kb_sweep (border + 4 parity phases, batched; statistics fused into the last sweep of each update)",
+        "roofline": {"bound": "hbm", "kernel": "kb_sweep4 (the 4 sweeps of an update, border + 4 parity phases each, batched; statistics of the relabelled pixels moved)",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if peak else None, "traffic": SWEEP_TRAFFIC_NCU["bytes_per_launch"],
                      "traffic_source": SWEEP_TRAFFIC_NCU["source"],

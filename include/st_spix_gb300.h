@@ -83,14 +83,14 @@ typedef struct stspix_config {
                             (default, exact and order-independent), 1 FP32 atomics (as
                             the reference; order-dependent), 2 FP64 atomics -- 1 and 2
                             exist for the accumulator precision study               */
-  int   sweep_schedule;  /* boundary sweeps per launch: 0 autotuned (default), 1 one,
+  int   sweep_schedule;  /* boundary sweeps per launch: 0 up to four (default), 1 one,
                             2 two whenever two remain; the labels are the same       */
-  int   sweep_tile;      /* tile width: 0 autotuned (default), or 16, 32, 64 (no
-                            timing; schedules 0 and 1 then run single sweeps of that
+  int   sweep_tile;      /* tile width: 0 chosen by the batch's size (default), or 16,
+                            32, 64 (schedules 0 and 1 then run single sweeps of that
                             width, schedule 2 two-sweep launches of that width)      */
-  int   sweep_queue;     /* single-sweep launches: 0 one block per tile (default), 1 a
-                            persistent work-queue kernel (one resident block set that
-                            takes tiles from an atomic counter); same labels         */
+  int   sweep_queue;     /* 1 runs single sweeps as a persistent work-queue kernel (one
+                            resident block set that takes tiles from an atomic
+                            counter); 0 one block per tile (default); same labels    */
   int   lab_ingest;      /* 0 frames used as given (default; the reference's
                             bist_forward ignores its rgb2lab flag), 1 every frame is
                             converted sRGB -> CIELAB (the reference's rgb2lab steps,
@@ -148,9 +148,9 @@ long long   stspix_kernel_launches(const stspix_ctx* ctx);
  * step whose frame sizes, capacities, iteration counts and configuration repeat is
  * captured on its second occurrence and replayed from then on).                    */
 long long   stspix_graph_replays(const stspix_ctx* ctx);
-/* The sweep autotuner's choices, entry idx (0..): *tiles_class = the batch's 32x32 tile
- * count class (4 log2 tiles), *single_w = the single-sweep tile width, *pair_w = the
- * two-sweep width (0: single sweeps only).  Returns 1 while idx is an entry, else 0.  */
+/* The tiles the default sweep schedule used, entry idx (0..): *tiles_class = the batch's
+ * 32x32 tile count class (4 log2 tiles), *single_w = *pair_w = the tile width of its
+ * launches.  Returns 1 while idx is an entry, else 0.                                 */
 int         stspix_sweep_choice(const stspix_ctx* ctx, int idx, int* tiles_class, int* single_w,
                                 int* pair_w);
 /* Enable (default) or disable the capture and replay of repeated batch steps; with

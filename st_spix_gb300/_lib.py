@@ -219,7 +219,7 @@ class Context:
         return int(self.lib.stspix_graph_replays(self.handle))
 
     def sweep_choices(self) -> list:
-        """The autotuner's (tile-count class, single width, pair width or 0) entries."""
+        """The default sweep schedule's (tile-count class, tile width, tile width) entries."""
         out, i = [], 0
         a, b, c = C.c_int(0), C.c_int(0), C.c_int(0)
         while self.lib.stspix_sweep_choice(self.handle, i, C.byref(a), C.byref(b), C.byref(c)):

@@ -74,7 +74,7 @@ struct List {
   int B = 0;
   int max_npix = 0, max_cap = 0, max_nprev = 0, max_w = 0, max_h = 0;
   bool any_prop = false;
-  std::vector<int> tiles_upto[3];  // sweep tiles (32-, 64-, 16-wide) of the first i slots
+  std::vector<int> tiles_upto[kSweepGeoms];  // sweep tiles of the first i slots, per tile size
   std::vector<long long> segs_upto;  // 32-pixel row segments of the first i slots
 };
 
@@ -111,10 +111,7 @@ struct stspix_ctx {
   // hole-fill loop graphs (conditional WHILE node), per (slot table, batch size)
   struct FillGraph { cudaGraph_t g; cudaGraphExec_t exec; };
   std::map<std::pair<const Slot*, int>, FillGraph> fill_graphs;
-  // sweep tile autotuner
-  std::map<std::pair<unsigned long long, int>, int> sweep_choice;  // (tile class, single forced) -> widths
-  cudaEvent_t tune_ev[kSweepVariants + 1] = {};
-  long long tunes = 0;
+  std::map<int, int> sweep_choice;  // four-sweep launches: size class -> tile (sweep_kernels)
   int accumulator = 0;            // cfg.accumulator of the batch being run
   int lab_ingest = 0;             // cfg.lab_ingest of the batch being run
   int* body_iters = nullptr;       // device: [0] fill-loop iterations run (launch count),
@@ -437,6 +434,9 @@ void preload_kernels() {
       (const void*)kb_sweep2_t32,
       (const void*)kb_sweep2_t16,
       (const void*)kb_sweep2_t64,
+      (const void*)kb_sweep4_s,
+      (const void*)kb_sweep4_m,
+      (const void*)kb_sweep4_l,
       (const void*)kb_sweepq_t32,
       (const void*)kb_sweepq_t64,
       (const void*)kb_sweepq_t16,
@@ -598,17 +598,16 @@ Slot make_slot(stspix_ctx* ctx, const FrameDesc& f, int cap) {
 List make_list(stspix_ctx* ctx, int off, const std::vector<Slot>& slots) {
   List L;
   L.d = ctx->d_slots + (size_t)off * ctx->bcap;
-  for (int v = 0; v < kSweepVariants; v++) L.tiles_upto[v].assign(1, 0);
+  for (int v = 0; v < kSweepGeoms; v++) L.tiles_upto[v].assign(1, 0);
   L.segs_upto.assign(1, 0);
   Slot* h = ctx->h_slots + (size_t)off * ctx->bcap;
   L.B = (int)slots.size();
   for (int i = 0; i < L.B; i++) {
     Slot s = slots[i];
-    for (int v = 0; v < kSweepVariants; v++) {
-      if (L.tiles_upto[v].empty()) L.tiles_upto[v].push_back(0);
+    for (int v = 0; v < kSweepGeoms; v++) {
       s.tile_base[v] = L.tiles_upto[v].back();
-      const int tw = kSweepTileW[v];
-      L.tiles_upto[v].push_back(s.tile_base[v] + ((s.W + tw - 1) / tw) * ((s.H + 31) / 32));
+      const int tw = kGeomW[v], th = kGeomH[v];
+      L.tiles_upto[v].push_back(s.tile_base[v] + ((s.W + tw - 1) / tw) * ((s.H + th - 1) / th));
     }
     if (L.segs_upto.empty()) L.segs_upto.push_back(0);
     L.segs_upto.push_back(L.segs_upto.back() + (long long)s.H * ((s.W + 31) / 32));
@@ -671,203 +670,104 @@ int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
   return STSPIX_OK;
 }
 
+// The sweep kernels by sweeps per launch (one, two, four) and tile.
+struct SweepKernel {
+  void (*fn)(const Slot*, int, int, int, float, float, int, int);
+  const char* name;
+  int geom, threads, smem;
+};
+#define SWEEP_KERNEL(k, geom, threads) SweepKernel{k, #k, geom, threads, k##_smem()}
+const SweepKernel (*sweep_kernels())[3] {
+  static const SweepKernel t[3][3] = {
+      {SWEEP_KERNEL(kb_sweep_t32, 0, 256), SWEEP_KERNEL(kb_sweep_t64, 1, 256),
+       SWEEP_KERNEL(kb_sweep_t16, 2, 256)},
+      {SWEEP_KERNEL(kb_sweep2_t32, 0, 256), SWEEP_KERNEL(kb_sweep2_t64, 1, 256),
+       SWEEP_KERNEL(kb_sweep2_t16, 2, 256)},
+      {SWEEP_KERNEL(kb_sweep4_s, 0, 512), SWEEP_KERNEL(kb_sweep4_m, 1, 256),
+       SWEEP_KERNEL(kb_sweep4_l, 3, 256)}};
+  return t;
+}
+#undef SWEEP_KERNEL
+
 // update_seg (update_seg.cu:281-311): niters_seg fused sweeps ping-ponging between
 // the labels and a scratch buffer; the border mask is only built when the next
 // iteration's merge reads it.
+// *cur: the buffer that holds the labels, 0 the slot's labels (seg), 1 the scratch
+// (seg_alt); a launch reads buffer *cur and writes the other.  keep: the next step only
+// sweeps again and needs no labels in seg (statistics kept by the sweeps), so an odd
+// number of launches is not copied back.
 // fuse_stats: every sweep launch moves the statistics of the pixels it relabels
-// (incremental statistics, see kb_sweep_t*), so the statistics stay those of the
+// (incremental statistics, see sweep_tile), so the statistics stay those of the
 // current labels and the next update_params skips its clear and accumulate passes.
-// Not while tuning (the trial launches rerun the same sweep).  *fused tells whether
-// that happened.
-// first_active: the first sweep is an active-set sweep too (mode 2): only the
-// previous call's last-sweep changes (change plane 1) and the pixels next to a label
-// whose record the posterior between the calls changed can decide differently.  For
-// calls that follow one with *chg_ok set, with only an incremental posterior between.
-// *chg_ok: this call ran no tuning trials and an even number of launches, so change
-// plane 1 holds its last sweep's changes.
+// first_active: the first sweep scores only the pixels next to a change of the previous
+// call's last launch or to a label whose record the posterior between the calls changed
+// (mode 2).  For calls that follow one with *chg_ok set, with only an incremental
+// posterior between.
+// *chg_ok: this call copied no labels, so the change plane of its last launch and the two
+// label buffers are as that launch left them.
 int update_seg(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
-               const stspix_config& cfg, bool need_border, bool fuse_stats, bool* fused,
-               bool first_active = false, bool* chg_ok = nullptr) {
+               const stspix_config& cfg, bool need_border, bool keep, bool fuse_stats,
+               bool first_active, int* cur, bool* chg_ok) {
   ctx->cur_fam = STSPIX_FAM_SWEEP;
   const int nseg = cfg.niters_seg;
-  *fused = false;
-  if (chg_ok) *chg_ok = false;
-  // the first sweep of the call scores every border pixel; the later ones only the
-  // active set next to the previous sweep's changes (same labels, see kb_sweep_t*).
-  // Launch j reads the labels of parity j & 1 and writes the other buffer.
-  auto sweep1 = [&](int v, int parity, int mode, int stats) {
-    const unsigned g = (unsigned)std::max(1, L.tiles_upto[v][nb]);
-    if (cfg.sweep_queue) {
-      // persistent work queue: the blocks the SMs hold at once (6 per SM), at most one
-      // per tile
-      unsigned* q = (unsigned*)(ctx->body_iters + 2);
-      const unsigned gq = std::min<unsigned>(g, 6u * (unsigned)ctx->num_sms);
-      const int nt = (int)g;
-      if (v == 1)
-        LAUNCHG(kb_sweepq_t64, gq, 256, L.d, nb, nt, q, parity, cfg.sigma2_app, cfg.potts, mode,
-                stats);
-      else if (v == 2)
-        LAUNCHG(kb_sweepq_t16, gq, 256, L.d, nb, nt, q, parity, cfg.sigma2_app, cfg.potts, mode,
-                stats);
-      else
-        LAUNCHG(kb_sweepq_t32, gq, 256, L.d, nb, nt, q, parity, cfg.sigma2_app, cfg.potts, mode,
-                stats);
-      return;
-    }
-    if (v == 1)
-      LAUNCHG(kb_sweep_t64, g, 256, L.d, nb, parity, cfg.sigma2_app, cfg.potts, mode, stats);
-    else if (v == 2)
-      LAUNCHG(kb_sweep_t16, g, 256, L.d, nb, parity, cfg.sigma2_app, cfg.potts, mode, stats);
-    else
-      LAUNCHG(kb_sweep_t32, g, 256, L.d, nb, parity, cfg.sigma2_app, cfg.potts, mode, stats);
-  };
-  auto sweep2 = [&](int v, int parity, int mode, int stats) {   // v: 0 (32 wide), 1 (64), 2 (16)
-    const unsigned g = (unsigned)std::max(1, L.tiles_upto[v][nb]);
-    if (v == 2)
-      LAUNCHG(kb_sweep2_t16, g, 256, L.d, nb, parity, cfg.sigma2_app, cfg.potts, mode, stats);
-    else if (v == 1)
-      LAUNCHG(kb_sweep2_t64, g, 256, L.d, nb, parity, cfg.sigma2_app, cfg.potts, mode, stats);
-    else
-      LAUNCHG(kb_sweep2_t32, g, 256, L.d, nb, parity, cfg.sigma2_app, cfg.potts, mode, stats);
-  };
-  // Tile autotuner: the first update of a batch size class runs its first sweep with
-  // every single-sweep tile width and (with three or more sweeps) its second and
-  // third sweeps with every two-sweep width, each on the same input (a launch reads
-  // only the labels at its start, so all write the same output); the class keeps the
-  // fastest single width and, when the best two-sweep launch beats two single ones,
-  // two-sweep launches.  The class is the number of 32x32 tiles of the sweeping slots
-  // in quarter octaves: the choice depends on how well the tiles fill the SMs, and
-  // mixed serving batches then tune a handful of times.
-  const int tl = std::max(1, L.tiles_upto[0][nb]);
-  // (a forced single-sweep schedule keeps its own entries: its tuning skips the pairs)
-  const auto key = std::make_pair((unsigned long long)std::floor(4.0 * std::log2((double)tl)),
-                                  cfg.sweep_schedule == 1 ? 1 : 0);
-  auto ch = ctx->sweep_choice.find(key);
-  int done = 0, launch = 0;
-  int v1 = 1, v2 = -1;      // best single-sweep width, two-sweep width (-1: none)
   int forced = -1;     // the width stspix_config.sweep_tile pins
   for (int c = 0; c < kSweepVariants; c++)
     if (kSweepTileW[c] == cfg.sweep_tile) forced = c;
-  if (cfg.sweep_schedule == 2) {
-    v1 = forced >= 0 ? forced : 0;
-    v2 = v1;
-  } else if (forced >= 0) {
-    v1 = forced;
-    v2 = -1;
-  } else if (ch != ctx->sweep_choice.end()) {
-    v1 = ch->second & 0xff;
-    v2 = cfg.sweep_schedule == 1 ? -1 : (ch->second >> 8) - 1;
-  } else if (ctx->capturing) {
-    v1 = 1;     // no timing inside a graph capture (a replayed batch was tuned before)
-    v2 = -1;
-  } else if (nseg > 0) {
-    // the whole call's launch count is known only after tuning; the clear rides on the
-    // first launch, the accumulation on the last (decided when it is issued)
-    // Every trial runs kTuneRounds times and keeps its fastest run: other streams of
-    // the device (concurrent lanes) only ever slow a run down.
-    float t1[kSweepVariants];
-    for (int r = 0; r < kTuneRounds; r++) {
-      CK(cudaEventRecord(ctx->tune_ev[0], st));
-      for (int c = 0; c < kSweepVariants; c++) {
-        sweep1(c, 0, 0, 0);
-        CK(cudaEventRecord(ctx->tune_ev[c + 1], st));
-      }
-      CK(cudaEventSynchronize(ctx->tune_ev[kSweepVariants]));
-      for (int c = 0; c < kSweepVariants; c++) {
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, ctx->tune_ev[c], ctx->tune_ev[c + 1]);
-        t1[c] = r == 0 ? ms : std::min(t1[c], ms);
-      }
-    }
-    float best1 = t1[0];
-    v1 = 0;
-    for (int c = 1; c < kSweepVariants; c++)
-      if (t1[c] < best1) { best1 = t1[c]; v1 = c; }
-    // Large batches keep the widest tile (the least halo work per pixel: 1.41 staged
-    // labels per pixel against 1.56 for 32x32) unless another width is 5 % faster:
-    // with other lanes' kernels on the SMs the total work decides, and timings of
-    // 64x32 and 32x32 alone differ by less than their noise (batches of 8 480x854
-    // frames on three lanes: 1545 frames/s when one lane picked 32x32, 1635-1642
-    // with 64x32 on all).
-    if (tl >= kPairMaxTiles && t1[1] <= kWideMargin * best1) {
-      best1 = t1[1];
-      v1 = 1;
-    }
-    done = 1;
-    launch = 1;
-    // Large batches keep single sweeps: a two-sweep launch holds more registers (4
-    // blocks per SM against 6), which costs more than its timing alone shows once other
-    // lanes' kernels share the SMs (batches of 8 480x854 frames on three lanes: 1532-1535
-    // frames/s when one lane picked 64x32 pairs, 1624-1631 with single sweeps on all).
-    if (nseg >= 3 && cfg.sweep_schedule == 0 && tl < kPairMaxTiles) {
-      // a two-sweep launch is an active-set sweep plus a full-listing one: with four or
-      // more sweeps the second sweep runs alone (timed, active set) and the pair covers
-      // the third and fourth, and the pair is compared with that sweep plus a full one
-      float ref = 2.f * best1;
-      if (nseg >= 4) {
-        float ms1 = 0.f;
-        for (int r = 0; r < kTuneRounds; r++) {
-          CK(cudaEventRecord(ctx->tune_ev[0], st));
-          sweep1(v1, launch & 1, 1, 0);
-          CK(cudaEventRecord(ctx->tune_ev[1], st));
-          CK(cudaEventSynchronize(ctx->tune_ev[1]));
-          float ms = 0.f;
-          cudaEventElapsedTime(&ms, ctx->tune_ev[0], ctx->tune_ev[1]);
-          ms1 = r == 0 ? ms : std::min(ms1, ms);
-        }
-        ref = best1 + ms1;
-        done = 2;
-        launch = 2;
-      }
-      // (both pair runs write the same labels; neither moves statistics, which would
-      // count them twice: a tuned call ends with a full statistics pass)
-      float t2[kSweepVariants];
-      for (int r = 0; r < kTuneRounds; r++) {
-        CK(cudaEventRecord(ctx->tune_ev[0], st));
-        for (int c = 0; c < kSweepVariants; c++) {
-          sweep2(c, launch & 1, 1, 0);
-          CK(cudaEventRecord(ctx->tune_ev[c + 1], st));
-        }
-        CK(cudaEventSynchronize(ctx->tune_ev[kSweepVariants]));
-        for (int c = 0; c < kSweepVariants; c++) {
-          float ms = 0.f;
-          cudaEventElapsedTime(&ms, ctx->tune_ev[c], ctx->tune_ev[c + 1]);
-          t2[c] = r == 0 ? ms : std::min(t2[c], ms);
-        }
-      }
-      float best2 = t2[0];
-      int b2 = 0;
-      for (int c = 1; c < kSweepVariants; c++)
-        if (t2[c] < best2) { best2 = t2[c]; b2 = c; }
-      v2 = best2 < ref ? b2 : -1;
-      done += 2;
-      launch += 1;
-    }
-    ctx->sweep_choice[key] = v1 | ((v2 + 1) << 8);
-    ctx->tunes++;
-    if (done >= nseg) {
-      if (launch & 1) LAUNCHB(kb_copy_labels, pix_units(L.max_npix), L, nb);
-      if (need_border) {
-        ctx->cur_fam = STSPIX_FAM_MERGE;
-        LAUNCHB(kb_find_border, pix_units(L.max_npix), L, nb);
-      }
-      return STSPIX_OK;
-    }
+  const bool queue = cfg.sweep_queue != 0;
+  // sweeps per launch: four, or one or two as stspix_config.sweep_schedule / _tile / _queue pin
+  const int per = queue || cfg.sweep_schedule == 1 ? 1
+                  : cfg.sweep_schedule == 2 ? 2 : forced >= 0 ? 1 : 4;
+  auto sweep_queue = [&](int v, int mode, int stats) {
+    // persistent work queue: the blocks the SMs hold at once (4 per SM), at most one per tile
+    unsigned* q = (unsigned*)(ctx->body_iters + 2);
+    const int nt = std::max(1, L.tiles_upto[v][nb]);
+    const unsigned gq = std::min<unsigned>((unsigned)nt, 4u * (unsigned)ctx->num_sms);
+    if (v == 1)
+      LAUNCHG(kb_sweepq_t64, gq, 256, L.d, nb, nt, q, *cur, cfg.sigma2_app, cfg.potts, mode, stats);
+    else if (v == 2)
+      LAUNCHG(kb_sweepq_t16, gq, 256, L.d, nb, nt, q, *cur, cfg.sigma2_app, cfg.potts, mode, stats);
+    else
+      LAUNCHG(kb_sweepq_t32, gq, 256, L.d, nb, nt, q, *cur, cfg.sigma2_app, cfg.potts, mode, stats);
+  };
+  auto sweep = [&](const SweepKernel& k, int ns, int mode, int stats) {
+    cudaEvent_t pe = prof_begin(ctx, st);
+    launch_k(k.fn, dim3((unsigned)std::max(1, L.tiles_upto[k.geom][nb])), dim3(k.threads),
+             (size_t)k.smem, st, ctx->capturing ? 0 : 1, (const Slot*)L.d, nb, *cur, ns,
+             cfg.sigma2_app, cfg.potts, mode, stats);
+    ctx->launches++;
+    prof_end(ctx, st, pe, k.name);
+  };
+  // The tile of the four-sweep launches, by the number of 32x32 tiles of the sweeping slots.
+  // Up to two per SM the launch is one tile's chain of phases: small tiles of 512 threads
+  // (a phase's pixels in one round).  Above eight per SM the total work decides: the tallest
+  // tile (the least halo); in between 64x32.  Measured, us for 3 frames of one video (20
+  // iterations; 2 frames in the batches), 32x32 / 64x32 / 64x48:
+  //   240x320 (80 tiles)     4204 / 4358 / 4569      360x640 (240)      4471 / 4479 / 4673
+  //   480x854 (405)          5546 / 5002 / 5129      720x1280 (920)     7358 / 5667 / 5729
+  //   4 x 480x854 (1620)     7472 / 5188 / 4771      1080x1920 (2040)  12165 / 8273 / 8089
+  const int tl = std::max(1, L.tiles_upto[0][nb]);
+  int v;
+  if (per == 4) {
+    v = tl <= kSmallTilesPerSm * ctx->num_sms ? 0 : tl <= kMidTilesPerSm * ctx->num_sms ? 1 : 2;
+    // recorded per size class (quarter octaves of the tile count) for stspix_sweep_choice
+    ctx->sweep_choice[(int)std::floor(4.0 * std::log2((double)tl))] = v;
+  } else {
+    v = forced >= 0 ? forced : per == 2 ? 0 : 1;
   }
-  const bool untuned = done == 0;             // no tuning trials in this call
-  const bool fuse = fuse_stats && untuned;
-  while (done < nseg) {
-    const bool pair = v2 >= 0 && nseg - done >= 2;
-    const int deltas = fuse ? 1 : 0;
-    const int mode = done > 0 ? 1 : (first_active && untuned ? 2 : 0);
-    if (pair) sweep2(v2, launch & 1, mode, deltas);
-    else sweep1(v1, launch & 1, mode, deltas);
-    done += pair ? 2 : 1;
-    launch++;
+  for (int done = 0; done < nseg;) {
+    const int ns = std::min(per, nseg - done);
+    const int mode = done > 0 ? 1 : first_active ? 2 : 0;
+    if (queue) sweep_queue(v, mode, fuse_stats ? 1 : 0);
+    else sweep(sweep_kernels()[per == 4 ? 2 : per - 1][v], ns, mode, fuse_stats ? 1 : 0);
+    *cur ^= 1;
+    done += ns;
   }
-  *fused = fuse;
-  if (chg_ok) *chg_ok = untuned && launch > 0 && (launch & 1) == 0;
-  if (launch & 1) LAUNCHB(kb_copy_labels, pix_units(L.max_npix), L, nb);
+  *chg_ok = nseg > 0;
+  if (*cur && !(keep && fuse_stats)) {
+    LAUNCHB(kb_copy_labels, pix_units(L.max_npix), L, nb);
+    *cur = 0;
+    *chg_ok = false;
+  }
   if (need_border) {
     ctx->cur_fam = STSPIX_FAM_MERGE;
     LAUNCHB(kb_find_border, pix_units(L.max_npix), L, nb);
@@ -952,7 +852,8 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
   // pass); the int64 accumulator only
   bool stats_ready = false;
   const bool fuse = ctx->accumulator == 0;
-  bool chg_ok = false;      // the previous update_seg left its last changes in plane 1
+  bool chg_ok = false;      // the previous update_seg left its changes and label buffers
+  int cur = 0;              // the label buffer the next sweep reads (see update_seg)
   for (int idx = 0; idx < maxn; idx++) {
     while (nb > 0 && nit[nb - 1] <= idx) nb--;
     if (stop_after >= 0 && idx == stop_after) {
@@ -983,11 +884,13 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
     const int nx = idx + 1;
     const bool merge_next = nx < maxn && nx > cfg.sm_start && nx % P == P / 2;
     const bool fuse_now = fuse && nx < maxn && !(stop_after >= 0 && nx == stop_after);
-    bool fused = false;
-    if ((r = update_seg(ctx, st, L, nb, cfg, merge_next || stop_after >= 0, fuse_now, &fused,
-                        first_active, &chg_ok)))
+    // the next iteration only sweeps, over the same slots: it reads the labels where they are
+    const bool sm_next = nx > cfg.sm_start && (nx % P == 0 || nx % P == P / 2);
+    const bool keep = fuse_now && stop_after < 0 && !sm_next && nit[nb - 1] > nx;
+    if ((r = update_seg(ctx, st, L, nb, cfg, merge_next || stop_after >= 0, keep, fuse_now,
+                        first_active, &cur, &chg_ok)))
       return r;
-    stats_ready = fused;
+    stats_ready = fuse_now;
   }
   if (stop_after >= 0) {
     if (extra_update && (r = update_params(ctx, st, L, L.B))) return r;
@@ -1637,7 +1540,6 @@ int stspix_create(stspix_ctx** out, int device) {
   cudaMemset(ctx->body_iters, 0, 4 * sizeof(int));
   cudaEventCreate(&ctx->batch_ev[0]);
   cudaEventCreate(&ctx->batch_ev[1]);
-  for (auto& e : ctx->tune_ev) cudaEventCreate(&e);
   cudaDeviceSynchronize();
   *out = ctx;
   return STSPIX_OK;
@@ -1653,7 +1555,6 @@ int stspix_destroy(stspix_ctx* ctx) {
   drop_fill_graphs(ctx);
   free_list(ctx->ctl_bufs);
   cudaFree(ctx->body_iters);
-  for (auto e : ctx->tune_ev) if (e) cudaEventDestroy(e);
   if (ctx->body_iters_host) cudaFreeHost(ctx->body_iters_host);
   prof_harvest(ctx);
   for (auto& e : ctx->frame_ev) { ctx->ev_free.push_back(e.a); ctx->ev_free.push_back(e.b); }
@@ -2122,11 +2023,11 @@ int stspix_sweep_choice(const stspix_ctx* ctx, int idx, int* tiles_class, int* s
                         int* pair_w) {
   if (!ctx || idx < 0) return 0;
   for (const auto& kv : ctx->sweep_choice) {
-    if (kv.first.second != 0 || idx-- > 0) continue;   // autotuned entries only
-    const int v1 = kv.second & 0xff, v2 = (kv.second >> 8) - 1;
-    if (tiles_class) *tiles_class = (int)kv.first.first;
-    if (single_w) *single_w = kSweepTileW[v1];
-    if (pair_w) *pair_w = v2 >= 0 ? kSweepTileW[v2] : 0;
+    if (idx-- > 0) continue;
+    if (tiles_class) *tiles_class = kv.first;
+    const int w = kGeomW[sweep_kernels()[2][kv.second].geom];
+    if (single_w) *single_w = w;
+    if (pair_w) *pair_w = w;
     return 1;
   }
   return 0;

@@ -27,11 +27,13 @@ constexpr int kFxSqShift = 20;
 constexpr int kFxFlowShift = 24;
 constexpr int kFillBreakIter = 1000;      // fill_missing.cu: break_iter
 constexpr int kSweepVariants = 3;         // sweep tile shapes: 32x32, 64x32, 16x32
-constexpr int kTuneRounds = 3;            // timed runs per autotuner trial (fastest kept)
 constexpr int kMaxBatchGraphs = 64;       // captured batch steps kept per context
-constexpr float kWideMargin = 1.05f;      // large batches: 64x32 unless 5 % slower
-constexpr int kPairMaxTiles = 2048;       // two-sweep launches only below this many 32x32 tiles
+// 32x32 tiles per SM up to which four-sweep launches take 32x32 and 64x32 tiles
+// (64x48 above; measured in update_seg)
+constexpr int kSmallTilesPerSm = 2, kMidTilesPerSm = 8;
 constexpr int kSweepTileW[kSweepVariants] = {32, 64, 16};
+constexpr int kSweepGeoms = 4;            // sweep tile sizes: the widths above, 64x48
+constexpr int kGeomW[kSweepGeoms] = {32, 64, 16, 64}, kGeomH[kSweepGeoms] = {32, 32, 32, 48};
 constexpr int kRelabelChunk = 64;         // previous superpixels per relabel-compare block
 
 // Packed record read by the boundary sweep: the fields calc_joint reads
@@ -169,7 +171,7 @@ struct Slot {
   double* pscache;         // [3*(cap+2)]: the prior shape term of the last full posterior
   int* post_ids;           // [cap+2]: ids of the running posterior (kb_post_list)
   Scalars* sc;
-  int tile_base[3];        // first sweep tile of this slot in the batch (32-, 64-, 16-wide)
+  int tile_base[kSweepGeoms];  // first sweep tile of this slot in the batch, per tile size
 };
 
 // kb_scalars operations.

@@ -819,50 +819,61 @@ __host__ __device__ constexpr SimpleBits simple_bits() {
 }
 __constant__ SimpleBits c_simple_bits = simple_bits();
 
-__device__ __forceinline__ void joint(float c0, float c1, float c2, int x, int y,
-                                      const SweepRec& r, int k, float s2, float neigh_neq,
-                                      float beta, float* best, int* best_label) {
+// calc_joint's score of label record r for a pixel with neq neighbours of other labels.
+__device__ __forceinline__ float joint(float c0, float c1, float c2, int x, int y,
+                                       const SweepRec& r, float s2, int neq, float beta) {
   float res = -1000;
   const float x0 = c0 - r.mu_r;
   const float x1 = c1 - r.mu_g;
   const float x2 = c2 - r.mu_b;
   int d0 = x - r.mxi, d1 = y - r.myi;   // == (int)(x - mu_x), see SweepRec
-  if ((r.frac & 1) && d0 >= 1) d0 -= 1;
-  if ((r.frac & 2) && d1 >= 1) d1 -= 1;
+  d0 -= min(max(d0, 0), r.frac & 1);
+  d1 -= min(max(d1, 0), (r.frac >> 1) & 1);
   res = res - (x0 * x0 + x1 * x1 + x2 * x2) / s2;
   res = res - (float)(d0 * d0) * r.isx - (float)(d1 * d1) * r.isz - (float)(2 * d0 * d1) * r.isy;
   res = res - r.logdet;
-  res = res - beta * neigh_neq;
-  res = res - (float)(100 * (r.count <= 10));
-  if (res > *best) { *best = res; *best_label = k; }
+  // (float)neq for 0 <= neq < 2^23 without a conversion
+  res = res - beta * (__uint_as_float(0x4b000000u | (unsigned)neq) - 8388608.f);
+  res = res - (r.count <= 10 ? 100.f : 0.f);
+  return res;
 }
 
 // ---------------------------------------------------------------------------
-// Fused sweep: border pass + the four parity phases of one sweep in one launch.
-// A block owns a TX x TY tile and stages labels of the tile plus a 4-pixel halo
-// (phase k is evaluated on the tile grown by 3-k pixels, so every label a tile
-// pixel depends on is produced inside the block exactly as the four separate
-// launches produce it), the image and the border mask of the tile plus 3 pixels.
-// Labels are read from seg_in (labels at the sweep start) and the tile is
-// written to seg_out, so neighbouring blocks never see each other's updates.
+// Fused sweeps: border pass + the four parity phases of up to NS sweeps in one launch.
+// A block owns a TX x TY tile and stages the labels of the tile plus a halo of 4 NS
+// pixels.  Sweep s of the ns sweeps of a launch evaluates phase k on the tile grown by
+// 4 (ns - s) - 1 - k pixels, so every label a tile pixel depends on is produced inside
+// the block exactly as separate launches produce it.  Labels are read from seg_in
+// (labels at the launch's start) and the tile is written to seg_out, so neighbouring
+// blocks never see each other's updates.
 //
 // The grid is the list of tiles of every frame of the batch (frame i owns tiles
 // [tile_base, tile_base + its tile count)); a block finds its frame by binary
 // search, so frames of uneven size cost what their tiles cost.
+//
+// What bounds it: not bytes (a batch's labels stay in L2) but the instructions and the
+// dependent round trips of a tile.  Per launch a tile pays the launch, the slot lookup,
+// the staging round trip and the write-back once, however many sweeps it runs, and after
+// the first sweep only the pixels next to a change are scored, so four sweeps per launch
+// win although the halo is wider (64 x 32 tile: 3 staged labels per tile pixel against
+// 4 x 1.41 in four launches, 2.6 scored pixels in the first sweep against 1.15).  In
+// between, a phase is a list of its pixels (two barriers), so that the few pixels of a
+// late sweep fill warps instead of leaving one active lane per warp.  Measured on batches
+// of 8 480x854 frames, the four sweeps of an update: 200-225 us early in a propagated
+// frame, 79-95 us late, as four launches of a kernel that scored every border pixel
+// within 4 pixels of a change; now 115-170 and 44-50 us (64x32 tiles, 256 threads).  A
+// scored pixel takes about 300 instructions of its warp, and a phase of one pixel about
+// 2100 cycles (list, 3x3 labels, records, scores, marks: one dependent chain).
 constexpr int kReach = 4;             // a sweep's labels depend on labels this far away
 
-// NS sweeps per launch (1 or 2): the label halo is 4 NS pixels; sweep s of the launch
-// lists and scores the tile grown by G = 4 (NS - s) - 1 pixels (phase k on the tile
-// grown by G - k), so after sweep s the labels of the tile grown by 4 (NS - s - 1)
-// are exactly those of NS separate launches.
 // Incremental statistics.  Between two update_params of the BASS loop the labels
 // change only in the sweeps, so the statistics of the new labels are those of the old
-// ones plus, for every pixel a sweep relabels from C to bl, its contribution moved
+// ones plus, for every pixel a launch relabels from C to bl, its contribution moved
 // from C to bl.  A sweep block collects the moves of its tile's own pixels in a small
 // table in shared memory (label -> count and sums, 32-bit fields: colours split into
-// 16-bit parts, positions relative to the tile) and adds each touched label's net
-// change to its 64-bit global sums once per launch.  Integer sums, so the result is
-// identical to clearing and summing every pixel again.
+// 16-bit parts, positions relative to the tile; at most 2048 pixels move) and adds each
+// touched label's net change to its 64-bit global sums once per launch.  Integer sums, so the result is identical to clearing and
+// summing every pixel again.
 constexpr int kDeltaTab = 64;         // labels a tile's moves can touch (a power of two)
 
 struct DeltaTab {
@@ -886,16 +897,16 @@ __device__ __forceinline__ int delta_slot(DeltaTab& tb, int k) {
 }
 
 // pixel (gx, gy), tile origin (tx0, ty0), moved from label C to label b.
-__device__ __forceinline__ void delta_move(DeltaTab& tb, const SpDev& sp, int C, int b, int gx,
-                                           int gy, int tx0, int ty0, float c0, float c1,
+__device__ __forceinline__ void delta_move(DeltaTab& tb, int* count, long long* sums, int C, int b,
+                                           int gx, int gy, int tx0, int ty0, float c0, float c1,
                                            float c2) {
-  const bool unit = c0 >= 0.f && c0 <= 1.f && c1 >= 0.f && c1 <= 1.f && c2 >= 0.f && c2 <= 1.f;
+  const bool unit = unit_colour(c0) && unit_colour(c1) && unit_colour(c2);
   const int sc = unit ? delta_slot(tb, C) : -1;
   const int sb = unit ? delta_slot(tb, b) : -1;
   if (sc >= 0 && sb >= 0) {
     // colours in [0, 1]: the fixed-point value is one exact conversion, at most 2^28
-    const unsigned q0 = __float2uint_rn(c0 * 0x1p28f), q1 = __float2uint_rn(c1 * 0x1p28f),
-                   q2 = __float2uint_rn(c2 * 0x1p28f);
+    const unsigned q0 = fx_unit(c0, kFxAppShift), q1 = fx_unit(c1, kFxAppShift),
+                   q2 = fx_unit(c2, kFxAppShift);
     const int x = gx - tx0, y = gy - ty0;
     const int d[12] = {1, (int)(q0 & 0xFFFF), (int)(q0 >> 16), (int)(q1 & 0xFFFF), (int)(q1 >> 16),
                        (int)(q2 & 0xFFFF), (int)(q2 >> 16), x, y, x * x, x * y, y * y};
@@ -910,10 +921,10 @@ __device__ __forceinline__ void delta_move(DeltaTab& tb, const SpDev& sp, int C,
   const long long q[3] = {fx_q(c0, kFxAppShift), fx_q(c1, kFxAppShift), fx_q(c2, kFxAppShift)};
   const long long X = gx, Y = gy;
   const long long d[8] = {q[0], q[1], q[2], X, Y, X * X, X * Y, Y * Y};
-  unsigned long long* ab = (unsigned long long*)(sp.acc + 8 * (size_t)b);
-  unsigned long long* ac = (unsigned long long*)(sp.acc + 8 * (size_t)C);
-  atomicAdd(&sp.count[b], 1);
-  atomicSub(&sp.count[C], 1);
+  unsigned long long* ab = (unsigned long long*)(sums + 8 * (size_t)b);
+  unsigned long long* ac = (unsigned long long*)(sums + 8 * (size_t)C);
+  atomicAdd(&count[b], 1);
+  atomicSub(&count[C], 1);
 #pragma unroll
   for (int f = 0; f < 8; f++) {
     atomicAdd(ab + f, (unsigned long long)d[f]);
@@ -922,7 +933,8 @@ __device__ __forceinline__ void delta_move(DeltaTab& tb, const SpDev& sp, int C,
 }
 
 // The table's net changes to the global sums (block-wide; after the last phase).
-__device__ __forceinline__ void delta_flush(DeltaTab& tb, const SpDev& sp, int tx0, int ty0) {
+__device__ __forceinline__ void delta_flush(DeltaTab& tb, int* count, long long* sums, int tx0,
+                                            int ty0) {
   for (int i = threadIdx.x; i < kDeltaTab; i += blockDim.x) {
     const int k = tb.key[i];
     if (k < 0) continue;
@@ -933,532 +945,514 @@ __device__ __forceinline__ void delta_flush(DeltaTab& tb, const SpDev& sp, int t
                             (long long)v[6] * 65536 + v[5], n * X + sx, n * Y + sy,
                             n * X * X + 2 * X * sx + v[9], n * X * Y + X * sy + Y * sx + v[10],
                             n * Y * Y + 2 * Y * sy + v[11]};
-    unsigned long long* acc = (unsigned long long*)(sp.acc + 8 * (size_t)k);
-    atomicAdd(&sp.count[k], v[0]);
+    unsigned long long* acc = (unsigned long long*)(sums + 8 * (size_t)k);
+    atomicAdd(&count[k], v[0]);
 #pragma unroll
     for (int f = 0; f < 8; f++) atomicAdd(acc + f, (unsigned long long)d[f]);
   }
 }
 
+// Bits [0, n) of a 32-bit word (n clamped to 0..32), and bits [a, b) of word w of a row
+// of 32-pixel words.
+__device__ __forceinline__ unsigned bits32_below(int n) {
+  return ~__funnelshift_lc(0u, 0xffffffffu, (unsigned)max(n, 0));
+}
+__device__ __forceinline__ unsigned range32(int a, int b, int w) {
+  return bits32_below(b - 32 * w) & ~bits32_below(a - 32 * w);
+}
+
+// Shared memory of a sweep block.  Masks are rows of 32-pixel words over the label
+// region (bit x & 31 of word x >> 5 of row y = label-region pixel (x, y)).
 template <int TX, int TY, int NS>
 struct SweepTile {
-  static constexpr int kSH = 4 * NS;                                 // label halo
+  static constexpr int kSH = kReach * NS;                            // label halo
   static constexpr int kG0 = kSH - 1;                                // first sweep's growth
-  static constexpr int kLX = TX + 2 * kSH, kLY = TY + 2 * kSH;      // staged labels
-  static constexpr int kMaxList = (TX / 2 + kG0) * (TY / 2 + kG0);
-  static_assert(TX + 2 * kG0 < 256 && TY + 2 * kG0 < 256, "list entries pack (ly << 8) | lx");
-  static_assert(kLX <= 128, "a label-region row is at most two 64-bit words");
-  int L[kLX * kLY];
-  unsigned short list[4][kMaxList];   // border pixels of each parity phase, (ly << 8) | lx
-  int cnt[4];
-  // active-set sweeps: change flags of the label region as row bitmasks (bit x of
-  // row y = label-region pixel (x, y)), dilated by 4 pixels
-  unsigned long long act[2][kLY];
-  // label edges of the label region as row bitmasks: bit x of edE[.][y] is set when
-  // pixel (x, y) and its right neighbour differ, of edS[.][y] when (x, y) and the pixel
-  // below differ
-  unsigned long long edE[2][kLY];
-  unsigned long long edS[2][kLY];
-  // pixels of the tile whose label the launch's last sweep changed, as row bitmasks
-  // over label-region columns (the change flags the launch writes)
-  unsigned long long chg[TY][2];
-  DeltaTab delta;                     // statistics moves of the tile's pixels (deltas on)
+  static constexpr int kLX = TX + 2 * kSH, kLY = TY + 2 * kSH;       // staged labels
+  static constexpr int kCK = (kLX + 31) / 32;                        // words per row
+  static constexpr int kClass = (TX / 2 + kG0) * (TY / 2 + kG0);     // a phase's pixels
+  static constexpr int kRowsOut = 32 < TY ? 16 : TY;                 // rows per write-back pass
+  static constexpr int kMaxList = kClass > TX * kRowsOut ? kClass : TX * kRowsOut;
+  static_assert(kLX < 256 && kLY < 256 && TY % kRowsOut == 0, "list entries pack (y << 8) | x");
+  static_assert(kLX % 8 == 0 && kLY % 8 == 0, "8-pixel groups, rows in whole warp spans");
+  static_assert(kSH % 2 == 0 && TX % 16 == 0 && TY % 2 == 0, "region parity = image parity");
+  __align__(16) int L[kLX * kLY];
+  unsigned short list[kMaxList];      // pixels of the running phase, (y << 8) | x
+  int cnt[2][4];                      // list lengths by phase, alternating between sweeps
+  int wcnt;                           // length of the write-back list
+  int neg;                            // a staged label is negative (outside the image)
+  union {
+    struct {
+      // label edges: edE bit set when a pixel and its right neighbour differ, edS when a
+      // pixel and the one below differ.  Built at staging, kept current by the relabels.
+      unsigned edE[kLY][kCK], edS[kLY][kCK];
+      unsigned seed[kLY][kCK];        // changed pixels the first sweep starts from
+      unsigned dirty[kLY][kCK];       // pixels to score at their next phase (see sweep_tile)
+      unsigned bm[kLY][kCK];          // border pixels at the start of the running sweep
+    };
+    DeltaTab delta;                   // after the sweeps: statistics moves of the tile's pixels
+  };
+  unsigned sin[kLY][kCK];             // pixels where seg_out differs from seg_in at the start
+  unsigned all[kLY][kCK];             // tile pixels relabelled by this launch
 };
 
-// Bit masks over a label-region row (two 64-bit words, bit x of word x >> 6).
-__host__ __device__ constexpr unsigned long long bits_below(int n) {
-  return n <= 0 ? 0ull : n >= 64 ? ~0ull : ((1ull << n) - 1ull);
-}
-// bits [a, b) of word w
-__host__ __device__ constexpr unsigned long long range_word(int a, int b, int w) {
-  return bits_below(b - 64 * w) & ~bits_below(a - 64 * w);
-}
-constexpr unsigned long long kEvenBits = 0x5555555555555555ull;
-constexpr unsigned long long kOddBits = 0xAAAAAAAAAAAAAAAAull;
-
-// Active-set sweeps.  The parameters are fixed across the sweeps of one update_seg
-// call and a pixel's decision depends only on its 3x3 labels (after the earlier
-// phases of the sweep), its colour and the parameters, so a pixel of phase k can
-// only change if a label within Chebyshev distance k + 1 <= 4 changed during the
-// previous sweep or earlier in this one.  Sweeps after the first of a call (mode 1)
-// therefore list only the border pixels within 4 pixels of a change flagged by the
-// previous sweep (chg_in), and a tile whose whole label region saw no change keeps
-// its labels.  Every sweep writes its own change flags (chg_out).
-// One sweep inside a launch: list the border pixels of each parity class on the tile
-// grown by G (phase k on the tile grown by G - k), then score them phase by phase in
-// shared memory.  OFF = label-region offset of the grown-by-G region; use_act: only
-// pixels flagged in sm.act (active-set sweeps).
-// The 32-bit chunk ballots of a label-region row as its two 64-bit words.
-template <int kCK>
-__device__ __forceinline__ void pack_row(const unsigned (&b)[kCK], unsigned long long* w0,
-                                         unsigned long long* w1) {
-  unsigned long long lo = b[0], hi = 0;
-  if (kCK > 1) lo |= (unsigned long long)b[1 % kCK] << 32;
-  if (kCK > 2) hi = b[2 % kCK];
-  if (kCK > 3) hi |= (unsigned long long)b[3 % kCK] << 32;
-  *w0 = lo; *w1 = hi;
-}
-
-// STAGED: the label edges of the staged rows are already in sm.edE / sm.edS (computed
-// from the staging registers, rows in contiguous spans of kLY / 8 per warp) except the
-// lower edges of each span's last row, which need the next warp's first row.
-template <int TX, int TY, int NS, int G, bool STAGED>
-__device__ __forceinline__ void sweep_pass(const Slot& S, SweepTile<TX, TY, NS>& sm,
-                                           const unsigned* lut_bits, int tx0, int ty0,
-                                           float s2, float potts, bool use_act, bool last,
-                                           bool deltas) {
-  constexpr int kLX = SweepTile<TX, TY, NS>::kLX;
-  constexpr int kLY = SweepTile<TX, TY, NS>::kLY;
-  constexpr int kSH = SweepTile<TX, TY, NS>::kSH;
-  constexpr int OFF = kSH - G;
-  constexpr int kIY = TY + 2 * G;
-  constexpr int kCK = (kLX + 31) / 32;
-  static_assert(OFF >= 1, "every listed pixel has its 4 neighbours in the label region");
-  int* L = sm.L;
-  auto& list = sm.list;
-  int* cnt = sm.cnt;
-  const int H = S.H, W = S.W;
-  const float* __restrict__ img = S.img;
-  const SweepRec* __restrict__ rec = S.sp.rec;
-  const SpDev& spd = S.sp;
-  const int cap = S.sp.cap;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int ix0 = tx0 - G, iy0 = ty0 - G;
-  const int rx0 = tx0 - kSH, ry0 = ty0 - kSH;
-  // Border mask at the sweep start (find_border_pixels, seg_utils.cu:164-195) as row
-  // bitmasks: a pixel is a border pixel when one of its 4 neighbours carries another
-  // label (labels outside the image are staged as -1, so in-image pixels of the image's
-  // edge rows and columns count as border pixels as in the reference).  First the
-  // edges of the label region, one warp per row in 32-pixel chunks (rows with no
-  // change in reach are skipped in active-set sweeps).
-  if (STAGED) {
-    constexpr int kSpan = kLY / 8;
-    const int ay = warp * kSpan + kSpan - 1;   // this warp's span's last row
-    if (ay + 1 < kLY) {
-      unsigned d[kCK];
-#pragma unroll
-      for (int c = 0; c < kCK; c++) {
-        const int x = lane + 32 * c;
-        const bool in = x < kLX;
-        const int v = in ? L[ay * kLX + x] : -1;
-        const int dn = in ? L[(ay + 1) * kLX + x] : v;
-        d[c] = __ballot_sync(0xffffffffu, v != dn);
-      }
-      if (lane == 0) pack_row<kCK>(d, &sm.edS[0][ay], &sm.edS[1][ay]);
-    }
-  } else {
-    for (int ay = OFF - 1 + warp; ay < OFF + kIY; ay += nwarps) {
-      if (use_act) {
-        const int an = min(ay + 1, kLY - 1);
-        if (!(sm.act[0][ay] | sm.act[1][ay] | sm.act[0][an] | sm.act[1][an])) continue;
-      }
-      unsigned e[kCK], d[kCK];
-#pragma unroll
-      for (int c = 0; c < kCK; c++) {
-        const int x = lane + 32 * c;
-        const bool in = x < kLX;
-        const int v = in ? L[ay * kLX + x] : -1;
-        const int r = (x + 1 < kLX) ? L[ay * kLX + x + 1] : v;
-        const int dn = (in && ay + 1 < kLY) ? L[(ay + 1) * kLX + x] : v;
-        e[c] = __ballot_sync(0xffffffffu, v != r);
-        d[c] = __ballot_sync(0xffffffffu, v != dn);
-      }
-      if (lane == 0) {
-        pack_row<kCK>(e, &sm.edE[0][ay], &sm.edE[1][ay]);
-        pack_row<kCK>(d, &sm.edS[0][ay], &sm.edS[1][ay]);
-      }
-    }
-  }
-  __syncthreads();
-  // Then the border pixels of each parity class inside the tile grown by G minus the
-  // class (the class's phase), one warp per row: the row's border mask, restricted to
-  // the image, the active set and the two classes of the row's y parity, is counted
-  // per class (one shared atomic per class and row) and its set bits appended in
-  // ascending x order.
-  {
-    const unsigned lt = (1u << lane) - 1u;
-    const unsigned long long img0 = range_word(-rx0, W - rx0, 0);
-    const unsigned long long img1 = range_word(-rx0, W - rx0, 1);
-    for (int ly = warp; ly < kIY; ly += nwarps) {
-      const int gy = iy0 + ly;
-      if (gy < 0 || gy >= H) continue;
-      const int ay = ly + OFF;                   // label-region row
-      unsigned long long m0 = img0, m1 = img1;
-      if (use_act) {
-        m0 &= sm.act[0][ay];
-        m1 &= sm.act[1][ay];
-        if (!(m0 | m1)) continue;
-      }
-      const int cy = gy & 1;
-      // the two classes of this row: (xo << 1) | cy, listed on the tile grown by
-      // G - class; x parity of a label-region column equals that of the image column.
-      // The column masks of the four classes are constants of the template.
-      constexpr unsigned long long A00 = range_word(kSH - G, kSH + TX + G, 0) & kEvenBits;
-      constexpr unsigned long long A01 = range_word(kSH - G, kSH + TX + G, 1) & kEvenBits;
-      constexpr unsigned long long B00 = range_word(kSH - G + 2, kSH + TX + G - 2, 0) & kOddBits;
-      constexpr unsigned long long B01 = range_word(kSH - G + 2, kSH + TX + G - 2, 1) & kOddBits;
-      constexpr unsigned long long A10 = range_word(kSH - G + 1, kSH + TX + G - 1, 0) & kEvenBits;
-      constexpr unsigned long long A11 = range_word(kSH - G + 1, kSH + TX + G - 1, 1) & kEvenBits;
-      constexpr unsigned long long B10 = range_word(kSH - G + 3, kSH + TX + G - 3, 0) & kOddBits;
-      constexpr unsigned long long B11 = range_word(kSH - G + 3, kSH + TX + G - 3, 1) & kOddBits;
-      const int ga = G - cy, gb = G - (2 | cy);
-      const int ry = ay - kSH;                   // row relative to the tile
-      const bool ya = ry >= -ga && ry < TY + ga, yb = ry >= -gb && ry < TY + gb;
-      const unsigned long long k0 = (ya ? (cy ? A10 : A00) : 0ull) | (yb ? (cy ? B10 : B00) : 0ull);
-      const unsigned long long k1 = (ya ? (cy ? A11 : A01) : 0ull) | (yb ? (cy ? B11 : B01) : 0ull);
-      const unsigned long long e0 = sm.edE[0][ay], e1 = sm.edE[1][ay];
-      const unsigned long long b0 = e0 | (e0 << 1) | sm.edS[0][ay] | sm.edS[0][ay - 1];
-      const unsigned long long b1 =
-          e1 | (e1 << 1) | (e0 >> 63) | sm.edS[1][ay] | sm.edS[1][ay - 1];
-      m0 &= b0 & k0;
-      m1 &= b1 & k1;
-      if (!(m0 | m1)) continue;
-      const int na = __popcll(m0 & kEvenBits) + __popcll(m1 & kEvenBits);
-      const int nb = __popcll(m0 & kOddBits) + __popcll(m1 & kOddBits);
-      int base = 0;
-      if (lane < 2) {
-        const int n = lane ? nb : na;
-        if (n) base = atomicAdd(&cnt[(lane << 1) | cy], n);
-      }
-      int base_a = __shfl_sync(0xffffffffu, base, 0);
-      int base_b = __shfl_sync(0xffffffffu, base, 1);
-      const bool odd = lane & 1;
-      const unsigned mine = odd ? 0xAAAAAAAAu : 0x55555555u;
-      unsigned short* out = list[((int)odd << 1) | cy];
-#pragma unroll
-      for (int c = 0; c < kCK; c++) {
-        const unsigned w = (unsigned)((c < 2 ? m0 : m1) >> (32 * (c & 1)));
-        if (!w) continue;
-        const int ax = 32 * c + lane;
-        if ((w >> lane) & 1u) {
-          const int pos = (odd ? base_b : base_a) + __popc(w & mine & lt);
-          out[pos] = (unsigned short)((ly << 8) | (ax - OFF));
-        }
-        base_a += __popc(w & 0x55555555u);
-        base_b += __popc(w & 0xAAAAAAAAu);
-      }
-    }
-  }
-  __syncthreads();
-  for (int ph = 0; ph < 4; ph++) {
-    const int n = cnt[ph];
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-      const int bi = list[ph][j];
-      const int lxi = bi & 255, lyi = bi >> 8;
-      int gx = ix0 + lxi, gy = iy0 + lyi;
-      int p = (lyi + OFF) * kLX + (lxi + OFF);
-      // the pixel's colour is loaded first: its latency overlaps the simple-point tests
-      const float* pix = img + 3 * ((size_t)gy * W + gx);
-      const float c0 = __ldg(pix), c1 = __ldg(pix + 1), c2 = __ldg(pix + 2);
-      int C = L[p];
-      if (C < 0 || C >= cap) continue;
-      const int N = L[p - kLX], S = L[p + kLX], Wl = L[p - 1], E = L[p + 1];
-      const int NW = L[p - kLX - 1], NE = L[p - kLX + 1], SW = L[p + kLX - 1],
-                SE = L[p + kLX + 1];
-      // simple-point codes of the four candidates: bit i set when neighbour i
-      // (NW,N,NE,W,E,SW,S,SE) carries the candidate or lies outside the image;
-      // equal candidates share one code; differing neighbours = 8 - popcount
-      const int nb[8] = {NW, N, NE, Wl, E, SW, S, SE};
-      unsigned m1 = 0;
-#pragma unroll
-      for (int q = 0; q < 8; q++) m1 |= (unsigned)(nb[q] == -1) << q;
-      auto code = [&](int v) {
-        unsigned c = m1;
-#pragma unroll
-        for (int q = 0; q < 8; q++) c |= (unsigned)(nb[q] == v) << q;
-        return c;
-      };
-      const unsigned cN = code(N);
-      const unsigned cW = (Wl == N) ? cN : code(Wl);
-      const unsigned cS = (S == N) ? cN : (S == Wl) ? cW : code(S);
-      const unsigned cE = (E == N) ? cN : (E == Wl) ? cW : (E == S) ? cS : code(E);
-      auto simple = [&](unsigned c) { return (lut_bits[c >> 5] >> (c & 31)) & 1u; };
-      if (!simple(cN) || !simple(cW) || !simple(cS) || !simple(cE)) continue;
-      const int dN = 8 - __popc(cN), dW = 8 - __popc(cW), dS = 8 - __popc(cS),
-                dE = 8 - __popc(cE);
-      if (N >= cap || S >= cap || Wl >= cap || E >= cap) continue;
-      float best = -9999.f;
-      int bl = C;
-      if (N >= 0) joint(c0, c1, c2, gx, gy, rec[N], N, s2, (float)dN, potts, &best, &bl);
-      if (S != N && S >= 0) joint(c0, c1, c2, gx, gy, rec[S], S, s2, (float)dS, potts, &best, &bl);
-      if (Wl != S && Wl != N && Wl >= 0)
-        joint(c0, c1, c2, gx, gy, rec[Wl], Wl, s2, (float)dW, potts, &best, &bl);
-      if (E != Wl && E != S && E != N && E >= 0)
-        joint(c0, c1, c2, gx, gy, rec[E], E, s2, (float)dE, potts, &best, &bl);
-      if (rec[C].count <= 2 && bl == C) {
-        if (N >= 0) bl = N;
-        else if (E >= 0) bl = E;
-        else if (S >= 0) bl = S;
-        else if (Wl >= 0) bl = Wl;
-      }
-      if (bl != C) {
-        L[p] = bl;
-        // a tile pixel changed by the launch's last sweep: its change flag (each pixel
-        // is scored once per sweep, so a changed pixel keeps its new label); with
-        // deltas, the move of its statistics from C to bl
-        const int ty = lyi + OFF - kSH, ax = lxi + OFF;
-        if (ty >= 0 && ty < TY && ax >= kSH && ax < kSH + TX) {
-          if (last) atomicOr(&sm.chg[ty][ax >> 6], 1ull << (ax & 63));
-          if (deltas) delta_move(sm.delta, spd, C, bl, gx, gy, tx0, ty0, c0, c1, c2);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  (void)rx0; (void)ry0;
+// The slot fields a sweep reads, loaded together (one round trip; the slot table is read
+// from L2 by every block).
+struct SweepSlot {
+  const int* in;
+  int* out;
+  const uint16_t* chg_in;
+  uint16_t* chg_out;
+  const float* img;
+  const SweepRec* rec;
+  const uint8_t* recchg;
+  int* count;
+  long long* acc;
+  int H, W, cap, tile0;
+};
+__device__ __forceinline__ SweepSlot sweep_slot(const Slot& S, int parity, int v) {
+  SweepSlot r;
+  int* a = S.seg;
+  int* b = S.seg_alt;
+  uint8_t* c0 = S.chg[0];
+  uint8_t* c1 = S.chg[1];
+  r.img = S.img;
+  r.rec = S.sp.rec;
+  r.recchg = S.recchg;
+  r.count = S.sp.count;
+  r.acc = S.sp.acc;
+  r.H = S.H; r.W = S.W; r.cap = S.cap;
+  r.tile0 = S.tile_base[v];
+  r.in = parity ? b : a;
+  r.out = parity ? a : b;
+  r.chg_in = (const uint16_t*)(parity ? c0 : c1);
+  r.chg_out = (uint16_t*)(parity ? c1 : c0);
+  return r;
 }
 
-// Active-set sweeps.  The parameters are fixed across the sweeps of one update_seg
-// call and a pixel's decision depends only on its 3x3 labels (after the earlier
-// phases of the sweep), its colour and the parameters, so a pixel of phase k can
-// only change if a label within Chebyshev distance k + 1 <= 4 changed during the
-// previous sweep or earlier in this one.  Sweeps after the first of a call (mode 1)
-// therefore list only the border pixels within 4 pixels of a change flagged by the
-// previous sweep (chg_in), and a tile whose whole label region saw no change keeps
-// its labels.  Every launch writes the change flags of its last sweep (chg_out); in
-// a two-sweep launch the second sweep lists every border pixel.
-template <int TX, int TY, int NS>
-__device__ __forceinline__ void sweep_tile(const Slot& S, int bx, int by, int parity, float s2,
+// The three 16-byte words of label k's record.
+__device__ __forceinline__ SweepRec load_rec(const SweepRec* __restrict__ rec, int k) {
+  union { SweepRec r; uint4 q[3]; } u;
+  const uint4* p = (const uint4*)(rec + k);
+#pragma unroll
+  for (int i = 0; i < 3; i++) u.q[i] = __ldg(p + i);
+  return u.r;
+}
+
+// What a sweep scores.  The parameters are fixed across the sweeps of one update_seg
+// call, and a pixel's decision depends only on its 3x3 labels at its phase, its colour
+// and the records of its own and its 4-neighbours' labels.  So a pixel whose 3x3 labels
+// and records have not changed since it was last scored keeps its label, and only the
+// others, the dirty pixels, are scored: a relabelled pixel makes its 3x3 dirty, a phase
+// scores the dirty pixels of its class that were border pixels at the start of the sweep
+// (the reference's border mask is built once per sweep) and clears their bits; a dirty
+// pixel that was no border pixel then stays dirty.  The first sweep of a launch starts
+// from
+//   mode 0: every border pixel (seg_out holds nothing of use);
+//   mode 1: the pixels within 1 of a change of the previous launch of the call (chg_in);
+//   mode 2: within 1 of a change of the previous call's last launch, or of a pixel of a
+//           label whose record the posterior between the calls changed.
+// A pixel of phase k depends, through the phases before it, on labels within Chebyshev
+// distance k + 1 <= 4, so the label region holds everything a tile pixel depends on.
+// A launch writes the union of its sweeps' changes (chg_out): a superset of the last
+// sweep's, and every pixel where seg_out and seg_in differ.  So when a launch in mode 1
+// or 2 starts, seg_out (the labels before the previous launch) equals seg_in but at the
+// pixels of chg_in, and only those and the launch's own changes are stored.
+//
+// NT: threads of the block.
+template <int TX, int TY, int NS, int NT>
+__device__ __forceinline__ void sweep_tile(const SweepSlot& S, int bx, int by, int ns, float s2,
                                            float potts, SweepTile<TX, TY, NS>& sm,
                                            const unsigned* lut_bits, int mode, int deltas) {
-  constexpr int kTX = TX, kTY = TY;
-  constexpr int kSH = SweepTile<TX, TY, NS>::kSH;
-  constexpr int kLX = SweepTile<TX, TY, NS>::kLX, kLY = SweepTile<TX, TY, NS>::kLY;
+  using Tile = SweepTile<TX, TY, NS>;
+  constexpr int kSH = Tile::kSH, kLX = Tile::kLX, kLY = Tile::kLY, kCK = Tile::kCK;
+  constexpr int kWords = kLY * kCK, kWarps = NT / 32;
   int* L = sm.L;
-  int* cnt = sm.cnt;
-
   const int H = S.H, W = S.W;
-  const int* __restrict__ seg_in = parity ? S.seg_alt : S.seg;
-  int* __restrict__ seg_out = parity ? S.seg : S.seg_alt;
-  if (threadIdx.x < 4) cnt[threadIdx.x] = 0;
-  const int tx0 = bx * kTX, ty0 = by * kTY;
+  const int* __restrict__ seg_in = S.in;
+  int* __restrict__ seg_out = S.out;
+  const int tx0 = bx * TX, ty0 = by * TY;
   const int rx0 = tx0 - kSH, ry0 = ty0 - kSH;        // label region origin
   // change flags: one bit per pixel, rows of P16 16-bit words (bit x & 15 of word
   // x >> 4); a tile's x origin is a multiple of 16, so every word has one writer
-  const uint16_t* __restrict__ chg_in = (const uint16_t*)S.chg[parity ^ 1];
-  uint16_t* __restrict__ chg_out = (uint16_t*)S.chg[parity];
+  const uint16_t* __restrict__ chg_in = S.chg_in;
+  uint16_t* __restrict__ chg_out = S.chg_out;
   const int P16 = (W + 15) >> 4;
-  // The label region is loaded first, into registers: warp w takes rows w, w + 8, ...
-  // in 32-label chunks, every load issued before any is used, so the block waits for
-  // one memory round trip (overlapping the change-flag loads of active-set sweeps).
+  const int cap = S.cap;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kRW = kLY / 8, kCK = (kLX + 31) / 32;   // warp w: rows kRW w .. kRW w + kRW - 1
-  static_assert(kLY % 8 == 0, "label-region rows in whole warp spans");
-  int lv[kRW][kCK];
-  if (rx0 >= 0 && ry0 >= 0 && rx0 + kLX <= W && ry0 + kLY <= H) {
-    // the label region lies inside the frame (most tiles): one row pointer per row,
-    // no per-label bounds but the region's width
-    const int* base = seg_in + (size_t)(ry0 + warp * kRW) * W + rx0 + lane;
+
+  // --- staging: the label region to shared memory, a span of rows per warp; every load
+  // of a thread is issued before the first store (one memory round trip)
+  {
+    constexpr int kRW = (kLY + kWarps - 1) / kWarps;      // warp w: rows w, w + kWarps, ..
+    int lv[kRW][kCK];
+    if (rx0 >= 0 && ry0 >= 0 && rx0 + kLX <= W && ry0 + kLY <= H) {
+      // inside the frame (most tiles): one row pointer per row
+      const int* base = seg_in + (size_t)(ry0 + warp) * W + rx0 + lane;
+      const size_t step = (size_t)kWarps * W;
 #pragma unroll
-    for (int a = 0; a < kRW; a++) {
+      for (int a = 0; a < kRW; a++)
 #pragma unroll
-      for (int c = 0; c < kCK; c++)
-        lv[a][c] = (lane + 32 * c < kLX) ? base[(size_t)a * W + 32 * c] : -1;
-    }
-  } else {
-#pragma unroll
-    for (int a = 0; a < kRW; a++) {
-      const int r = warp * kRW + a, gy = ry0 + r;
-      const bool row_ok = r < kLY && gy >= 0 && gy < H;
-#pragma unroll
-      for (int c = 0; c < kCK; c++) {
-        const int x = lane + 32 * c, gx = rx0 + x;
-        lv[a][c] = (row_ok && x < kLX && gx >= 0 && gx < W) ? seg_in[gy * W + gx] : -1;
-      }
-    }
-  }
-  // tile pixels of the staging layout: (a, c) -> label-region (r, x)
-  auto in_tile = [&](int r, int x) {
-    return r >= kSH && r < kSH + kTY && x >= kSH && x < kSH + kTX && ry0 + r < H && rx0 + x < W;
-  };
-  if (mode) {
-    unsigned long long* a0 = sm.act[0];
-    unsigned long long* a1 = sm.act[1];
-    if (mode == 2) {
-      // first sweep after an incremental posterior: besides the previous sweep's changes,
-      // every pixel whose label or 4-neighbour's label got a new record may decide
-      // differently.  The label-region pixels whose label's record changed, as row
-      // bitmasks (from the staging registers; sm.edE is free until the edges below).
-      const int cap = S.sp.cap;
+        for (int c = 0; c < kCK; c++)
+          lv[a][c] = (kLX % 32 == 0 || lane + 32 * c < kLX) &&
+                             (kLY % kWarps == 0 || a * kWarps + warp < kLY)
+                         ? base[a * step + 32 * c] : -1;
+    } else {
 #pragma unroll
       for (int a = 0; a < kRW; a++) {
-        const int rr = warp * kRW + a;
-        unsigned q[kCK];
+        const int gy = ry0 + a * kWarps + warp;
 #pragma unroll
         for (int c = 0; c < kCK; c++) {
-          const int v = lv[a][c];
-          q[c] = __ballot_sync(0xffffffffu, v >= 0 && v < cap && S.recchg[v] != 0);
+          const int x = lane + 32 * c, gx = rx0 + x;
+          lv[a][c] = (gy >= 0 && gy < H && a * kWarps + warp < kLY && x < kLX && gx >= 0 && gx < W)
+                         ? seg_in[(size_t)gy * W + gx] : -1;
         }
-        if (lane == 0) pack_row<kCK>(q, &sm.edE[0][rr], &sm.edE[1][rr]);
+      }
+    }
+    // the changes of the previous launch, meanwhile
+    for (int i = threadIdx.x; i < kWords; i += NT) {
+      unsigned w = 0;
+      if (mode) {
+        const int r = i / kCK, c = i - r * kCK;
+        const int gy = ry0 + r, x = rx0 + 32 * c;
+        const int w0 = x >> 4, off = x & 15;         // x >= -16: the shift floors
+        if (gy >= 0 && gy < H) {
+          const uint16_t* row = chg_in + (size_t)gy * P16;
+          unsigned long long v = 0;
+#pragma unroll
+          for (int k = 0; k < (kSH % 16 ? 3 : 2); k++)
+            if (w0 + k >= 0 && w0 + k < P16) v |= (unsigned long long)row[w0 + k] << (16 * k);
+          w = (unsigned)(v >> off) & range32(0, kLX, c);
+        }
+      }
+      (&sm.sin[0][0])[i] = w;
+      (&sm.all[0][0])[i] = 0;
+    }
+    if (threadIdx.x < 8) (&sm.cnt[0][0])[threadIdx.x] = 0;
+    if (threadIdx.x == 8) { sm.wcnt = 0; sm.neg = 0; }
+#pragma unroll
+    for (int a = 0; a < kRW; a++)
+#pragma unroll
+      for (int c = 0; c < kCK; c++)
+        if ((kLX % 32 == 0 || lane + 32 * c < kLX) &&
+            (kLY % kWarps == 0 || a * kWarps + warp < kLY))
+          L[(a * kWarps + warp) * kLX + lane + 32 * c] = lv[a][c];
+  }
+  __syncthreads();
+  // --- label edges and seeds, 8 pixels of a row per thread: bytes of the mask rows.
+  // A border pixel (find_border_pixels, seg_utils.cu:164-195) is one with an edge to any of
+  // its 4 neighbours; labels outside the image are staged as -1, so in-image pixels of the
+  // image's edge rows and columns count as border pixels as in the reference.
+  bool seed = false;
+  {
+    constexpr int kGrp = kLX / 8;
+    const uint8_t* __restrict__ recchg = S.recchg;
+    int sign = 0;
+    for (int i = threadIdx.x; i < kGrp * kLY; i += NT) {
+      const int r = i / kGrp, g = i - r * kGrp;
+      const int* row = L + r * kLX + 8 * g;
+      const int* below = r + 1 < kLY ? row + kLX : row;
+      const int4 va = *(const int4*)row, vb = *(const int4*)(row + 4);
+      const int4 da = *(const int4*)below, db = *(const int4*)(below + 4);
+      const int v[9] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w,
+                        g + 1 < kGrp ? row[8] : vb.w};
+      const int d[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+      unsigned e = 0, s = 0;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        e |= (unsigned)(v[q] != v[q + 1]) << q;
+        s |= (unsigned)(v[q] != d[q]) << q;
+        sign |= v[q];
+      }
+      ((uint8_t*)sm.edE[r])[g] = (uint8_t)e;
+      ((uint8_t*)sm.edS[r])[g] = (uint8_t)s;
+      if (mode) {
+        unsigned q8 = ((const uint8_t*)sm.sin[r])[g];
+        if (mode == 2) {
+#pragma unroll
+          for (int q = 0; q < 8; q++)
+            q8 |= (unsigned)((unsigned)v[q] < (unsigned)cap && recchg[v[q]] != 0) << q;
+        }
+        ((uint8_t*)sm.seed[r])[g] = (uint8_t)q8;
+        seed |= q8 != 0;
+      }
+    }
+    if (sign < 0) sm.neg = 1;
+    // bytes past the region's columns in a row's last word
+    if (kGrp % 4)
+      for (int r = threadIdx.x; r < kLY; r += NT)
+#pragma unroll
+        for (int g = kGrp; g < 4 * kCK; g++) {
+          ((uint8_t*)sm.edE[r])[g] = 0;
+          ((uint8_t*)sm.edS[r])[g] = 0;
+          ((uint8_t*)sm.seed[r])[g] = 0;
+        }
+  }
+  constexpr int kTW = TX / 16;
+  if (!__syncthreads_or(seed || mode == 0)) {
+    // nothing within reach changed: the tile keeps its labels, which seg_out holds
+    for (int i = threadIdx.x; i < TY * kTW; i += NT) {
+      const int gy = ty0 + i / kTW, wi = (tx0 >> 4) + i % kTW;
+      if (gy < H && wi < P16) chg_out[(size_t)gy * P16 + wi] = 0;
+    }
+    return;
+  }
+  // --- the sweeps
+  const float* __restrict__ img = S.img;
+  const SweepRec* __restrict__ rec = S.rec;
+  const bool neg = sm.neg != 0;
+  // the grid of a phase: 16-pixel half words of the rows of one y parity
+  constexpr int kHalves = 2 * kCK, kItems = kLY / 2 * kHalves;
+  for (int s = 0; s < ns; s++) {
+    const int cur = s & 1;
+    const int G = kReach * (ns - s) - 1;
+    // border mask at the sweep's start, inside the image and the tile grown by G; the
+    // first sweep's dirty pixels
+    bool any = false;
+    for (int i = threadIdx.x; i < kWords; i += NT) {
+      const int ay = i / kCK, c = i - ay * kCK;
+      unsigned m = 0;
+      if (ay >= max(kSH - G, -ry0) && ay < min(kSH + TY + G, H - ry0)) {
+        const unsigned e = sm.edE[ay][c];
+        m = e | (e << 1) | sm.edS[ay][c] | sm.edS[ay - 1][c];
+        if (kCK > 1 && c > 0) m |= sm.edE[ay][c - 1] >> 31;
+        m &= range32(max(kSH - G, -rx0), min(kSH + TX + G, W - rx0), c);
+      }
+      sm.bm[ay][c] = m;
+      unsigned d = 0xffffffffu;
+      if (s > 0) {
+        d = sm.dirty[ay][c];
+      } else {
+        if (mode) {
+          unsigned p = 0, w = 0, n = 0;
+#pragma unroll
+          for (int k = -1; k <= 1; k++) {
+            const int r = ay + k;
+            if (r < 0 || r >= kLY) continue;
+            w |= sm.seed[r][c];
+            if (kCK > 1 && c > 0) p |= sm.seed[r][c - 1];
+            if (kCK > 1 && c + 1 < kCK) n |= sm.seed[r][c + 1 < kCK ? c + 1 : c];
+          }
+          d = w | __funnelshift_l(p, w, 1) | __funnelshift_r(w, n, 1);
+        }
+        sm.dirty[ay][c] = d;
+      }
+      any |= (m & d) != 0;
+    }
+    if (threadIdx.x < 4) sm.cnt[cur ^ 1][threadIdx.x] = 0;
+    if (!__syncthreads_or(any)) break;   // nothing to score: nor in the later sweeps
+    for (int ph = 0; ph < 4; ph++) {
+      // the phase's pixels: dirty border pixels of the class ((x parity << 1) | y parity)
+      // on the tile grown by G - ph, listed by warp scans and one shared atomic per warp
+      const int g = G - ph;
+      for (int base = 0; base < kItems; base += NT) {
+        const int i = base + (int)threadIdx.x;
+        const int ay = 2 * (i / kHalves) + (ph & 1), h = i % kHalves, w = h >> 1;
+        unsigned m = 0;
+        if (ay >= kSH - g && ay < kSH + TY + g) {
+          m = sm.dirty[ay][w] & sm.bm[ay][w] & ((h & 1) ? 0xffff0000u : 0x0000ffffu) &
+              ((ph & 2) ? 0xAAAAAAAAu : 0x55555555u) & range32(kSH - g, kSH + TX + g, w);
+          if (m) atomicAnd(&sm.dirty[ay][w], ~m);
+        }
+        if (__any_sync(0xffffffffu, m != 0)) {
+          const int n = __popc(m);
+          int inc = n;
+#pragma unroll
+          for (int k = 1; k < 32; k <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, k);
+            if (lane >= k) inc += t;
+          }
+          int at = 0;
+          if (lane == 31) at = atomicAdd(&sm.cnt[cur][ph], inc);
+          at = __shfl_sync(0xffffffffu, at, 31) + inc - n;
+          const int ent = (ay << 8) | (32 * w);
+          for (; m; m &= m - 1) sm.list[at++] = (unsigned short)(ent + __ffs(m) - 1);
+        }
+      }
+      __syncthreads();
+      const int n = sm.cnt[cur][ph];
+      if (!n) continue;                               // block-uniform
+      for (int j = threadIdx.x; j < n; j += NT) {
+        const int ent = sm.list[j];
+        const int ax = ent & 255, ay = ent >> 8;
+        const int gx = rx0 + ax, gy = ry0 + ay;
+        const int p = ay * kLX + ax;
+        // the loads first (colour, 3x3 labels, then the records of the first two
+        // candidates: most border pixels have two), so their round trips overlap the
+        // simple-point tests
+        const float* pix = img + 3 * ((size_t)gy * W + gx);
+        const float c0 = __ldg(pix), c1 = __ldg(pix + 1), c2 = __ldg(pix + 2);
+        const int C = L[p];
+        const int N = L[p - kLX], So = L[p + kLX], Wl = L[p - 1], E = L[p + 1];
+        const int nb[8] = {L[p - kLX - 1], N, L[p - kLX + 1], Wl, E, L[p + kLX - 1], So,
+                           L[p + kLX + 1]};
+        // the distinct candidates in the order N, S, W, E (nothing to choose when every
+        // neighbour took this pixel's label since the sweep began)
+        const bool hS = So != N, hW = Wl != N && Wl != So, hE = E != N && E != So && E != Wl;
+        const int nc = 1 + hS + hW + hE;
+        if ((unsigned)C >= (unsigned)cap || (nc == 1 && N == C) || N >= cap || So >= cap ||
+            Wl >= cap || E >= cap)
+          continue;
+        const int k1 = hS ? So : hW ? Wl : hE ? E : N;
+        const int k2 = hS && hW ? Wl : E;
+        const SweepRec r0 = load_rec(rec, max(N, 0));
+        const SweepRec r1 = load_rec(rec, max(k1, 0));
+        // simple-point codes of the candidates: bit i set when neighbour i
+        // (NW,N,NE,W,E,SW,S,SE) carries the candidate or lies outside the image;
+        // differing neighbours = 8 - popcount
+        unsigned m1 = 0;
+        if (neg) {                                    // block-uniform
+#pragma unroll
+          for (int q = 0; q < 8; q++) m1 |= (unsigned)(nb[q] == -1) << q;
+        }
+        auto code = [&](int v) {
+          unsigned c = m1;
+#pragma unroll
+          for (int q = 0; q < 8; q++) c |= (unsigned)(nb[q] == v) << q;
+          return c;
+        };
+        auto simple = [&](unsigned c) { return (lut_bits[c >> 5] >> (c & 31)) & 1u; };
+        const unsigned d0 = code(N), d1 = code(k1);
+        if (!(simple(d0) & simple(d1))) continue;
+        unsigned d2 = 0, d3 = 0;
+        if (nc > 2) {
+          d2 = code(k2);
+          if (!simple(d2)) continue;
+          if (nc > 3) {
+            d3 = code(E);
+            if (!simple(d3)) continue;
+          }
+        }
+        // (both scores in one straight line: their chains overlap)
+        const float s0 = joint(c0, c1, c2, gx, gy, r0, s2, 8 - __popc(d0), potts);
+        const float s1 = joint(c0, c1, c2, gx, gy, r1, s2, 8 - __popc(d1), potts);
+        float best = -9999.f;
+        int bl = C;
+        if (N >= 0 && s0 > best) { best = s0; bl = N; }
+        if (nc > 1 && k1 >= 0 && s1 > best) { best = s1; bl = k1; }
+        if (nc > 2) {
+          if (k2 >= 0) {
+            const float t = joint(c0, c1, c2, gx, gy, load_rec(rec, k2), s2, 8 - __popc(d2), potts);
+            if (t > best) { best = t; bl = k2; }
+          }
+          if (nc > 3 && E >= 0) {
+            const float t = joint(c0, c1, c2, gx, gy, load_rec(rec, E), s2, 8 - __popc(d3), potts);
+            if (t > best) { best = t; bl = E; }
+          }
+        }
+        if (bl == C) {
+          const int n_c = N == C ? r0.count : k1 == C ? r1.count : __ldg(&rec[C].count);
+          if (n_c <= 2) {
+            if (N >= 0) bl = N;
+            else if (E >= 0) bl = E;
+            else if (So >= 0) bl = So;
+            else if (Wl >= 0) bl = Wl;
+          }
+        }
+        if (bl != C) {
+          L[p] = bl;
+          const int wx = ax >> 5;
+          const unsigned bit = 1u << (ax & 31);
+          // its 3x3 is dirty
+          const unsigned long long three = 7ull << ((ax & 31) + 31);   // bits 31.. = word wx
+          const unsigned mid = (unsigned)(three >> 32), lo = (unsigned)three & 0x80000000u;
+#pragma unroll
+          for (int k = -1; k <= 1; k++) {
+            atomicOr(&sm.dirty[ay + k][wx], mid);
+            if (lo) atomicOr(&sm.dirty[ay + k][wx - 1], lo);
+            if (bit >> 31) atomicOr(&sm.dirty[ay + k][wx + 1], 1u);
+          }
+          // and its four edges change (the pixels of a phase are never 4-neighbours, so
+          // each edge has one writer; words are shared)
+          atomicXor(&sm.edE[ay][wx], (C != E) != (bl != E) ? bit : 0u);
+          atomicXor(&sm.edE[ay][(ax - 1) >> 5],
+                    (C != Wl) != (bl != Wl) ? 1u << ((ax - 1) & 31) : 0u);
+          atomicXor(&sm.edS[ay][wx], (C != So) != (bl != So) ? bit : 0u);
+          atomicXor(&sm.edS[ay - 1][wx], (C != N) != (bl != N) ? bit : 0u);
+          if (ay >= kSH && ay < kSH + TY && ax >= kSH && ax < kSH + TX)
+            atomicOr(&sm.all[ay][wx], bit);
+        }
       }
       __syncthreads();
     }
-    // each row of the label region: its change bits from the previous sweep's plane
-    // (kNW 16-bit words starting at word rx0 >> 4, shifted by the region's offset in
-    // the first word), then dilated by the reach horizontally
-    constexpr int kNW = (kLX + 15) / 16 + 1;
-    static_assert(kNW <= 8 && kLX <= 128, "a label-region row spans at most 8 words");
-    const int w0 = rx0 >> 4;                     // rx0 >= -8: arithmetic shift floors
-    const int off = rx0 - (w0 << 4);             // 16 - halo, in 1..15
-    unsigned long long h0 = 0, h1 = 0;
-    bool nz = false;
-    const int r = threadIdx.x;
-    if (r < kLY) {
-      const int gy = ry0 + r;
-      unsigned long long lo = 0, hi = 0;
-      if (gy >= 0 && gy < H) {
-        const uint16_t* row = chg_in + (size_t)gy * P16;
-#pragma unroll
-        for (int k = 0; k < kNW; k++) {
-          const int wi = w0 + k;
-          const unsigned long long v = (wi >= 0 && wi < P16) ? (unsigned long long)row[wi] : 0ull;
-          if (k < 4) lo |= v << (16 * k);
-          else hi |= v << (16 * (k - 4));
-        }
-      }
-      unsigned long long f0 = (lo >> off) | (hi << (64 - off));
-      unsigned long long f1 = hi >> off;
-      if (mode == 2) {
-        // changed records seed the active set one pixel further out (a pixel reads the
-        // records of its 4-neighbours' labels)
-        unsigned long long q0 = sm.edE[0][r], q1 = sm.edE[1][r];
-        if (r > 0) { q0 |= sm.edE[0][r - 1]; q1 |= sm.edE[1][r - 1]; }
-        if (r + 1 < kLY) { q0 |= sm.edE[0][r + 1]; q1 |= sm.edE[1][r + 1]; }
-        f0 |= q0 | (q0 << 1) | (q0 >> 1) | (q1 << 63);
-        f1 |= q1 | (q1 << 1) | (q1 >> 1) | (q0 >> 63);
-      }
-      if (kLX < 64) { f0 &= (1ull << (kLX & 63)) - 1ull; f1 = 0; }
-      else if (kLX < 128) { f1 &= (1ull << ((kLX - 64) & 63)) - 1ull; }
-      nz = (f0 | f1) != 0;
-      h0 = f0; h1 = f1;
-#pragma unroll
-      for (int sft = 1; sft <= kReach; sft++) {
-        h0 |= (f0 << sft) | (f0 >> sft) | (f1 << (64 - sft));
-        h1 |= (f1 << sft) | (f1 >> sft) | (f0 >> (64 - sft));
-      }
-      a0[r] = h0;
-      a1[r] = h1;
-    }
-    if (!__syncthreads_or(nz)) {
-      // nothing within reach changed: the tile keeps its labels (for every sweep of
-      // the launch: a later sweep can only move pixels within reach of an earlier
-      // change, and there is none in the label region)
-#pragma unroll
-      for (int a = 0; a < kRW; a++) {
-        const int rr = warp * kRW + a;
-#pragma unroll
-        for (int c = 0; c < kCK; c++) {
-          const int x = lane + 32 * c;
-          if (rr < kLY && x < kLX && in_tile(rr, x))
-            seg_out[(size_t)(ry0 + rr) * W + (rx0 + x)] = lv[a][c];
-        }
-      }
-      // zero change words of the tile's rows
-      constexpr int kTW = kTX / 16;
-      for (int i = threadIdx.x; i < kTY * kTW; i += blockDim.x) {
-        const int gy = ty0 + i / kTW, wi = (tx0 >> 4) + i % kTW;
-        if (gy < H && wi < P16) chg_out[(size_t)gy * P16 + wi] = 0;
-      }
-      return;
-    }
-    // vertical dilation
-    unsigned long long v0 = 0, v1 = 0;
-    if (r < kLY) {
-      for (int k = max(0, r - kReach); k <= min(kLY - 1, r + kReach); k++) {
-        v0 |= a0[k]; v1 |= a1[k];
-      }
-    }
-    __syncthreads();
-    if (r < kLY) { a0[r] = v0; a1[r] = v1; }
-    // (the barrier after the label stores below orders these before the border pass)
   }
-  // labels to shared memory (colours are not staged: the scored border pixels read
-  // theirs from global memory), and the label edges of the warp's rows from the
-  // registers: right neighbours by shuffles, lower neighbours from the next row of
-  // the span (the span's last row waits for the shared copy, see sweep_pass)
-#pragma unroll
-  for (int a = 0; a < kRW; a++) {
-    const int r = warp * kRW + a;
-    unsigned e[kCK], d[kCK];
-#pragma unroll
-    for (int c = 0; c < kCK; c++) {
-      const int x = lane + 32 * c;
-      const int v = lv[a][c];
-      if (x < kLX) L[r * kLX + x] = v;
-      int right = __shfl_down_sync(0xffffffffu, v, 1);
-      const int nxt = __shfl_sync(0xffffffffu, lv[a][c + 1 < kCK ? c + 1 : c], 0);
-      if (lane == 31) right = c + 1 < kCK ? nxt : v;
-      e[c] = __ballot_sync(0xffffffffu, x + 1 < kLX && v != right);
-      d[c] = __ballot_sync(0xffffffffu, x < kLX && a + 1 < kRW && v != lv[a + 1 < kRW ? a + 1 : a][c]);
-    }
-    if (lane == 0) {
-      pack_row<kCK>(e, &sm.edE[0][r], &sm.edE[1][r]);
-      if (a + 1 < kRW) pack_row<kCK>(d, &sm.edS[0][r], &sm.edS[1][r]);
-    }
-  }
+  // --- write-back.  The pixels where seg_out is behind (mode 0: every pixel of the tile is
+  // stored) are listed like a phase's, kRowsOut rows at a time, and a relabelled one moves
+  // its statistics from the label it had at the launch's start to the one it has now.
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * kTY; i += blockDim.x) (&sm.chg[0][0])[i] = 0ull;
-  if (deltas) {
-    for (int i = threadIdx.x; i < kDeltaTab; i += blockDim.x) {
-      sm.delta.key[i] = -1;
-#pragma unroll
-      for (int f = 0; f < 12; f++) sm.delta.v[i][f] = 0;
+  if (deltas)
+    for (int i = threadIdx.x; i < kDeltaTab * 13; i += NT)
+      ((int*)&sm.delta)[i] = i < kDeltaTab ? -1 : 0;
+  if (mode == 0)
+    for (int i = threadIdx.x; i < TX * TY; i += NT) {
+      const int x = i % TX + kSH, y = i / TX + kSH;
+      const int gx = rx0 + x, gy = ry0 + y;
+      if (gx < W && gy < H) seg_out[(size_t)gy * W + gx] = L[y * kLX + x];
     }
-  }
-  // (the listing barrier of the first pass orders these clears before any use)
-  if (NS == 1) {
-    sweep_pass<TX, TY, NS, 4 * NS - 1, true>(S, sm, lut_bits, tx0, ty0, s2, potts, mode != 0,
-                                             true, deltas != 0);
-  } else {
-    sweep_pass<TX, TY, NS, 4 * NS - 1, true>(S, sm, lut_bits, tx0, ty0, s2, potts, mode != 0,
-                                             false, deltas != 0);
-    if (threadIdx.x < 4) cnt[threadIdx.x] = 0;   // fresh lists (the phases' last barrier
-                                                 // ordered every read of the counts)
-    sweep_pass<TX, TY, NS, 3, false>(S, sm, lut_bits, tx0, ty0, s2, potts, false, true,
-                                     deltas != 0);
-  }
-  if (deltas) delta_flush(sm.delta, S.sp, tx0, ty0);   // after the last phase's barrier
-  // write back the tile (a warp covers 32 consecutive pixels of a row; 16-wide tiles:
-  // two rows), then the change words of the last sweep: word i of a tile row holds
-  // tile columns 16 i .. 16 i + 15 = label-region columns kSH + 16 i ..
-  for (int i = threadIdx.x; i < kTX * kTY; i += blockDim.x) {
-    const int x = i % kTX, y = i / kTX;
-    const int gx = tx0 + x, gy = ty0 + y;
-    if (gx < W && gy < H) seg_out[(size_t)gy * W + gx] = L[(y + kSH) * kLX + (x + kSH)];
-  }
-  constexpr int kTW = kTX / 16;
-  for (int i = threadIdx.x; i < kTY * kTW; i += blockDim.x) {
+  // change words: word q of a tile row holds label-region columns kSH + 16 q ..
+  for (int i = threadIdx.x; i < TY * kTW; i += NT) {
     const int y = i / kTW, q = i % kTW;
     const int gy = ty0 + y, wi = (tx0 >> 4) + q;
     if (gy < H && wi < P16) {
-      const int b0 = kSH + 16 * q;
-      const unsigned long long lo = sm.chg[y][0], hi = sm.chg[y][1];
-      const unsigned long long v = b0 < 64 ? ((lo >> b0) | (b0 > 48 ? hi << (64 - b0) : 0ull))
-                                           : (hi >> (b0 - 64));
-      chg_out[(size_t)gy * P16 + wi] = (uint16_t)v;
+      const int b = kSH + 16 * q, c = b >> 5;
+      const unsigned lo = sm.all[y + kSH][c];
+      const unsigned hi = c + 1 < kCK ? sm.all[y + kSH][c + 1 < kCK ? c + 1 : c] : 0u;
+      chg_out[(size_t)gy * P16 + wi] = (uint16_t)__funnelshift_r(lo, hi, b & 31);
     }
   }
+  for (int y0 = kSH; y0 < kSH + TY; y0 += Tile::kRowsOut) {
+    for (int i = threadIdx.x; i < Tile::kRowsOut * kCK; i += NT) {
+      const int y = i / kCK + y0, c = i % kCK;
+      unsigned m = (sm.sin[y][c] & (mode ? range32(kSH, kSH + TX, c) : 0u)) | sm.all[y][c];
+      if (m) {
+        int at = atomicAdd(&sm.wcnt, __popc(m));
+        for (const int ent = (y << 8) | (32 * c); m; m &= m - 1)
+          sm.list[at++] = (unsigned short)(ent + __ffs(m) - 1);
+      }
+    }
+    __syncthreads();
+    const int nw = sm.wcnt;
+    for (int j = threadIdx.x; j < nw; j += NT) {
+      const int ent = sm.list[j];
+      const int ax = ent & 255, ay = ent >> 8;
+      const int gx = rx0 + ax, gy = ry0 + ay;
+      const size_t g = (size_t)gy * W + gx;
+      const int b = L[ay * kLX + ax];
+      if (mode) seg_out[g] = b;
+      if (deltas && ((sm.all[ay][ax >> 5] >> (ax & 31)) & 1u)) {
+        const int o = seg_in[g];
+        if (o != b) {
+          const float* pix = img + 3 * g;
+          delta_move(sm.delta, S.count, S.acc, o, b, gx, gy, tx0, ty0, __ldg(pix),
+                     __ldg(pix + 1), __ldg(pix + 2));
+        }
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) sm.wcnt = 0;
+    if (y0 + Tile::kRowsOut < kSH + TY) __syncthreads();
+  }
+  if (deltas) delta_flush(sm.delta, S.count, S.acc, tx0, ty0);
 }
 
-template <int TX, int TY, int NS>
+template <int TX, int TY, int NS, int NT>
 __device__ __forceinline__ void sweep_flat(const Slot* __restrict__ slots, int B, int parity,
-                                           float s2, float potts, int mode, int deltas) {
-  __shared__ SweepTile<TX, TY, NS> sm;
+                                           int ns, float s2, float potts, int mode, int deltas) {
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  SweepTile<TX, TY, NS>& sm = *(SweepTile<TX, TY, NS>*)sweep_smem;
   __shared__ unsigned lut_bits[8];
   if (threadIdx.x < 8) lut_bits[threadIdx.x] = c_simple_bits.w[threadIdx.x];
-  const int v = TX == 32 ? 0 : TX == 64 ? 1 : 2;   // which tile_base of the slots
+  constexpr int v = TY == 48 ? 3 : TX == 32 ? 0 : TX == 64 ? 1 : 2;   // the tile size (kGeomW)
   const int t = blockIdx.x;
   int lo = 0, hi = B - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (slots[mid].tile_base[v] <= t) lo = mid; else hi = mid - 1;
   }
-  const Slot& S = slots[lo];
-  const int tl = t - S.tile_base[v];
+  const SweepSlot S = sweep_slot(slots[lo], parity, v);
+  const int tl = t - S.tile0;
   const int tiles_x = (S.W + TX - 1) / TX;
-  sweep_tile<TX, TY, NS>(S, tl % tiles_x, tl / tiles_x, parity, s2, potts, sm, lut_bits, mode,
-                         deltas);
+  sweep_tile<TX, TY, NS, NT>(S, tl % tiles_x, tl / tiles_x, ns, s2, potts, sm, lut_bits, mode,
+                             deltas);
 }
 
 // Persistent work-queue form of the single-sweep launch: a resident set of blocks
@@ -1487,11 +1481,11 @@ __device__ __forceinline__ void sweep_queue(const Slot* __restrict__ slots, int 
       const int mid = (lo + hi + 1) >> 1;
       if (slots[mid].tile_base[v] <= t) lo = mid; else hi = mid - 1;
     }
-    const Slot& S = slots[lo];
-    const int tl = t - S.tile_base[v];
+    const SweepSlot S = sweep_slot(slots[lo], parity, v);
+    const int tl = t - S.tile0;
     const int tiles_x = (S.W + TX - 1) / TX;
-    sweep_tile<TX, TY, 1>(S, tl % tiles_x, tl / tiles_x, parity, s2, potts, sm, lut_bits, mode,
-                          deltas);
+    sweep_tile<TX, TY, 1, 256>(S, tl % tiles_x, tl / tiles_x, 1, s2, potts, sm, lut_bits, mode,
+                               deltas);
     __syncthreads();          // the tile's shared memory and `next` are free again
   }
   if (threadIdx.x == 0) {
@@ -1512,29 +1506,34 @@ __device__ __forceinline__ void sweep_queue(const Slot* __restrict__ slots, int 
     pdl_enter();                                                                             \
     sweep_queue<TX, 32>(slots, B, ntiles, queue, parity, s2, potts, mode, deltas);           \
   }
-STSPIX_SWEEPQ_KERNEL(kb_sweepq_t32, 32, 6)
-STSPIX_SWEEPQ_KERNEL(kb_sweepq_t64, 64, 6)
-STSPIX_SWEEPQ_KERNEL(kb_sweepq_t16, 16, 6)
+STSPIX_SWEEPQ_KERNEL(kb_sweepq_t32, 32, 4)
+STSPIX_SWEEPQ_KERNEL(kb_sweepq_t64, 64, 4)
+STSPIX_SWEEPQ_KERNEL(kb_sweepq_t16, 16, 4)
 #undef STSPIX_SWEEPQ_KERNEL
 
-// One block per tile of the batch (grid = the batch's total tile count), one sweep
-// (kb_sweep_t*) or two consecutive sweeps (kb_sweep2_t*) per launch.
-// mode 0: every border pixel (first sweep of an update_seg call); 1: active set.
-// deltas 1: move the statistics of every relabelled tile pixel (incremental
-// statistics: the sums of the labels at the call's start stay current); 0: not.
-#define STSPIX_SWEEP_KERNEL(name, TX, NS, MINB)                                          \
-  __global__ void __launch_bounds__(256, MINB) name(const Slot* __restrict__ slots, int B, \
-                                                    int parity, float s2, float potts,     \
-                                                    int mode, int deltas) {                \
-    pdl_enter();                                                                          \
-    sweep_flat<TX, 32, NS>(slots, B, parity, s2, potts, mode, deltas);                    \
-  }
-STSPIX_SWEEP_KERNEL(kb_sweep_t32, 32, 1, 6)
-STSPIX_SWEEP_KERNEL(kb_sweep_t64, 64, 1, 6)
-STSPIX_SWEEP_KERNEL(kb_sweep_t16, 16, 1, 6)
-STSPIX_SWEEP_KERNEL(kb_sweep2_t32, 32, 2, 4)
-STSPIX_SWEEP_KERNEL(kb_sweep2_t16, 16, 2, 4)
-STSPIX_SWEEP_KERNEL(kb_sweep2_t64, 64, 2, 4)
+// One block per tile of the batch (grid = the batch's total tile count), ns sweeps per
+// launch: up to one (kb_sweep_t*), two (kb_sweep2_t*) or four (kb_sweep4_*, see the rule in
+// update_seg).  Dynamic shared memory: the SweepTile (kb_sweep*_smem).
+// mode: what the first sweep scores (see sweep_tile).  deltas 1: move the statistics of
+// every relabelled tile pixel (incremental statistics: the sums of the labels at the
+// call's start stay current); 0: not.
+#define STSPIX_SWEEP_KERNEL(name, TX, TY, NS, NT, MINB)                                      \
+  __global__ void __launch_bounds__(NT, MINB) name(const Slot* __restrict__ slots, int B,    \
+                                                   int parity, int ns, float s2,             \
+                                                   float potts, int mode, int deltas) {      \
+    pdl_enter();                                                                             \
+    sweep_flat<TX, TY, NS, NT>(slots, B, parity, ns, s2, potts, mode, deltas);               \
+  }                                                                                          \
+  int name##_smem() { return (int)sizeof(SweepTile<TX, TY, NS>); }
+STSPIX_SWEEP_KERNEL(kb_sweep_t32, 32, 32, 1, 256, 4)
+STSPIX_SWEEP_KERNEL(kb_sweep_t64, 64, 32, 1, 256, 4)
+STSPIX_SWEEP_KERNEL(kb_sweep_t16, 16, 32, 1, 256, 4)
+STSPIX_SWEEP_KERNEL(kb_sweep2_t32, 32, 32, 2, 256, 4)
+STSPIX_SWEEP_KERNEL(kb_sweep2_t16, 16, 32, 2, 256, 4)
+STSPIX_SWEEP_KERNEL(kb_sweep2_t64, 64, 32, 2, 256, 4)
+STSPIX_SWEEP_KERNEL(kb_sweep4_s, 32, 32, 4, 512, 2)
+STSPIX_SWEEP_KERNEL(kb_sweep4_m, 64, 32, 4, 256, 4)
+STSPIX_SWEEP_KERNEL(kb_sweep4_l, 64, 48, 4, 256, 4)
 #undef STSPIX_SWEEP_KERNEL
 
 // ---------------------------------------------------------------------------

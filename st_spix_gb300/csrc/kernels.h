@@ -40,28 +40,31 @@ __global__ void k_label_stats_out(int n, int mode, const long long* iacc, const 
                                   const double* dacc, double* out);
 __global__ void kb_store_sample(const Slot* slots);
 __global__ void kb_find_border(const Slot* slots);
-// boundary sweep, one block per 32x32 / 64x32 / 16x32 tile of the batch
-__global__ void kb_sweep_t32(const Slot* slots, int B, int parity, float s2, float potts,
-                             int mode, int deltas);
-__global__ void kb_sweep_t64(const Slot* slots, int B, int parity, float s2, float potts,
-                             int mode, int deltas);
-__global__ void kb_sweep_t16(const Slot* slots, int B, int parity, float s2, float potts,
-                             int mode, int deltas);
-// the same single sweep as a persistent work-queue kernel (queue: 2 counters, zero
-// between launches)
+// boundary sweeps, one block per tile of the batch, ns sweeps per launch: 1 (kb_sweep_t*:
+// 32x32, 64x32 and 16x32 tiles), up to 2 (kb_sweep2_t*), up to 4 (kb_sweep4_*: 32x32 tiles
+// of 512 threads, 64x32 and 64x48 tiles of 256); name_smem: dynamic shared memory in bytes
+#define STSPIX_DECL_SWEEP(name)                                                             \
+  __global__ void name(const Slot* slots, int B, int parity, int ns, float s2, float potts, \
+                       int mode, int deltas);                                               \
+  int name##_smem();
+STSPIX_DECL_SWEEP(kb_sweep_t32)
+STSPIX_DECL_SWEEP(kb_sweep_t64)
+STSPIX_DECL_SWEEP(kb_sweep_t16)
+STSPIX_DECL_SWEEP(kb_sweep2_t32)
+STSPIX_DECL_SWEEP(kb_sweep2_t64)
+STSPIX_DECL_SWEEP(kb_sweep2_t16)
+STSPIX_DECL_SWEEP(kb_sweep4_s)
+STSPIX_DECL_SWEEP(kb_sweep4_m)
+STSPIX_DECL_SWEEP(kb_sweep4_l)
+#undef STSPIX_DECL_SWEEP
+// the single sweep as a persistent work-queue kernel (queue: 2 counters, zero between
+// launches)
 __global__ void kb_sweepq_t32(const Slot* slots, int B, int ntiles, unsigned* queue, int parity,
                               float s2, float potts, int mode, int deltas);
 __global__ void kb_sweepq_t64(const Slot* slots, int B, int ntiles, unsigned* queue, int parity,
                               float s2, float potts, int mode, int deltas);
 __global__ void kb_sweepq_t16(const Slot* slots, int B, int ntiles, unsigned* queue, int parity,
                               float s2, float potts, int mode, int deltas);
-// two consecutive sweeps per launch (8-pixel halo)
-__global__ void kb_sweep2_t32(const Slot* slots, int B, int parity, float s2, float potts,
-                              int mode, int deltas);
-__global__ void kb_sweep2_t16(const Slot* slots, int B, int parity, float s2, float potts,
-                              int mode, int deltas);
-__global__ void kb_sweep2_t64(const Slot* slots, int B, int parity, float s2, float potts,
-                              int mode, int deltas);
 __global__ void kb_copy_labels(const Slot* slots);
 __global__ void kb_read_params(const Slot* slots);
 __global__ void kb_save_prev(const Slot* slots);
