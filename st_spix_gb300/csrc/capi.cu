@@ -321,7 +321,7 @@ constexpr long long kPixBytes = 1 + 5 * 4 + 8 + 4 + 2;        // border, d1 d2 s
 constexpr long long kSpDevBytes = 4 + 1 + 1 + 4 + 4 + 4 + 12 + 16 + 24 + 8 + 12 + 16 + 24 + 24 + 24 +
                                   64 + (long long)sizeof(SweepRec);
 constexpr long long kSmBytes = 4 + 24 + 24 + 4 + 4 + 4 + 4 + 4 + 1 + 8;
-constexpr long long kAuxBytes = 5 * 1 + 6 * 4 + 16 + 8 + 4 + 16 + 8 + 8 + 72 + 4 + 1 + 24;
+constexpr long long kAuxBytes = 5 * 1 + 6 * 4 + 16 + 8 + 4 + 16 + 8 + 8 + 72 + 1 + 24;
 constexpr long long kParamBytes = 12 + 12 + 16 + 24 + 4 + 16 + 24 + 24 + 4 + 4 + 4 + 4 + 4;
 
 // Make sure slot position i holds npix pixels and sp_cap superpixels.  Growing
@@ -363,7 +363,7 @@ int ensure_slot(stspix_ctx* ctx, int i, int npix, int sp_cap) {
     AL(L, s.fs, 2 * c2); AL(L, s.fds, 2 * c2); AL(L, s.ss, c2);
     AL(L, s.centers, 2 * c2); AL(L, s.rbest, c2); AL(L, s.ccbest, c2);
     AL(L, s.bbox, 4 * c2);
-    AL(L, s.snap, 9 * c2); AL(L, s.post_ids, c2); AL(L, s.recchg, c2);
+    AL(L, s.snap, 9 * c2); AL(L, s.recchg, c2);
     AL(L, s.pscache, 3 * c2);
     w.sp_cap = cap;
   }
@@ -425,7 +425,6 @@ void preload_kernels() {
       (const void*)kb_clear_stats,
       (const void*)kb_accumulate,
       (const void*)kb_posterior,
-      (const void*)kb_post_list,
       (const void*)kb_store_sample,
       (const void*)kb_find_border,
       (const void*)kb_sweep_t32,
@@ -650,7 +649,7 @@ void accumulate_fp(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, int 
 
 // stats_ready: the last sweep of the preceding update_seg already cleared and added
 // the statistics of the first nb slots (see update_seg).
-// incremental: only the ids whose sums changed since their last posterior (kb_post_list);
+// incremental: only the ids whose sums changed since their last posterior;
 // only where nothing but sweeps ran since the previous posterior of every slot.
 int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
                   bool stats_ready = false, bool incremental = false) {
@@ -661,9 +660,8 @@ int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
   }
   if (ctx->accumulator) accumulate_fp(ctx, st, L, nb, ctx->accumulator);
   ctx->cur_fam = STSPIX_FAM_POSTERIOR;
-  LAUNCHB(kb_post_list, L.max_cap, L, nb, incremental ? 1 : 0);
-  // groups of 32 listed ids, about four blocks per SM over the batch (a block loops
-  // when a slot lists more groups)
+  // groups of 32 ids, about four blocks per SM over the batch (a block loops over a slot's
+  // further groups)
   const unsigned pg = (unsigned)std::min<long long>((L.max_cap + 31) / 32,
                                                     std::max(32, (4 * ctx->num_sms + nb - 1) / nb));
   LAUNCHG(kb_posterior, dim3(pg, (unsigned)nb), 128, L.d, incremental ? 1 : 0);

@@ -120,8 +120,6 @@ struct Scalars {
   // (class counts, write cursors)
   int fl_n, fl_prev, fl_iter, fl_done, fl_fill;
   int fl_cnt[4], fl_pos[4];
-  // posterior work list: ids listed, blocks of the posterior launch done
-  int npost, post_done;
 };
 
 // One frame of a batch: its inputs, outputs, workspace and scalars.  Kernels take
@@ -169,7 +167,6 @@ struct Slot {
   long long* snap;         // [9*(cap+2)]: count and the 8 sums each id's posterior last saw
   uint8_t* recchg;         // [cap+2]: the last posterior changed the id's SweepRec
   double* pscache;         // [3*(cap+2)]: the prior shape term of the last full posterior
-  int* post_ids;           // [cap+2]: ids of the running posterior (kb_post_list)
   Scalars* sc;
   int tile_base[kSweepGeoms];  // first sweep tile of this slot in the batch, per tile size
 };
@@ -211,7 +208,7 @@ __device__ __forceinline__ long long fx_q(float v, int shift) {
   return (long long)__float2int_rz(h) * 262144LL + (long long)__float2int_rn(l);
 }
 __device__ __forceinline__ double fx_unq(long long q, int shift) {
-  return ldexp((double)q, -shift);
+  return (double)q * (1.0 / (double)(1u << shift));   // a power of two: exact
 }
 // Full-warp sum of a 64-bit integer by 32-bit reductions: v = hi * 2^24 + lo with lo in
 // [0, 2^24), so the lo parts of 32 lanes stay below 2^29; |v| < 2^54 per lane.

@@ -483,199 +483,177 @@ __device__ __forceinline__ void smooth_prior(double in_x, double in_y, double in
 // mean and scatter; then warps 0-2 one smoothed covariance entry each, then warps 0-2
 // one inverse entry each and warp 3 the log determinant.  Every value is the same
 // expression as a single-thread evaluation, exchanged through shared memory.
-// k: this lane's id (-1: none).  cached: the prior shape term is read from S.pscache,
-// which the last full posterior wrote (incremental posteriors: the priors, flags and
-// sample covariance it depends on change only in the steps followed by a full one).
-__device__ __forceinline__ void posterior_ids(const Slot& S, int k, bool cached) {
-  __shared__ double v_ps[3][32], v_raw[3][32], v_m[2][32], v_s[3][32], v_i[4][32];
-  __shared__ float v_app[3][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const SpDev& sp = S.sp;
-  const bool inr = k >= 0 && k < sp.cap;
-  // every load of the id is issued before any is used (one memory round trip): the
-  // count and flags, and the fields this warp's part of the posterior reads
-  int count_int = 0;
-  uint8_t valid = 0, prop = 0;
-  float pc = 0.f;
-  long long a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0;
-  double q0 = 0, q1 = 0, q2 = 0, i0 = 0, i1 = 0, i2 = 0;
-  const long long* a = sp.acc + 8 * (size_t)k;
-  if (inr) {
-    count_int = sp.count[k];
-    valid = sp.valid[k];
-    if (w == 0) { a0 = a[0]; a1 = a[1]; a2 = a[2]; }
-    else if (w == 1) {
-      pc = sp.prior_count[k];
-      if (cached) {
-        q0 = S.pscache[3 * (size_t)k]; q1 = S.pscache[3 * (size_t)k + 1];
-        q2 = S.pscache[3 * (size_t)k + 2];
-      } else {
-        prop = sp.prop[k];
-        q0 = sp.sample_sigma_shape[3 * k]; q1 = sp.sample_sigma_shape[3 * k + 1];
-        q2 = sp.sample_sigma_shape[3 * k + 2];
-        i0 = sp.prior_icov[3 * k]; i1 = sp.prior_icov[3 * k + 1]; i2 = sp.prior_icov[3 * k + 2];
-      }
-    } else if (w == 2) { a0 = a[3]; a1 = a[4]; a2 = a[5]; a3 = a[6]; a4 = a[7]; }
-    if (w != 1) pc = sp.prior_count[k];
-  }
-  const bool live = valid && count_int > 0;
-  if (w == 0 && inr) {
-    if (valid && count_int <= 0) sp.valid[k] = 0;
-    if (!live) {
-      for (int c = 0; c < 3; c++) { sp.mu_app[3 * k + c] = 0.f; sp.sigma_shape[3 * k + c] = 0.0; }
-      sp.mu_shape[2 * k] = 0.0; sp.mu_shape[2 * k + 1] = 0.0;
-    }
-  }
-  if (!__syncthreads_or(live)) return;
-  const double count = count_int * 1.0;
-  const double total_count = (double)count_int + pc * 50;
-  if (live) {
-    if (w == 0) {
-      // colour means (fixed-point sums, R1)
-      const long long ac[3] = {a0, a1, a2};
-      for (int c = 0; c < 3; c++) {
-        const float m = (float)(fx_unq(ac[c], kFxAppShift) / count);
-        sp.mu_app[3 * k + c] = m;
-        v_app[c][lane] = m;
-      }
-    } else if (w == 1) {
-      // prior shape term (calc_simple_update with _add_sigma_smoothing)
-      if (cached) {
-        v_ps[0][lane] = q0; v_ps[1][lane] = q1; v_ps[2][lane] = q2;
-      } else {
-        double px, py, pz;
-        if (prop) {
-          smooth_prior(q0, q1, q2, (int)pc, pc, S.sp_size, &px, &py, &pz);
-        } else {
-          px = i0; py = i1; pz = i2;
-        }
-        double pr_det = px * pz - py * py;
-        if (!(pr_det > 0)) atomicExch(&S.sc->status, STSPIX_ERR_DEGENERATE);
-        pr_det = sqrt(pr_det);
-        const double t0 = pc / pr_det * px, t1 = pc / pr_det * py, t2 = pc / pr_det * pz;
-        v_ps[0][lane] = t0; v_ps[1][lane] = t1; v_ps[2][lane] = t2;
-        S.pscache[3 * (size_t)k] = t0; S.pscache[3 * (size_t)k + 1] = t1;
-        S.pscache[3 * (size_t)k + 2] = t2;
-      }
-    } else if (w == 2) {
-      // shape mean and scatter
-      const double mx = a0 / count, my = a1 / count;
-      sp.mu_shape[2 * k] = mx; sp.mu_shape[2 * k + 1] = my;
-      v_m[0][lane] = mx; v_m[1][lane] = my;
-      v_raw[0][lane] = a2 - count * mx * mx;
-      v_raw[1][lane] = a3 - count * mx * my;
-      v_raw[2][lane] = a4 - count * my * my;
-    }
-  }
-  __syncthreads();
-  if (live && w < 3) v_s[w][lane] = (pc * v_ps[w][lane] + v_raw[w][lane]) / (total_count + 3.0);
-  __syncthreads();
-  if (live) {
-    double sx = v_s[0][lane], sy = v_s[1][lane], sz = v_s[2][lane];
-    double det = sx * sz - sy * sy;
-    if (det <= 0) {
-      sx = sx + 0.00001;
-      sz = sz + 0.00001;
-      det = sx * sz - sy * sy;
-      if (det <= 0) det = 0.00001;
-    }
-    if (w == 0) v_i[0][lane] = sz / det;
-    else if (w == 1) v_i[1][lane] = -sy / det;
-    else if (w == 2) v_i[2][lane] = sx / det;
-    else v_i[3][lane] = log(det);
-  }
-  __syncthreads();
-  if (live && w == 0) {
-    const double ix = v_i[0][lane], iy = v_i[1][lane], iz = v_i[2][lane], ld = v_i[3][lane];
-    const double mx = v_m[0][lane], my = v_m[1][lane];
-    sp.sigma_shape[3 * k] = ix; sp.sigma_shape[3 * k + 1] = iy; sp.sigma_shape[3 * k + 2] = iz;
-    sp.logdet[k] = ld;
-    SweepRec r;
-    r.mu_r = v_app[0][lane]; r.mu_g = v_app[1][lane]; r.mu_b = v_app[2][lane];
-    r.logdet = (float)ld;
-    const double fx = floor(mx), fy = floor(my);
-    r.mxi = (int)fx; r.myi = (int)fy;
-    r.frac = (mx != fx ? 1 : 0) | (my != fy ? 2 : 0);
-    r.isx = (float)ix; r.isy = (float)iy; r.isz = (float)iz; r.pad = 0.f;
-    r.count = count_int;
-    // the sweeps of the next update score again only the pixels next to a changed record
-    const uint4* o = (const uint4*)&sp.rec[k];
-    const uint4* nw = (const uint4*)&r;
-    bool same = true;
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      const uint4 a = o[q], b = nw[q];
-      same &= a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w;
-    }
-    if (!same) S.recchg[k] = 1;
-    sp.rec[k] = r;
-  }
-}
-
-// The posterior's work list (ids 0 .. max_spix, below cap): every id, or with
-// `incremental` only the ids whose count or sums differ from those its posterior last
-// saw.  Between two posteriors of the outer loop only the sweeps run, which change no
-// other input of the posterior (priors, flags and the sample covariance change in the
-// split, merge and relabel steps and at the frame's set-up, whose posteriors are full),
-// so an id with equal sums would get the values it already holds (the same
-// expressions of the same inputs).  Listed ids record their sums; the list's order
-// varies, each id's result does not.
-__global__ void kb_post_list(const Slot* __restrict__ slots, int incremental) {
-  pdl_enter();
-  SLOT_Y;
-  const int last = min(S.sp.cap - 1, S.sc->max_spix);
-  if ((int)(blockIdx.x * blockDim.x) > last) return;     // block-uniform
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  bool want = false;
-  if (k <= last) {
-    S.recchg[k] = 0;                       // set by kb_posterior when the record changes
-    const long long* a = S.sp.acc + 8 * (size_t)k;
-    long long* snap = S.snap + 9 * (size_t)k;
-    long long cur[9];
-#pragma unroll
-    for (int f = 0; f < 8; f++) cur[f] = a[f];
-    cur[8] = S.sp.count[k];
-    want = !incremental;
-    if (incremental) {
-#pragma unroll
-      for (int f = 0; f < 9; f++) want |= cur[f] != snap[f];
-    }
-    if (want) {
-#pragma unroll
-      for (int f = 0; f < 9; f++) snap[f] = cur[f];
-    }
-  }
-  const unsigned m = __ballot_sync(0xffffffffu, want);
-  if (!m) return;
-  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-  int base = 0;
-  if (lane == leader) base = atomicAdd(&S.sc->npost, __popc(m));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  const int pos = base + __popc(m & ((1u << lane) - 1));
-  if (want && pos < S.sp.cap) S.post_ids[pos] = k;     // at most cap ids are listed
-}
-
-// Grid: x blocks per slot, each taking groups of 32 listed ids x, x + gridDim.x, ...
-// A group's barriers are block-uniform, and the first barrier of the next group follows
-// every read of the previous one's shared values.  The last block of a slot to finish
-// clears the list for the next posterior (every block read the list length first).
+//
+// incremental: only the ids whose count or sums differ from those their posterior last saw
+// (S.snap) are computed.  Between two posteriors of the outer loop only the sweeps run,
+// which change no other input of the posterior (priors, flags and the sample covariance
+// change in the split, merge and relabel steps and at the frame's set-up, whose posteriors
+// are full), so an id with equal sums would get the values it already holds (the same
+// expressions of the same inputs).  The prior shape term is read from S.pscache then, which
+// the last full posterior wrote.
+//
+// Every load of a group, the old record and the snapshot among them, is issued before any
+// is used, and the ids are compared where they are computed: what bounds a launch is the
+// chain launch - slot - loads - FP64 - store, one group per block on most frames.  With
+// a work list of the changed ids built by a kernel of its own a posterior took 10.5 us on
+// a 240x320 frame, 13.4 on 720x1280 and 17.1 on 8 frames of 480x854; now 5.7, 7.5 and 11.6.
 __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slots,
                                                     int incremental) {
   pdl_enter();
   SLOT_Y;
-  Scalars* sc = S.sc;
-  const int n = min(*(volatile int*)&sc->npost, S.sp.cap);
-  for (int g = blockIdx.x; g * 32 < n; g += gridDim.x) {
-    const int i = g * 32 + (threadIdx.x & 31);
-    posterior_ids(S, i < n ? S.post_ids[i] : -1, incremental != 0);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(&sc->post_done, 1) == (int)gridDim.x - 1) {
-      sc->npost = 0;
-      sc->post_done = 0;
-      __threadfence();
+  __shared__ double v_ps[3][32], v_raw[3][32], v_m[2][32], v_s[3][32], v_i[4][32];
+  __shared__ float v_app[3][32];
+  __shared__ int s_diff[2][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const SpDev& sp = S.sp;
+  const int cap = sp.cap;
+  const int last = min(cap - 1, S.sc->max_spix);
+  for (int g = blockIdx.x;; g += gridDim.x) {
+    const int k = 32 * g + lane;
+    // warp 0: colour sums, count and record; warp 1: the prior; warp 2: position sums
+    int count_int = 0;
+    uint8_t valid = 0, prop = 0;
+    float pc = 0.f;
+    long long a[5] = {0, 0, 0, 0, 0}, o[5] = {0, 0, 0, 0, 0}, ocount = 0;
+    double q0 = 0, q1 = 0, q2 = 0, i0 = 0, i1 = 0, i2 = 0;
+    uint4 orec[3];
+    if (k < cap) {
+      const long long* acc = sp.acc + 8 * (size_t)k;
+      const long long* snap = S.snap + 9 * (size_t)k;
+      count_int = sp.count[k];
+      valid = sp.valid[k];
+      pc = sp.prior_count[k];
+      if (w == 0) {
+#pragma unroll
+        for (int f = 0; f < 3; f++) { a[f] = acc[f]; o[f] = snap[f]; }
+        ocount = snap[8];
+#pragma unroll
+        for (int q = 0; q < 3; q++) orec[q] = ((const uint4*)&sp.rec[k])[q];
+      } else if (w == 1) {
+        if (incremental) {
+          q0 = S.pscache[3 * (size_t)k]; q1 = S.pscache[3 * (size_t)k + 1];
+          q2 = S.pscache[3 * (size_t)k + 2];
+        } else {
+          prop = sp.prop[k];
+          q0 = sp.sample_sigma_shape[3 * k]; q1 = sp.sample_sigma_shape[3 * k + 1];
+          q2 = sp.sample_sigma_shape[3 * k + 2];
+          i0 = sp.prior_icov[3 * k]; i1 = sp.prior_icov[3 * k + 1]; i2 = sp.prior_icov[3 * k + 2];
+        }
+      } else if (w == 2) {
+#pragma unroll
+        for (int f = 0; f < 5; f++) { a[f] = acc[3 + f]; o[f] = snap[3 + f]; }
+      }
+    }
+    if (32 * g > last) return;                     // block-uniform
+    const bool inr = k <= last;
+    if (w == 0 || w == 2) {
+      bool diff = !incremental;
+#pragma unroll
+      for (int f = 0; f < 5; f++) diff |= a[f] != o[f];
+      if (w == 0) diff |= ocount != count_int;
+      s_diff[w >> 1][lane] = inr && diff;
+    }
+    __syncthreads();
+    const bool want = s_diff[0][lane] | s_diff[1][lane];
+    const bool live = want && valid && count_int > 0;
+    if (want) {
+      long long* snap = S.snap + 9 * (size_t)k;
+      if (w == 0) {
+#pragma unroll
+        for (int f = 0; f < 3; f++) snap[f] = a[f];
+        snap[8] = count_int;
+        if (valid && count_int <= 0) sp.valid[k] = 0;
+        if (!live) {
+          for (int c = 0; c < 3; c++) { sp.mu_app[3 * k + c] = 0.f; sp.sigma_shape[3 * k + c] = 0.0; }
+          sp.mu_shape[2 * k] = 0.0; sp.mu_shape[2 * k + 1] = 0.0;
+        }
+      } else if (w == 2) {
+#pragma unroll
+        for (int f = 0; f < 5; f++) snap[3 + f] = a[f];
+      }
+    }
+    // (the sweeps of the next update score again only the pixels next to a changed record)
+    if (w == 0 && inr && !live) S.recchg[k] = 0;
+    if (!__syncthreads_or(live)) continue;
+    const double count = count_int * 1.0;
+    const double total_count = (double)count_int + pc * 50;
+    if (live) {
+      if (w == 0) {
+        // colour means (fixed-point sums, R1)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const float m = (float)(fx_unq(a[c], kFxAppShift) / count);
+          sp.mu_app[3 * k + c] = m;
+          v_app[c][lane] = m;
+        }
+      } else if (w == 1) {
+        // prior shape term (calc_simple_update with _add_sigma_smoothing)
+        if (incremental) {
+          v_ps[0][lane] = q0; v_ps[1][lane] = q1; v_ps[2][lane] = q2;
+        } else {
+          double px, py, pz;
+          if (prop) {
+            smooth_prior(q0, q1, q2, (int)pc, pc, S.sp_size, &px, &py, &pz);
+          } else {
+            px = i0; py = i1; pz = i2;
+          }
+          double pr_det = px * pz - py * py;
+          if (!(pr_det > 0)) atomicExch(&S.sc->status, STSPIX_ERR_DEGENERATE);
+          pr_det = sqrt(pr_det);
+          const double t0 = pc / pr_det * px, t1 = pc / pr_det * py, t2 = pc / pr_det * pz;
+          v_ps[0][lane] = t0; v_ps[1][lane] = t1; v_ps[2][lane] = t2;
+          S.pscache[3 * (size_t)k] = t0; S.pscache[3 * (size_t)k + 1] = t1;
+          S.pscache[3 * (size_t)k + 2] = t2;
+        }
+      } else if (w == 2) {
+        // shape mean and scatter
+        const double mx = a[0] / count, my = a[1] / count;
+        sp.mu_shape[2 * k] = mx; sp.mu_shape[2 * k + 1] = my;
+        v_m[0][lane] = mx; v_m[1][lane] = my;
+        v_raw[0][lane] = a[2] - count * mx * mx;
+        v_raw[1][lane] = a[3] - count * mx * my;
+        v_raw[2][lane] = a[4] - count * my * my;
+      }
+    }
+    __syncthreads();
+    if (live && w < 3) v_s[w][lane] = (pc * v_ps[w][lane] + v_raw[w][lane]) / (total_count + 3.0);
+    __syncthreads();
+    if (live) {
+      double sx = v_s[0][lane], sy = v_s[1][lane], sz = v_s[2][lane];
+      double det = sx * sz - sy * sy;
+      if (det <= 0) {
+        sx = sx + 0.00001;
+        sz = sz + 0.00001;
+        det = sx * sz - sy * sy;
+        if (det <= 0) det = 0.00001;
+      }
+      if (w == 0) v_i[0][lane] = sz / det;
+      else if (w == 1) v_i[1][lane] = -sy / det;
+      else if (w == 2) v_i[2][lane] = sx / det;
+      else v_i[3][lane] = log(det);
+    }
+    __syncthreads();
+    if (live && w == 0) {
+      const double ix = v_i[0][lane], iy = v_i[1][lane], iz = v_i[2][lane], ld = v_i[3][lane];
+      const double mx = v_m[0][lane], my = v_m[1][lane];
+      sp.sigma_shape[3 * k] = ix; sp.sigma_shape[3 * k + 1] = iy; sp.sigma_shape[3 * k + 2] = iz;
+      sp.logdet[k] = ld;
+      SweepRec r;
+      r.mu_r = v_app[0][lane]; r.mu_g = v_app[1][lane]; r.mu_b = v_app[2][lane];
+      r.logdet = (float)ld;
+      const double fx = floor(mx), fy = floor(my);
+      r.mxi = (int)fx; r.myi = (int)fy;
+      r.frac = (mx != fx ? 1 : 0) | (my != fy ? 2 : 0);
+      r.isx = (float)ix; r.isy = (float)iy; r.isz = (float)iz; r.pad = 0.f;
+      r.count = count_int;
+      const uint4* nw = (const uint4*)&r;
+      bool same = true;
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+        same &= orec[q].x == nw[q].x && orec[q].y == nw[q].y && orec[q].z == nw[q].z &&
+                orec[q].w == nw[q].w;
+      S.recchg[k] = same ? 0 : 1;
+      sp.rec[k] = r;
     }
   }
 }
@@ -1584,7 +1562,6 @@ __global__ void kb_scalars(const Slot* __restrict__ slots, int B, int op) {
       sc->fill_iters = 0;
       sc->ninvalid = 0;
       sc->tmp0 = sc->tmp1 = sc->tmp2 = 0;
-      sc->npost = sc->post_done = 0;
       sc->nspix = 0;
       if (S.mode) { sc->max_spix = S.n_prev - 1; sc->nbuf_logical = 10 * S.n_prev; }
       else { sc->max_spix = 0; sc->nbuf_logical = 30 * S.nraw; }
