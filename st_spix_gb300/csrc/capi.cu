@@ -73,6 +73,7 @@ struct List {
   Slot* d = nullptr;               // device table
   int B = 0;
   int max_npix = 0, max_cap = 0, max_nprev = 0, max_w = 0, max_h = 0;
+  int max_words = 0;               // 16-pixel change words
   bool any_prop = false;
   std::vector<int> tiles_upto[kSweepGeoms];  // sweep tiles of the first i slots, per tile size
   std::vector<long long> segs_upto;  // 32-pixel row segments of the first i slots
@@ -616,6 +617,7 @@ List make_list(stspix_ctx* ctx, int off, const std::vector<Slot>& slots) {
     // a bound on n_prev that depends on the capacity only (grids over previous ids)
     if (s.mode) L.max_nprev = std::max(L.max_nprev, (s.cap - 2) / 10);
     L.max_w = std::max(L.max_w, s.W);
+    L.max_words = std::max(L.max_words, s.H * ((s.W + 15) / 16));
     L.max_h = std::max(L.max_h, s.H);
     if (s.mode) L.any_prop = true;
   }
@@ -652,10 +654,10 @@ void accumulate_fp(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, int 
 // incremental: only the ids whose sums changed since their last posterior;
 // only where nothing but sweeps ran since the previous posterior of every slot.
 int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
-                  bool stats_ready = false, bool incremental = false) {
+                  bool stats_ready = false, bool incremental = false, bool clear_all = false) {
   ctx->cur_fam = STSPIX_FAM_STATS;
   if (!stats_ready) {
-    LAUNCHB(kb_clear_stats, L.max_cap, L, nb);
+    LAUNCHB(kb_clear_stats, L.max_cap, L, nb, clear_all ? 1 : 0);
     LAUNCHG(kb_accumulate, acc_blocks(ctx, L, nb), 256, L.d, nb);
   }
   if (ctx->accumulator) accumulate_fp(ctx, st, L, nb, ctx->accumulator);
@@ -762,7 +764,7 @@ int update_seg(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
   }
   *chg_ok = nseg > 0;
   if (*cur && !(keep && fuse_stats)) {
-    LAUNCHB(kb_copy_labels, pix_units(L.max_npix), L, nb);
+    LAUNCHB(kb_copy_labels, L.max_words, L, nb);
     *cur = 0;
     *chg_ok = false;
   }
@@ -820,10 +822,10 @@ int run_relabel(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
 }
 
 int run_merge(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmConsts& K,
-              const stspix_config& cfg, int dir_b, int dir_p) {
+              const stspix_config& cfg, int dir_b, int dir_p, bool use_border) {
   ctx->cur_fam = STSPIX_FAM_MERGE;
   LAUNCHB(kb_merge_clear, L.max_cap + 2, L, nb);
-  LAUNCHB(kb_merge_candidates, pix_units(L.max_npix), L, nb, dir_b, dir_p);
+  LAUNCHB(kb_merge_candidates, pix_units(L.max_npix), L, nb, dir_b, dir_p, use_border ? 1 : 0);
   LAUNCHB(kb_sm_clear, L.max_cap + 2, L, nb);
   LAUNCHG(kb_sm_accumulate, dim3(tiles64(L), (unsigned)nb), kThreads, L.d, 0);
   LAUNCHG(kb_merge_single, dim3((unsigned)((L.max_cap + 31) / 32), (unsigned)nb), 128, L.d, K);
@@ -859,7 +861,7 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
       return STSPIX_OK;
     }
     // after the first iteration only the sweeps ran since every slot's last posterior
-    if ((r = update_params(ctx, st, L, nb, stats_ready, idx > 0))) return r;
+    if ((r = update_params(ctx, st, L, nb, stats_ready, idx > 0, idx == 0))) return r;
     stats_ready = false;
     // the first sweep is an active-set one when only sweeps and that incremental
     // posterior ran since the previous update_seg
@@ -875,17 +877,18 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
       if (idx % P == P / 2) {
         count_p += 1;  // propagated frames step the direction again before merging
         if (L.any_prop && (r = run_relabel(ctx, st, L, nb, cfg))) return r;
-        if ((r = run_merge(ctx, st, L, nb, K, cfg, count_b % 2, count_p % 2))) return r;
+        if ((r = run_merge(ctx, st, L, nb, K, cfg, count_b % 2, count_p % 2, P == 1))) return r;
         if ((r = update_params(ctx, st, L, nb))) return r;
       }
     }
     const int nx = idx + 1;
-    const bool merge_next = nx < maxn && nx > cfg.sm_start && nx % P == P / 2;
+    // (the merge reads the border mask only where a split comes in between: P = 1)
+    const bool border_next = P == 1 && nx < maxn && nx > cfg.sm_start;
     const bool fuse_now = fuse && nx < maxn && !(stop_after >= 0 && nx == stop_after);
     // the next iteration only sweeps, over the same slots: it reads the labels where they are
     const bool sm_next = nx > cfg.sm_start && (nx % P == 0 || nx % P == P / 2);
     const bool keep = fuse_now && stop_after < 0 && !sm_next && nit[nb - 1] > nx;
-    if ((r = update_seg(ctx, st, L, nb, cfg, merge_next || stop_after >= 0, keep, fuse_now,
+    if ((r = update_seg(ctx, st, L, nb, cfg, border_next, keep, fuse_now,
                         first_active, &cur, &chg_ok)))
       return r;
     stats_ready = fuse_now;
@@ -931,7 +934,7 @@ int compact(stspix_ctx* ctx, cudaStream_t st, const List& L) {
 }
 
 // run_bass set-up (bass.cu:221-262) on the BASS slots.
-int bass_init(stspix_ctx* ctx, cudaStream_t st, const List& L) {
+int bass_init(stspix_ctx* ctx, cudaStream_t st, const List& L, const stspix_config& cfg) {
   if (L.B <= 0) return STSPIX_OK;
   ctx->cur_fam = STSPIX_FAM_OTHER;
   LAUNCHG(kb_init_hex, dim3(tiles64(L), (unsigned)L.B), kThreads, L.d);
@@ -942,11 +945,11 @@ int bass_init(stspix_ctx* ctx, cudaStream_t st, const List& L) {
   LAUNCHB(kb_remap, pix_units(L.max_npix), L, L.B, 0);
   LAUNCHS(kb_scalars, L, L.B, (int)kOpAfterHex);
   LAUNCHB(kb_init_bass_params, L.max_cap, L, L.B);
-  LAUNCHB(kb_clear_stats, L.max_cap, L, L.B);
+  LAUNCHB(kb_clear_stats, L.max_cap, L, L.B, 1);
   LAUNCHG(kb_accumulate, acc_blocks(ctx, L, L.B), 256, L.d, L.B);
   if (ctx->accumulator) accumulate_fp(ctx, st, L, L.B, ctx->accumulator);
   LAUNCHB(kb_init_prior_mu, L.max_cap, L, L.B);
-  LAUNCHB(kb_find_border, pix_units(L.max_npix), L, L.B);
+  if (cfg.sm_period == 1) LAUNCHB(kb_find_border, pix_units(L.max_npix), L, L.B);
   return STSPIX_OK;
 }
 
@@ -1150,7 +1153,7 @@ struct BatchOut {
 // fractions for the 4/8/12 ladder), and the tail, from the propagated initialisation
 // to the parameter read-out, for known iteration counts and no partial stop.
 int batch_head(stspix_ctx* ctx, cudaStream_t st, int stages, const List& La, const List& Lb,
-               const List& Lp) {
+               const List& Lp, const stspix_config& cfg) {
   int r;
   if ((r = upload(ctx, st, La, 0)) || (r = upload(ctx, st, Lb, 1)) || (r = upload(ctx, st, Lp, 2)))
     return r;
@@ -1158,7 +1161,7 @@ int batch_head(stspix_ctx* ctx, cudaStream_t st, int stages, const List& La, con
   LAUNCHS(kb_scalars, La, La.B, (int)kOpBegin);
   if (ctx->lab_ingest) LAUNCHB(kb_lab_ingest, La.max_npix, La, La.B);
   if ((stages & kStageShift) && (r = shift_fill(ctx, st, Lp))) return r;
-  return bass_init(ctx, st, Lb);
+  return bass_init(ctx, st, Lb, cfg);
 }
 
 int batch_tail(stspix_ctx* ctx, cudaStream_t st, const List& Lp, const List& Ls, bool ls_own,
@@ -1326,7 +1329,7 @@ int run_batch(stspix_ctx* ctx, cudaStream_t st, std::vector<FrameDesc>& fr,
   if ((stages & kStageSeg) && stop_after < 0 && !split_dir && !ctx->prof_on && ctx->graphs_on) {
     const std::string key = batch_signature(fr, caps, nit, stages, cfg);
     r = run_graphed(ctx, st, key + "h",
-                    [&](cudaStream_t s) { return batch_head(ctx, s, stages, La, Lb, Lp); });
+                    [&](cudaStream_t s) { return batch_head(ctx, s, stages, La, Lb, Lp, cfg); });
     if (r) return r;
     if (need_ladder) {
       if ((r = read_scalars(ctx, st, B))) return r;
@@ -1360,7 +1363,7 @@ int run_batch(stspix_ctx* ctx, cudaStream_t st, std::vector<FrameDesc>& fr,
     }
     return STSPIX_OK;
   }
-  if ((r = bass_init(ctx, st, Lb))) return r;
+  if ((r = bass_init(ctx, st, Lb, cfg))) return r;
   if (need_ladder) {
     if ((r = read_scalars(ctx, st, B))) return r;
     for (int i = 0; i < B; i++) {

@@ -191,6 +191,12 @@ constexpr int kPixPerThread = 4;
        j_ < kPixPerThread && t - (int)threadIdx.x < (n); j_++, t += (int)blockDim.x)
 #define SLOT_Z const Slot& S = slots[blockIdx.z]
 
+// Ids in use: 0 .. max_spix, below the capacity (ids above are never valid).  The per-id
+// steps of the loop stop here: a slot's capacity is 10 or 30 times what it uses.
+__device__ __forceinline__ int live_ids(const Slot& S) {
+  return min(S.cap, S.sc->max_spix + 1);
+}
+
 // ---------------------------------------------------------------------------
 // Device helpers shared by the kernels.
 // round(v * 2^shift) (round half to even, as llrintf(ldexpf(v, shift))) for

@@ -113,38 +113,61 @@ __global__ void kb_mark_present(const Slot* __restrict__ slots, int mode) {
   }
 }
 
-// One block per slot: exclusive scan of n byte flags (n up to a few 10^5), each
-// counted as 0 or 1 (the split acceptance flags of propagated frames carry extra bits).
-//   mode 0: hex-id presence (n = nraw)        -> total = live hex ids
-//   mode 1: split acceptance (n = cap)        -> total = accepted splits
-//   mode 2: relabel mint flags (n = cap)      -> total = minted ids
-//   mode 3: final presence (n = max_spix+1-lo) -> total = live new ids
-__global__ void kb_scan(const Slot* __restrict__ slots, int mode) {
+// One block of 1024 threads per slot: exclusive scan of n byte flags (n up to a few 10^5),
+// each counted as 0 or 1 (the split acceptance flags of propagated frames carry extra bits).
+//   mode 0: hex-id presence (n = nraw)           -> total = live hex ids
+//   mode 1: split acceptance (n = ids in use)    -> total = accepted splits
+//   mode 2: relabel mint flags (n = ids in use)  -> total = minted ids
+//   mode 3: final presence (n = max_spix+1-lo)   -> total = live new ids
+// A thread takes 16 flags (one 16-byte load; the arrays start on 256-byte boundaries and end
+// at least 2 entries past cap, so the tail is read byte by byte), a warp and then the block
+// are scanned by shuffles.  Bound: two block-wide steps per 16384 flags.  Over all cap ids
+// with serial chunks a scan took 82 us on a 2160x3840 frame (cap 400,000, 13,000 in use).
+__global__ void __launch_bounds__(1024) kb_scan(const Slot* __restrict__ slots, int mode) {
   pdl_enter();
   const Slot& S = slots[blockIdx.x];
   if (mode == 2 && !S.mode) return;  // mint flags exist on propagated slots only
-  __shared__ int part[1024];
-  const int T = blockDim.x;
+  __shared__ int part[32];
   const uint8_t* flags = (mode == 1) ? S.accept : (mode == 2) ? S.mint : S.flags;
-  int n = (mode == 0) ? S.nraw : (mode == 3) ? S.sc->tmp2 : S.cap;
+  const int n = (mode == 0) ? S.nraw : (mode == 3) ? S.sc->tmp2 : live_ids(S);
   int* excl = S.excl;
   int* total = (mode == 0) ? &S.sc->nspix : (mode == 3) ? &S.sc->tmp1 : &S.sc->tmp2;
-  if (n < 0) n = 0;
-  int chunk = (n + T - 1) / T;
-  int b = threadIdx.x * chunk, e = min(n, b + chunk);
-  int s = 0;
-  for (int i = b; i < e; i++) s += flags[i] != 0;
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int off = 1; off < T; off <<= 1) {
-    int v = threadIdx.x >= off ? part[threadIdx.x - off] : 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int run = 0;
+  for (int base = 0; base < n; base += 16 * 1024) {
+    const int i = base + 16 * (int)threadIdx.x;
+    unsigned bits = 0;                           // bit q: flag i + q
+    if (i + 16 <= n) {
+      const uint4 v = *(const uint4*)(flags + i);
+      const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int q = 0; q < 16; q++) bits |= (unsigned)(((w[q >> 2] >> (8 * (q & 3))) & 0xffu) != 0) << q;
+    } else {
+      for (int q = 0; q < 16 && i + q < n; q++) bits |= (unsigned)(flags[i + q] != 0) << q;
+    }
+    const int c = __popc(bits);
+    int inc = c;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, k);
+      if (lane >= k) inc += t;
+    }
+    if (lane == 31) part[warp] = inc;
     __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
+    int p = part[lane], pi = p;                  // every warp scans the 32 warp totals
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, pi, k);
+      if (lane >= k) pi += t;
+    }
+    const int before = run + __shfl_sync(0xffffffffu, pi - p, warp) + inc - c;
+#pragma unroll
+    for (int q = 0; q < 16; q++)
+      if (i + q < n) excl[i + q] = before + __popc(bits & ((1u << q) - 1u));
+    run += __shfl_sync(0xffffffffu, pi, 31);
+    __syncthreads();                             // part is free for the next tile
   }
-  int run = threadIdx.x ? part[threadIdx.x - 1] : 0;
-  for (int i = b; i < e; i++) { excl[i] = run; run += flags[i] != 0; }
-  if (threadIdx.x == T - 1) *total = part[T - 1];
+  if (threadIdx.x == 0) *total = run;
 }
 
 __global__ void kb_remap(const Slot* __restrict__ slots, int mode) {
@@ -658,13 +681,14 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
   }
 }
 
-// clear_fields + the helper memset (update_params.cu:54-88, :26): zero the counts
-// and the sums of every slot.
-__global__ void kb_clear_stats(const Slot* __restrict__ slots) {
+// clear_fields + the helper memset (update_params.cu:54-88, :26): zero the counts and
+// the sums of every slot, of all ids (once per frame) or of the ids in use (a step that
+// raises max_spix is followed by such a clear, so an id's sums start at zero).
+__global__ void kb_clear_stats(const Slot* __restrict__ slots, int all) {
   pdl_enter();
   SLOT_Y;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= S.sp.cap) return;
+  if (k >= (all ? S.sp.cap : live_ids(S))) return;
   S.sp.count[k] = 0;
   long long* a = S.sp.acc + 8 * (size_t)k;
 #pragma unroll
@@ -1594,10 +1618,22 @@ __global__ void kb_save_prev(const Slot* __restrict__ slots) {
   FOR_PIX(i, S.npix) S.resident_labels[i] = S.seg[i];
 }
 
+// The labels back from seg_alt to seg after a launch that read seg: only the pixels that
+// launch changed (change plane 0) differ.  A thread takes one 16-pixel change word.
 __global__ void kb_copy_labels(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
-  FOR_PIX(i, S.npix) S.seg[i] = S.seg_alt[i];
+  const int W = S.W, P16 = (W + 15) >> 4;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= S.H * P16) return;
+  unsigned m = ((const uint16_t*)S.chg[0])[i];
+  if (!m) return;
+  const int y = i / P16;
+  const size_t g = (size_t)y * W + 16 * (i - y * P16);
+  for (; m; m &= m - 1) {
+    const int q = __ffs(m) - 1;
+    S.seg[g + q] = S.seg_alt[g + q];
+  }
 }
 
 __global__ void k_dump_state(SpDev sp, stspix_state_dump d) {

@@ -701,11 +701,13 @@ __global__ void kb_relabel_init(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
   if (!S.mode) return;
+  // (a minted id is at most 2 max_spix + 1)
+  const int n_ids = live_ids(S);
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S.cap + 2) return;
-  S.living[s] = 0;
+  if (s >= min(S.cap, 2 * n_ids)) return;
   S.src_of[s] = -1;
-  if (s >= S.cap) return;
+  if (s >= n_ids) return;
+  S.living[s] = 0;
   S.rbest[s] = ((unsigned long long)__float_as_uint(10000.f) << 32) | 0x7fffffffull;
   S.ss[s] = 0.f;
 }
@@ -791,11 +793,11 @@ __global__ void kb_relabel_mark(const Slot* __restrict__ slots, float thresh_rep
   int* __restrict__ rid = S.rid;
   uint8_t* __restrict__ mint = S.mint;
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= cap) return;
+  const int nspix = sc->max_spix + 1;
+  if (s >= min(cap, nspix)) return;
   mint[s] = 0;
   rid[s] = -1;
-  const int nspix = sc->max_spix + 1;
-  if (s >= nspix || !living[s]) return;
+  if (!living[s]) return;
   unsigned long long b = best[s];
   float delta = __uint_as_float((unsigned)(b >> 32));
   int c = (int)(unsigned)(b & 0xffffffffull);
@@ -815,7 +817,7 @@ __global__ void kb_relabel_ids(const Slot* __restrict__ slots) {
   int* __restrict__ rid = S.rid;
   int* __restrict__ src_of = S.src_of;
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= cap) return;
+  if (s >= live_ids(S)) return;
   if (mint[s]) rid[s] = sc->max_spix + 1 + excl[s];
   int n = rid[s];
   if (n >= 0 && n < cap) atomicMax(&src_of[n], s);
@@ -833,7 +835,7 @@ __global__ void kb_relabel_params(const Slot* __restrict__ slots) {
   const int* __restrict__ src_of = S.src_of;
   const int n_prev = S.n_prev;
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= sp.cap) return;
+  if (s >= live_ids(S)) return;
   int n = rid[s];
   if (n < 0 || n >= sp.cap) return;
   sp.valid[s] = 0;
@@ -884,7 +886,7 @@ __global__ void kb_count_revived(const Slot* __restrict__ slots) {
   SLOT_Y;
   if (!S.mode) return;
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S.cap) return;
+  if (s >= live_ids(S)) return;
   if (S.rid[s] >= 0 && !S.mint[s]) atomicAdd(&S.sc->nrevived, 1);
 }
 

@@ -31,7 +31,7 @@ __global__ void kb_split_seed(const Slot* __restrict__ slots, int dir_bass, int 
   const SpDev& sp = S.sp;
   const int direction = S.mode ? dir_prop : dir_bass;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= sp.cap) return;
+  if (k >= live_ids(S)) return;
   int* bb = S.bbox + 4 * (size_t)k;
   bb[0] = INT32_MAX; bb[1] = -1; bb[2] = INT32_MAX; bb[3] = -1;
   if (!S.sc->tmp0 /*split_on*/ || !sp.valid[k]) return;
@@ -439,13 +439,14 @@ __global__ void kb_split_partition(const Slot* __restrict__ slots) {
   }
 }
 
-// Clear the split/merge sums (cap + 2 entries).
+// Clear the split/merge sums of the ids in use and of their second halves (a split gives
+// the second half of id k the label k + max_spix + 1).
 __global__ void kb_sm_clear(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
   const SmDev& sm = S.sm;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= S.cap + 2) return;
+  if (k >= min(S.cap + 2, 2 * (S.sc->max_spix + 1))) return;
   sm.count[k] = 0;
   sm.ninvalid[k] = 0;
 #pragma unroll
@@ -600,13 +601,14 @@ __global__ void __launch_bounds__(128) kb_split_decide(const Slot* __restrict__ 
   Scalars* sc = S.sc;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
-  if ((int)blockIdx.x * 32 >= sp.cap) return;             // block-uniform
+  const int n_ids = live_ids(S);
+  if ((int)blockIdx.x * 32 >= n_ids) return;              // block-uniform
   __shared__ double t_lr[3][3][32], t_log[3][32];
   // the preconditions, evaluated alike by every warp
   bool ok = false;
   int s = 0;
   double cnt[3] = {0, 0, 0};                                // k's half, s's half, whole
-  if (k < sp.cap) {
+  if (k < n_ids) {
     if (w == 0) S.accept[k] = 0;
     if (sc->tmp0 && sp.valid[k]) {
       s = k + sc->tmp1;
@@ -672,7 +674,7 @@ __global__ void kb_split_commit(const Slot* __restrict__ slots) {
   const int* __restrict__ excl = S.excl;
   const int prop_mode = S.mode;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= sp.cap) return;
+  if (k >= live_ids(S)) return;
   uint8_t fl = accept[k];
   if (!fl) return;
   int snew = sc->max_spix + 1 + excl[k];
@@ -742,7 +744,11 @@ __global__ void kb_split_end(const Slot* __restrict__ slots, int B) {
 // ---------------------------------------------------------------------------
 // Merge candidates (calc_merge_candidate, split_merge.cu:719-755;
 // calc_merge_candidate_p, split_merge_prop.cu:1808-1845).
-__global__ void kb_merge_candidates(const Slot* __restrict__ slots, int dir_bass, int dir_prop) {
+// A pixel whose neighbour in the direction carries another label is a border pixel (now, and
+// when the reference built its mask: a relabel in between maps equal labels to equal ones),
+// so the mask is read (use_border) only where a split came between the two.
+__global__ void kb_merge_candidates(const Slot* __restrict__ slots, int dir_bass, int dir_prop,
+                                    int use_border) {
   pdl_enter();
   SLOT_Y;
   const int* __restrict__ seg = S.seg;
@@ -754,7 +760,7 @@ __global__ void kb_merge_candidates(const Slot* __restrict__ slots, int dir_bass
   const int cap = S.cap;
   int* __restrict__ pair = S.sm.pair;
   FOR_PIX(idx, H * W) {
-    if (!border[idx]) continue;
+    if (use_border && !border[idx]) continue;
     const int x = idx % W, y = idx / W;
     const int C = seg[idx];
     if (C < 0 || C >= cap) continue;
@@ -785,11 +791,12 @@ __global__ void __launch_bounds__(128) kb_merge_single(const Slot* __restrict__ 
   const SmDev& sm = S.sm;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
-  if ((int)blockIdx.x * 32 >= sp.cap) return;             // block-uniform
+  const int n_ids = live_ids(S);
+  if ((int)blockIdx.x * 32 >= n_ids) return;              // block-uniform
   __shared__ double t_lr[3][32], t_log[32];
   bool ok = false;
   double n = 0;
-  if (k < sp.cap) {
+  if (k < n_ids) {
     if (w == 0) sm.flag[k] = 0;
     ok = sp.valid[k] && sm.pair[k] >= 0;
     if (ok) n = sp.count[k];
@@ -818,7 +825,7 @@ __global__ void __launch_bounds__(128) kb_merge_decide(const Slot* __restrict__ 
   Scalars* sc = S.sc;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
-  const int n_ids = min(sp.cap, sc->max_spix + 1);
+  const int n_ids = live_ids(S);
   if ((int)blockIdx.x * 32 >= n_ids) return;              // block-uniform
   __shared__ double t_lr[3][32], t_log[32];
   bool ok = false;
@@ -860,12 +867,12 @@ __global__ void __launch_bounds__(128) kb_merge_decide(const Slot* __restrict__ 
   }
 }
 
-// Merge set-up: candidate pairs unset, claims at +inf (cap + 2 entries).
+// Merge set-up: candidate pairs unset, claims at +inf.
 __global__ void kb_merge_clear(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= S.cap + 2) return;
+  if (k >= live_ids(S)) return;
   S.sm.pair[k] = -1;
   S.sm.claim[k] = 0x7f7f7f7f;
 }
@@ -878,7 +885,7 @@ __global__ void kb_merge_flag(const Slot* __restrict__ slots) {
   const SmDev& sm = S.sm;
   uint8_t* __restrict__ valid0 = S.valid0;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= sp.cap) return;
+  if (k >= live_ids(S)) return;
   valid0[k] = sp.valid[k];
   int f = sm.pair[k];
   sm.target[k] = f;
@@ -897,7 +904,7 @@ __global__ void kb_merge_remove(const Slot* __restrict__ slots) {
   const uint8_t* __restrict__ valid0 = S.valid0;
   const int prop_mode = S.mode;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= sp.cap) return;
+  if (k >= live_ids(S)) return;
   int s = sm.pair[k];
   if (s < 0) return;
   bool is_cycle = sm.pair[s] == k;

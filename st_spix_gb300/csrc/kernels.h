@@ -27,7 +27,7 @@ __global__ void kb_compact_gather(const Slot* slots);
 __global__ void kb_compact_scatter(const Slot* slots);
 __global__ void kb_init_bass_params(const Slot* slots);
 __global__ void kb_init_prior_mu(const Slot* slots);
-__global__ void kb_clear_stats(const Slot* slots);
+__global__ void kb_clear_stats(const Slot* slots, int all);
 __global__ void kb_accumulate(const Slot* slots, int B);
 __global__ void kb_posterior(const Slot* slots, int incremental);
 __global__ void kb_accumulate_fp(const Slot* slots, int mode);
@@ -83,7 +83,7 @@ __global__ void kb_split_commit(const Slot* slots);
 __global__ void kb_split_apply(const Slot* slots);
 __global__ void kb_split_end(const Slot* slots, int B);
 __global__ void kb_merge_clear(const Slot* slots);
-__global__ void kb_merge_candidates(const Slot* slots, int dir_bass, int dir_prop);
+__global__ void kb_merge_candidates(const Slot* slots, int dir_bass, int dir_prop, int use_border);
 __global__ void kb_merge_single(const Slot* slots, SmConsts K);
 __global__ void kb_merge_decide(const Slot* slots, SmConsts K, float merge_alpha);
 __global__ void kb_merge_flag(const Slot* slots);

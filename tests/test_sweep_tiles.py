@@ -37,3 +37,27 @@ def test_four_sweep_launches_match_the_oracle(H, W, sp, niters, niters_seg, lo, 
                                                              prop_niters=niters), True)
     assert st == 0
     np.testing.assert_array_equal(out.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("H,W,sp,niters,period", [
+    (96, 128, 15, 9, 1),         # split and merge in one step: the merge reads the border mask
+    (96, 128, 15, 9, 2),
+    (97, 131, 9, 10, 3),
+    (300, 300, 2, 6, 4),         # 23,000 ids: scans of more than one tile
+])
+def test_split_merge_periods_match_the_oracle(H, W, sp, niters, period):
+    from st_spix_gb300 import bist_cuda, synth
+    vid, flows, _ = synth.voronoi_video(H, W, 2, max(3, H * W // 900), 0.05, seed=period,
+                                        max_shift=3.0)
+    out = bist_cuda.bist_forward(torch.from_numpy(vid).cuda(), torch.from_numpy(flows).cuda(),
+                                 niters, sp, 0.5, 0.009 ** 2, float(np.log(0.5)), 0.0, True, False,
+                                 sm_period=period, prop_niters=niters)
+    glog = bist_cuda.frame_log()
+    st, ref, _ = O.bist_forward(vid, flows, O.default_config(niters=niters, sp_size=sp,
+                                                             sm_period=period,
+                                                             prop_niters=niters), True)
+    assert st == 0
+    np.testing.assert_array_equal(out.cpu().numpy(), ref)
+    olog = O.last_log()
+    assert (glog.nsplits, glog.nmerges, glog.nrevived, glog.nminted) == \
+        (olog.nsplits, olog.nmerges, olog.nrevived, olog.nminted)
