@@ -847,11 +847,12 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
   const int P = cfg.sm_period > 0 ? cfg.sm_period : 4;
   const int maxn = L.B ? nit[0] : 0;
   int nb = L.B;
-  // the statistics of the first nb slots were kept current by the previous
-  // iteration's sweeps (incremental statistics; integer sums, so identical to a full
-  // pass); the int64 accumulator only
-  bool stats_ready = false;
+  // the statistics of the first nb slots are those of their labels: from the frames'
+  // initialisation when all are plain BASS, and after the previous iteration's sweeps
+  // kept them current (incremental statistics; integer sums, so identical to a full
+  // pass; the int64 accumulator only)
   const bool fuse = ctx->accumulator == 0;
+  bool stats_ready = fuse && !L.any_prop;
   bool chg_ok = false;      // the previous update_seg left its changes and label buffers
   int cur = 0;              // the label buffer the next sweep reads (see update_seg)
   for (int idx = 0; idx < maxn; idx++) {
@@ -884,10 +885,10 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
     const int nx = idx + 1;
     // (the merge reads the border mask only where a split comes in between: P = 1)
     const bool border_next = P == 1 && nx < maxn && nx > cfg.sm_start;
-    const bool fuse_now = fuse && nx < maxn && !(stop_after >= 0 && nx == stop_after);
+    const bool fuse_now = fuse && !(stop_after >= 0 && nx == stop_after);
     // the next iteration only sweeps, over the same slots: it reads the labels where they are
     const bool sm_next = nx > cfg.sm_start && (nx % P == 0 || nx % P == P / 2);
-    const bool keep = fuse_now && stop_after < 0 && !sm_next && nit[nb - 1] > nx;
+    const bool keep = fuse_now && stop_after < 0 && nx < maxn && !sm_next && nit[nb - 1] > nx;
     if ((r = update_seg(ctx, st, L, nb, cfg, border_next, keep, fuse_now,
                         first_active, &cur, &chg_ok)))
       return r;
@@ -899,7 +900,10 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
   }
   // final update_params + store_sample; slots that finished earlier were untouched
   // since, so running theirs here is the same as running it right after their loop
-  if ((r = update_params(ctx, st, L, L.B, false, maxn > 0))) return r;
+  // (and their statistics are current too: with fuse every sweep moved them)
+  if ((r = update_params(ctx, st, L, L.B, fuse && maxn > 0 && nit[L.B - 1] > 0, maxn > 0,
+                         maxn == 0)))
+    return r;
   ctx->cur_fam = STSPIX_FAM_POSTERIOR;
   LAUNCHB(kb_store_sample, L.max_cap, L, L.B);
   return STSPIX_OK;
