@@ -200,17 +200,12 @@ int stspix_get_marked_video(stspix_ctx* ctx, void* stream,
                             const float* color, int T, int H, int W, int nftrs,
                             float* marked_out);
 
-/* get_marked_video without any allocation.  No counterpart in the reference: it is
- * for callers that must not allocate device memory while they run (a process that
+/* get_marked_video without a context.  No counterpart in the reference: it is for
+ * callers that must not allocate device memory while they run (a process that
  * reserves its GPU memory up front, a plugin whose host owns every allocation, a
- * real-time loop).  The border-mask scratch lives in a 16 MiB array compiled into
- * the library (held on every GPU that loads it until exit); T*H*W above 2^24 pixels
- * returns STSPIX_ERR_TOO_LARGE.  Frames have 3 channels (else STSPIX_ERR_ARG).  No
- * context is needed; it runs on `stream`, which must belong to the current device
- * (else STSPIX_ERR_ARG).  All calls share that one array, so calls that overlap on
- * the GPU race and must be serialised by the caller.  The first call on a device
- * looks up the array's address and caches it for the process; make it before any
- * stream capture, and do not use the entry point across a cudaDeviceReset.       */
+ * real-time loop).  T*H*W above 2^24 pixels returns STSPIX_ERR_TOO_LARGE.  Frames have
+ * 3 channels (else STSPIX_ERR_ARG).  It runs on `stream`, which must belong to the
+ * current device (else STSPIX_ERR_ARG).                                           */
 int stspix_get_marked_video_noalloc(void* stream, const float* vid, const int32_t* spix,
                                     const float* color, int T, int H, int W, int nftrs,
                                     float* marked_out);

@@ -74,7 +74,7 @@ def bist_forward(vid: torch.Tensor, flows: torch.Tensor, niters: int, sp_size: i
         if flows.dim() != 4 or flows.shape[0] < T - 1 or tuple(flows.shape[1:]) != (H, W, 2):
             raise RuntimeError("flows must be [T-1,H,W,2] (or longer) in video mode")
     cfg = make_config(niters, sp_size, potts, sigma2_app, alpha, split_alpha, **extra)
-    out = torch.zeros((T, H, W), dtype=torch.int32, device=vid.device)
+    out = torch.empty((T, H, W), dtype=torch.int32, device=vid.device)
     ctx = _ctx(vid.device)
     with torch.cuda.device(vid.device):
         st = ctx.lib.stspix_bist_forward(ctx.handle, _stream(vid.device), vid.data_ptr(),
@@ -96,7 +96,7 @@ def get_marked_video(vid: torch.Tensor, spix: torch.Tensor, color: torch.Tensor)
         raise RuntimeError("color must have one value per channel")
     color = color.to(device=vid.device, dtype=torch.float32).contiguous()
     spix = spix.to(torch.int32).contiguous()
-    marked = torch.zeros((T, H, W, F), dtype=torch.float32, device=vid.device)
+    marked = torch.empty((T, H, W, F), dtype=torch.float32, device=vid.device)
     ctx = _ctx(vid.device)
     with torch.cuda.device(vid.device):
         st = ctx.lib.stspix_get_marked_video(ctx.handle, _stream(vid.device), vid.data_ptr(),
@@ -156,7 +156,7 @@ def run_bass(img: torch.Tensor, **cfg_kw):
     H, W = img.shape[:2]
     cfg = make_config(**cfg_kw)
     params = SuperpixelParams(30 * hex_count(H, W, cfg.sp_size), img.device)
-    labels = torch.zeros((H, W), dtype=torch.int32, device=img.device)
+    labels = torch.empty((H, W), dtype=torch.int32, device=img.device)
     ps = params.struct()
     n = C.c_int(0)
     ctx = _ctx(img.device)
@@ -192,7 +192,7 @@ def run_prop(img: torch.Tensor, niters: int, filled: torch.Tensor, shifted: torc
     H, W = img.shape[:2]
     cfg = make_config(**cfg_kw)
     out = SuperpixelParams(10 * params_prev.n, img.device)
-    labels = torch.zeros((H, W), dtype=torch.int32, device=img.device)
+    labels = torch.empty((H, W), dtype=torch.int32, device=img.device)
     pprev = params_prev.struct()
     ps = out.struct()
     n = C.c_int(0)

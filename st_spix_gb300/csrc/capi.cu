@@ -411,7 +411,7 @@ void preload_kernels() {
       (const void*)k_init_hex,
       (const void*)k_find_border,
       (const void*)k_find_border_end,
-      (const void*)k_overlay,
+      (const void*)k_marked,
       (const void*)k_dump_state,
       (const void*)kb_scalars,
       (const void*)kb_init_hex,
@@ -2697,12 +2697,10 @@ int stspix_get_marked_video(stspix_ctx* ctx, void* stream, const float* vid, con
   if ((r = check_size(ctx, H, W))) return r;
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
-  long long n = (long long)T * H * W;
-  uint8_t* border = nullptr;
-  CK(cudaMallocAsync((void**)&border, (size_t)std::max(n, 1LL), st));
-  LAUNCH(k_find_border_end, n, spix, border, H, W, T);
-  LAUNCH(k_overlay, n, marked_out, vid, color, border, n);
-  CK(cudaFreeAsync(border, st));
+  const long long n = (long long)T * H * W;
+  if (n > 0)
+    LAUNCHG(k_marked, (unsigned)((n + kMarkPix - 1) / kMarkPix), 256, marked_out, vid, spix, color,
+            H, W, n);
   CK(cudaGetLastError());
   return STSPIX_OK;
 }

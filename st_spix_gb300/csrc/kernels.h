@@ -13,8 +13,9 @@ namespace stspix {
 __global__ void k_init_hex(int* seg, int H, int W, double Hh, double w, int nx, int ny);
 __global__ void k_find_border(const int* seg, uint8_t* border, int H, int W);
 __global__ void k_find_border_end(const int* seg, uint8_t* border, int H, int W, int nframes);
-__global__ void k_overlay(float* out, const float* img, const float* color,
-                          const uint8_t* border, long long n);
+constexpr int kMarkPix = 1024;            // pixels per block of k_marked (256 threads)
+__global__ void k_marked(float* out, const float* vid, const int* spix, const float* color, int H,
+                         int W, long long n);
 __global__ void k_dump_state(SpDev sp, stspix_state_dump d);
 
 __global__ void kb_scalars(const Slot* slots, int B, int op);
