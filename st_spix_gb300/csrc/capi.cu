@@ -122,6 +122,15 @@ struct stspix_ctx {
   long long body_iters_seen = 0;
   // bist_forward's stream state
   stspix_video* fwd = nullptr;
+  // device scratch of the quality entry points, kept between calls up to kScratchMax
+  // bytes (an allocation per call gave its memory back to the driver at every
+  // synchronisation: 200 us a call).  ev marks its last use: a call on another stream
+  // waits for it.
+  struct { char* p = nullptr; size_t bytes = 0; cudaEvent_t ev = nullptr; cudaStream_t st = nullptr;
+           bool used = false; } scratch;
+  // pinned staging of small results (kPinBytes)
+  char* pin = nullptr;
+  cudaEvent_t range_ev = nullptr;
   // profiling (CUDA events on the launching stream)
   int prof_on = 0;
   int cur_fam = STSPIX_FAM_OTHER;
@@ -1566,6 +1575,10 @@ int stspix_destroy(stspix_ctx* ctx) {
   for (auto e : ctx->ev_free) cudaEventDestroy(e);
   for (auto e : ctx->batch_ev) if (e) cudaEventDestroy(e);
   if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
+  if (ctx->scratch.p) cudaFree(ctx->scratch.p);
+  if (ctx->scratch.ev) cudaEventDestroy(ctx->scratch.ev);
+  if (ctx->range_ev) cudaEventDestroy(ctx->range_ev);
+  if (ctx->pin) cudaFreeHost(ctx->pin);
   if (ctx->sc_host) cudaFreeHost(ctx->sc_host);
   if (ctx->h_slots) cudaFreeHost(ctx->h_slots);
   delete ctx;
@@ -2106,24 +2119,73 @@ int stspix_label_stats(stspix_ctx* ctx, void* stream, const float* img, const in
 
 // ---- quality metrics (evaluate.py) ------------------------------------------------
 namespace {
-// Scratch of one evaluation, carved from one allocation (256-byte aligned pieces).
+constexpr size_t kScratchMax = size_t(256) << 20, kPinBytes = size_t(1) << 20;
+
+// `bytes` of device scratch for work on st: the context's own (grown to the next power of
+// two; growing synchronises the device), or, above kScratchMax, an allocation of this call.
+// Released by the destructor, after which nothing more is launched on it.
+struct Scratch {
+  stspix_ctx* ctx;
+  cudaStream_t st;
+  char* p = nullptr;
+  bool own = false;
+  Scratch(stspix_ctx* c, cudaStream_t s) : ctx(c), st(s) {}
+  ~Scratch() {
+    if (!p) return;
+    if (own) { cudaFreeAsync(p, st); return; }
+    ctx->scratch.used = cudaEventRecord(ctx->scratch.ev, st) == cudaSuccess;
+    ctx->scratch.st = st;
+  }
+  int get(size_t bytes) {
+    auto& k = ctx->scratch;
+    if (bytes > kScratchMax) {
+      CK(cudaMallocAsync((void**)&p, bytes, st));
+      own = true;
+      return STSPIX_OK;
+    }
+    if (bytes > k.bytes) {
+      std::lock_guard<std::mutex> lk(g_device_mu);
+      size_t n = size_t(1) << 20;
+      while (n < bytes) n <<= 1;
+      CK(cudaDeviceSynchronize());
+      if (k.p) cudaFree(k.p);
+      k.p = nullptr;
+      k.bytes = 0;
+      k.used = false;
+      CK(cudaMalloc((void**)&k.p, n));
+      k.bytes = n;
+      if (!k.ev) CK(cudaEventCreateWithFlags(&k.ev, cudaEventDisableTiming));
+    }
+    if (k.used && k.st != st) CK(cudaStreamWaitEvent(st, k.ev, 0));
+    p = k.p;
+    return STSPIX_OK;
+  }
+};
+
+int ensure_pin(stspix_ctx* ctx) {
+  if (!ctx->pin) CK(cudaMallocHost((void**)&ctx->pin, kPinBytes));
+  return STSPIX_OK;
+}
+
+// Scratch of one evaluation, carved from one allocation (256-byte aligned pieces).  The
+// pieces from `live` to `sa3` are the results the host reads, in one copy.
 struct QualityScratch {
   int* cnt;                    // [T*S]   per-frame id sizes
   double* fsum;                // [T*S*3] per-frame id colour sums
+  double* mean;                // [T*S*3] pooled colours
   double* vsum;                // [S*3]   video-wide id colour sums
   double* msum;                // [T*3]   per-frame colour sums
-  double* pix2;                // [T]     sum (v - mean)^2
-  double* pix2s;               // [T]     the same at x255 scale
+  long long* ntot;             // [S]     total size over the video
+  int* J;                      // [T*S*G1] id x ground-truth overlaps
+  unsigned long long* live;    // [T]     ids alive per frame
+  double* stdv;                // [S]     size std over the frames alive (-1: < 2)
   double* sse;                 // [T]     sum (v - pooled)^2
   double* pool2;               // [T]     sum (pooled - mean)^2, per-frame pooling
-  double* pool3;               // [T]     the same, video pooling at x255
-  unsigned long long* live;    // [T]     ids alive per frame
-  long long* ntot;             // [S]     total size over the video
-  double* stdv;                // [S]     size std over the frames alive (-1: < 2)
-  int* J;                      // [T*S*G1] id x ground-truth overlaps
+  double* cross;               // [T]     sum (F - n pooled)(pooled - mean)
+  double* pool3;               // [T]     as pool2, video pooling at x255
   unsigned long long *ue, *sa, *gsize;   // [T*G1]
   unsigned long long *ue3, *sa3;         // [G1]
-  size_t bytes;
+  size_t bytes, results;       // total, and where the results start
 };
 
 QualityScratch quality_layout(char* base, long long T, long long S, long long G1, bool colour,
@@ -2136,21 +2198,24 @@ QualityScratch quality_layout(char* base, long long T, long long S, long long G1
     return p;
   };
   q.cnt = (int*)take(4 * T * S);
-  q.live = (unsigned long long*)take(8 * T);
   q.ntot = (long long*)take(8 * S);
-  q.stdv = (double*)take(8 * S);
   if (colour) {
     q.fsum = (double*)take(24 * T * S);
+    q.mean = (double*)take(24 * T * S);
     q.vsum = (double*)take(24 * S);
     q.msum = (double*)take(24 * T);
-    q.pix2 = (double*)take(8 * T);
-    q.pix2s = (double*)take(8 * T);
+  }
+  if (gt) q.J = (int*)take(4 * T * S * G1);
+  q.results = off;
+  q.live = (unsigned long long*)take(8 * T);
+  q.stdv = (double*)take(8 * S);
+  if (colour) {
     q.sse = (double*)take(8 * T);
     q.pool2 = (double*)take(8 * T);
+    q.cross = (double*)take(8 * T);
     q.pool3 = (double*)take(8 * T);
   }
   if (gt) {
-    q.J = (int*)take(4 * T * S * G1);
     q.ue = (unsigned long long*)take(8 * T * G1);
     q.sa = (unsigned long long*)take(8 * T * G1);
     q.gsize = (unsigned long long*)take(8 * T * G1);
@@ -2163,21 +2228,56 @@ QualityScratch quality_layout(char* base, long long T, long long S, long long G1
 
 constexpr size_t kQualityMaxScratch = size_t(64) << 30;
 
-int label_range(stspix_ctx* ctx, cudaStream_t st, const int32_t* a, long long n, int out[2]) {
-  int* mm = nullptr;
-  CK(cudaMallocAsync((void**)&mm, 2 * sizeof(int), st));
-  LAUNCHG(k_q_range_init, 1, 32, mm);
-  const long long nb = std::min<long long>((n + kThreads - 1) / kThreads, 4LL * ctx->num_sms);
-  LAUNCHG(k_q_range, (unsigned)std::max(1LL, nb), kThreads, a, n, mm);
-  CK(cudaMemcpyAsync(out, mm, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(cudaFreeAsync(mm, st));
+// The results of an evaluation on the host: one copy into the pinned staging (or, when
+// larger, into buf), then the stream is synchronised.  Returns where `results` starts.
+int quality_results(stspix_ctx* ctx, cudaStream_t st, const char* base, const QualityScratch& q,
+                    std::vector<char>& buf, const char** out) {
+  const size_t n = q.bytes - q.results;
+  int r = ensure_pin(ctx);
+  if (r) return r;
+  char* dst = ctx->pin;
+  if (n > kPinBytes) {
+    buf.resize(n);
+    dst = buf.data();
+  }
+  CK(cudaMemcpyAsync(dst, base + q.results, n, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  CK(cudaGetLastError());
+  *out = dst;
   return STSPIX_OK;
 }
 
+// Smallest and largest of the n labels of a (and of b), launched on st; range_get waits for
+// them: out[0..1] of a, out[2..3] of b.  mm: four words of device scratch.
+int range_launch(stspix_ctx* ctx, cudaStream_t st, int* mm, const int32_t* a, const int32_t* b,
+                 long long n) {
+  int r = ensure_pin(ctx);
+  if (r) return r;
+  LAUNCHG(k_q_range_init, 1, 32, mm);
+  const long long nb = std::min<long long>((n + kThreads - 1) / kThreads, 4LL * ctx->num_sms);
+  LAUNCHG(k_q_range, dim3((unsigned)std::max(1LL, nb), b ? 2 : 1), kThreads, a, b, n, mm);
+  CK(cudaMemcpyAsync(ctx->pin, mm, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (!ctx->range_ev) CK(cudaEventCreateWithFlags(&ctx->range_ev, cudaEventDisableTiming));
+  CK(cudaEventRecord(ctx->range_ev, st));
+  return STSPIX_OK;
+}
+int range_get(stspix_ctx* ctx, int out[4]) {
+  CK(cudaEventSynchronize(ctx->range_ev));
+  memcpy(out, ctx->pin, 4 * sizeof(int));
+  return STSPIX_OK;
+}
+int label_range(stspix_ctx* ctx, cudaStream_t st, const int32_t* a, const int32_t* b, long long n,
+                int out[4]) {
+  Scratch mm(ctx, st);
+  int r;
+  if ((r = mm.get(4 * sizeof(int)))) return r;
+  if ((r = range_launch(ctx, st, (int*)mm.p, a, b, n))) return r;
+  return range_get(ctx, out);
+}
+
 // tex / szv from the per-frame live counts and per-id stds (evaluate.py:287-327).
-void size_scores(const std::vector<unsigned long long>& live, const std::vector<double>& stdv,
-                 int T, long long S, double* tex, double* szv) {
+void size_scores(const unsigned long long* live, const double* stdv, int T, long long S,
+                 double* tex, double* szv) {
   double a = 0;
   for (int t = 0; t < T; t++) a += (double)live[t] / (double)S;
   *tex = a / T;
@@ -2189,6 +2289,10 @@ void size_scores(const std::vector<unsigned long long>& live, const std::vector<
 }
 
 unsigned q_blocks(long long n) { return (unsigned)std::max(1LL, (n + kThreads - 1) / kThreads); }
+// 64 x 32 tiles of an H x W frame (warp_block)
+unsigned q_tiles(int H, int W) {
+  return (unsigned)(((long long)(W + 63) / 64) * ((H + 31LL) / 32));
+}
 }  // namespace
 
 int stspix_label_range(stspix_ctx* ctx, void* stream, const int32_t* labels, long long n,
@@ -2196,8 +2300,8 @@ int stspix_label_range(stspix_ctx* ctx, void* stream, const int32_t* labels, lon
   if (!ctx || !labels || !out || n < 1) return fail(ctx, STSPIX_ERR_ARG, "bad argument");
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
-  int mm[2];
-  int r = label_range(ctx, st, labels, n, mm);
+  int mm[4];
+  int r = label_range(ctx, st, labels, nullptr, n, mm);
   if (r) return r;
   out[0] = mm[0];
   out[1] = mm[1];
@@ -2210,17 +2314,17 @@ int stspix_count_spix(stspix_ctx* ctx, void* stream, const int32_t* spix, int T,
     return fail(ctx, STSPIX_ERR_ARG, "bad argument");
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
-  int mm[2];
-  int r = label_range(ctx, st, spix, (long long)T * npix, mm);
+  int mm[4];
+  int r = label_range(ctx, st, spix, nullptr, (long long)T * npix, mm);
   if (r) return r;
   if (mm[0] < id_offset || (long long)mm[1] >= (long long)id_offset + nids)
     return fail(ctx, STSPIX_ERR_ARG, "ids %d..%d outside [%d, %lld)", mm[0], mm[1], id_offset,
                 (long long)id_offset + nids);
   CK(cudaMemsetAsync(counts, 0, sizeof(int32_t) * (size_t)T * nids, st));
-  const long long segs = (long long)T * ((npix + 31) / 32);
-  const unsigned nb = (unsigned)std::max(1LL, std::min<long long>((segs + 7) / 8, 8LL * ctx->num_sms));
-  LAUNCHG(k_q_accum, nb, kThreads, nullptr, spix, nullptr, T, 1, (int)npix, id_offset, nids, 1,
-          counts, nullptr, nullptr, nullptr, nullptr);
+  // (rows of 64 pixels: the frame's width is not known here)
+  const int H = (int)((npix + 63) / 64);
+  LAUNCHG(k_q_count, dim3(q_tiles(H, 64), (unsigned)T), kThreads, spix, npix, H, 64, id_offset,
+          nids, counts);
   CK(cudaGetLastError());
   return STSPIX_OK;
 }
@@ -2232,20 +2336,19 @@ int stspix_size_variation(stspix_ctx* ctx, void* stream, const int32_t* counts, 
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
   QualityScratch q = quality_layout(nullptr, T, S, 1, false, false);
-  char* base = nullptr;
-  CK(cudaMallocAsync((void**)&base, q.bytes, st));
-  q = quality_layout(base, T, S, 1, false, false);
-  CK(cudaMemsetAsync(base, 0, q.bytes, st));
-  LAUNCHG(k_q_id_time, q_blocks(S), kThreads, counts, T, S, q.ntot, q.stdv);
-  LAUNCHG(k_q_frame_ids, dim3(q_blocks(S), T), kThreads, counts, nullptr, nullptr, q.ntot,
-          nullptr, S, 1, q.live, nullptr, nullptr);
-  std::vector<unsigned long long> live(T);
-  std::vector<double> stdv(S);
-  CK(cudaMemcpyAsync(live.data(), q.live, 8 * (size_t)T, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(stdv.data(), q.stdv, 8 * (size_t)S, cudaMemcpyDeviceToHost, st));
-  CK(cudaFreeAsync(base, st));
-  CK(cudaStreamSynchronize(st));
-  CK(cudaGetLastError());
+  Scratch mem(ctx, st);
+  int r;
+  if ((r = mem.get(q.bytes))) return r;
+  q = quality_layout(mem.p, T, S, 1, false, false);
+  CK(cudaMemsetAsync(mem.p, 0, q.bytes, st));
+  LAUNCHG(k_q_id_time, q_blocks(S), kThreads, counts, nullptr, T, S, q.ntot, q.stdv, nullptr);
+  LAUNCHG(k_q_frame_ids, dim3(q_blocks(S), T), kThreads, counts, nullptr, nullptr, nullptr, q.ntot,
+          nullptr, S, 1, q.live, nullptr, nullptr, nullptr);
+  std::vector<char> buf;
+  const char* res;
+  if ((r = quality_results(ctx, st, mem.p, q, buf, &res))) return r;
+  const auto* live = (const unsigned long long*)res;
+  const auto* stdv = (const double*)(res + ((char*)q.stdv - (char*)q.live));
   size_scores(live, stdv, T, S, tex, szv);
   if (ave_nsp) {
     double a = 0;
@@ -2263,31 +2366,28 @@ int stspix_sp_pooling(stspix_ctx* ctx, void* stream, const float* vid, const int
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
   const long long npix = (long long)H * W, n = T * npix, TS = (long long)T * nids;
-  int mm[2];
-  int r = label_range(ctx, st, spix, n, mm);
-  if (r) return r;
-  if (mm[0] < 0 || mm[1] >= nids)
-    return fail(ctx, STSPIX_ERR_ARG, "ids %d..%d outside [0, %d)", mm[0], mm[1], nids);
-  // counts, per-frame id sums, and the video-wide id / per-frame sums that the
-  // accumulation pass also produces
+  // the range check's words, counts and per-frame id sums.  The kernels skip ids out of
+  // range, so all of them are launched before the host waits for the range alone.
   const size_t cbytes = (4 * (size_t)TS + 255) & ~size_t(255);
-  const size_t bytes = cbytes + 24 * ((size_t)TS + nids + T);
-  char* base = nullptr;
-  CK(cudaMallocAsync((void**)&base, bytes, st));
-  CK(cudaMemsetAsync(base, 0, bytes, st));
-  int* cnt = (int*)base;
-  double* fsum = (double*)(base + cbytes);
-  double* vsum = fsum + 3 * (size_t)TS;
-  double* msum = vsum + 3 * (size_t)nids;
-  const long long segs = (long long)T * H * ((W + 31) / 32);
-  const unsigned nb = (unsigned)std::max(1LL, std::min<long long>((segs + 7) / 8, 8LL * ctx->num_sms));
-  LAUNCHG(k_q_accum, nb, kThreads, vid, spix, nullptr, T, H, W, 0, nids, 1, cnt, fsum, vsum, msum,
-          nullptr);
+  const size_t bytes = 256 + cbytes + 24 * (size_t)TS;
+  Scratch mem(ctx, st);
+  int r;
+  if ((r = mem.get(bytes))) return r;
+  if ((r = range_launch(ctx, st, (int*)mem.p, spix, nullptr, n))) return r;
+  CK(cudaMemsetAsync(mem.p + 256, 0, bytes - 256, st));
+  int* cnt = (int*)(mem.p + 256);
+  double* fsum = (double*)(mem.p + 256 + cbytes);
+  LAUNCHG(k_q_accum, dim3(q_tiles(H, W), (unsigned)T), kThreads, vid, spix, nullptr, npix, H, W, 0,
+          nids, 1, cnt, fsum, nullptr);
   LAUNCHG(k_q_down, q_blocks(TS), kThreads, cnt, fsum, TS, down);
   if (pooled)
-    LAUNCHG(k_q_pool_write, q_blocks(n), kThreads, spix, (int)npix, 0, nids, n, down, pooled);
-  CK(cudaFreeAsync(base, st));
+    LAUNCHG(k_q_pool_write, (unsigned)((n + kMarkPix - 1) / kMarkPix), kThreads, spix, (int)npix,
+            nids, n, down, pooled);
   CK(cudaGetLastError());
+  int mm[4];
+  if ((r = range_get(ctx, mm))) return r;
+  if (mm[0] < 0 || mm[1] >= nids)
+    return fail(ctx, STSPIX_ERR_ARG, "ids %d..%d outside [0, %d)", mm[0], mm[1], nids);
   return STSPIX_OK;
 }
 
@@ -2475,11 +2575,11 @@ int stspix_legacy_split_disconnected(stspix_ctx* ctx, void* stream, int32_t* spi
   if (!ctx || !spix || !split_starts || !max_nsplits || H < 1 || W < 1 || nspix < 1 ||
       (long long)H * W > INT_MAX / 2)
     return fail(ctx, STSPIX_ERR_ARG, "bad argument");
-  int r, rng[2];
+  int r, rng[4];
   const int npix = H * W;
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
-  if ((r = label_range(ctx, st, spix, npix, rng))) return r;
+  if ((r = label_range(ctx, st, spix, nullptr, npix, rng))) return r;
   if (rng[0] < 0 || rng[1] >= nspix)
     return fail(ctx, STSPIX_ERR_ARG, "labels must lie in [0, %d) (got %d..%d)", nspix, rng[0],
                 rng[1]);
@@ -2541,10 +2641,11 @@ int stspix_evaluate(stspix_ctx* ctx, void* stream, const float* vid, const int32
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
   const long long npix = (long long)H * W, n = T * npix;
-  int sr[2], gr[2] = {0, 0};
-  int r = label_range(ctx, st, spix, n, sr);
+  int mm[4];
+  int r = label_range(ctx, st, spix, gt, n, mm);
   if (r) return r;
-  if (gt && (r = label_range(ctx, st, gt, n, gr))) return r;
+  const int* sr = mm;
+  const int gr[2] = {gt ? mm[2] : 0, gt ? mm[3] : 0};
   if (gt && gr[0] < 0) return fail(ctx, STSPIX_ERR_ARG, "negative ground-truth id %d", gr[0]);
   const long long S = (long long)sr[1] - sr[0] + 1, G1 = gt ? (long long)gr[1] + 1 : 1;
   if (S > INT_MAX || G1 > INT_MAX) return fail(ctx, STSPIX_ERR_TOO_LARGE, "id range too large");
@@ -2552,57 +2653,40 @@ int stspix_evaluate(stspix_ctx* ctx, void* stream, const float* vid, const int32
   if (q.bytes > kQualityMaxScratch || (gt && (double)T * S * G1 > 2e9))
     return fail(ctx, STSPIX_ERR_TOO_LARGE, "evaluation tables of %zu bytes (T=%d, ids=%lld, "
                 "ground-truth ids=%lld) exceed the limit", q.bytes, T, S, G1);
-  char* base = nullptr;
-  CK(cudaMallocAsync((void**)&base, q.bytes, st));
-  q = quality_layout(base, T, S, G1, true, gt != nullptr);
-  CK(cudaMemsetAsync(base, 0, q.bytes, st));
-  const long long segs = (long long)T * H * ((W + 31) / 32);
-  const unsigned nb = (unsigned)std::max(1LL, std::min<long long>((segs + 7) / 8, 8LL * ctx->num_sms));
-  LAUNCHG(k_q_accum, nb, kThreads, vid, spix, gt, T, H, W, sr[0], (int)S, (int)G1, q.cnt, q.fsum,
-          q.vsum, q.msum, q.J);
+  Scratch mem(ctx, st);
+  if ((r = mem.get(q.bytes))) return r;
+  q = quality_layout(mem.p, T, S, G1, true, gt != nullptr);
+  CK(cudaMemsetAsync(mem.p, 0, q.bytes, st));
+  LAUNCHG(k_q_accum, dim3(q_tiles(H, W), (unsigned)T), kThreads, vid, spix, gt, npix, H, W, sr[0],
+          (int)S, (int)G1, q.cnt, q.fsum, q.J);
+  LAUNCHG(k_q_mean, dim3(q_blocks(S), T), kThreads, q.cnt, q.fsum, (int)S, q.mean, q.msum);
   const unsigned rx = (unsigned)std::max(1LL, std::min<long long>(q_blocks(npix), 8LL * ctx->num_sms / T + 1));
-  LAUNCHG(k_q_resid, dim3(rx, T), kThreads, vid, spix, (int)npix, sr[0], (int)S, q.cnt, q.fsum,
-          q.msum, q.pix2, q.pix2s, q.sse);
-  LAUNCHG(k_q_id_time, q_blocks(S), kThreads, q.cnt, T, (int)S, q.ntot, q.stdv);
-  LAUNCHG(k_q_frame_ids, dim3(q_blocks(S), T), kThreads, q.cnt, q.fsum, q.vsum, q.ntot, q.msum,
-          (int)S, (int)npix, q.live, q.pool2, q.pool3);
-  if (gt) {
-    LAUNCHG(k_q_uesa_frame, dim3(q_blocks(S), T), kThreads, q.cnt, q.J, (int)S, (int)G1, q.ue,
-            q.sa, q.gsize);
-    LAUNCHG(k_q_uesa_id, q_blocks(S), kThreads, q.cnt, q.J, q.ntot, T, (int)S, (int)G1, q.ue3,
-            q.sa3);
-  }
+  LAUNCHG(k_q_resid, dim3(rx, T), kThreads, vid, spix, (int)npix, sr[0], (int)S, q.mean, q.sse);
+  LAUNCHG(k_q_id_time, q_blocks(S), kThreads, q.cnt, q.fsum, T, (int)S, q.ntot, q.stdv, q.vsum);
+  LAUNCHG(k_q_frame_ids, dim3(q_blocks(S), T), kThreads, q.cnt, q.fsum, q.mean, q.vsum, q.ntot,
+          q.msum, (int)S, (int)npix, q.live, q.pool2, q.cross, q.pool3);
+  if (gt)
+    LAUNCHG(k_q_uesa, dim3((unsigned)((S + kQUesaIds - 1) / kQUesaIds), q_blocks(G1)), kThreads,
+            q.cnt, q.J, q.ntot, T, (int)S, (int)G1, q.ue, q.sa, q.gsize, q.ue3, q.sa3);
   // per-frame / per-id results to the host
-  std::vector<double> pix2(T), pix2s(T), sse(T), pool2(T), pool3(T), stdv(S);
-  std::vector<unsigned long long> live(T), ue, sa, gsize, ue3, sa3;
-  auto d2h = [&](void* dst, const void* src, size_t bytes) {
-    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+  std::vector<char> buf;
+  const char* out_h;
+  if ((r = quality_results(ctx, st, mem.p, q, buf, &out_h))) return r;
+  auto on_host = [&](const auto* d) {
+    return (decltype(d))(out_h + ((const char*)d - (mem.p + q.results)));
   };
-  CK(d2h(pix2.data(), q.pix2, 8 * (size_t)T));
-  CK(d2h(pix2s.data(), q.pix2s, 8 * (size_t)T));
-  CK(d2h(sse.data(), q.sse, 8 * (size_t)T));
-  CK(d2h(pool2.data(), q.pool2, 8 * (size_t)T));
-  CK(d2h(pool3.data(), q.pool3, 8 * (size_t)T));
-  CK(d2h(live.data(), q.live, 8 * (size_t)T));
-  CK(d2h(stdv.data(), q.stdv, 8 * (size_t)S));
-  if (gt) {
-    ue.resize(T * G1); sa.resize(T * G1); gsize.resize(T * G1); ue3.resize(G1); sa3.resize(G1);
-    CK(d2h(ue.data(), q.ue, 8 * (size_t)(T * G1)));
-    CK(d2h(sa.data(), q.sa, 8 * (size_t)(T * G1)));
-    CK(d2h(gsize.data(), q.gsize, 8 * (size_t)(T * G1)));
-    CK(d2h(ue3.data(), q.ue3, 8 * (size_t)G1));
-    CK(d2h(sa3.data(), q.sa3, 8 * (size_t)G1));
-  }
-  CK(cudaFreeAsync(base, st));
-  CK(cudaStreamSynchronize(st));
-  CK(cudaGetLastError());
+  const auto *live = on_host(q.live), *ue = on_host(q.ue), *sa = on_host(q.sa),
+             *gsize = on_host(q.gsize), *ue3 = on_host(q.ue3), *sa3 = on_host(q.sa3);
+  const auto *stdv = on_host(q.stdv), *sse = on_host(q.sse), *pool2 = on_host(q.pool2),
+             *cross = on_host(q.cross), *pool3 = on_host(q.pool3);
 
   stspix_quality res{};
   size_scores(live, stdv, T, S, &res.tex, &res.szv);
   double ev = 0, ev3 = 0, ps = 0, nsp = 0;
   for (int t = 0; t < T; t++) {
-    ev += pool2[t] / (pix2[t] + 1e-10);
-    ev3 += pool3[t] / (pix2s[t] + 1e-10);
+    const double pix2 = sse[t] + 2 * cross[t] + pool2[t];   // sum (v - frame mean)^2
+    ev += pool2[t] / (pix2 + 1e-10);
+    ev3 += pool3[t] / (65025.0 * pix2 + 1e-10);
     const double mse = sse[t] / (3.0 * npix);
     ps += mse > 0 ? 10.0 * std::log10(1.0 / mse) : INFINITY;
     nsp += (double)live[t];

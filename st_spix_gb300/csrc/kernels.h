@@ -129,23 +129,25 @@ __global__ void k_lab2rgb(const float* lab, float* rgb, long long npix);
 __global__ void k_rescale_u8(const uint8_t* in, float* out, long long nvals, float mval);
 
 // k_quality.cu
-constexpr int kQGtShared = 256;
+constexpr int kQUesaIds = 4;              // ids per thread of k_q_uesa
 __global__ void k_q_range_init(int* mm);
-__global__ void k_q_range(const int32_t* a, long long n, int* mm);
-__global__ void k_q_accum(const float* vid, const int32_t* spix, const int32_t* gt, int T, int H,
-                          int W, int off, int S, int G1, int* cnt, double* fsum, double* vsum,
-                          double* msum, int* J);
+__global__ void k_q_range(const int32_t* a, const int32_t* b, long long n, int* mm);
+__global__ void k_q_accum(const float* vid, const int32_t* spix, const int32_t* gt, long long npix,
+                          int H, int W, int off, int S, int G1, int* cnt, double* fsum, int* J);
+__global__ void k_q_count(const int32_t* spix, long long npix, int H, int W, int off, int S,
+                          int* cnt);
+__global__ void k_q_id_time(const int* cnt, const double* fsum, int T, int S, long long* ntot,
+                            double* std_out, double* vsum);
+__global__ void k_q_mean(const int* cnt, const double* fsum, int S, double* mean, double* msum);
 __global__ void k_q_resid(const float* vid, const int32_t* spix, int npix, int off, int S,
-                          const int* cnt, const double* fsum, const double* msum, double* pix2,
-                          double* pix2s, double* sse);
-__global__ void k_q_id_time(const int* cnt, int T, int S, long long* ntot, double* std_out);
-__global__ void k_q_frame_ids(const int* cnt, const double* fsum, const double* vsum,
-                              const long long* ntot, const double* msum, int S, int npix,
-                              unsigned long long* live, double* pool2, double* pool3);
-__global__ void k_q_uesa_frame(const int* cnt, const int* J, int S, int G1, unsigned long long* ue,
-                               unsigned long long* sa, unsigned long long* size);
-__global__ void k_q_uesa_id(const int* cnt, const int* J, const long long* ntot, int T, int S,
-                            int G1, unsigned long long* ue3, unsigned long long* sa3);
+                          const double* mean, double* sse);
+__global__ void k_q_frame_ids(const int* cnt, const double* fsum, const double* mean,
+                              const double* vsum, const long long* ntot, const double* msum, int S,
+                              int npix, unsigned long long* live, double* pool2, double* cross,
+                              double* pool3);
+__global__ void k_q_uesa(const int* cnt, const int* J, const long long* ntot, int T, int S, int G1,
+                         unsigned long long* ue, unsigned long long* sa, unsigned long long* size,
+                         unsigned long long* ue3, unsigned long long* sa3);
 __global__ void k_q_down(const int* cnt, const double* fsum, long long TS, float* down);
 
 // k_legacy.cu
@@ -163,7 +165,7 @@ __global__ void k_vpool_mean(const double* sum, const unsigned long long* cnt, l
                              int F, float* down, float* counts);
 __global__ void k_vpool_write(const float* down, const int32_t* seg, int T, long long npix, int F,
                               int nspix, float* pooled);
-__global__ void k_q_pool_write(const int32_t* spix, int npix, int off, int S, long long n,
+__global__ void k_q_pool_write(const int32_t* spix, int npix, int S, long long n,
                                const float* down, float* pooled);
 __global__ void k_lmark_ids(const int32_t* spix, long long n, int nids, uint8_t* present);
 __global__ void k_lupdate_prior(const uint8_t* present, int nids, int prev_nspix, int invert,
