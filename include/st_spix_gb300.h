@@ -273,6 +273,10 @@ int stspix_bass_partial(stspix_ctx* ctx, void* stream, const float* img, int H, 
  * (rgb2lab.cu:184 rescale_image_kernel).  Pixels with a NaN channel are left
  * unwritten, as in the reference.                                              */
 int stspix_rgb2lab(stspix_ctx* ctx, void* stream, const float* rgb, float* lab, long long npix);
+/* The same conversion with the first channel blue (first_blue 1) or red (0), into a buffer
+ * that holds nothing yet: a pixel with a NaN channel gets its input values.         */
+int stspix_rgb2lab_copy(stspix_ctx* ctx, void* stream, const float* rgb, float* lab,
+                        long long npix, int first_blue);
 int stspix_lab2rgb(stspix_ctx* ctx, void* stream, const float* lab, float* rgb, long long npix);
 int stspix_rescale_u8(stspix_ctx* ctx, void* stream, const uint8_t* in, float* out,
                       long long nvals, float scale);

@@ -221,11 +221,16 @@ def kernel_launches(device=None) -> int:
 def rgb2lab(img: torch.Tensor) -> torch.Tensor:
     """f32 [...,3] (first channel read as blue, as the reference) -> CIELAB stored as
     (L/-100, a/100, b/100), rgb2lab.cu:51-122."""
+    return _rgb2lab(img, 1)
+
+
+def _rgb2lab(img: torch.Tensor, first_blue: int) -> torch.Tensor:
     _check_input(img, "img")
-    out = img.clone()
+    # every whole pixel is written (one with a NaN channel as it was)
+    out = torch.empty_like(img) if img.numel() % 3 == 0 else img.clone()
     ctx = _ctx(img.device)
-    ctx.check(ctx.lib.stspix_rgb2lab(ctx.handle, _stream(img.device), img.data_ptr(),
-                                     out.data_ptr(), img.numel() // 3))
+    ctx.check(ctx.lib.stspix_rgb2lab_copy(ctx.handle, _stream(img.device), img.data_ptr(),
+                                          out.data_ptr(), img.numel() // 3, first_blue))
     return out
 
 

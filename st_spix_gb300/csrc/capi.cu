@@ -2062,7 +2062,17 @@ int stspix_rgb2lab(stspix_ctx* ctx, void* stream, const float* rgb, float* lab,
   if (!ctx || !rgb || !lab || npix < 0) return fail(ctx, STSPIX_ERR_ARG, "bad argument");
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
-  LAUNCH(k_rgb2lab, npix, rgb, lab, npix, 1);
+  LAUNCH(k_rgb2lab, npix, rgb, lab, npix, 1, 0);
+  CK(cudaGetLastError());
+  return STSPIX_OK;
+}
+
+int stspix_rgb2lab_copy(stspix_ctx* ctx, void* stream, const float* rgb, float* lab,
+                        long long npix, int first_blue) {
+  if (!ctx || !rgb || !lab || npix < 0) return fail(ctx, STSPIX_ERR_ARG, "bad argument");
+  cudaSetDevice(ctx->device);
+  cudaStream_t st = (cudaStream_t)stream;
+  LAUNCH(k_rgb2lab, npix, rgb, lab, npix, first_blue ? 1 : 0, 1);
   CK(cudaGetLastError());
   return STSPIX_OK;
 }
@@ -2083,7 +2093,7 @@ int stspix_rescale_u8(stspix_ctx* ctx, void* stream, const uint8_t* in, float* o
     return fail(ctx, STSPIX_ERR_ARG, "bad argument");
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
-  LAUNCH(k_rescale_u8, nvals, in, out, nvals, scale);
+  LAUNCH(k_rescale_u8, (nvals + 3) / 4, in, out, nvals, scale);
   CK(cudaGetLastError());
   return STSPIX_OK;
 }
@@ -2460,7 +2470,7 @@ int stspix_legacy_rgb_to_lab(stspix_ctx* ctx, void* stream, const float* rgb, fl
   if (!ctx || !rgb || !lab || npix < 0) return fail(ctx, STSPIX_ERR_ARG, "bad argument");
   cudaSetDevice(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
-  LAUNCH(k_rgb2lab, npix, rgb, lab, npix, 0);
+  LAUNCH(k_rgb2lab, npix, rgb, lab, npix, 0, 0);
   CK(cudaGetLastError());
   return STSPIX_OK;
 }

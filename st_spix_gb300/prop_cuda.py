@@ -247,12 +247,7 @@ def fill_missing(spix, centers, missing, break_iter):
 
 def rgb_to_lab(img):
     """prop/rgb2lab.cu:167 (channels read in RGB order)."""
-    _check_input(img, "img")
-    out = img.clone()
-    ctx = _ctx(img.device)
-    ctx.check(ctx.lib.stspix_legacy_rgb_to_lab(ctx.handle, _stream(img.device), img.data_ptr(),
-                                               out.data_ptr(), img.numel() // 3))
-    return out
+    return bist_cuda._rgb2lab(img, 0)
 
 
 def lab_to_rgb(img):
