@@ -662,8 +662,10 @@ void accumulate_fp(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, int 
 // the statistics of the first nb slots (see update_seg).
 // incremental: only the ids whose sums changed since their last posterior;
 // only where nothing but sweeps ran since the previous posterior of every slot.
+// log64: the log determinants in FP64 (see kb_posterior).
 int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
-                  bool stats_ready = false, bool incremental = false, bool clear_all = false) {
+                  bool stats_ready = false, bool incremental = false, bool clear_all = false,
+                  bool log64 = false) {
   ctx->cur_fam = STSPIX_FAM_STATS;
   if (!stats_ready) {
     LAUNCHB(kb_clear_stats, L.max_cap, L, nb, clear_all ? 1 : 0);
@@ -675,7 +677,8 @@ int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
   // further groups)
   const unsigned pg = (unsigned)std::min<long long>((L.max_cap + 31) / 32,
                                                     std::max(32, (4 * ctx->num_sms + nb - 1) / nb));
-  LAUNCHG(kb_posterior, dim3(pg, (unsigned)nb), 128, L.d, incremental ? 1 : 0);
+  LAUNCHG(kb_posterior, dim3(pg, (unsigned)nb), 128, L.d, incremental ? 1 : 0,
+          log64 ? 1 : 0);
   return STSPIX_OK;
 }
 
@@ -864,14 +867,19 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
   bool stats_ready = fuse && !L.any_prop;
   bool chg_ok = false;      // the previous update_seg left its changes and label buffers
   int cur = 0;              // the label buffer the next sweep reads (see update_seg)
+  const bool state = stop_after >= 0;       // the caller reads the state, not the parameters
+  auto params = [&](const List& l, int n, bool ready = false, bool incremental = false,
+                    bool all = false) {
+    return update_params(ctx, st, l, n, ready, incremental, all, state);
+  };
   for (int idx = 0; idx < maxn; idx++) {
     while (nb > 0 && nit[nb - 1] <= idx) nb--;
     if (stop_after >= 0 && idx == stop_after) {
-      if (extra_update && (r = update_params(ctx, st, L, nb))) return r;
+      if (extra_update && (r = params(L, nb))) return r;
       return STSPIX_OK;
     }
     // after the first iteration only the sweeps ran since every slot's last posterior
-    if ((r = update_params(ctx, st, L, nb, stats_ready, idx > 0, idx == 0))) return r;
+    if ((r = params(L, nb, stats_ready, idx > 0, idx == 0))) return r;
     stats_ready = false;
     // the first sweep is an active-set one when only sweeps and that incremental
     // posterior ran since the previous update_seg
@@ -882,13 +890,13 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
         count_b += 1;
         count_p += 1;
         if ((r = run_split(ctx, st, L, nb, K, cfg, count_b % 2 + 1, count_p % 2 + 1))) return r;
-        if ((r = update_params(ctx, st, L, nb))) return r;
+        if ((r = params(L, nb))) return r;
       }
       if (idx % P == P / 2) {
         count_p += 1;  // propagated frames step the direction again before merging
         if (L.any_prop && (r = run_relabel(ctx, st, L, nb, cfg))) return r;
         if ((r = run_merge(ctx, st, L, nb, K, cfg, count_b % 2, count_p % 2, P == 1))) return r;
-        if ((r = update_params(ctx, st, L, nb))) return r;
+        if ((r = params(L, nb))) return r;
       }
     }
     const int nx = idx + 1;
@@ -904,14 +912,13 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
     stats_ready = fuse_now;
   }
   if (stop_after >= 0) {
-    if (extra_update && (r = update_params(ctx, st, L, L.B))) return r;
+    if (extra_update && (r = params(L, L.B))) return r;
     return STSPIX_OK;
   }
   // final update_params + store_sample; slots that finished earlier were untouched
   // since, so running theirs here is the same as running it right after their loop
   // (and their statistics are current too: with fuse every sweep moved them)
-  if ((r = update_params(ctx, st, L, L.B, fuse && maxn > 0 && nit[L.B - 1] > 0, maxn > 0,
-                         maxn == 0)))
+  if ((r = params(L, L.B, fuse && maxn > 0 && nit[L.B - 1] > 0, maxn > 0, maxn == 0)))
     return r;
   ctx->cur_fam = STSPIX_FAM_POSTERIOR;
   LAUNCHB(kb_store_sample, L.max_cap, L, L.B);

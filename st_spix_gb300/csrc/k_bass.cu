@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.h"
+#include "ff.h"
 #include "kernels.h"
 
 namespace stspix {
@@ -512,12 +513,16 @@ __device__ __forceinline__ void smooth_prior(double in_x, double in_y, double in
   *oz = (pc * sp_size + count * in_z) / (total_count + 3.0);
 }
 
-// One block = 32 consecutive ids, four warps splitting each id's FP64 chain (this part
-// issues FP64 slowly, so one warp per id set would serialise the whole chain on one
-// scheduler): warp 0 the colour means, warp 1 the prior shape term, warp 2 the shape
-// mean and scatter; then warps 0-2 one smoothed covariance entry each, then warps 0-2
-// one inverse entry each and warp 3 the log determinant.  Every value is the same
-// expression as a single-thread evaluation, exchanged through shared memory.
+// One block = 32 consecutive ids, four warps.  Every value is that of the reference's FP64
+// expression, bit for bit, but an FP64 instruction here occupies its scheduler for 64 cycles
+// (measured: a dependent or an independent one, one lane or 32; a division 564, log 2100),
+// so their number on the longest warp is what a launch lasts.  The four warps sit on four
+// schedulers and share the work out: warps 1 and 2 take the x and y means and scatters,
+// warp 0 the mixed one, each then one entry of the smoothed covariance and of its inverse;
+// warp 3 the prior, the reciprocal of the smoothing's denominator and the log determinant.
+// Quotients of one divisor share its reciprocal (correctly rounded all the same, see ff.h),
+// and where only a float is kept (colour means, the record's log determinant) it is computed
+// in pairs of floats, FP64 only next to a rounding boundary.
 //
 // incremental: only the ids whose count or sums differ from those their posterior last saw
 // (S.snap) are computed.  Between two posteriors of the outer loop only the sweeps run,
@@ -527,29 +532,37 @@ __device__ __forceinline__ void smooth_prior(double in_x, double in_y, double in
 // expressions of the same inputs).  The prior shape term is read from S.pscache then, which
 // the last full posterior wrote.
 //
+// log64: sp.logdet in FP64 (the state read-out); otherwise its float, which is all that the
+// records and the parameter read-out take of it.
+//
 // Every load of a group, the old record and the snapshot among them, is issued before any
-// is used, and the ids are compared where they are computed: what bounds a launch is the
-// chain launch - slot - loads - FP64 - store, one group per block on most frames.  With
-// a work list of the changed ids built by a kernel of its own a posterior took 10.5 us on
-// a 240x320 frame, 13.4 on 720x1280 and 17.1 on 8 frames of 480x854; now 5.7, 7.5 and 11.6.
+// is used, and the ids are compared where they are computed: on most frames, with one group
+// per block, a launch is the chain launch - slot - loads - FP64 - store.  With a work list of
+// the changed ids built by a kernel of its own a posterior took 10.5 us on a 240x320 frame,
+// 13.4 on 720x1280 and 17.1 on 8 frames of 480x854; without it, but with a division per
+// quotient and the log in FP64, 5.7, 7.6 and 11.6 (and 32.4 on 16 frames of mixed sizes);
+// now 5.0, 6.5, 9.4 (and 23.3).
 __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slots,
-                                                    int incremental) {
+                                                    int incremental, int log64) {
   pdl_enter();
   SLOT_Y;
-  __shared__ double v_ps[3][32], v_raw[3][32], v_m[2][32], v_s[3][32], v_i[4][32];
-  __shared__ float v_app[3][32];
-  __shared__ int s_diff[2][32];
+  __shared__ double v_ps[3][32], v_den[3][32], v_m[2][32], v_s[3][32], v_ld[32];
+  __shared__ float v_i[3][32];
+  __shared__ int v_pos[2][32];
+  __shared__ unsigned s_diff[3];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const SpDev& sp = S.sp;
   const int cap = sp.cap;
   const int last = min(cap - 1, S.sc->max_spix);
+  // the sums and the covariance entry (xx, xy, yy) of a warp
+  const int f0 = w == 0 ? 0 : w == 1 ? 3 : 4;
+  const int f1 = w == 0 ? 6 : w == 1 ? 5 : 7, ent = w == 0 ? 1 : w == 1 ? 0 : 2;
   for (int g = blockIdx.x;; g += gridDim.x) {
     const int k = 32 * g + lane;
-    // warp 0: colour sums, count and record; warp 1: the prior; warp 2: position sums
     int count_int = 0;
     uint8_t valid = 0, prop = 0;
     float pc = 0.f;
-    long long a[5] = {0, 0, 0, 0, 0}, o[5] = {0, 0, 0, 0, 0}, ocount = 0;
+    long long a[4] = {0, 0, 0, 0}, o[4] = {0, 0, 0, 0}, ocount = 0;
     double q0 = 0, q1 = 0, q2 = 0, i0 = 0, i1 = 0, i2 = 0;
     uint4 orec[3];
     if (k < cap) {
@@ -558,74 +571,71 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
       count_int = sp.count[k];
       valid = sp.valid[k];
       pc = sp.prior_count[k];
-      if (w == 0) {
+      if (w < 3) {
+        a[0] = acc[f0]; o[0] = snap[f0];
+        a[3] = acc[f1]; o[3] = snap[f1];
+        if (incremental) q0 = S.pscache[3 * (size_t)k + ent];
+        if (w == 0) {
+          a[1] = acc[1]; o[1] = snap[1];
+          a[2] = acc[2]; o[2] = snap[2];
+          ocount = snap[8];
 #pragma unroll
-        for (int f = 0; f < 3; f++) { a[f] = acc[f]; o[f] = snap[f]; }
-        ocount = snap[8];
-#pragma unroll
-        for (int q = 0; q < 3; q++) orec[q] = ((const uint4*)&sp.rec[k])[q];
-      } else if (w == 1) {
-        if (incremental) {
-          q0 = S.pscache[3 * (size_t)k]; q1 = S.pscache[3 * (size_t)k + 1];
-          q2 = S.pscache[3 * (size_t)k + 2];
-        } else {
-          prop = sp.prop[k];
-          q0 = sp.sample_sigma_shape[3 * k]; q1 = sp.sample_sigma_shape[3 * k + 1];
-          q2 = sp.sample_sigma_shape[3 * k + 2];
-          i0 = sp.prior_icov[3 * k]; i1 = sp.prior_icov[3 * k + 1]; i2 = sp.prior_icov[3 * k + 2];
+          for (int q = 0; q < 3; q++) orec[q] = ((const uint4*)&sp.rec[k])[q];
         }
-      } else if (w == 2) {
-#pragma unroll
-        for (int f = 0; f < 5; f++) { a[f] = acc[3 + f]; o[f] = snap[3 + f]; }
+      } else if (!incremental) {
+        prop = sp.prop[k];
+        q0 = sp.sample_sigma_shape[3 * k]; q1 = sp.sample_sigma_shape[3 * k + 1];
+        q2 = sp.sample_sigma_shape[3 * k + 2];
+        i0 = sp.prior_icov[3 * k]; i1 = sp.prior_icov[3 * k + 1]; i2 = sp.prior_icov[3 * k + 2];
       }
     }
     if (32 * g > last) return;                     // block-uniform
     const bool inr = k <= last;
-    if (w == 0 || w == 2) {
+    if (w < 3) {
       bool diff = !incremental;
 #pragma unroll
-      for (int f = 0; f < 5; f++) diff |= a[f] != o[f];
+      for (int f = 0; f < 4; f++) diff |= a[f] != o[f];
       if (w == 0) diff |= ocount != count_int;
-      s_diff[w >> 1][lane] = inr && diff;
+      const unsigned m = __ballot_sync(0xffffffffu, inr && diff);
+      if (lane == 0) s_diff[w] = m;
     }
     __syncthreads();
-    const bool want = s_diff[0][lane] | s_diff[1][lane];
+    const bool want = ((s_diff[0] | s_diff[1] | s_diff[2]) >> lane) & 1u;
     const bool live = want && valid && count_int > 0;
-    if (want) {
-      long long* snap = S.snap + 9 * (size_t)k;
-      if (w == 0) {
-#pragma unroll
-        for (int f = 0; f < 3; f++) snap[f] = a[f];
-        snap[8] = count_int;
-        if (valid && count_int <= 0) sp.valid[k] = 0;
-        if (!live) {
-          for (int c = 0; c < 3; c++) { sp.mu_app[3 * k + c] = 0.f; sp.sigma_shape[3 * k + c] = 0.0; }
-          sp.mu_shape[2 * k] = 0.0; sp.mu_shape[2 * k + 1] = 0.0;
-        }
-      } else if (w == 2) {
-#pragma unroll
-        for (int f = 0; f < 5; f++) snap[3 + f] = a[f];
-      }
-    }
+    const bool any = __any_sync(0xffffffffu, live);          // the same in every warp
     // (the sweeps of the next update score again only the pixels next to a changed record)
     if (w == 0 && inr && !live) S.recchg[k] = 0;
-    if (!__syncthreads_or(live)) continue;
-    const double count = count_int * 1.0;
-    const double total_count = (double)count_int + pc * 50;
+    double r0 = 0, nd = 0;
+    float app[3] = {0.f, 0.f, 0.f};                // warp 0: the mean colour
     if (live) {
+      nd = to_double(count_int);
       if (w == 0) {
         // colour means (fixed-point sums, R1)
+        const float y = __frcp_rn((float)count_int);
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const float m = (float)(fx_unq(a[c], kFxAppShift) / count);
-          sp.mu_app[3 * k + c] = m;
-          v_app[c][lane] = m;
-        }
-      } else if (w == 1) {
+        for (int c = 0; c < 3; c++)
+          if (!mean_ff(a[c], count_int, y, &app[c]))
+            app[c] = (float)(fx_unq(a[c], kFxAppShift) / nd);
+        r0 = to_double(a[3]);
+      } else if (w < 3) {
+        // shape mean and scatter, of x or of y
+        const double y = recip34(nd, (float)count_int), s = to_double(a[0]);
+        const double m = div_int(a[0], s, nd, y);
+        v_m[w - 1][lane] = m;
+        r0 = to_double(a[3]) - nd * m * m;
+        sp.mu_shape[2 * k + w - 1] = m;
+        // floor and has-fraction, in the bits below and above
+        bool frac;
+        const int fl = floor_bits(m, &frac);
+        v_pos[w - 1][lane] = (int)((unsigned)fl << 1) | (frac ? 1 : 0);
+      } else {
+        const double total_count = nd + pc * 50;
+        const double den = total_count + 3.0;
+        v_den[0][lane] = den;
+        v_den[1][lane] = recip34(den, pc >= 0.f ? (float)count_int + pc * 50 + 3.f : 0.f);
+        v_den[2][lane] = pc;
         // prior shape term (calc_simple_update with _add_sigma_smoothing)
-        if (incremental) {
-          v_ps[0][lane] = q0; v_ps[1][lane] = q1; v_ps[2][lane] = q2;
-        } else {
+        if (!incremental) {
           double px, py, pz;
           if (prop) {
             smooth_prior(q0, q1, q2, (int)pc, pc, S.sp_size, &px, &py, &pz);
@@ -640,19 +650,38 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
           S.pscache[3 * (size_t)k] = t0; S.pscache[3 * (size_t)k + 1] = t1;
           S.pscache[3 * (size_t)k + 2] = t2;
         }
-      } else if (w == 2) {
-        // shape mean and scatter
-        const double mx = a[0] / count, my = a[1] / count;
-        sp.mu_shape[2 * k] = mx; sp.mu_shape[2 * k + 1] = my;
-        v_m[0][lane] = mx; v_m[1][lane] = my;
-        v_raw[0][lane] = a[2] - count * mx * mx;
-        v_raw[1][lane] = a[3] - count * mx * my;
-        v_raw[2][lane] = a[4] - count * my * my;
       }
     }
     __syncthreads();
-    if (live && w < 3) v_s[w][lane] = (pc * v_ps[w][lane] + v_raw[w][lane]) / (total_count + 3.0);
+    if (want) {
+      // (behind the first barrier's reads, beside the FP64 work)
+      long long* snap = S.snap + 9 * (size_t)k;
+      if (w < 3) {
+        snap[f0] = a[0];
+        snap[f1] = a[3];
+      }
+      if (w == 0) {
+        snap[1] = a[1];
+        snap[2] = a[2];
+        snap[8] = count_int;
+        if (valid && count_int <= 0) sp.valid[k] = 0;
+#pragma unroll
+        for (int c = 0; c < 3; c++) sp.mu_app[3 * k + c] = app[c];
+        if (!live) {
+          for (int c = 0; c < 3; c++) sp.sigma_shape[3 * k + c] = 0.0;
+          sp.mu_shape[2 * k] = 0.0; sp.mu_shape[2 * k + 1] = 0.0;
+        }
+      }
+    }
+    if (!any) continue;
+    // the smoothed covariance, an entry per warp
+    if (live && w < 3) {
+      if (w == 0) r0 = r0 - nd * v_m[0][lane] * v_m[1][lane];
+      const double ps = incremental ? q0 : v_ps[ent][lane];
+      v_s[ent][lane] = div_recip(v_den[2][lane] * ps + r0, v_den[0][lane], v_den[1][lane]);
+    }
     __syncthreads();
+    // its inverse and log determinant
     if (live) {
       double sx = v_s[0][lane], sy = v_s[1][lane], sz = v_s[2][lane];
       double det = sx * sz - sy * sy;
@@ -662,24 +691,26 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
         det = sx * sz - sy * sy;
         if (det <= 0) det = 0.00001;
       }
-      if (w == 0) v_i[0][lane] = sz / det;
-      else if (w == 1) v_i[1][lane] = -sy / det;
-      else if (w == 2) v_i[2][lane] = sx / det;
-      else v_i[3][lane] = log(det);
+      if (w < 3) {
+        const double v = (w == 0 ? -sy : w == 1 ? sz : sx) / det;
+        sp.sigma_shape[3 * k + ent] = v;
+        v_i[ent][lane] = (float)v;
+      } else {
+        float l;
+        v_ld[lane] = !log64 && log_ff(det, &l) ? (double)l : log(det);
+      }
     }
     __syncthreads();
     if (live && w == 0) {
-      const double ix = v_i[0][lane], iy = v_i[1][lane], iz = v_i[2][lane], ld = v_i[3][lane];
-      const double mx = v_m[0][lane], my = v_m[1][lane];
-      sp.sigma_shape[3 * k] = ix; sp.sigma_shape[3 * k + 1] = iy; sp.sigma_shape[3 * k + 2] = iz;
+      const double ld = v_ld[lane];
       sp.logdet[k] = ld;
       SweepRec r;
-      r.mu_r = v_app[0][lane]; r.mu_g = v_app[1][lane]; r.mu_b = v_app[2][lane];
+      r.mu_r = app[0]; r.mu_g = app[1]; r.mu_b = app[2];
       r.logdet = (float)ld;
-      const double fx = floor(mx), fy = floor(my);
-      r.mxi = (int)fx; r.myi = (int)fy;
-      r.frac = (mx != fx ? 1 : 0) | (my != fy ? 2 : 0);
-      r.isx = (float)ix; r.isy = (float)iy; r.isz = (float)iz; r.pad = 0.f;
+      const int px = v_pos[0][lane], py = v_pos[1][lane];
+      r.mxi = (int)((unsigned)px >> 1); r.myi = (int)((unsigned)py >> 1);
+      r.frac = (px & 1) | ((py & 1) << 1);
+      r.isx = v_i[0][lane]; r.isy = v_i[1][lane]; r.isz = v_i[2][lane]; r.pad = 0.f;
       r.count = count_int;
       const uint4* nw = (const uint4*)&r;
       bool same = true;

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.h"
+#include "ff.h"
 #include "pdl.h"
 
 namespace stspix {
@@ -63,27 +64,8 @@ __device__ __noinline__ void rgb2lab_fp64(float cR, float cG, float cB, float* l
 // branches, with larger values or an infinity, takes the FP64 steps: about 1 pixel in 10^5
 // of a bright frame; of the dark ones those of exactly equal channels (the differences
 // cancel), but for black.
-struct FF {
-  float h, l;
-};
-#define FF_CONST(x) FF{(float)(x), (float)((x) - (double)(float)(x))}
 constexpr float kFFMargin = 0x1p-43f;
 
-// RN(h + e) into *out; false when a value within `margin` of it may round elsewhere.
-__device__ __forceinline__ bool ff_round(float h, float e, float margin, float* out) {
-  const float up = h + (e + margin), dn = h + (e - margin);
-  *out = up;
-  return up == dn;
-}
-// The rounding error of s = a + b.
-__device__ __forceinline__ float sum_err(float a, float b, float s) {
-  const float bb = s - a;
-  return (a - (s - bb)) + (b - bb);
-}
-// a k - p for p = RN(a.h k.h), k a constant pair.
-__device__ __forceinline__ float mul_err(FF a, FF k, float p) {
-  return fmaf(a.l, k.h, fmaf(a.h, k.l, fmaf(a.h, k.h, -p)));
-}
 __device__ __forceinline__ bool lin_ff(float c, FF* r) {
   // (the largest float not above 0.04045 is its rounding)
   if (c <= 0.04045f) {

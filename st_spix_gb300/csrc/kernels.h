@@ -30,7 +30,7 @@ __global__ void kb_init_bass_params(const Slot* slots);
 __global__ void kb_init_prior_mu(const Slot* slots);
 __global__ void kb_clear_stats(const Slot* slots, int all);
 __global__ void kb_accumulate(const Slot* slots, int B);
-__global__ void kb_posterior(const Slot* slots, int incremental);
+__global__ void kb_posterior(const Slot* slots, int incremental, int log64);
 __global__ void kb_accumulate_fp(const Slot* slots, int mode);
 __global__ void kb_accumulate_fp_store(const Slot* slots, int mode);
 __global__ void kb_accumulate_fp_clear(const Slot* slots);
