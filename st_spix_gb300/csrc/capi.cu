@@ -273,11 +273,28 @@ void launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStrea
       LAUNCHG(kernel, dim3(blocks_for(n_), (unsigned)(nb)), kThreads, (L).d, ##__VA_ARGS__); \
   } while (0)
 
+// A per-id kernel (FOR_ID loops) over n ids per slot.
+#define LAUNCHI(kernel, n, L, nb, ...)                                         \
+  do {                                                                         \
+    if ((n) > 0 && (nb) > 0)                                                   \
+      LAUNCHG(kernel, dim3(id_blocks(ctx, (n), kThreads, (nb)), (unsigned)(nb)), kThreads, \
+              (L).d, ##__VA_ARGS__);                                           \
+  } while (0)
+
 // One thread per slot.
 #define LAUNCHS(kernel, L, nb, ...)                                            \
   do {                                                                         \
     if ((nb) > 0) LAUNCHG(kernel, blocks_for(nb), kThreads, (L).d, (nb), ##__VA_ARGS__); \
   } while (0)
+
+// Blocks per slot of a kernel over n ids, `per` a block, whose blocks loop: no more than 8
+// per SM over the batch.  A slot's capacity is 10 to 30 times the ids in use, and one block
+// per 32 ids of the largest capacity launched mostly empty ones: a merge decision over 16
+// frames of 240 to 1080 rows took 93 us so, 22 with this bound (a clear of per-id bytes 13.4 and 3.2).
+unsigned id_blocks(const stspix_ctx* ctx, long long n, int per, int nb) {
+  const long long most = std::max(8, (8 * ctx->num_sms + nb - 1) / nb);
+  return (unsigned)std::max(1LL, std::min((n + per - 1) / per, most));
+}
 
 template <typename T>
 int alloc(stspix_ctx* ctx, std::vector<Buf>& list, T** p, size_t n) {
@@ -459,7 +476,6 @@ void preload_kernels() {
       (const void*)kb_split_bfs,
       (const void*)kb_split_bfs_big,
       (const void*)kb_split_partition,
-      (const void*)kb_sm_clear,
       (const void*)kb_sm_accumulate,
       (const void*)kb_split_decide,
       (const void*)kb_split_commit,
@@ -499,7 +515,7 @@ void preload_kernels() {
       (const void*)kb_relabel_params,
       (const void*)kb_relabel_apply,
       (const void*)kb_relabel_end,
-      (const void*)kb_count_revived,
+
       (const void*)kb_accumulate_fp, (const void*)kb_accumulate_fp_store,
       (const void*)kb_accumulate_fp_clear, (const void*)k_label_stats,
       (const void*)k_label_stats_out,
@@ -668,16 +684,13 @@ int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
                   bool log64 = false) {
   ctx->cur_fam = STSPIX_FAM_STATS;
   if (!stats_ready) {
-    LAUNCHB(kb_clear_stats, L.max_cap, L, nb, clear_all ? 1 : 0);
+    LAUNCHI(kb_clear_stats, 4LL * L.max_cap, L, nb, clear_all ? 1 : 0);
     LAUNCHG(kb_accumulate, acc_blocks(ctx, L, nb), 256, L.d, nb);
   }
   if (ctx->accumulator) accumulate_fp(ctx, st, L, nb, ctx->accumulator);
   ctx->cur_fam = STSPIX_FAM_POSTERIOR;
-  // groups of 32 ids, about four blocks per SM over the batch (a block loops over a slot's
-  // further groups)
-  const unsigned pg = (unsigned)std::min<long long>((L.max_cap + 31) / 32,
-                                                    std::max(32, (4 * ctx->num_sms + nb - 1) / nb));
-  LAUNCHG(kb_posterior, dim3(pg, (unsigned)nb), 128, L.d, incremental ? 1 : 0,
+  const unsigned pg = id_blocks(ctx, L.max_cap, 32, nb);     // groups of 32 ids
+  LAUNCHG(kb_posterior, dim3((unsigned)nb, pg), 128, L.d, incremental ? 1 : 0,
           log64 ? 1 : 0);
   return STSPIX_OK;
 }
@@ -792,7 +805,7 @@ int run_split(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmC
   ctx->cur_fam = STSPIX_FAM_SPLIT;
   LAUNCHS(kb_split_begin, L, nb);
   LAUNCHB(kb_split_clear, pix_units(L.max_npix), L, nb);
-  LAUNCHB(kb_split_seed, L.max_cap, L, nb, dir_b, dir_p);
+  LAUNCHI(kb_split_seed, L.max_cap, L, nb, dir_b, dir_p);
   LAUNCHG(kb_bbox, dim3(tiles64(L), (unsigned)nb), kThreads, L.d);
   LAUNCHG(kb_split_bfs, dim3(256, (unsigned)nb), 128, L.d, dir_b, dir_p);  // 1024 warps per slot
   {
@@ -803,12 +816,11 @@ int run_split(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmC
     prof_end(ctx, st, pe_, "kb_split_bfs_big");
   }
   LAUNCHB(kb_split_partition, pix_units(L.max_npix), L, nb);
-  LAUNCHB(kb_sm_clear, L.max_cap + 2, L, nb);
   LAUNCHG(kb_sm_accumulate, dim3(tiles64(L), (unsigned)nb), kThreads, L.d, 1);
-  LAUNCHG(kb_split_decide, dim3((unsigned)((L.max_cap + 31) / 32), (unsigned)nb), 128, L.d, K,
+  LAUNCHG(kb_split_decide, dim3((unsigned)nb, id_blocks(ctx, L.max_cap, 32, nb)), 128, L.d, K,
           cfg.split_alpha);
   LAUNCHG(kb_scan, (unsigned)nb, 1024, L.d, 1);
-  LAUNCHB(kb_split_commit, L.max_cap, L, nb);
+  LAUNCHI(kb_split_commit, L.max_cap, L, nb);
   LAUNCHB(kb_split_apply, pix_units(L.max_npix), L, nb);
   LAUNCHS(kb_split_end, L, nb);
   return STSPIX_OK;
@@ -818,17 +830,16 @@ int run_split(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmC
 int run_relabel(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
                 const stspix_config& cfg) {
   ctx->cur_fam = STSPIX_FAM_MERGE;
-  LAUNCHB(kb_relabel_init, L.max_cap + 2, L, nb);
+  LAUNCHI(kb_relabel_init, L.max_cap + 2, L, nb);
   LAUNCHG(kb_living, dim3(tiles64(L), (unsigned)nb), kThreads, L.d);
   dim3 g(blocks_for(L.max_cap),
          (unsigned)std::max(1, (L.max_nprev + kRelabelChunk - 1) / kRelabelChunk), (unsigned)nb);
   LAUNCHG(kb_relabel_compare, g, kThreads, L.d);
-  LAUNCHB(kb_relabel_mark, L.max_cap, L, nb, cfg.thresh_relabel, cfg.thresh_new);
+  LAUNCHI(kb_relabel_mark, L.max_cap, L, nb, cfg.thresh_relabel, cfg.thresh_new);
   LAUNCHG(kb_scan, (unsigned)nb, 1024, L.d, 2);
-  LAUNCHB(kb_relabel_ids, L.max_cap, L, nb);
-  LAUNCHB(kb_relabel_params, L.max_cap, L, nb);
+  LAUNCHI(kb_relabel_ids, L.max_cap, L, nb);
+  LAUNCHI(kb_relabel_params, L.max_cap, L, nb);
   LAUNCHB(kb_relabel_apply, pix_units(L.max_npix), L, nb);
-  LAUNCHB(kb_count_revived, L.max_cap, L, nb);
   LAUNCHS(kb_relabel_end, L, nb);
   return STSPIX_OK;
 }
@@ -836,15 +847,14 @@ int run_relabel(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
 int run_merge(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmConsts& K,
               const stspix_config& cfg, int dir_b, int dir_p, bool use_border) {
   ctx->cur_fam = STSPIX_FAM_MERGE;
-  LAUNCHB(kb_merge_clear, L.max_cap + 2, L, nb);
+  LAUNCHI(kb_merge_clear, L.max_cap + 2, L, nb);
   LAUNCHB(kb_merge_candidates, pix_units(L.max_npix), L, nb, dir_b, dir_p, use_border ? 1 : 0);
-  LAUNCHB(kb_sm_clear, L.max_cap + 2, L, nb);
   LAUNCHG(kb_sm_accumulate, dim3(tiles64(L), (unsigned)nb), kThreads, L.d, 0);
-  LAUNCHG(kb_merge_single, dim3((unsigned)((L.max_cap + 31) / 32), (unsigned)nb), 128, L.d, K);
-  LAUNCHG(kb_merge_decide, dim3((unsigned)((L.max_cap + 31) / 32), (unsigned)nb), 128, L.d, K,
+  LAUNCHG(kb_merge_single, dim3((unsigned)nb, id_blocks(ctx, L.max_cap, 32, nb)), 128, L.d, K);
+  LAUNCHG(kb_merge_decide, dim3((unsigned)nb, id_blocks(ctx, L.max_cap, 32, nb)), 128, L.d, K,
           cfg.merge_alpha);
-  LAUNCHB(kb_merge_flag, L.max_cap, L, nb);
-  LAUNCHB(kb_merge_remove, L.max_cap, L, nb);
+  LAUNCHI(kb_merge_flag, L.max_cap, L, nb);
+  LAUNCHI(kb_merge_remove, L.max_cap, L, nb);
   LAUNCHB(kb_merge_apply, pix_units(L.max_npix), L, nb);
   return STSPIX_OK;
 }
@@ -921,7 +931,7 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
   if ((r = params(L, L.B, fuse && maxn > 0 && nit[L.B - 1] > 0, maxn > 0, maxn == 0)))
     return r;
   ctx->cur_fam = STSPIX_FAM_POSTERIOR;
-  LAUNCHB(kb_store_sample, L.max_cap, L, L.B);
+  LAUNCHI(kb_store_sample, L.max_cap, L, L.B);
   return STSPIX_OK;
 }
 
@@ -935,19 +945,19 @@ int split_only(stspix_ctx* ctx, cudaStream_t st, const List& L, const stspix_con
   if ((r = run_split(ctx, st, L, L.B, K, cfg, dir, dir))) return r;
   if ((r = update_params(ctx, st, L, L.B))) return r;
   ctx->cur_fam = STSPIX_FAM_POSTERIOR;
-  LAUNCHB(kb_store_sample, L.max_cap, L, L.B);
+  LAUNCHI(kb_store_sample, L.max_cap, L, L.B);
   return STSPIX_OK;
 }
 
 // compactify_new_superpixels (compact_spix.cu:41-89) for ids >= lo, moving params.
 int compact(stspix_ctx* ctx, cudaStream_t st, const List& L) {
   ctx->cur_fam = STSPIX_FAM_OTHER;
-  LAUNCHB(kb_clear_flags, L.max_cap + 2, L, L.B);
+  LAUNCHI(kb_clear_flags, L.max_cap + 2, L, L.B);
   LAUNCHS(kb_scalars, L, L.B, (int)kOpCompactN);
   LAUNCHB(kb_mark_present, pix_units(L.max_npix), L, L.B, 1);
   LAUNCHG(kb_scan, (unsigned)L.B, 1024, L.d, 3);
-  LAUNCHB(kb_compact_gather, L.max_cap, L, L.B);
-  LAUNCHB(kb_compact_scatter, L.max_cap, L, L.B);
+  LAUNCHI(kb_compact_gather, L.max_cap, L, L.B);
+  LAUNCHI(kb_compact_scatter, L.max_cap, L, L.B);
   LAUNCHB(kb_remap, pix_units(L.max_npix), L, L.B, 1);
   LAUNCHS(kb_scalars, L, L.B, (int)kOpCompactEnd);
   return STSPIX_OK;
@@ -959,16 +969,16 @@ int bass_init(stspix_ctx* ctx, cudaStream_t st, const List& L, const stspix_conf
   ctx->cur_fam = STSPIX_FAM_OTHER;
   LAUNCHG(kb_init_hex, dim3(tiles64(L), (unsigned)L.B), kThreads, L.d);
   // compact the hex ids (extract_unique_ids + compactify, bass.cu:251-252)
-  LAUNCHB(kb_clear_flags, L.max_cap + 2, L, L.B);
+  LAUNCHI(kb_clear_flags, L.max_cap + 2, L, L.B);
   LAUNCHB(kb_mark_present, pix_units(L.max_npix), L, L.B, 0);
   LAUNCHG(kb_scan, (unsigned)L.B, 1024, L.d, 0);
   LAUNCHB(kb_remap, pix_units(L.max_npix), L, L.B, 0);
   LAUNCHS(kb_scalars, L, L.B, (int)kOpAfterHex);
-  LAUNCHB(kb_init_bass_params, L.max_cap, L, L.B);
-  LAUNCHB(kb_clear_stats, L.max_cap, L, L.B, 1);
+  LAUNCHI(kb_init_bass_params, L.max_cap, L, L.B);
+  LAUNCHI(kb_clear_stats, 4LL * L.max_cap, L, L.B, 1);
   LAUNCHG(kb_accumulate, acc_blocks(ctx, L, L.B), 256, L.d, L.B);
   if (ctx->accumulator) accumulate_fp(ctx, st, L, L.B, ctx->accumulator);
-  LAUNCHB(kb_init_prior_mu, L.max_cap, L, L.B);
+  LAUNCHI(kb_init_prior_mu, L.max_cap, L, L.B);
   if (cfg.sm_period == 1) LAUNCHB(kb_find_border, pix_units(L.max_npix), L, L.B);
   return STSPIX_OK;
 }
@@ -1135,7 +1145,7 @@ int shift_fill(stspix_ctx* ctx, cudaStream_t st, const List& L) {
 int prop_init(stspix_ctx* ctx, cudaStream_t st, const List& L) {
   if (L.B <= 0) return STSPIX_OK;
   ctx->cur_fam = STSPIX_FAM_OTHER;
-  LAUNCHB(kb_write_params, L.max_cap, L, L.B);
+  LAUNCHI(kb_write_params, L.max_cap, L, L.B);
   LAUNCHG(kb_mark_active, dim3(tiles64(L), (unsigned)L.B), kThreads, L.d);
   return STSPIX_OK;
 }
@@ -1192,7 +1202,7 @@ int batch_tail(stspix_ctx* ctx, cudaStream_t st, const List& Lp, const List& Ls,
   const SmConsts K = sm_constants(cfg);
   if ((r = bass_loop(ctx, st, Ls, nit_sorted, cfg, K, -1, 0))) return r;
   if ((r = compact(ctx, st, Ls))) return r;
-  LAUNCHB(kb_read_params, Ls.max_cap, Ls, Ls.B);
+  LAUNCHI(kb_read_params, Ls.max_cap, Ls, Ls.B);
   LAUNCHB(kb_save_prev, pix_units(Ls.max_npix), Ls, Ls.B);
   return STSPIX_OK;
 }
@@ -1406,7 +1416,7 @@ int run_batch(stspix_ctx* ctx, cudaStream_t st, std::vector<FrameDesc>& fr,
   }
   if (stop_after < 0) {
     if ((r = compact(ctx, st, Ls))) return r;
-    LAUNCHB(kb_read_params, Ls.max_cap, Ls, Ls.B);
+    LAUNCHI(kb_read_params, Ls.max_cap, Ls, Ls.B);
     LAUNCHB(kb_save_prev, pix_units(Ls.max_npix), Ls, Ls.B);
   }
   return finish();

@@ -61,6 +61,12 @@ __device__ __forceinline__ int spread_id(int j) {
 #define FOR_SP(k, n)                                                              \
   for (int j_ = threadIdx.x, k = spread_id(j_); k < (n); j_ += blockDim.x, k = spread_id(j_))
 
+// Light per-id kernels: the ids [lo, n) strided over the grid (see id_blocks).
+#define FOR_ID_FROM(k, lo, n)                                                      \
+  for (int k = (lo) + (int)(blockIdx.x * blockDim.x + threadIdx.x), k##_end = (n); \
+       k < k##_end; k += (int)(gridDim.x * blockDim.x))
+#define FOR_ID(k, n) FOR_ID_FROM(k, 0, n)
+
 // Per-superpixel working state, structure of arrays, `cap` entries each.
 struct SpDev {
   int cap;
@@ -175,6 +181,12 @@ struct Slot {
 enum { kOpBegin = 0, kOpAfterHex = 1, kOpCompactN = 2, kOpCompactEnd = 3 };
 
 #define SLOT_Y const Slot& S = slots[blockIdx.y]
+// The slot as the fast grid dimension, for kernels whose few busy blocks of each slot come
+// first and are long: they then start first and spread over the SMs (with the slot as the
+// slow one and a multiple of the SM count per slot, every slot's land on the same SMs: a
+// split decision over 8 frames of 480x854 took 47 us so, 18 this way).  The slots are rotated
+// from row to row, so the blocks of one large slot among many spread too.
+#define SLOT_X const Slot& S = slots[(blockIdx.x + blockIdx.y) % gridDim.x]
 // Light per-pixel kernels: thread i of block b takes the pixels
 // kPixPerThread * blockDim.x * b + i + blockDim.x * j (j < kPixPerThread), coalesced, so
 // a launch has a quarter of the blocks of one pixel per thread (block scheduling and the

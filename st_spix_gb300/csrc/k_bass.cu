@@ -202,25 +202,25 @@ __global__ void kb_compact_gather(const Slot* __restrict__ slots) {
   const uint8_t* flags = S.flags;
   const int* excl = S.excl;
   const int lo = S.lo;
-  int v = lo + blockIdx.x * blockDim.x + threadIdx.x;
-  if (v > S.sc->max_spix || v >= sp.cap) return;
-  if (!flags[v - lo]) return;
-  int j = excl[v - lo];
-  for (int c = 0; c < 3; c++) {
-    tmp.mu_app[3 * j + c] = sp.mu_app[3 * v + c];
-    tmp.prior_mu_app[3 * j + c] = sp.prior_mu_app[3 * v + c];
-    tmp.sigma_shape[3 * j + c] = sp.sigma_shape[3 * v + c];
-    tmp.prior_sigma_shape[3 * j + c] = sp.prior_sigma_shape[3 * v + c];
-    tmp.sample_sigma_shape[3 * j + c] = sp.sample_sigma_shape[3 * v + c];
+  FOR_ID_FROM(v, lo, min(S.sc->max_spix + 1, sp.cap)) {
+    if (!flags[v - lo]) continue;
+    int j = excl[v - lo];
+    for (int c = 0; c < 3; c++) {
+      tmp.mu_app[3 * j + c] = sp.mu_app[3 * v + c];
+      tmp.prior_mu_app[3 * j + c] = sp.prior_mu_app[3 * v + c];
+      tmp.sigma_shape[3 * j + c] = sp.sigma_shape[3 * v + c];
+      tmp.prior_sigma_shape[3 * j + c] = sp.prior_sigma_shape[3 * v + c];
+      tmp.sample_sigma_shape[3 * j + c] = sp.sample_sigma_shape[3 * v + c];
+    }
+    for (int c = 0; c < 2; c++) {
+      tmp.mu_shape[2 * j + c] = sp.mu_shape[2 * v + c];
+      tmp.prior_mu_shape[2 * j + c] = sp.prior_mu_shape[2 * v + c];
+    }
+    tmp.logdet[j] = sp.logdet[v];
+    tmp.count[j] = sp.count[v];
+    tmp.prior_count[j] = sp.prior_count[v];
+    tmp.valid[j] = sp.valid[v];
   }
-  for (int c = 0; c < 2; c++) {
-    tmp.mu_shape[2 * j + c] = sp.mu_shape[2 * v + c];
-    tmp.prior_mu_shape[2 * j + c] = sp.prior_mu_shape[2 * v + c];
-  }
-  tmp.logdet[j] = sp.logdet[v];
-  tmp.count[j] = sp.count[v];
-  tmp.prior_count[j] = sp.prior_count[v];
-  tmp.valid[j] = sp.valid[v];
 }
 
 // fill_old_params_from_new (compact_spix.cu:268-290).
@@ -230,25 +230,24 @@ __global__ void kb_compact_scatter(const Slot* __restrict__ slots) {
   const SpDev& sp = S.sp;
   const SpDev& tmp = S.tmp;
   const int lo = S.lo;
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= S.sc->tmp1) return;
-  int d = lo + j;
-  if (d >= sp.cap) return;
-  for (int c = 0; c < 3; c++) {
-    sp.mu_app[3 * d + c] = tmp.mu_app[3 * j + c];
-    sp.prior_mu_app[3 * d + c] = tmp.prior_mu_app[3 * j + c];
-    sp.sigma_shape[3 * d + c] = tmp.sigma_shape[3 * j + c];
-    sp.prior_sigma_shape[3 * d + c] = tmp.prior_sigma_shape[3 * j + c];
-    sp.sample_sigma_shape[3 * d + c] = tmp.sample_sigma_shape[3 * j + c];
+  FOR_ID(j, min(S.sc->tmp1, sp.cap - lo)) {
+    int d = lo + j;
+    for (int c = 0; c < 3; c++) {
+      sp.mu_app[3 * d + c] = tmp.mu_app[3 * j + c];
+      sp.prior_mu_app[3 * d + c] = tmp.prior_mu_app[3 * j + c];
+      sp.sigma_shape[3 * d + c] = tmp.sigma_shape[3 * j + c];
+      sp.prior_sigma_shape[3 * d + c] = tmp.prior_sigma_shape[3 * j + c];
+      sp.sample_sigma_shape[3 * d + c] = tmp.sample_sigma_shape[3 * j + c];
+    }
+    for (int c = 0; c < 2; c++) {
+      sp.mu_shape[2 * d + c] = tmp.mu_shape[2 * j + c];
+      sp.prior_mu_shape[2 * d + c] = tmp.prior_mu_shape[2 * j + c];
+    }
+    sp.logdet[d] = tmp.logdet[j];
+    sp.count[d] = tmp.count[j];
+    sp.prior_count[d] = tmp.prior_count[j];
+    sp.valid[d] = tmp.valid[j];
   }
-  for (int c = 0; c < 2; c++) {
-    sp.mu_shape[2 * d + c] = tmp.mu_shape[2 * j + c];
-    sp.prior_mu_shape[2 * d + c] = tmp.prior_mu_shape[2 * j + c];
-  }
-  sp.logdet[d] = tmp.logdet[j];
-  sp.count[d] = tmp.count[j];
-  sp.prior_count[d] = tmp.prior_count[j];
-  sp.valid[d] = tmp.valid[j];
 }
 
 // ---------------------------------------------------------------------------
@@ -261,26 +260,26 @@ __global__ void kb_init_bass_params(const Slot* __restrict__ slots) {
   const int sp_size = S.sp_size;
   const SpDev& sp = S.sp;
   const int npix = S.npix;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= sp.cap) return;
-  int nspix = S.sc->nspix;
-  int count = (int)(npix / (1. * nspix));
-  sp.prior_sigma_shape[3 * k] = 1.0 / sp_size;
-  sp.prior_sigma_shape[3 * k + 1] = 0.;
-  sp.prior_sigma_shape[3 * k + 2] = 1.0 / sp_size;
-  sp.prior_icov[3 * k] = 1; sp.prior_icov[3 * k + 1] = 0; sp.prior_icov[3 * k + 2] = 1;
-  sp.prop[k] = 0;
-  sp.icount[k] = 0.f;
-  sp.sm_count[k] = 0;
-  for (int c = 0; c < 3; c++) {
-    sp.mu_app[3 * k + c] = 0.f; sp.prior_mu_app[3 * k + c] = 0.f;
-    sp.sigma_shape[3 * k + c] = 0.0; sp.sample_sigma_shape[3 * k + c] = 0.0;
+  FOR_ID(k, sp.cap) {
+    int nspix = S.sc->nspix;
+    int count = (int)(npix / (1. * nspix));
+    sp.prior_sigma_shape[3 * k] = 1.0 / sp_size;
+    sp.prior_sigma_shape[3 * k + 1] = 0.;
+    sp.prior_sigma_shape[3 * k + 2] = 1.0 / sp_size;
+    sp.prior_icov[3 * k] = 1; sp.prior_icov[3 * k + 1] = 0; sp.prior_icov[3 * k + 2] = 1;
+    sp.prop[k] = 0;
+    sp.icount[k] = 0.f;
+    sp.sm_count[k] = 0;
+    for (int c = 0; c < 3; c++) {
+      sp.mu_app[3 * k + c] = 0.f; sp.prior_mu_app[3 * k + c] = 0.f;
+      sp.sigma_shape[3 * k + c] = 0.0; sp.sample_sigma_shape[3 * k + c] = 0.0;
+    }
+    for (int c = 0; c < 2; c++) { sp.mu_shape[2 * k + c] = 0.0; sp.prior_mu_shape[2 * k + c] = 0.0; }
+    sp.logdet[k] = 0.0;
+    sp.count[k] = 0;
+    if (k < nspix) { sp.valid[k] = 1; sp.prior_count[k] = (float)count; }
+    else { sp.valid[k] = 0; sp.prior_count[k] = 0.f; }
   }
-  for (int c = 0; c < 2; c++) { sp.mu_shape[2 * k + c] = 0.0; sp.prior_mu_shape[2 * k + c] = 0.0; }
-  sp.logdet[k] = 0.0;
-  sp.count[k] = 0;
-  if (k < nspix) { sp.valid[k] = 1; sp.prior_count[k] = (float)count; }
-  else { sp.valid[k] = 0; sp.prior_count[k] = 0.f; }
 }
 
 // prior_mu_app := initial mean (calc_summ_stats, update_params.cu:142-203).
@@ -289,13 +288,13 @@ __global__ void kb_init_prior_mu(const Slot* __restrict__ slots) {
   SLOT_Y;
   if (S.mode) return;
   const SpDev& sp = S.sp;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= S.sc->nspix || k >= sp.cap) return;
-  int n = sp.count[k];
-  double c = n;
-  for (int ch = 0; ch < 3; ch++)
-    sp.prior_mu_app[3 * k + ch] =
-        n > 0 ? (float)(fx_unq(sp.acc[8 * k + ch], kFxAppShift) / c) : 0.f;
+  FOR_ID(k, min(S.sc->nspix, sp.cap)) {
+    int n = sp.count[k];
+    double c = n;
+    for (int ch = 0; ch < 3; ch++)
+      sp.prior_mu_app[3 * k + ch] =
+          n > 0 ? (float)(fx_unq(sp.acc[8 * k + ch], kFxAppShift) / c) : 0.f;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -541,11 +540,11 @@ __device__ __forceinline__ void smooth_prior(double in_x, double in_y, double in
 // the changed ids built by a kernel of its own a posterior took 10.5 us on a 240x320 frame,
 // 13.4 on 720x1280 and 17.1 on 8 frames of 480x854; without it, but with a division per
 // quotient and the log in FP64, 5.7, 7.6 and 11.6 (and 32.4 on 16 frames of mixed sizes);
-// now 5.0, 6.5, 9.4 (and 23.3).
+// now 5.0, 6.5, 7.9 (and 17.9; the last step the spread of the groups, see SLOT_X).
 __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slots,
                                                     int incremental, int log64) {
   pdl_enter();
-  SLOT_Y;
+  SLOT_X;
   __shared__ double v_ps[3][32], v_den[3][32], v_m[2][32], v_s[3][32], v_ld[32];
   __shared__ float v_i[3][32];
   __shared__ int v_pos[2][32];
@@ -557,7 +556,7 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
   // the sums and the covariance entry (xx, xy, yy) of a warp
   const int f0 = w == 0 ? 0 : w == 1 ? 3 : 4;
   const int f1 = w == 0 ? 6 : w == 1 ? 5 : 7, ent = w == 0 ? 1 : w == 1 ? 0 : 2;
-  for (int g = blockIdx.x;; g += gridDim.x) {
+  for (int g = blockIdx.y;; g += gridDim.y) {
     const int k = 32 * g + lane;
     int count_int = 0;
     uint8_t valid = 0, prop = 0;
@@ -730,12 +729,10 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
 __global__ void kb_clear_stats(const Slot* __restrict__ slots, int all) {
   pdl_enter();
   SLOT_Y;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= (all ? S.sp.cap : live_ids(S))) return;
-  S.sp.count[k] = 0;
-  long long* a = S.sp.acc + 8 * (size_t)k;
-#pragma unroll
-  for (int c = 0; c < 8; c++) a[c] = 0;
+  const int n = all ? S.sp.cap : live_ids(S);
+  ulonglong2* acc = (ulonglong2*)S.sp.acc;           // 8 sums, 64 bytes, per id
+  FOR_ID(k, n) S.sp.count[k] = 0;
+  FOR_ID(q, 4 * n) acc[q] = make_ulonglong2(0, 0);
 }
 
 // store_sample_sigma_shape_k (update_params.cu:397-438).
@@ -1644,30 +1641,30 @@ __global__ void kb_read_params(const Slot* __restrict__ slots) {
   SLOT_Y;
   const SpDev& sp = S.sp;
   const stspix_params& out = S.pout;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
   int n = S.sc->nspix;
-  if (i >= n || i >= out.capacity || i >= sp.cap) return;
-  bool upd = sp.count[i] > 0;
-  for (int c = 0; c < 3; c++) {
-    float m = sp.mu_app[3 * i + c];
-    out.mu_app[3 * i + c] = m;
-    out.prior_mu_app[3 * i + c] = upd ? m : sp.prior_mu_app[3 * i + c];
-    double s = sp.sigma_shape[3 * i + c];
-    out.sigma_shape[3 * i + c] = s;
-    out.prior_sigma_shape[3 * i + c] = upd ? s : sp.prior_sigma_shape[3 * i + c];
-    out.sample_sigma_shape[3 * i + c] = sp.sample_sigma_shape[3 * i + c];
+  FOR_ID(i, min(n, min(out.capacity, sp.cap))) {
+    bool upd = sp.count[i] > 0;
+    for (int c = 0; c < 3; c++) {
+      float m = sp.mu_app[3 * i + c];
+      out.mu_app[3 * i + c] = m;
+      out.prior_mu_app[3 * i + c] = upd ? m : sp.prior_mu_app[3 * i + c];
+      double s = sp.sigma_shape[3 * i + c];
+      out.sigma_shape[3 * i + c] = s;
+      out.prior_sigma_shape[3 * i + c] = upd ? s : sp.prior_sigma_shape[3 * i + c];
+      out.sample_sigma_shape[3 * i + c] = sp.sample_sigma_shape[3 * i + c];
+    }
+    for (int c = 0; c < 2; c++) {
+      double m = sp.mu_shape[2 * i + c];
+      out.mu_shape[2 * i + c] = m;
+      out.prior_mu_shape[2 * i + c] = upd ? m : sp.prior_mu_shape[2 * i + c];
+    }
+    out.logdet_sigma_shape[i] = (float)sp.logdet[i];
+    out.counts[i] = sp.count[i];
+    out.invalid_counts[i] = sp.icount[i];
+    out.sm_counts[i] = sp.sm_count[i];
+    out.prior_counts[i] = sp.prior_count[i];
+    out.ids[i] = i;
   }
-  for (int c = 0; c < 2; c++) {
-    double m = sp.mu_shape[2 * i + c];
-    out.mu_shape[2 * i + c] = m;
-    out.prior_mu_shape[2 * i + c] = upd ? m : sp.prior_mu_shape[2 * i + c];
-  }
-  out.logdet_sigma_shape[i] = (float)sp.logdet[i];
-  out.counts[i] = sp.count[i];
-  out.invalid_counts[i] = sp.icount[i];
-  out.sm_counts[i] = sp.sm_count[i];
-  out.prior_counts[i] = sp.prior_count[i];
-  out.ids[i] = i;
 }
 
 // Per-slot scalar steps, one thread per slot.
@@ -1704,8 +1701,7 @@ __global__ void kb_scalars(const Slot* __restrict__ slots, int B, int op) {
 __global__ void kb_clear_flags(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < S.cap + 2) S.flags[k] = 0;
+  FOR_ID(k, S.cap + 2) S.flags[k] = 0;
 }
 
 // Keep a copy of the finished labels where the slot's video stream resides.

@@ -627,46 +627,46 @@ __global__ void kb_write_params(const Slot* __restrict__ slots) {
   const SpDev& sp = S.sp;
   const stspix_params& pp = S.pprev;
   const int n = S.n_prev, sp_size = S.sp_size;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= sp.cap) return;
-  if (i < n) {
-    for (int c = 0; c < 3; c++) {
-      sp.mu_app[3 * i + c] = pp.mu_app[3 * i + c];
-      sp.prior_mu_app[3 * i + c] = pp.prior_mu_app[3 * i + c];
-      sp.sigma_shape[3 * i + c] = pp.sigma_shape[3 * i + c];
-      sp.prior_sigma_shape[3 * i + c] = pp.prior_sigma_shape[3 * i + c];
-      sp.sample_sigma_shape[3 * i + c] = pp.sample_sigma_shape[3 * i + c];
+  FOR_ID(i, sp.cap) {
+    if (i < n) {
+      for (int c = 0; c < 3; c++) {
+        sp.mu_app[3 * i + c] = pp.mu_app[3 * i + c];
+        sp.prior_mu_app[3 * i + c] = pp.prior_mu_app[3 * i + c];
+        sp.sigma_shape[3 * i + c] = pp.sigma_shape[3 * i + c];
+        sp.prior_sigma_shape[3 * i + c] = pp.prior_sigma_shape[3 * i + c];
+        sp.sample_sigma_shape[3 * i + c] = pp.sample_sigma_shape[3 * i + c];
+      }
+      for (int c = 0; c < 2; c++) {
+        sp.mu_shape[2 * i + c] = pp.mu_shape[2 * i + c];
+        sp.prior_mu_shape[2 * i + c] = pp.prior_mu_shape[2 * i + c];
+      }
+      sp.logdet[i] = pp.logdet_sigma_shape[i];
+      double px = pp.prior_sigma_shape[3 * i], py = pp.prior_sigma_shape[3 * i + 1],
+             pz = pp.prior_sigma_shape[3 * i + 2];
+      double pr_det = px * pz - py * py;
+      sp.prior_icov[3 * i] = pz / pr_det;
+      sp.prior_icov[3 * i + 1] = py / pr_det;
+      sp.prior_icov[3 * i + 2] = px / pr_det;
+      sp.count[i] = pp.counts[i];
+      sp.icount[i] = pp.invalid_counts[i];
+      sp.sm_count[i] = pp.sm_counts[i];
+      sp.prior_count[i] = pp.prior_counts[i];
+    } else {
+      for (int c = 0; c < 3; c++) {
+        sp.mu_app[3 * i + c] = 0.f; sp.prior_mu_app[3 * i + c] = 0.f;
+        sp.sigma_shape[3 * i + c] = 0.0; sp.sample_sigma_shape[3 * i + c] = 0.0;
+        sp.prior_icov[3 * i + c] = 0.0;
+      }
+      sp.prior_sigma_shape[3 * i] = 1.0 / sp_size;
+      sp.prior_sigma_shape[3 * i + 1] = 0;
+      sp.prior_sigma_shape[3 * i + 2] = 1.0 / sp_size;
+      for (int c = 0; c < 2; c++) { sp.mu_shape[2 * i + c] = 0.0; sp.prior_mu_shape[2 * i + c] = 0.0; }
+      sp.logdet[i] = 0.0;
+      sp.count[i] = 0; sp.icount[i] = 0.f; sp.sm_count[i] = 0; sp.prior_count[i] = 0.f;
     }
-    for (int c = 0; c < 2; c++) {
-      sp.mu_shape[2 * i + c] = pp.mu_shape[2 * i + c];
-      sp.prior_mu_shape[2 * i + c] = pp.prior_mu_shape[2 * i + c];
-    }
-    sp.logdet[i] = pp.logdet_sigma_shape[i];
-    double px = pp.prior_sigma_shape[3 * i], py = pp.prior_sigma_shape[3 * i + 1],
-           pz = pp.prior_sigma_shape[3 * i + 2];
-    double pr_det = px * pz - py * py;
-    sp.prior_icov[3 * i] = pz / pr_det;
-    sp.prior_icov[3 * i + 1] = py / pr_det;
-    sp.prior_icov[3 * i + 2] = px / pr_det;
-    sp.count[i] = pp.counts[i];
-    sp.icount[i] = pp.invalid_counts[i];
-    sp.sm_count[i] = pp.sm_counts[i];
-    sp.prior_count[i] = pp.prior_counts[i];
-  } else {
-    for (int c = 0; c < 3; c++) {
-      sp.mu_app[3 * i + c] = 0.f; sp.prior_mu_app[3 * i + c] = 0.f;
-      sp.sigma_shape[3 * i + c] = 0.0; sp.sample_sigma_shape[3 * i + c] = 0.0;
-      sp.prior_icov[3 * i + c] = 0.0;
-    }
-    sp.prior_sigma_shape[3 * i] = 1.0 / sp_size;
-    sp.prior_sigma_shape[3 * i + 1] = 0;
-    sp.prior_sigma_shape[3 * i + 2] = 1.0 / sp_size;
-    for (int c = 0; c < 2; c++) { sp.mu_shape[2 * i + c] = 0.0; sp.prior_mu_shape[2 * i + c] = 0.0; }
-    sp.logdet[i] = 0.0;
-    sp.count[i] = 0; sp.icount[i] = 0.f; sp.sm_count[i] = 0; sp.prior_count[i] = 0.f;
+    sp.valid[i] = 0;
+    sp.prop[i] = 0;
   }
-  sp.valid[i] = 0;
-  sp.prop[i] = 0;
 }
 
 __global__ void kb_mark_active(const Slot* __restrict__ slots) {
@@ -703,13 +703,13 @@ __global__ void kb_relabel_init(const Slot* __restrict__ slots) {
   if (!S.mode) return;
   // (a minted id is at most 2 max_spix + 1)
   const int n_ids = live_ids(S);
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= min(S.cap, 2 * n_ids)) return;
-  S.src_of[s] = -1;
-  if (s >= n_ids) return;
-  S.living[s] = 0;
-  S.rbest[s] = ((unsigned long long)__float_as_uint(10000.f) << 32) | 0x7fffffffull;
-  S.ss[s] = 0.f;
+  FOR_ID(s, min(S.cap, 2 * n_ids)) {
+    S.src_of[s] = -1;
+    if (s >= n_ids) continue;
+    S.living[s] = 0;
+    S.rbest[s] = ((unsigned long long)__float_as_uint(10000.f) << 32) | 0x7fffffffull;
+    S.ss[s] = 0.f;
+  }
 }
 
 __global__ void kb_living(const Slot* __restrict__ slots) {
@@ -786,24 +786,26 @@ __global__ void kb_relabel_mark(const Slot* __restrict__ slots, float thresh_rep
   SLOT_Y;
   if (!S.mode) return;
   const int cap = S.cap;
-  const Scalars* __restrict__ sc = S.sc;
+  Scalars* sc = S.sc;
   const uint8_t* __restrict__ living = S.living;
   const unsigned long long* __restrict__ best = S.rbest;
   const float* __restrict__ ss = S.ss;
   int* __restrict__ rid = S.rid;
   uint8_t* __restrict__ mint = S.mint;
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int nspix = sc->max_spix + 1;
-  if (s >= min(cap, nspix)) return;
-  mint[s] = 0;
-  rid[s] = -1;
-  if (!living[s]) return;
-  unsigned long long b = best[s];
-  float delta = __uint_as_float((unsigned)(b >> 32));
-  int c = (int)(unsigned)(b & 0xffffffffull);
-  bool revive = (delta < thresh_replace) && (c < nspix) && (c != s);
-  if (revive) rid[s] = c;
-  else if (ss[s] > thresh_new) mint[s] = 1;
+  FOR_ID(s, min(cap, nspix)) {
+    mint[s] = 0;
+    rid[s] = -1;
+    if (!living[s]) continue;
+    unsigned long long b = best[s];
+    float delta = __uint_as_float((unsigned)(b >> 32));
+    int c = (int)(unsigned)(b & 0xffffffffull);
+    bool revive = (delta < thresh_replace) && (c < nspix) && (c != s);
+    if (revive) {
+      rid[s] = c;
+      atomicAdd(&sc->nrevived, 1);
+    } else if (ss[s] > thresh_new) mint[s] = 1;
+  }
 }
 
 __global__ void kb_relabel_ids(const Slot* __restrict__ slots) {
@@ -816,12 +818,12 @@ __global__ void kb_relabel_ids(const Slot* __restrict__ slots) {
   const int* __restrict__ excl = S.excl;
   int* __restrict__ rid = S.rid;
   int* __restrict__ src_of = S.src_of;
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= live_ids(S)) return;
-  if (mint[s]) rid[s] = sc->max_spix + 1 + excl[s];
-  int n = rid[s];
-  if (n >= 0 && n < cap) atomicMax(&src_of[n], s);
-  else if (n >= cap) atomicExch(&sc->status, STSPIX_ERR_CAPACITY);
+  FOR_ID(s, live_ids(S)) {
+    if (mint[s]) rid[s] = sc->max_spix + 1 + excl[s];
+    int n = rid[s];
+    if (n >= 0 && n < cap) atomicMax(&src_of[n], s);
+    else if (n >= cap) atomicExch(&sc->status, STSPIX_ERR_CAPACITY);
+  }
 }
 
 // relabel_spix_kernel parameter copies (relabel.cu:86-120), from the largest
@@ -834,23 +836,23 @@ __global__ void kb_relabel_params(const Slot* __restrict__ slots) {
   const int* __restrict__ rid = S.rid;
   const int* __restrict__ src_of = S.src_of;
   const int n_prev = S.n_prev;
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= live_ids(S)) return;
-  int n = rid[s];
-  if (n < 0 || n >= sp.cap) return;
-  sp.valid[s] = 0;
-  if (src_of[n] != s) return;
-  sp.count[n] = sp.count[s];
-  sp.icount[n] = sp.icount[s];
-  sp.valid[n] = 1;
-  if (n >= n_prev) {
-    sp.prop[n] = 0;
-    sp.prior_count[n] = sp.prior_count[s];
-    for (int c = 0; c < 3; c++) {
-      sp.prior_sigma_shape[3 * n + c] = sp.prior_sigma_shape[3 * s + c];
-      sp.sample_sigma_shape[3 * n + c] = sp.sample_sigma_shape[3 * s + c];
-      sp.prior_mu_app[3 * n + c] = sp.prior_mu_app[3 * s + c];
-      sp.prior_icov[3 * n + c] = sp.prior_icov[3 * s + c];
+  FOR_ID(s, live_ids(S)) {
+    int n = rid[s];
+    if (n < 0 || n >= sp.cap) continue;
+    sp.valid[s] = 0;
+    if (src_of[n] != s) continue;
+    sp.count[n] = sp.count[s];
+    sp.icount[n] = sp.icount[s];
+    sp.valid[n] = 1;
+    if (n >= n_prev) {
+      sp.prop[n] = 0;
+      sp.prior_count[n] = sp.prior_count[s];
+      for (int c = 0; c < 3; c++) {
+        sp.prior_sigma_shape[3 * n + c] = sp.prior_sigma_shape[3 * s + c];
+        sp.sample_sigma_shape[3 * n + c] = sp.sample_sigma_shape[3 * s + c];
+        sp.prior_mu_app[3 * n + c] = sp.prior_mu_app[3 * s + c];
+        sp.prior_icov[3 * n + c] = sp.prior_icov[3 * s + c];
+      }
     }
   }
 }
@@ -881,13 +883,5 @@ __global__ void kb_relabel_end(const Slot* __restrict__ slots, int B) {
   sc->max_spix += m;
 }
 
-__global__ void kb_count_revived(const Slot* __restrict__ slots) {
-  pdl_enter();
-  SLOT_Y;
-  if (!S.mode) return;
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= live_ids(S)) return;
-  if (S.rid[s] >= 0 && !S.mint[s]) atomicAdd(&S.sc->nrevived, 1);
-}
 
 }  // namespace stspix

@@ -10,7 +10,6 @@
 
 namespace stspix {
 
-
 // ---------------------------------------------------------------------------
 // Split seeds (init_split, split_merge.cu:803-844): seed s (0, 1) of superpixel k is
 // the pixel one step from its mean position along +direction (s = 0) or -direction
@@ -25,19 +24,35 @@ __device__ __forceinline__ int split_seed_index(const Slot& S, int k, int s, int
   return S.seg[ind] == k ? (int)ind : -1;
 }
 
+// The split/merge sums cover the ids in use and their second halves (a split gives the
+// second half of id k the label k + max_spix + 1); the first per-id kernel of a step clears
+// them.
+__device__ __forceinline__ int sm_ids(const Slot& S) {
+  return min(S.cap + 2, 2 * (S.sc->max_spix + 1));
+}
+__device__ __forceinline__ void sm_clear(const SmDev& sm, int k) {
+  sm.count[k] = 0;
+  sm.ninvalid[k] = 0;
+#pragma unroll
+  for (int c = 0; c < 3; c++) { sm.s[3 * (size_t)k + c] = 0; sm.sq[3 * (size_t)k + c] = 0; }
+}
+
 __global__ void kb_split_seed(const Slot* __restrict__ slots, int dir_bass, int dir_prop) {
   pdl_enter();
   SLOT_Y;
   const SpDev& sp = S.sp;
   const int direction = S.mode ? dir_prop : dir_bass;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= live_ids(S)) return;
-  int* bb = S.bbox + 4 * (size_t)k;
-  bb[0] = INT32_MAX; bb[1] = -1; bb[2] = INT32_MAX; bb[3] = -1;
-  if (!S.sc->tmp0 /*split_on*/ || !sp.valid[k]) return;
-  for (int s = 0; s < 2; s++) {
-    const int ind = split_seed_index(S, k, s, direction);
-    if (ind >= 0) (s == 0 ? S.d1 : S.d2)[ind] = 1;
+  const int n_ids = live_ids(S);
+  FOR_ID(k, sm_ids(S)) {
+    sm_clear(S.sm, k);
+    if (k >= n_ids) continue;
+    int* bb = S.bbox + 4 * (size_t)k;
+    bb[0] = INT32_MAX; bb[1] = -1; bb[2] = INT32_MAX; bb[3] = -1;
+    if (!S.sc->tmp0 /*split_on*/ || !sp.valid[k]) continue;
+    for (int s = 0; s < 2; s++) {
+      const int ind = split_seed_index(S, k, s, direction);
+      if (ind >= 0) (s == 0 ? S.d1 : S.d2)[ind] = 1;
+    }
   }
 }
 
@@ -439,20 +454,6 @@ __global__ void kb_split_partition(const Slot* __restrict__ slots) {
   }
 }
 
-// Clear the split/merge sums of the ids in use and of their second halves (a split gives
-// the second half of id k the label k + max_spix + 1).
-__global__ void kb_sm_clear(const Slot* __restrict__ slots) {
-  pdl_enter();
-  SLOT_Y;
-  const SmDev& sm = S.sm;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= min(S.cap + 2, 2 * (S.sc->max_spix + 1))) return;
-  sm.count[k] = 0;
-  sm.ninvalid[k] = 0;
-#pragma unroll
-  for (int c = 0; c < 3; c++) { sm.s[3 * (size_t)k + c] = 0; sm.sq[3 * (size_t)k + c] = 0; }
-}
-
 // sum_by_label over split/merge labels (split_merge.cu:862-891,
 // split_merge_prop.cu:1942-2018): count, colour sums, square sums, invalid count.
 // split: labels = split labels, invalid counts against the shifted labels (prop
@@ -595,72 +596,73 @@ __device__ __forceinline__ bool near_tie(double h) { return fabs(h + 2.0) < 1e-6
 __global__ void __launch_bounds__(128) kb_split_decide(const Slot* __restrict__ slots, SmConsts K,
                                                        float split_alpha) {
   pdl_enter();
-  SLOT_Y;
+  SLOT_X;
   const SpDev& sp = S.sp;
   const SmDev& sm = S.sm;
   Scalars* sc = S.sc;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int k = blockIdx.x * 32 + lane;
   const int n_ids = live_ids(S);
-  if ((int)blockIdx.x * 32 >= n_ids) return;              // block-uniform
   __shared__ double t_lr[3][3][32], t_log[3][32];
-  // the preconditions, evaluated alike by every warp
-  bool ok = false;
-  int s = 0;
-  double cnt[3] = {0, 0, 0};                                // k's half, s's half, whole
-  if (k < n_ids) {
-    if (w == 0) S.accept[k] = 0;
-    if (sc->tmp0 && sp.valid[k]) {
-      s = k + sc->tmp1;
-      if (s < sc->nbuf_logical && s < sp.cap + 2) {
-        cnt[2] = sp.count[k];
-        cnt[0] = sm.count[k];
-        cnt[1] = sm.count[s];
-        ok = cnt[2] >= 1 && cnt[0] >= 1 && cnt[1] >= 1 && cnt[2] == cnt[0] + cnt[1];
+  for (int g = blockIdx.y; 32 * g < n_ids; g += gridDim.y) {  // the same for the block
+    const int k = 32 * g + lane;
+    // the preconditions, evaluated alike by every warp
+    bool ok = false;
+    int s = 0;
+    double cnt[3] = {0, 0, 0};                                // k's half, s's half, whole
+    if (k < n_ids) {
+      if (w == 0) S.accept[k] = 0;
+      if (sc->tmp0 && sp.valid[k]) {
+        s = k + sc->tmp1;
+        if (s < sc->nbuf_logical && s < sp.cap + 2) {
+          cnt[2] = sp.count[k];
+          cnt[0] = sm.count[k];
+          cnt[1] = sm.count[s];
+          ok = cnt[2] >= 1 && cnt[0] >= 1 && cnt[1] >= 1 && cnt[2] == cnt[0] + cnt[1];
+        }
       }
     }
-  }
-  if (!__syncthreads_or(ok)) return;
-  if (ok) {
-    if (w < 3) {
+    if (!__syncthreads_or(ok)) continue;              // block-uniform
+    if (ok) {
+      if (w < 3) {
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        long long sv, qv;
-        if (w == 0) { sv = sm.s[3 * (size_t)k + c]; qv = sm.sq[3 * (size_t)k + c]; }
-        else if (w == 1) { sv = sm.s[3 * (size_t)s + c]; qv = sm.sq[3 * (size_t)s + c]; }
-        else { sv = sp.acc[8 * (size_t)k + c]; qv = sm.sq[3 * (size_t)k + c] + sm.sq[3 * (size_t)s + c]; }
-        const double nm = w == 0 ? cnt[0] : (w == 1 ? cnt[1] : cnt[2]);
-        t_lr[w][c][lane] = marginal_lr(nm, K, sv, qv, false);
+        for (int c = 0; c < 3; c++) {
+          long long sv, qv;
+          if (w == 0) { sv = sm.s[3 * (size_t)k + c]; qv = sm.sq[3 * (size_t)k + c]; }
+          else if (w == 1) { sv = sm.s[3 * (size_t)s + c]; qv = sm.sq[3 * (size_t)s + c]; }
+          else { sv = sp.acc[8 * (size_t)k + c]; qv = sm.sq[3 * (size_t)k + c] + sm.sq[3 * (size_t)s + c]; }
+          const double nm = w == 0 ? cnt[0] : (w == 1 ? cnt[1] : cnt[2]);
+          t_lr[w][c][lane] = marginal_lr(nm, K, sv, qv, false);
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < 3; m++) t_log[m][lane] = log(cnt[m]);
       }
-    } else {
-#pragma unroll
-      for (int m = 0; m < 3; m++) t_log[m][lane] = log(cnt[m]);
     }
-  }
-  __syncthreads();
-  if (w != 0 || !ok) return;
-  double mm[3];
+    __syncthreads();
+    if (w != 0 || !ok) continue;
+    double mm[3];
 #pragma unroll
-  for (int m = 0; m < 3; m++)
-    mm[m] = marginal_sum(cnt[m], K, t_lr[m][0][lane], t_lr[m][1][lane], t_lr[m][2][lane],
-                         t_log[m][lane]);
-  const double count_k = cnt[0], count_s = cnt[1];
-  double h = mm[0] + mm[1] - mm[2] + split_alpha;
-  uint8_t fl = 1;
-  if (S.mode) {
-    bool is_prop = sp.prop[k];
-    int ninv_k = sm.ninvalid[k], ninv_s = sm.ninvalid[s];
-    bool prop_k = (ninv_k <= ninv_s);
-    float iperc_k = (float)(ninv_k / (1.0 * count_k));
-    float iperc_s = (float)(ninv_k / (1.0 * count_s));  // reference uses ninvalid_k here
-    float iperc = prop_k ? iperc_k : iperc_s;
-    iperc = is_prop ? iperc : 1.0f;
-    h = h - 2 * (1.0 - iperc);
-    if (prop_k || !is_prop) fl |= 8;   // select
-    if (prop_k) fl |= 16;              // keep prior count on k
+    for (int m = 0; m < 3; m++)
+      mm[m] = marginal_sum(cnt[m], K, t_lr[m][0][lane], t_lr[m][1][lane], t_lr[m][2][lane],
+                           t_log[m][lane]);
+    const double count_k = cnt[0], count_s = cnt[1];
+    double h = mm[0] + mm[1] - mm[2] + split_alpha;
+    uint8_t fl = 1;
+    if (S.mode) {
+      bool is_prop = sp.prop[k];
+      int ninv_k = sm.ninvalid[k], ninv_s = sm.ninvalid[s];
+      bool prop_k = (ninv_k <= ninv_s);
+      float iperc_k = (float)(ninv_k / (1.0 * count_k));
+      float iperc_s = (float)(ninv_k / (1.0 * count_s));  // reference uses ninvalid_k here
+      float iperc = prop_k ? iperc_k : iperc_s;
+      iperc = is_prop ? iperc : 1.0f;
+      h = h - 2 * (1.0 - iperc);
+      if (prop_k || !is_prop) fl |= 8;   // select
+      if (prop_k) fl |= 16;              // keep prior count on k
+    }
+    if (near_tie(h)) atomicAdd(&sc->near_ties, 1);
+    if (h > -2) S.accept[k] = fl;
   }
-  if (near_tie(h)) atomicAdd(&sc->near_ties, 1);
-  if (h > -2) S.accept[k] = fl;
 }
 
 // Split commit: new id = max_spix + 1 + rank (R2), prior counts.
@@ -673,35 +675,35 @@ __global__ void kb_split_commit(const Slot* __restrict__ slots) {
   const uint8_t* __restrict__ accept = S.accept;
   const int* __restrict__ excl = S.excl;
   const int prop_mode = S.mode;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= live_ids(S)) return;
-  uint8_t fl = accept[k];
-  if (!fl) return;
-  int snew = sc->max_spix + 1 + excl[k];
-  sm.newid[k] = snew;
-  if (snew >= sp.cap) { atomicExch(&sc->status, STSPIX_ERR_CAPACITY); sm.newid[k] = -1; return; }
-  if (!prop_mode) {
-    float pcn = (float)fmax(sp.prior_count[k] / 2.0, 8.0);
-    sp.prior_count[k] = pcn;
-    sp.prior_count[snew] = pcn;
-  } else {
-    float pc = sp.prior_count[k];
-    float half = (float)fmax(pc / 2.0, 36.0);
-    if (fl & 16) {
-      sp.prior_count[k] = pc;
-      sp.prior_count[snew] = (float)(pc / 2.);
+  FOR_ID(k, live_ids(S)) {
+    uint8_t fl = accept[k];
+    if (!fl) continue;
+    int snew = sc->max_spix + 1 + excl[k];
+    sm.newid[k] = snew;
+    if (snew >= sp.cap) { atomicExch(&sc->status, STSPIX_ERR_CAPACITY); sm.newid[k] = -1; continue; }
+    if (!prop_mode) {
+      float pcn = (float)fmax(sp.prior_count[k] / 2.0, 8.0);
+      sp.prior_count[k] = pcn;
+      sp.prior_count[snew] = pcn;
     } else {
-      sp.prior_count[k] = half;
-      sp.prior_count[snew] = half;
-      double pcs = half;
-      sp.prior_icov[3 * k] = pcs; sp.prior_icov[3 * k + 1] = 0; sp.prior_icov[3 * k + 2] = pcs;
+      float pc = sp.prior_count[k];
+      float half = (float)fmax(pc / 2.0, 36.0);
+      if (fl & 16) {
+        sp.prior_count[k] = pc;
+        sp.prior_count[snew] = (float)(pc / 2.);
+      } else {
+        sp.prior_count[k] = half;
+        sp.prior_count[snew] = half;
+        double pcs = half;
+        sp.prior_icov[3 * k] = pcs; sp.prior_icov[3 * k + 1] = 0; sp.prior_icov[3 * k + 2] = pcs;
+      }
+      sp.prop[snew] = 0;
+      sp.icount[k] = (float)(sp.icount[k] / 2.0);
+      double pcs = sp.prior_count[snew];
+      sp.prior_icov[3 * snew] = pcs; sp.prior_icov[3 * snew + 1] = 0; sp.prior_icov[3 * snew + 2] = pcs;
     }
-    sp.prop[snew] = 0;
-    sp.icount[k] = (float)(sp.icount[k] / 2.0);
-    double pcs = sp.prior_count[snew];
-    sp.prior_icov[3 * snew] = pcs; sp.prior_icov[3 * snew + 1] = 0; sp.prior_icov[3 * snew + 2] = pcs;
+    sp.valid[snew] = 1;
   }
-  sp.valid[snew] = 1;
 }
 
 // split_sp (split_merge.cu:1002-1031) / split_sp_p (split_merge_prop.cu:2317-2350).
@@ -786,30 +788,31 @@ __global__ void kb_merge_candidates(const Slot* __restrict__ slots, int dir_bass
 // per 32 ids: warps 0-2 one channel's log ratio each, warp 3 the log count, warp 0 adds.
 __global__ void __launch_bounds__(128) kb_merge_single(const Slot* __restrict__ slots, SmConsts K) {
   pdl_enter();
-  SLOT_Y;
+  SLOT_X;
   const SpDev& sp = S.sp;
   const SmDev& sm = S.sm;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int k = blockIdx.x * 32 + lane;
   const int n_ids = live_ids(S);
-  if ((int)blockIdx.x * 32 >= n_ids) return;              // block-uniform
   __shared__ double t_lr[3][32], t_log[32];
-  bool ok = false;
-  double n = 0;
-  if (k < n_ids) {
-    if (w == 0) sm.flag[k] = 0;
-    ok = sp.valid[k] && sm.pair[k] >= 0;
-    if (ok) n = sp.count[k];
+  for (int g = blockIdx.y; 32 * g < n_ids; g += gridDim.y) {  // the same for the block
+    const int k = 32 * g + lane;
+    bool ok = false;
+    double n = 0;
+    if (k < n_ids) {
+      if (w == 0) sm.flag[k] = 0;
+      ok = sp.valid[k] && sm.pair[k] >= 0;
+      if (ok) n = sp.count[k];
+    }
+    if (!__syncthreads_or(ok)) continue;              // block-uniform
+    if (ok) {
+      if (w < 3) t_lr[w][lane] = marginal_lr(n, K, sp.acc[8 * (size_t)k + w], sm.sq[3 * (size_t)k + w], true);
+      else t_log[lane] = log(n);
+    }
+    __syncthreads();
+    if (w != 0 || !ok) continue;
+    sm.msingle[k] = marginal_sum(n, K, t_lr[0][lane], t_lr[1][lane], t_lr[2][lane], t_log[lane]);
+    sm.flag[k] = 16;
   }
-  if (!__syncthreads_or(ok)) return;
-  if (ok) {
-    if (w < 3) t_lr[w][lane] = marginal_lr(n, K, sp.acc[8 * (size_t)k + w], sm.sq[3 * (size_t)k + w], true);
-    else t_log[lane] = log(n);
-  }
-  __syncthreads();
-  if (w != 0 || !ok) return;
-  sm.msingle[k] = marginal_sum(n, K, t_lr[0][lane], t_lr[1][lane], t_lr[2][lane], t_log[lane]);
-  sm.flag[k] = 16;
 }
 
 // calc_merge_stats_step2 + update_merge_flag (split_merge_orig.cu:555-656), R3.  One
@@ -819,51 +822,52 @@ __global__ void __launch_bounds__(128) kb_merge_single(const Slot* __restrict__ 
 __global__ void __launch_bounds__(128) kb_merge_decide(const Slot* __restrict__ slots, SmConsts K,
                                                        float merge_alpha) {
   pdl_enter();
-  SLOT_Y;
+  SLOT_X;
   const SpDev& sp = S.sp;
   const SmDev& sm = S.sm;
   Scalars* sc = S.sc;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int k = blockIdx.x * 32 + lane;
   const int n_ids = live_ids(S);
-  if ((int)blockIdx.x * 32 >= n_ids) return;              // block-uniform
   __shared__ double t_lr[3][32], t_log[32];
-  bool ok = false;
-  int f = -1;
-  double count_k = 0, count_f = 0;
-  if (k < n_ids && sp.valid[k]) {
-    f = sm.pair[k];
-    if (f >= 0 && sp.valid[f]) {
-      count_k = sp.count[k];
-      count_f = sp.count[k] + sp.count[f];
-      ok = count_k >= 1 && count_f >= 1;
+  for (int g = blockIdx.y; 32 * g < n_ids; g += gridDim.y) {  // the same for the block
+    const int k = 32 * g + lane;
+    bool ok = false;
+    int f = -1;
+    double count_k = 0, count_f = 0;
+    if (k < n_ids && sp.valid[k]) {
+      f = sm.pair[k];
+      if (f >= 0 && sp.valid[f]) {
+        count_k = sp.count[k];
+        count_f = sp.count[k] + sp.count[f];
+        ok = count_k >= 1 && count_f >= 1;
+      }
     }
-  }
-  if (!__syncthreads_or(ok)) return;
-  const bool calc = ok && (sm.flag[f] & 16);
-  if (calc) {
-    if (w < 3) {
-      const long long sv = sp.acc[8 * (size_t)k + w] + sp.acc[8 * (size_t)f + w];
-      const long long qv = sm.sq[3 * (size_t)k + w] + sm.sq[3 * (size_t)f + w];
-      t_lr[w][lane] = marginal_lr(count_f, K, sv, qv, true);
+    if (!__syncthreads_or(ok)) continue;              // block-uniform
+    const bool calc = ok && (sm.flag[f] & 16);
+    if (calc) {
+      if (w < 3) {
+        const long long sv = sp.acc[8 * (size_t)k + w] + sp.acc[8 * (size_t)f + w];
+        const long long qv = sm.sq[3 * (size_t)k + w] + sm.sq[3 * (size_t)f + w];
+        t_lr[w][lane] = marginal_lr(count_f, K, sv, qv, true);
+      } else {
+        t_log[lane] = log(count_f);
+      }
+    }
+    __syncthreads();
+    if (w != 0 || !ok) continue;
+    double h;
+    if (!calc) {
+      h = -INFINITY;
     } else {
-      t_log[lane] = log(count_f);
+      const double m_merged =
+          marginal_sum(count_f, K, t_lr[0][lane], t_lr[1][lane], t_lr[2][lane], t_log[lane]);
+      h = m_merged - (K.log_alpha + sm.msingle[k] + sm.msingle[f]) + merge_alpha;
     }
-  }
-  __syncthreads();
-  if (w != 0 || !ok) return;
-  double h;
-  if (!calc) {
-    h = -INFINITY;
-  } else {
-    const double m_merged =
-        marginal_sum(count_f, K, t_lr[0][lane], t_lr[1][lane], t_lr[2][lane], t_log[lane]);
-    h = m_merged - (K.log_alpha + sm.msingle[k] + sm.msingle[f]) + merge_alpha;
-  }
-  if (near_tie(h)) atomicAdd(&sc->near_ties, 1);
-  if (h > -2) {
-    sm.flag[k] |= 1;  // only thread k writes flag[k] here; readers use bit 16 only
-    atomicMin(&sm.claim[f], k);
+    if (near_tie(h)) atomicAdd(&sc->near_ties, 1);
+    if (h > -2) {
+      sm.flag[k] |= 1;  // only thread k writes flag[k] here; readers use bit 16 only
+      atomicMin(&sm.claim[f], k);
+    }
   }
 }
 
@@ -871,10 +875,13 @@ __global__ void __launch_bounds__(128) kb_merge_decide(const Slot* __restrict__ 
 __global__ void kb_merge_clear(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= live_ids(S)) return;
-  S.sm.pair[k] = -1;
-  S.sm.claim[k] = 0x7f7f7f7f;
+  const int n_ids = live_ids(S);
+  FOR_ID(k, sm_ids(S)) {
+    sm_clear(S.sm, k);
+    if (k >= n_ids) continue;
+    S.sm.pair[k] = -1;
+    S.sm.claim[k] = 0x7f7f7f7f;
+  }
 }
 
 // merge flag := accepted and claimant of its target; snapshot valid; target := pair.
@@ -884,14 +891,14 @@ __global__ void kb_merge_flag(const Slot* __restrict__ slots) {
   const SpDev& sp = S.sp;
   const SmDev& sm = S.sm;
   uint8_t* __restrict__ valid0 = S.valid0;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= live_ids(S)) return;
-  valid0[k] = sp.valid[k];
-  int f = sm.pair[k];
-  sm.target[k] = f;
-  uint8_t fl = sm.flag[k];
-  if ((fl & 1) && f >= 0 && sm.claim[f] == k) fl |= 2;
-  sm.flag[k] = fl;
+  FOR_ID(k, live_ids(S)) {
+    valid0[k] = sp.valid[k];
+    int f = sm.pair[k];
+    sm.target[k] = f;
+    uint8_t fl = sm.flag[k];
+    if ((fl & 1) && f >= 0 && sm.claim[f] == k) fl |= 2;
+    sm.flag[k] = fl;
+  }
 }
 
 // remove_sp (split_merge.cu:1035-1080) / remove_sp_p (split_merge_prop.cu:2353-2449).
@@ -903,29 +910,29 @@ __global__ void kb_merge_remove(const Slot* __restrict__ slots) {
   Scalars* sc = S.sc;
   const uint8_t* __restrict__ valid0 = S.valid0;
   const int prop_mode = S.mode;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= live_ids(S)) return;
-  int s = sm.pair[k];
-  if (s < 0) return;
-  bool is_cycle = sm.pair[s] == k;
-  if (!valid0[k] || !valid0[s]) return;
-  bool mk = sm.flag[k] & 2, ms = sm.flag[s] & 2;
-  if (!prop_mode) {
-    if (mk && (!ms || (is_cycle && k < s))) {
-      sm.flag[k] |= 4;
-      sp.valid[k] = 0;
-      sp.prior_count[s] = sp.prior_count[k] + sp.prior_count[s];
-      atomicAdd(&sc->nmerges, 1);
-    }
-  } else {
-    bool cond_c = is_cycle && sp.prop[k];
-    if (mk && (!ms || cond_c)) {
-      int r = k, t = s;
-      if (sp.prop[k]) { sm.target[s] = k; r = s; t = k; }
-      sm.flag[r] |= 4;  // each superpixel has at most one remover (single writer)
-      sp.valid[r] = 0;
-      sp.prior_count[t] = sp.prior_count[r] + sp.prior_count[t];
-      atomicAdd(&sc->nmerges, 1);
+  FOR_ID(k, live_ids(S)) {
+    int s = sm.pair[k];
+    if (s < 0) continue;
+    bool is_cycle = sm.pair[s] == k;
+    if (!valid0[k] || !valid0[s]) continue;
+    bool mk = sm.flag[k] & 2, ms = sm.flag[s] & 2;
+    if (!prop_mode) {
+      if (mk && (!ms || (is_cycle && k < s))) {
+        sm.flag[k] |= 4;
+        sp.valid[k] = 0;
+        sp.prior_count[s] = sp.prior_count[k] + sp.prior_count[s];
+        atomicAdd(&sc->nmerges, 1);
+      }
+    } else {
+      bool cond_c = is_cycle && sp.prop[k];
+      if (mk && (!ms || cond_c)) {
+        int r = k, t = s;
+        if (sp.prop[k]) { sm.target[s] = k; r = s; t = k; }
+        sm.flag[r] |= 4;  // each superpixel has at most one remover (single writer)
+        sp.valid[r] = 0;
+        sp.prior_count[t] = sp.prior_count[r] + sp.prior_count[t];
+        atomicAdd(&sc->nmerges, 1);
+      }
     }
   }
 }

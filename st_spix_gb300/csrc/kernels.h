@@ -77,7 +77,6 @@ __global__ void kb_bbox(const Slot* slots);
 __global__ void kb_split_bfs(const Slot* slots, int dir_bass, int dir_prop);
 __global__ void kb_split_bfs_big(const Slot* slots);
 __global__ void kb_split_partition(const Slot* slots);
-__global__ void kb_sm_clear(const Slot* slots);
 __global__ void kb_sm_accumulate(const Slot* slots, int split);
 __global__ void kb_split_decide(const Slot* slots, SmConsts K, float split_alpha);
 __global__ void kb_split_commit(const Slot* slots);
@@ -120,7 +119,6 @@ __global__ void kb_relabel_ids(const Slot* slots);
 __global__ void kb_relabel_params(const Slot* slots);
 __global__ void kb_relabel_apply(const Slot* slots);
 __global__ void kb_relabel_end(const Slot* slots, int B);
-__global__ void kb_count_revived(const Slot* slots);
 
 // k_color.cu
 __global__ void k_rgb2lab(const float* rgb, float* lab, long long npix, int first_blue,
