@@ -1135,6 +1135,82 @@ __device__ __forceinline__ SweepRec load_rec(const SweepRec* __restrict__ rec, i
   return u.r;
 }
 
+// Scores and relabels the n <= threads / 4 listed pixels of a phase, four lanes to a pixel:
+// lane q takes candidate q of N, S, W, E (its simple-point code, record and score), two
+// exchanges find the best, and each lane updates its edge.  The result is that of one thread
+// per pixel (a repeated candidate scores the same, so the first of the best stands), in a
+// third of the dependent instructions: a phase of few pixels lasts one warp's chain, about
+// 350 instructions with a thread per pixel.  Up to a quarter of the block's threads in pixels:
+// above, one round no longer holds them (half, in two rounds, was 1 to 2 % slower, two lanes
+// to a pixel there too, all in rounds 12 %).  With the listing by atomics (below) a launch on
+// a 240x320 frame fell from 18.7 to 14.5 us, on 720x1280 from 43.4 to 37.8, on 8 frames of
+// 480x854 from 83.4 to 75.4.
+template <int TX, int TY, int NS>
+__device__ __forceinline__ void sweep_quad(const SweepSlot& S, SweepTile<TX, TY, NS>& sm, int rx0,
+                                           int ry0, int n, float s2, float potts,
+                                           const unsigned* lut_bits, bool neg) {
+  using Tile = SweepTile<TX, TY, NS>;
+  constexpr int kSH = Tile::kSH, kLX = Tile::kLX;
+  int* L = sm.L;
+  const int lane = threadIdx.x & 31, q = lane & 3, j = threadIdx.x >> 2;
+  const int W = S.W, cap = S.cap;
+  const bool act = j < n;
+  const int ent = sm.list[act ? j : 0];
+  const int ax = ent & 255, ay = ent >> 8;
+  const int gx = rx0 + ax, gy = ry0 + ay;
+  const int p = ay * kLX + ax;
+  const float* pix = S.img + 3 * ((size_t)gy * W + gx);
+  const float c0 = __ldg(pix), c1 = __ldg(pix + 1), c2 = __ldg(pix + 2);
+  const int v = L[p + (q < 2 ? (q ? kLX : -kLX) : (q == 2 ? -1 : 1))];
+  const int C = L[p];
+  const int N = L[p - kLX], So = L[p + kLX], Wl = L[p - 1], E = L[p + 1];
+  const int nb[8] = {L[p - kLX - 1], N, L[p - kLX + 1], Wl, E, L[p + kLX - 1], So, L[p + kLX + 1]};
+  const bool in = (unsigned)C < (unsigned)cap && max(max(N, So), max(Wl, E)) < cap &&
+                  !(N == C && So == C && Wl == C && E == C);
+  const SweepRec r = load_rec(S.rec, in ? max(v, 0) : 0);
+  const int n_c = __ldg(&S.rec[in ? C : 0].count);
+  unsigned d = 0, m1 = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) d |= (unsigned)(nb[i] == v) << i;
+  if (neg) {                                        // block-uniform
+#pragma unroll
+    for (int i = 0; i < 8; i++) m1 |= (unsigned)(nb[i] == -1) << i;
+    d |= m1;
+  }
+  const unsigned simple =
+      __ballot_sync(0xffffffffu, ((lut_bits[d >> 5] >> (d & 31)) & 1u) && in && act);
+  const float sc = joint(c0, c1, c2, gx, gy, r, s2, 8 - __popc(d), potts);
+  const bool cand = v >= 0 && sc > -9999.f;
+  float best = cand ? sc : -9999.f;
+  int bl = cand ? v : C;
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int ol = __shfl_xor_sync(0xffffffffu, bl, o);
+    if (ob > best || (ob == best && (lane & o))) { best = ob; bl = ol; }
+  }
+  if (((simple >> (lane & 28)) & 15u) != 15u) return;
+  if (bl == C && n_c <= 2) bl = N >= 0 ? N : E >= 0 ? E : So >= 0 ? So : Wl >= 0 ? Wl : C;
+  if (bl == C) return;
+  if (q == 0) {
+    L[p] = bl;
+    if (ay >= kSH && ay < kSH + TY && ax >= kSH && ax < kSH + TX)
+      atomicOr(&sm.all[ay][ax >> 5], 1u << (ax & 31));
+  }
+  if (q < 3) {                                      // row ay - 1 + q of its 3x3 is dirty
+    const unsigned long long three = 7ull << ((ax & 31) + 31);   // bits 31.. = word ax >> 5
+    unsigned* row = sm.dirty[ay - 1 + q] + (ax >> 5);
+    atomicOr(row, (unsigned)(three >> 32));
+    if (!(ax & 31)) atomicOr(row - 1, 0x80000000u);
+    if ((ax & 31) == 31) atomicOr(row + 1, 1u);
+  }
+  // the lane's edge: of N and S rows' edS, of W and E columns' edE (the pixels of a phase
+  // are never 4-neighbours, so each edge has one writer; words are shared)
+  const int ex = q == 2 ? ax - 1 : ax, ey = q == 0 ? ay - 1 : ay;
+  if ((C != v) != (bl != v))
+    atomicXor(q < 2 ? &sm.edS[ey][ex >> 5] : &sm.edE[ey][ex >> 5], 1u << (ex & 31));
+}
+
 // What a sweep scores.  The parameters are fixed across the sweeps of one update_seg
 // call, and a pixel's decision depends only on its 3x3 labels at its phase, its colour
 // and the records of its own and its 4-neighbours' labels.  So a pixel whose 3x3 labels
@@ -1297,8 +1373,9 @@ __device__ __forceinline__ void sweep_tile(const SweepSlot& S, int bx, int by, i
   const float* __restrict__ img = S.img;
   const SweepRec* __restrict__ rec = S.rec;
   const bool neg = sm.neg != 0;
-  // the grid of a phase: 16-pixel half words of the rows of one y parity
-  constexpr int kHalves = 2 * kCK, kItems = kLY / 2 * kHalves;
+  // the grid of a phase: words, or quarters, of the rows of one y parity
+  constexpr int kParts = kLY / 2 * 4 * kCK <= NT ? 4 : 1, kPartBits = 32 / kParts;
+  constexpr int kRowParts = kParts * kCK, kItems = kLY / 2 * kRowParts;
   for (int s = 0; s < ns; s++) {
     const int cur = s & 1;
     const int G = kReach * (ns - s) - 1;
@@ -1339,35 +1416,31 @@ __device__ __forceinline__ void sweep_tile(const SweepSlot& S, int bx, int by, i
     if (!__syncthreads_or(any)) break;   // nothing to score: nor in the later sweeps
     for (int ph = 0; ph < 4; ph++) {
       // the phase's pixels: dirty border pixels of the class ((x parity << 1) | y parity)
-      // on the tile grown by G - ph, listed by warp scans and one shared atomic per warp
+      // on the tile grown by G - ph, listed by a shared atomic per word, or quarter of a
+      // word where the threads suffice (a warp scan first took 8 % of a launch more on a
+      // 240x320 frame, 5 % on larger ones)
       const int g = G - ph;
-      for (int base = 0; base < kItems; base += NT) {
-        const int i = base + (int)threadIdx.x;
-        const int ay = 2 * (i / kHalves) + (ph & 1), h = i % kHalves, w = h >> 1;
-        unsigned m = 0;
-        if (ay >= kSH - g && ay < kSH + TY + g) {
-          m = sm.dirty[ay][w] & sm.bm[ay][w] & ((h & 1) ? 0xffff0000u : 0x0000ffffu) &
-              ((ph & 2) ? 0xAAAAAAAAu : 0x55555555u) & range32(kSH - g, kSH + TX + g, w);
-          if (m) atomicAnd(&sm.dirty[ay][w], ~m);
-        }
-        if (__any_sync(0xffffffffu, m != 0)) {
-          const int n = __popc(m);
-          int inc = n;
-#pragma unroll
-          for (int k = 1; k < 32; k <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, inc, k);
-            if (lane >= k) inc += t;
-          }
-          int at = 0;
-          if (lane == 31) at = atomicAdd(&sm.cnt[cur][ph], inc);
-          at = __shfl_sync(0xffffffffu, at, 31) + inc - n;
-          const int ent = (ay << 8) | (32 * w);
-          for (; m; m &= m - 1) sm.list[at++] = (unsigned short)(ent + __ffs(m) - 1);
+      for (int i = threadIdx.x; i < kItems; i += NT) {
+        const int ay = 2 * (i / kRowParts) + (ph & 1), h = i % kRowParts, w = h / kParts;
+        if (ay < kSH - g || ay >= kSH + TY + g) continue;
+        unsigned m = sm.dirty[ay][w] & sm.bm[ay][w] &
+                     ((0xffffffffu >> (32 - kPartBits)) << (kPartBits * (h % kParts))) &
+                     ((ph & 2) ? 0xAAAAAAAAu : 0x55555555u) & range32(kSH - g, kSH + TX + g, w);
+        if (m) {
+          atomicAnd(&sm.dirty[ay][w], ~m);
+          int at = atomicAdd(&sm.cnt[cur][ph], __popc(m));
+          for (const int ent = (ay << 8) | (32 * w); m; m &= m - 1)
+            sm.list[at++] = (unsigned short)(ent + __ffs(m) - 1);
         }
       }
       __syncthreads();
       const int n = sm.cnt[cur][ph];
       if (!n) continue;                               // block-uniform
+      if (n <= NT / 4) {                              // block-uniform
+        if (8 * warp < n) sweep_quad<TX, TY, NS>(S, sm, rx0, ry0, n, s2, potts, lut_bits, neg);
+        __syncthreads();
+        continue;
+      }
       for (int j = threadIdx.x; j < n; j += NT) {
         const int ent = sm.list[j];
         const int ax = ent & 255, ay = ent >> 8;
