@@ -927,7 +927,11 @@ __device__ __forceinline__ float joint(float c0, float c1, float c2, int x, int 
   d0 -= min(max(d0, 0), r.frac & 1);
   d1 -= min(max(d1, 0), (r.frac >> 1) & 1);
   res = res - (x0 * x0 + x1 * x1 + x2 * x2) / s2;
-  res = res - (float)(d0 * d0) * r.isx - (float)(d1 * d1) * r.isz - (float)(2 * d0 * d1) * r.isy;
+  // (float)(d0 * d0) and so on, by products of the floats (exact below 2^22, so the products
+  // round as the integers' conversions do)
+  const float f0 = __int_as_float(0x4b400000 + d0) - 12582912.f;
+  const float f1 = __int_as_float(0x4b400000 + d1) - 12582912.f;
+  res = res - f0 * f0 * r.isx - f1 * f1 * r.isz - 2.f * (f0 * f1) * r.isy;
   res = res - r.logdet;
   // (float)neq for 0 <= neq < 2^23 without a conversion
   res = res - beta * (__uint_as_float(0x4b000000u | (unsigned)neq) - 8388608.f);
@@ -1067,9 +1071,8 @@ struct SweepTile {
   static constexpr int kLX = TX + 2 * kSH, kLY = TY + 2 * kSH;       // staged labels
   static constexpr int kCK = (kLX + 31) / 32;                        // words per row
   static constexpr int kClass = (TX / 2 + kG0) * (TY / 2 + kG0);     // a phase's pixels
-  static constexpr int kRowsOut = 32 < TY ? 16 : TY;                 // rows per write-back pass
-  static constexpr int kMaxList = kClass > TX * kRowsOut ? kClass : TX * kRowsOut;
-  static_assert(kLX < 256 && kLY < 256 && TY % kRowsOut == 0, "list entries pack (y << 8) | x");
+  static constexpr int kMaxList = kClass > TX * TY ? kClass : TX * TY;
+  static_assert(kLX < 256 && kLY < 256, "list entries pack (y << 8) | x");
   static_assert(kLX % 8 == 0 && kLY % 8 == 0, "8-pixel groups, rows in whole warp spans");
   static_assert(kSH % 2 == 0 && TX % 16 == 0 && TY % 2 == 0, "region parity = image parity");
   __align__(16) int L[kLX * kLY];
@@ -1546,8 +1549,10 @@ __device__ __forceinline__ void sweep_tile(const SweepSlot& S, int bx, int by, i
     }
   }
   // --- write-back.  The pixels where seg_out is behind (mode 0: every pixel of the tile is
-  // stored) are listed like a phase's, kRowsOut rows at a time, and a relabelled one moves
-  // its statistics from the label it had at the launch's start to the one it has now.
+  // stored) are listed like a phase's, and a relabelled one moves its statistics
+  // from the label it had at the launch's start to the one it has now.
+  // (In one round: 16 rows at a time, three barriers and two memory round trips each, took
+  // 4 % of a launch of 64x48 tiles more.)
   __syncthreads();
   if (deltas)
     for (int i = threadIdx.x; i < kDeltaTab * 13; i += NT)
@@ -1569,39 +1574,37 @@ __device__ __forceinline__ void sweep_tile(const SweepSlot& S, int bx, int by, i
       chg_out[(size_t)gy * P16 + wi] = (uint16_t)__funnelshift_r(lo, hi, b & 31);
     }
   }
-  for (int y0 = kSH; y0 < kSH + TY; y0 += Tile::kRowsOut) {
-    for (int i = threadIdx.x; i < Tile::kRowsOut * kCK; i += NT) {
-      const int y = i / kCK + y0, c = i % kCK;
-      unsigned m = (sm.sin[y][c] & (mode ? range32(kSH, kSH + TX, c) : 0u)) | sm.all[y][c];
-      if (m) {
-        int at = atomicAdd(&sm.wcnt, __popc(m));
-        for (const int ent = (y << 8) | (32 * c); m; m &= m - 1)
-          sm.list[at++] = (unsigned short)(ent + __ffs(m) - 1);
-      }
+  for (int i = threadIdx.x; i < TY * kCK; i += NT) {
+    const int y = i / kCK + kSH, c = i % kCK;
+    unsigned m = (sm.sin[y][c] & (mode ? range32(kSH, kSH + TX, c) : 0u)) | sm.all[y][c];
+    if (m) {
+      int at = atomicAdd(&sm.wcnt, __popc(m));
+      for (const int ent = (y << 8) | (32 * c); m; m &= m - 1)
+        sm.list[at++] = (unsigned short)(ent + __ffs(m) - 1);
     }
-    __syncthreads();
-    const int nw = sm.wcnt;
-    for (int j = threadIdx.x; j < nw; j += NT) {
-      const int ent = sm.list[j];
-      const int ax = ent & 255, ay = ent >> 8;
-      const int gx = rx0 + ax, gy = ry0 + ay;
-      const size_t g = (size_t)gy * W + gx;
-      const int b = L[ay * kLX + ax];
-      if (mode) seg_out[g] = b;
-      if (deltas && ((sm.all[ay][ax >> 5] >> (ax & 31)) & 1u)) {
-        const int o = seg_in[g];
-        if (o != b) {
-          const float* pix = img + 3 * g;
-          delta_move(sm.delta, S.count, S.acc, o, b, gx, gy, tx0, ty0, __ldg(pix),
-                     __ldg(pix + 1), __ldg(pix + 2));
-        }
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) sm.wcnt = 0;
-    if (y0 + Tile::kRowsOut < kSH + TY) __syncthreads();
   }
-  if (deltas) delta_flush(sm.delta, S.count, S.acc, tx0, ty0);
+  __syncthreads();
+  const int nw = sm.wcnt;
+  for (int j = threadIdx.x; j < nw; j += NT) {
+    const int ent = sm.list[j];
+    const int ax = ent & 255, ay = ent >> 8;
+    const int gx = rx0 + ax, gy = ry0 + ay;
+    const size_t g = (size_t)gy * W + gx;
+    const int b = L[ay * kLX + ax];
+    if (mode) seg_out[g] = b;
+    if (deltas && ((sm.all[ay][ax >> 5] >> (ax & 31)) & 1u)) {
+      const int o = seg_in[g];
+      if (o != b) {
+        const float* pix = img + 3 * g;
+        delta_move(sm.delta, S.count, S.acc, o, b, gx, gy, tx0, ty0, __ldg(pix),
+                   __ldg(pix + 1), __ldg(pix + 2));
+      }
+    }
+  }
+  if (deltas) {
+    __syncthreads();
+    delta_flush(sm.delta, S.count, S.acc, tx0, ty0);
+  }
 }
 
 template <int TX, int TY, int NS, int NT>
