@@ -380,6 +380,7 @@ int ensure_slot(stspix_ctx* ctx, int i, int npix, int sp_cap) {
     size_t c2 = (size_t)cap + 2;
     SmDev& sm = s.sm;
     AL(L, sm.count, c2); AL(L, sm.s, 3 * c2); AL(L, sm.sq, 3 * c2);
+    AL(L, sm.pos, 5 * c2);
     AL(L, sm.ninvalid, c2); AL(L, sm.pair, c2); AL(L, sm.claim, c2);
     AL(L, sm.target, c2); AL(L, sm.newid, c2); AL(L, sm.flag, c2);
     AL(L, sm.msingle, c2);
@@ -476,7 +477,7 @@ void preload_kernels() {
       (const void*)kb_split_bfs,
       (const void*)kb_split_bfs_big,
       (const void*)kb_split_partition,
-      (const void*)kb_sm_accumulate,
+      (const void*)kb_sm_accumulate, (const void*)kb_sq_accumulate,
       (const void*)kb_split_decide,
       (const void*)kb_split_commit,
       (const void*)kb_split_apply,
@@ -674,14 +675,14 @@ void accumulate_fp(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, int 
   LAUNCHB(kb_accumulate_fp_store, L.max_cap, L, nb, mode);
 }
 
-// stats_ready: the last sweep of the preceding update_seg already cleared and added
-// the statistics of the first nb slots (see update_seg).
+// stats_ready: the statistics of the first nb slots are current (the sweeps, a split or a
+// merge moved them with the labels).
 // incremental: only the ids whose sums changed since their last posterior;
 // only where nothing but sweeps ran since the previous posterior of every slot.
-// log64: the log determinants in FP64 (see kb_posterior).
+// log64: the log determinants in FP64; merged: the sums left by a merge (see kb_posterior).
 int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
                   bool stats_ready = false, bool incremental = false, bool clear_all = false,
-                  bool log64 = false) {
+                  bool log64 = false, bool merged = false) {
   ctx->cur_fam = STSPIX_FAM_STATS;
   if (!stats_ready) {
     LAUNCHI(kb_clear_stats, 4LL * L.max_cap, L, nb, clear_all ? 1 : 0);
@@ -691,7 +692,7 @@ int update_params(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
   ctx->cur_fam = STSPIX_FAM_POSTERIOR;
   const unsigned pg = id_blocks(ctx, L.max_cap, 32, nb);     // groups of 32 ids
   LAUNCHG(kb_posterior, dim3((unsigned)nb, pg), 128, L.d, incremental ? 1 : 0,
-          log64 ? 1 : 0);
+          log64 ? 1 : 0, merged ? 1 : 0);
   return STSPIX_OK;
 }
 
@@ -816,7 +817,7 @@ int run_split(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmC
     prof_end(ctx, st, pe_, "kb_split_bfs_big");
   }
   LAUNCHB(kb_split_partition, pix_units(L.max_npix), L, nb);
-  LAUNCHG(kb_sm_accumulate, dim3(tiles64(L), (unsigned)nb), kThreads, L.d, 1);
+  LAUNCHG(kb_sm_accumulate, dim3(tiles64(L), (unsigned)nb), kThreads, L.d);
   LAUNCHG(kb_split_decide, dim3((unsigned)nb, id_blocks(ctx, L.max_cap, 32, nb)), 128, L.d, K,
           cfg.split_alpha);
   LAUNCHG(kb_scan, (unsigned)nb, 1024, L.d, 1);
@@ -849,13 +850,13 @@ int run_merge(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmC
   ctx->cur_fam = STSPIX_FAM_MERGE;
   LAUNCHI(kb_merge_clear, L.max_cap + 2, L, nb);
   LAUNCHB(kb_merge_candidates, pix_units(L.max_npix), L, nb, dir_b, dir_p, use_border ? 1 : 0);
-  LAUNCHG(kb_sm_accumulate, dim3(tiles64(L), (unsigned)nb), kThreads, L.d, 0);
+  LAUNCHG(kb_sq_accumulate, dim3(tiles64(L), (unsigned)nb), kThreads, L.d);
   LAUNCHG(kb_merge_single, dim3((unsigned)nb, id_blocks(ctx, L.max_cap, 32, nb)), 128, L.d, K);
   LAUNCHG(kb_merge_decide, dim3((unsigned)nb, id_blocks(ctx, L.max_cap, 32, nb)), 128, L.d, K,
           cfg.merge_alpha);
   LAUNCHI(kb_merge_flag, L.max_cap, L, nb);
   LAUNCHI(kb_merge_remove, L.max_cap, L, nb);
-  LAUNCHB(kb_merge_apply, pix_units(L.max_npix), L, nb);
+  LAUNCHB(kb_merge_apply, pix_units(L.max_npix), L, nb, ctx->accumulator == 0 ? 1 : 0);
   return STSPIX_OK;
 }
 
@@ -879,8 +880,8 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
   int cur = 0;              // the label buffer the next sweep reads (see update_seg)
   const bool state = stop_after >= 0;       // the caller reads the state, not the parameters
   auto params = [&](const List& l, int n, bool ready = false, bool incremental = false,
-                    bool all = false) {
-    return update_params(ctx, st, l, n, ready, incremental, all, state);
+                    bool all = false, bool merged = false) {
+    return update_params(ctx, st, l, n, ready, incremental, all, state, merged);
   };
   for (int idx = 0; idx < maxn; idx++) {
     while (nb > 0 && nit[nb - 1] <= idx) nb--;
@@ -900,13 +901,14 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
         count_b += 1;
         count_p += 1;
         if ((r = run_split(ctx, st, L, nb, K, cfg, count_b % 2 + 1, count_p % 2 + 1))) return r;
-        if ((r = params(L, nb))) return r;
+        // (the sums were current before the step, and it moved them with the labels)
+        if ((r = params(L, nb, fuse))) return r;
       }
       if (idx % P == P / 2) {
         count_p += 1;  // propagated frames step the direction again before merging
         if (L.any_prop && (r = run_relabel(ctx, st, L, nb, cfg))) return r;
         if ((r = run_merge(ctx, st, L, nb, K, cfg, count_b % 2, count_p % 2, P == 1))) return r;
-        if ((r = params(L, nb))) return r;
+        if ((r = params(L, nb, fuse, false, false, fuse))) return r;
       }
     }
     const int nx = idx + 1;

@@ -94,6 +94,7 @@ struct SmDev {
   int* count;
   long long* s;      // [3*(cap+2)]
   long long* sq;     // [3*(cap+2)]
+  long long* pos;    // [5*(cap+2)]: x, y, xx, xy, yy (split halves)
   int* ninvalid;
   int* pair;         // merge candidate (sm_pairs[2k+1])
   int* claim;        // merge claim (sm_pairs[2f])
@@ -237,12 +238,18 @@ __device__ __forceinline__ long long warp_sum64(long long v) {
          (long long)__reduce_add_sync(0xffffffffu, lo);
 }
 
-// Full-warp sum of 32-bit unsigned values (any value per lane): hi = v >> 24 < 2^8 and
-// lo < 2^24 summed separately.
-__device__ __forceinline__ long long warp_sum_u32(unsigned v) {
-  return (long long)__reduce_add_sync(0xffffffffu, v >> 24) * (1LL << 24) +
-         (long long)__reduce_add_sync(0xffffffffu, v & 0xFFFFFFu);
+// Full-warp sums of three 32-bit values of at most 2^31 each: the low 27 bits of 32 lanes fit
+// 32 bits, the high parts (at most 2^4, sums at most 2^9) share one word.
+__device__ __forceinline__ void warp_sum3_u31(const unsigned (&v)[3], long long (&out)[3]) {
+  const unsigned h = __reduce_add_sync(0xffffffffu, (v[0] >> 27) | (v[1] >> 27) << 10 |
+                                                        (v[2] >> 27) << 20);
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    out[c] = (long long)((h >> (10 * c)) & 1023u) * (1LL << 27) +
+             (long long)__reduce_add_sync(0xffffffffu, v[c] & 0x7FFFFFFu);
 }
+// All of n floats in [+0, 1], given the largest of their bit patterns (-0 is not, nor NaN).
+__device__ __forceinline__ bool unit_bits(unsigned max_bits) { return max_bits <= 0x3f800000u; }
 // Colours in [0, 1] (the usual RGB input): their 2^28 fixed point is one conversion and
 // fits 32 bits, and so does a lane's sum of 8 (< 2^31); squares at 2^20 likewise, and a
 // warp's sum of 256 of those (< 2^29) fits one 32-bit reduction.
@@ -263,17 +270,49 @@ __device__ __forceinline__ void label_rounds(const int (&lab)[8], unsigned pend,
     const unsigned any = __ballot_sync(0xffffffffu, pend != 0);
     if (!any) break;
     const int src = __ffs(any) - 1;
-    int first = -1;
-#pragma unroll
-    for (int i = 7; i >= 0; i--)
-      if ((pend >> i) & 1u) first = lab[i];
-    const int k = __shfl_sync(0xffffffffu, first, src);
+    const int r = __ffs(__shfl_sync(0xffffffffu, pend, src)) - 1;   // its first pending row
+    const bool b0 = r & 1, b1 = r & 2, b2 = r & 4;
+    const int v0 = b1 ? (b0 ? lab[3] : lab[2]) : (b0 ? lab[1] : lab[0]);
+    const int v1 = b1 ? (b0 ? lab[7] : lab[6]) : (b0 ? lab[5] : lab[4]);
+    const int k = __shfl_sync(0xffffffffu, b2 ? v1 : v0, src);
     unsigned m = 0;
 #pragma unroll
     for (int i = 0; i < 8; i++) m |= (unsigned)(lab[i] == k) << i;
     pend &= ~m;
     body(k, m, src);
   }
+}
+
+// Sums over the rows of a mask (8 bits) of their numbers, and of the squares << 8.
+__device__ __forceinline__ unsigned row_sums(unsigned m) {
+  // i = b0 + 2 b1 + 4 b2: i^2 = b0 + 4 b1 + 16 b2 + 4 b0 b1 + 8 b0 b2 + 16 b1 b2
+  const int p0 = __popc(m & 0xAA), p1 = __popc(m & 0xCC), p2 = __popc(m & 0xF0);
+  const int p01 = __popc(m & 0x88), p02 = __popc(m & 0xA0), p12 = __popc(m & 0xC0);
+  return (unsigned)(p0 + 2 * p1 + 4 * p2) |
+         (unsigned)(p0 + 4 * p1 + 16 * p2 + 4 * p01 + 8 * p02 + 16 * p12) << 8;
+}
+// Count and position moments of the warp's pixels of one label, relative to its 32 x 8
+// block: m the lane's rows, y = row_sums(m).  Two sums share a reduction's word.
+struct Moments {
+  int n, x, y, xx, xy, yy;
+};
+__device__ __forceinline__ Moments block_moments(unsigned m, unsigned y, unsigned lane) {
+  const unsigned n = __popc(m), sy = y & 255u;
+  const unsigned a = __reduce_add_sync(0xffffffffu, n | (n * lane) << 10);
+  const unsigned b = __reduce_add_sync(0xffffffffu, sy | (n * lane * lane) << 11);
+  const unsigned d = __reduce_add_sync(0xffffffffu, (y >> 8) | (lane * sy) << 13);
+  return Moments{(int)(a & 1023u), (int)(a >> 10), (int)(b & 2047u),
+                 (int)(b >> 11), (int)(d >> 13), (int)(d & 8191u)};
+}
+// Adds the moments of a block at (X, Y) to the sums of x, y, xx, xy, yy at p.
+__device__ __forceinline__ void add_moments(unsigned long long* p, const Moments& b, long long X,
+                                            long long Y) {
+  const long long n = b.n;
+  atomicAdd(p + 0, (unsigned long long)(n * X + b.x));
+  atomicAdd(p + 1, (unsigned long long)(n * Y + b.y));
+  atomicAdd(p + 2, (unsigned long long)(n * X * X + 2 * X * b.x + b.xx));
+  atomicAdd(p + 3, (unsigned long long)(n * X * Y + X * b.y + Y * b.x + b.xy));
+  atomicAdd(p + 4, (unsigned long long)(n * Y * Y + 2 * Y * b.y + b.yy));
 }
 
 // The 32 x 8 block of warp w of a block of the 64 x 32 tile grid of a W-wide frame:

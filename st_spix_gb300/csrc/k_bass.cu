@@ -309,7 +309,9 @@ __global__ void kb_init_prior_mu(const Slot* __restrict__ slots) {
 // [0, 1] are summed in 32 bits (one conversion each); others wait in the warp's shared
 // staging rows `cw` and are converted and summed in 64 bits in their label's round.
 // Integer sums: the totals do not depend on the grouping or the order of the adds.
-__device__ __forceinline__ void block_stats(const Slot& S, int bx, int by, float (*cw)[3][32]) {
+// ytab: row_sums of the 256 masks of rows.
+__device__ __forceinline__ void block_stats(const Slot& S, int bx, int by, float (*cw)[3][32],
+                                            const unsigned* ytab) {
   const int lane = threadIdx.x & 31;
   const int H = S.H, W = S.W;
   const SpDev& sp = S.sp;
@@ -317,8 +319,7 @@ __device__ __forceinline__ void block_stats(const Slot& S, int bx, int by, float
   const int gx = bx + lane;
   int lab[8];
   float c[8][3];
-  unsigned pend = 0;
-  bool unit = true;
+  unsigned pend = 0, top = 0;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     const int gy = by + i;
@@ -328,50 +329,37 @@ __device__ __forceinline__ void block_stats(const Slot& S, int bx, int by, float
 #pragma unroll
     for (int ch = 0; ch < 3; ch++) {
       c[i][ch] = in ? S.img[3 * g + ch] : 0.f;
-      unit &= unit_colour(c[i][ch]);
+      top = max(top, __float_as_uint(c[i][ch]));
     }
     if (lab[i] >= 0 && lab[i] < cap) pend |= 1u << i;
   }
   // the warp's totals of label k given its colour sums: count and position moments
-  // (relative to the block, so they fit 32 bits), one set of atomics
-  auto add = [&](int k, unsigned m, int src, long long S0, long long S1, long long S2) {
-    int sy = 0, syy = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-      if ((m >> i) & 1u) { sy += i; syy += i * i; }
-    const int n = __popc(m);
-    const int N = __reduce_add_sync(0xffffffffu, n);
-    const int SX = __reduce_add_sync(0xffffffffu, n * lane);
-    const int SXX = __reduce_add_sync(0xffffffffu, n * lane * lane);
-    const int SY = __reduce_add_sync(0xffffffffu, sy);
-    const int SYY = __reduce_add_sync(0xffffffffu, syy);
-    const int SXY = __reduce_add_sync(0xffffffffu, lane * sy);
+  // (relative to the block, two to a word), one set of atomics
+  auto add = [&](int k, unsigned m, int src, const long long (&St)[3]) {
+    const Moments b = block_moments(m, ytab[m], lane);
     if (lane == src) {
-      const long long ln = N, X = bx, Y = by;
       unsigned long long* acc = (unsigned long long*)(sp.acc + 8 * (size_t)k);
-      atomicAdd(&sp.count[k], N);
-      atomicAdd(acc + 0, (unsigned long long)S0);
-      atomicAdd(acc + 1, (unsigned long long)S1);
-      atomicAdd(acc + 2, (unsigned long long)S2);
-      atomicAdd(acc + 3, (unsigned long long)(ln * X + SX));
-      atomicAdd(acc + 4, (unsigned long long)(ln * Y + SY));
-      atomicAdd(acc + 5, (unsigned long long)(ln * X * X + 2 * X * SX + SXX));
-      atomicAdd(acc + 6, (unsigned long long)(ln * X * Y + X * SY + Y * SX + SXY));
-      atomicAdd(acc + 7, (unsigned long long)(ln * Y * Y + 2 * Y * SY + SYY));
+      atomicAdd(&sp.count[k], b.n);
+      atomicAdd(acc + 0, (unsigned long long)St[0]);
+      atomicAdd(acc + 1, (unsigned long long)St[1]);
+      atomicAdd(acc + 2, (unsigned long long)St[2]);
+      add_moments(acc + 3, b, bx, by);
     }
   };
-  if (__all_sync(0xffffffffu, unit)) {
+  if (__all_sync(0xffffffffu, unit_bits(top))) {
     unsigned q[8][3];
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
       for (int ch = 0; ch < 3; ch++) q[i][ch] = fx_unit(c[i][ch], kFxAppShift);
     label_rounds(lab, pend, [&](int k, unsigned m, int src) {
-      unsigned s0 = 0, s1 = 0, s2 = 0;
+      unsigned s[3] = {0, 0, 0};
 #pragma unroll
       for (int i = 0; i < 8; i++)
-        if ((m >> i) & 1u) { s0 += q[i][0]; s1 += q[i][1]; s2 += q[i][2]; }
-      add(k, m, src, warp_sum_u32(s0), warp_sum_u32(s1), warp_sum_u32(s2));
+        if ((m >> i) & 1u) { s[0] += q[i][0]; s[1] += q[i][1]; s[2] += q[i][2]; }
+      long long St[3];
+      warp_sum3_u31(s, St);
+      add(k, m, src, St);
     });
     return;
   }
@@ -383,14 +371,15 @@ __device__ __forceinline__ void block_stats(const Slot& S, int bx, int by, float
     for (int ch = 0; ch < 3; ch++) cw[i][ch][lane] = c[i][ch];
   __syncwarp();
   label_rounds(lab, pend, [&](int k, unsigned m, int src) {
-    long long s0 = 0, s1 = 0, s2 = 0;
+    long long s[3] = {0, 0, 0};
     for (unsigned mm = m; mm; mm &= mm - 1) {
       const int i = __ffs(mm) - 1;
-      s0 += fx_q(cw[i][0][lane], kFxAppShift);
-      s1 += fx_q(cw[i][1][lane], kFxAppShift);
-      s2 += fx_q(cw[i][2][lane], kFxAppShift);
+#pragma unroll
+      for (int ch = 0; ch < 3; ch++) s[ch] += fx_q(cw[i][ch][lane], kFxAppShift);
     }
-    add(k, m, src, warp_sum64(s0), warp_sum64(s1), warp_sum64(s2));
+#pragma unroll
+    for (int ch = 0; ch < 3; ch++) s[ch] = warp_sum64(s[ch]);
+    add(k, m, src, s);
   });
 }
 
@@ -411,8 +400,11 @@ __global__ void __launch_bounds__(256, 4) kb_accumulate(const Slot* __restrict__
   const int tiles_x = (S.W + 63) / 64;
   const int warp = threadIdx.x >> 5;
   __shared__ float cs[8][8][3][32];   // [warp][row][channel][lane]
+  __shared__ unsigned ytab[256];
+  ytab[threadIdx.x] = row_sums(threadIdx.x);
+  __syncthreads();
   block_stats(S, (tl % tiles_x) * 64 + (warp & 1) * 32, (tl / tiles_x) * 32 + (warp >> 1) * 8,
-              cs[warp]);
+              cs[warp], ytab);
 }
 
 // Accumulator precision study: colour sums by per-pixel FP32 (mode 1, as the
@@ -531,6 +523,8 @@ __device__ __forceinline__ void smooth_prior(double in_x, double in_y, double in
 // expressions of the same inputs).  The prior shape term is read from S.pscache then, which
 // the last full posterior wrote.
 //
+// merged: the sums come from a merge (S.tmp, see kb_merge_apply) and become the slot's.
+//
 // log64: sp.logdet in FP64 (the state read-out); otherwise its float, which is all that the
 // records and the parameter read-out take of it.
 //
@@ -542,7 +536,7 @@ __device__ __forceinline__ void smooth_prior(double in_x, double in_y, double in
 // quotient and the log in FP64, 5.7, 7.6 and 11.6 (and 32.4 on 16 frames of mixed sizes);
 // now 5.0, 6.5, 7.9 (and 17.9; the last step the spread of the groups, see SLOT_X).
 __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slots,
-                                                    int incremental, int log64) {
+                                                    int incremental, int log64, int merged) {
   pdl_enter();
   SLOT_X;
   __shared__ double v_ps[3][32], v_den[3][32], v_m[2][32], v_s[3][32], v_ld[32];
@@ -565,9 +559,9 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
     double q0 = 0, q1 = 0, q2 = 0, i0 = 0, i1 = 0, i2 = 0;
     uint4 orec[3];
     if (k < cap) {
-      const long long* acc = sp.acc + 8 * (size_t)k;
+      const long long* acc = (merged ? S.tmp.acc : sp.acc) + 8 * (size_t)k;
       const long long* snap = S.snap + 9 * (size_t)k;
-      count_int = sp.count[k];
+      count_int = (merged ? S.tmp.count : sp.count)[k];
       valid = sp.valid[k];
       pc = sp.prior_count[k];
       if (w < 3) {
@@ -658,6 +652,12 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
       if (w < 3) {
         snap[f0] = a[0];
         snap[f1] = a[3];
+      }
+      if (merged && w < 3) {
+        long long* acc = sp.acc + 8 * (size_t)k;
+        acc[f0] = a[0];
+        acc[f1] = a[3];
+        if (w == 0) { acc[1] = a[1]; acc[2] = a[2]; sp.count[k] = count_int; }
       }
       if (w == 0) {
         snap[1] = a[1];

@@ -35,6 +35,8 @@ __device__ __forceinline__ void sm_clear(const SmDev& sm, int k) {
   sm.ninvalid[k] = 0;
 #pragma unroll
   for (int c = 0; c < 3; c++) { sm.s[3 * (size_t)k + c] = 0; sm.sq[3 * (size_t)k + c] = 0; }
+#pragma unroll
+  for (int c = 0; c < 5; c++) sm.pos[5 * (size_t)k + c] = 0;
 }
 
 __global__ void kb_split_seed(const Slot* __restrict__ slots, int dir_bass, int dir_prop) {
@@ -457,7 +459,13 @@ __global__ void kb_split_partition(const Slot* __restrict__ slots) {
 // sum_by_label over split/merge labels (split_merge.cu:862-891,
 // split_merge_prop.cu:1942-2018): count, colour sums, square sums, invalid count.
 // split: labels = split labels, invalid counts against the shifted labels (prop
-// slots); merge: labels = current labels, ids < cap.
+// slots); merge: labels = current labels, ids < cap, and only the square sums, all that the
+// merge decisions read here (their counts and colour sums are the current statistics).
+// The split's halves also sum their positions: an accepted split takes them over as its
+// statistics (kb_split_commit), as a merge adds its ids' sums (kb_merge_apply), so neither is
+// followed by a clear and a pass over the pixels (5 and 27 us on 8 frames of 480x854; the
+// positions cost 4 here, the merge's sums 3).  What bounds it is its instructions (60 % of
+// the issue slots, 1300 a warp); the merge's passes took 33 us there with all sums, now 17.
 // Grid: the 64 x 32 tiles of a slot; warp w of a block owns the tile's 32 x 8 block
 // (w & 1, w >> 1), a lane one column of it.  The warp takes the block's labels one at a
 // time (the label of the lowest lane that still has pixels): each lane sums its pixels of
@@ -465,10 +473,9 @@ __global__ void kb_split_partition(const Slot* __restrict__ slots) {
 // one set of atomics.  Unit colours (all of the warp's in [0, 1]) are summed in 32 bits;
 // other colours wait in shared memory and a lane converts each pixel in its label's round.
 // Integer sums (R1): totals do not depend on the grouping.
-__global__ void __launch_bounds__(256, 4) kb_sm_accumulate(const Slot* __restrict__ slots, int split) {
-  pdl_enter();
-  SLOT_Y;
-  __shared__ float cs[8][8][3][32];   // [warp][row][channel][lane]
+template <bool split>
+__device__ __forceinline__ void sm_accumulate(const Slot& S, float (*cs)[8][3][32],
+                                              const unsigned* ytab) {
   const int H = S.H, W = S.W;
   int gx, by;
   if (!warp_block(W, H, gx, by)) return;
@@ -481,8 +488,7 @@ __global__ void __launch_bounds__(256, 4) kb_sm_accumulate(const Slot* __restric
   float (*cw)[3][32] = cs[warp];
   int lab[8];
   float c[8][3];
-  unsigned inv = 0, pend = 0;
-  bool unit = true;
+  unsigned inv = 0, pend = 0, top = 0;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     const int gy = by + i;
@@ -492,31 +498,39 @@ __global__ void __launch_bounds__(256, 4) kb_sm_accumulate(const Slot* __restric
 #pragma unroll
     for (int ch = 0; ch < 3; ch++) {
       c[i][ch] = in ? img[3 * g + ch] : 0.f;
-      unit &= unit_colour(c[i][ch]);
+      top = max(top, __float_as_uint(c[i][ch]));
     }
     if (shifted && in && shifted[g] < 0) inv |= 1u << i;
     if (lab[i] >= 0 && lab[i] < cap) pend |= 1u << i;
   }
   auto add = [&](int k, unsigned m, int src, const long long (&St)[3], const long long (&Qt)[3]) {
-    const int N = __reduce_add_sync(0xffffffffu, __popc(m));
-    const int NI = shifted ? __reduce_add_sync(0xffffffffu, __popc(m & inv)) : 0;
+    Moments b{};
+    int NI = 0;
+    if (split) {
+      b = block_moments(m, ytab[m], lane);
+      if (shifted) NI = __reduce_add_sync(0xffffffffu, __popc(m & inv));
+    }
     if (lane == src) {
-      atomicAdd(&sm.count[k], N);
-      if (NI) atomicAdd(&sm.ninvalid[k], NI);
+      if (split) {
+        atomicAdd(&sm.count[k], b.n);
+        if (NI) atomicAdd(&sm.ninvalid[k], NI);
+        add_moments((unsigned long long*)sm.pos + 5 * (size_t)k, b, gx - lane, by);
+      }
 #pragma unroll
       for (int ch = 0; ch < 3; ch++) {
-        atomicAdd((unsigned long long*)&sm.s[3 * (size_t)k + ch], (unsigned long long)St[ch]);
+        if (split)
+          atomicAdd((unsigned long long*)&sm.s[3 * (size_t)k + ch], (unsigned long long)St[ch]);
         atomicAdd((unsigned long long*)&sm.sq[3 * (size_t)k + ch], (unsigned long long)Qt[ch]);
       }
     }
   };
-  if (__all_sync(0xffffffffu, unit)) {
+  if (__all_sync(0xffffffffu, unit_bits(top))) {
     unsigned qs[8][3], qq[8][3];
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
       for (int ch = 0; ch < 3; ch++) {
-        qs[i][ch] = fx_unit(c[i][ch], kFxAppShift);
+        qs[i][ch] = split ? fx_unit(c[i][ch], kFxAppShift) : 0;
         qq[i][ch] = fx_unit(c[i][ch] * c[i][ch], kFxSqShift);
       }
     label_rounds(lab, pend, [&](int k, unsigned m, int src) {
@@ -525,14 +539,15 @@ __global__ void __launch_bounds__(256, 4) kb_sm_accumulate(const Slot* __restric
       for (int i = 0; i < 8; i++)
         if ((m >> i) & 1u) {
 #pragma unroll
-          for (int ch = 0; ch < 3; ch++) { s[ch] += qs[i][ch]; q[ch] += qq[i][ch]; }
+          for (int ch = 0; ch < 3; ch++) {
+            if (split) s[ch] += qs[i][ch];
+            q[ch] += qq[i][ch];
+          }
         }
-      long long St[3], Qt[3];
+      long long St[3] = {0, 0, 0}, Qt[3];
+      if (split) warp_sum3_u31(s, St);
 #pragma unroll
-      for (int ch = 0; ch < 3; ch++) {
-        St[ch] = warp_sum_u32(s[ch]);
-        Qt[ch] = (long long)__reduce_add_sync(0xffffffffu, q[ch]);
-      }
+      for (int ch = 0; ch < 3; ch++) Qt[ch] = (long long)__reduce_add_sync(0xffffffffu, q[ch]);
       add(k, m, src, St, Qt);
     });
     return;
@@ -551,15 +566,33 @@ __global__ void __launch_bounds__(256, 4) kb_sm_accumulate(const Slot* __restric
 #pragma unroll
       for (int ch = 0; ch < 3; ch++) {
         const float v = cw[i][ch][lane];
-        s[ch] += fx_q(v, kFxAppShift);
+        if (split) s[ch] += fx_q(v, kFxAppShift);
         q[ch] += fx_q(v * v, kFxSqShift);
       }
     }
     long long St[3], Qt[3];
 #pragma unroll
-    for (int ch = 0; ch < 3; ch++) { St[ch] = warp_sum64(s[ch]); Qt[ch] = warp_sum64(q[ch]); }
+    for (int ch = 0; ch < 3; ch++) {
+      St[ch] = split ? warp_sum64(s[ch]) : 0;
+      Qt[ch] = warp_sum64(q[ch]);
+    }
     add(k, m, src, St, Qt);
   });
+}
+__global__ void __launch_bounds__(256, 4) kb_sm_accumulate(const Slot* __restrict__ slots) {
+  pdl_enter();
+  SLOT_Y;
+  __shared__ float cs[8][8][3][32];   // [warp][row][channel][lane]
+  __shared__ unsigned ytab[256];
+  ytab[threadIdx.x] = row_sums(threadIdx.x);
+  __syncthreads();
+  sm_accumulate<true>(S, cs, ytab);
+}
+__global__ void __launch_bounds__(256, 4) kb_sq_accumulate(const Slot* __restrict__ slots) {
+  pdl_enter();
+  SLOT_Y;
+  __shared__ float cs[8][8][3][32];
+  sm_accumulate<false>(S, cs, nullptr);
 }
 
 // Marginal of one superpixel over the three colour channels, FP64: the
@@ -703,6 +736,24 @@ __global__ void kb_split_commit(const Slot* __restrict__ slots) {
       sp.prior_icov[3 * snew] = pcs; sp.prior_icov[3 * snew + 1] = 0; sp.prior_icov[3 * snew + 2] = pcs;
     }
     sp.valid[snew] = 1;
+    // the sums of the halves: the statistics after the split, without a pass over the pixels
+    const int half = k + sc->tmp1;
+    const bool second = !prop_mode || (fl & 8);      // the new id takes the second half
+    const int a = second ? k : half, b = second ? half : k;
+    sp.count[k] = sm.count[a];
+    sp.count[snew] = sm.count[b];
+    long long* ak = sp.acc + 8 * (size_t)k;
+    long long* an = sp.acc + 8 * (size_t)snew;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      ak[c] = sm.s[3 * (size_t)a + c];
+      an[c] = sm.s[3 * (size_t)b + c];
+    }
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+      ak[3 + c] = sm.pos[5 * (size_t)a + c];
+      an[3 + c] = sm.pos[5 * (size_t)b + c];
+    }
   }
 }
 
@@ -879,6 +930,10 @@ __global__ void kb_merge_clear(const Slot* __restrict__ slots) {
   FOR_ID(k, sm_ids(S)) {
     sm_clear(S.sm, k);
     if (k >= n_ids) continue;
+    S.tmp.count[k] = 0;
+    ulonglong2* acc = (ulonglong2*)(S.tmp.acc + 8 * (size_t)k);
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[c] = make_ulonglong2(0, 0);
     S.sm.pair[k] = -1;
     S.sm.claim[k] = 0x7f7f7f7f;
   }
@@ -937,13 +992,35 @@ __global__ void kb_merge_remove(const Slot* __restrict__ slots) {
   }
 }
 
-// merge_sp (split_merge.cu:984-1000).
-__global__ void kb_merge_apply(const Slot* __restrict__ slots) {
+// merge_sp (split_merge.cu:984-1000).  The statistics after the step need no pass over the
+// pixels: every pixel of label v before the step (and the relabel that precedes it on
+// propagated slots, S.rid) ends up with one label, so v's sums are added to that label's in
+// S.tmp (cleared by kb_merge_clear), which the posterior takes over.  An id that the relabel
+// revived or minted had no pixels; its count field holds its source's by then.
+__global__ void kb_merge_apply(const Slot* __restrict__ slots, int sums) {
   pdl_enter();
   SLOT_Y;
   int* __restrict__ seg = S.seg;
   const int cap = S.cap;
   const SmDev& sm = S.sm;
+  if (sums) {
+    const int prop_mode = S.mode;
+    FOR_ID(v, live_ids(S)) {
+      const int n = S.sp.count[v];
+      if (n <= 0 || (prop_mode && S.src_of[v] >= 0)) continue;
+      int k = v;
+      if (prop_mode) {
+        const int r = S.rid[v];
+        if (r >= 0 && r < cap) k = r;
+      }
+      if (sm.flag[k] & 4) k = sm.target[k];
+      atomicAdd(&S.tmp.count[k], n);
+      const long long* a = S.sp.acc + 8 * (size_t)v;
+      unsigned long long* t = (unsigned long long*)S.tmp.acc + 8 * (size_t)k;
+#pragma unroll
+      for (int c = 0; c < 8; c++) atomicAdd(t + c, (unsigned long long)a[c]);
+    }
+  }
   FOR_PIX(t, S.npix) {
     const int k = seg[t];
     if (k < 0 || k >= cap) continue;

@@ -30,7 +30,7 @@ __global__ void kb_init_bass_params(const Slot* slots);
 __global__ void kb_init_prior_mu(const Slot* slots);
 __global__ void kb_clear_stats(const Slot* slots, int all);
 __global__ void kb_accumulate(const Slot* slots, int B);
-__global__ void kb_posterior(const Slot* slots, int incremental, int log64);
+__global__ void kb_posterior(const Slot* slots, int incremental, int log64, int merged);
 __global__ void kb_accumulate_fp(const Slot* slots, int mode);
 __global__ void kb_accumulate_fp_store(const Slot* slots, int mode);
 __global__ void kb_accumulate_fp_clear(const Slot* slots);
@@ -77,7 +77,8 @@ __global__ void kb_bbox(const Slot* slots);
 __global__ void kb_split_bfs(const Slot* slots, int dir_bass, int dir_prop);
 __global__ void kb_split_bfs_big(const Slot* slots);
 __global__ void kb_split_partition(const Slot* slots);
-__global__ void kb_sm_accumulate(const Slot* slots, int split);
+__global__ void kb_sm_accumulate(const Slot* slots);
+__global__ void kb_sq_accumulate(const Slot* slots);
 __global__ void kb_split_decide(const Slot* slots, SmConsts K, float split_alpha);
 __global__ void kb_split_commit(const Slot* slots);
 __global__ void kb_split_apply(const Slot* slots);
@@ -88,7 +89,7 @@ __global__ void kb_merge_single(const Slot* slots, SmConsts K);
 __global__ void kb_merge_decide(const Slot* slots, SmConsts K, float merge_alpha);
 __global__ void kb_merge_flag(const Slot* slots);
 __global__ void kb_merge_remove(const Slot* slots);
-__global__ void kb_merge_apply(const Slot* slots);
+__global__ void kb_merge_apply(const Slot* slots, int sums);
 
 // k_prop.cu
 __global__ void kb_prop_clear(const Slot* slots);
