@@ -25,6 +25,10 @@ namespace stspix {
 constexpr int kFxAppShift = 28;
 constexpr int kFxSqShift = 20;
 constexpr int kFxFlowShift = 24;
+// The hole fill in one launch (kb_fill): a cluster of blocks per slot, each with two lists of
+// up to kFillList holes in shared memory; one block up to kFillSolo holes (a 720x1280 frame's
+// second fill takes 32 us in one block, 44 in a cluster; limits of 4,096 to 16,384 time alike).
+constexpr int kFillSolo = 4096, kFillList = 16384, kFillSmem = 2 * kFillList * 4;
 constexpr int kFillBreakIter = 1000;      // fill_missing.cu: break_iter
 constexpr int kSweepVariants = 3;         // sweep tile shapes: 32x32, 64x32, 16x32
 constexpr int kMaxBatchGraphs = 64;       // captured batch steps kept per context
@@ -138,7 +142,7 @@ struct Slot {
   const float* img;        // [npix*3] the colours the path reads
   const float* img_src;    // [npix*3] the caller's frame when it is converted to CIELAB
                            // into img at ingest (stspix_config.lab_ingest), else null
-  double inv_w, inv_h;     // 1 / W, 1 / H (the hole fill's quotients, see fill_quot)
+  float2 inv_w, inv_h;     // 1 / W, 1 / H as pairs of floats (the hole fill, see fill_quot)
   int* seg;                // working labels (the caller's output)
   int* seg_alt;            // ping-pong labels for the sweeps
   int H, W, npix;
@@ -169,6 +173,7 @@ struct Slot {
   long long* fs;
   float *fds, *ss;
   double* centers;
+  float4* centers_ff;      // [cap+2]: the centres as pairs of floats (x, y)
   unsigned long long *rbest, *ccbest;
   int* bbox;               // [4*(cap+2)]: x0, x1, y0, y1 per superpixel (split BFS)
   long long* snap;         // [9*(cap+2)]: count and the 8 sums each id's posterior last saw
