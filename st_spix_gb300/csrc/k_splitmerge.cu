@@ -39,33 +39,37 @@ __device__ __forceinline__ void sm_clear(const SmDev& sm, int k) {
   for (int c = 0; c < 5; c++) sm.pos[5 * (size_t)k + c] = 0;
 }
 
-__global__ void kb_split_seed(const Slot* __restrict__ slots, int dir_bass, int dir_prop) {
+// The second halves of a split, one bit per pixel: row y, word x >> 5, bit x & 31 (in the
+// buffer of the shift's hits, which only the shift and its fill use).  A superpixel's rows set
+// their bits by a few atomics; the pixels' own labels and this bit are the split labels.
+// (Before, the distances of every pixel were cleared, and compared into split labels that the
+// sums and the relabelling read: two passes over the pixels and 26 bytes of them more, 37 us
+// of a split of a 2160x3840 frame, 6 of a 480x854 one.)
+__device__ __forceinline__ unsigned* half_bits(const Slot& S) { return (unsigned*)S.hits; }
+__device__ __forceinline__ int half_pitch(const Slot& S) { return (S.W + 31) >> 5; }
+// Sets the bits b of the 64 pixels from x of a row of the bits.
+__device__ __forceinline__ void set_half(unsigned* row, int x, unsigned long long b) {
+  const int w = x >> 5, s = x & 31;
+  const unsigned lo = (unsigned)b, hi = (unsigned)(b >> 32);
+  const unsigned v[3] = {lo << s, __funnelshift_l(lo, hi, s), __funnelshift_l(hi, 0u, s)};
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+    if (v[i]) atomicOr(row + w + i, v[i]);
+}
+
+// Clears a split's sums and bits, and the boxes.
+__global__ void kb_split_clear(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
-  const SpDev& sp = S.sp;
-  const int direction = S.mode ? dir_prop : dir_bass;
   const int n_ids = live_ids(S);
   FOR_ID(k, sm_ids(S)) {
     sm_clear(S.sm, k);
     if (k >= n_ids) continue;
     int* bb = S.bbox + 4 * (size_t)k;
     bb[0] = INT32_MAX; bb[1] = -1; bb[2] = INT32_MAX; bb[3] = -1;
-    if (!S.sc->tmp0 /*split_on*/ || !sp.valid[k]) continue;
-    for (int s = 0; s < 2; s++) {
-      const int ind = split_seed_index(S, k, s, direction);
-      if (ind >= 0) (s == 0 ? S.d1 : S.d2)[ind] = 1;
-    }
   }
-}
-
-// d1 = d2 = -1 (unreached) before the split seeds.
-__global__ void kb_split_clear(const Slot* __restrict__ slots) {
-  pdl_enter();
-  SLOT_Y;
-  FOR_PIX(t, S.npix) {
-    S.d1[t] = -1;
-    S.d2[t] = -1;
-  }
+  unsigned* half = half_bits(S);
+  FOR_ID(q, S.H * half_pitch(S)) half[q] = 0;
 }
 
 __global__ void kb_split_begin(const Slot* __restrict__ slots, int B) {
@@ -238,7 +242,7 @@ __device__ void bfs_bits(int t, int k, int x0, int y0, int bw, int bh, int W,
 // read; only the comparison d1 > d2 is written, once, at the end.
 template <int R, int C>
 __device__ __forceinline__ void bfs_reg(int k, int x0, int y0, int bw, int bh, int W,
-                                        const int* __restrict__ seg, int* d1, int* d2,
+                                        const int* __restrict__ seg, unsigned* half,
                                         int seed1, int seed2) {
   using u64 = unsigned long long;
   const int lane = threadIdx.x & 31;
@@ -311,9 +315,10 @@ __device__ __forceinline__ void bfs_reg(int k, int x0, int y0, int bw, int bh, i
       for (int w = 0; w < C; w++) { f[j][w] = n[j][w]; v[j][w] |= n[j][w]; any |= n[j][w]; }
     return any;
   };
-  // The split's only use of the distances is d1 > d2 (kb_split_partition): true where seed
-  // 1 reaches a pixel and seed 2 reaches it strictly later or never.  early2: pixels seed 2
-  // reached in a layer where seed 1 had not (yet) reached them, seed 2 itself included.
+  // The split's only use of the distances is d1 > d2 (calc_seg_split, split_merge.cu:847-859):
+  // true where seed 1 reaches a pixel and seed 2 reaches it strictly later or never.  early2:
+  // pixels seed 2 reached in a layer where seed 1 had not (yet) reached them, seed 2 itself
+  // included.
   u64 early2[R][C];
 #pragma unroll
   for (int j = 0; j < R; j++)
@@ -329,31 +334,14 @@ __device__ __forceinline__ void bfs_reg(int k, int x0, int y0, int bw, int bh, i
       for (int w = 0; w < C; w++) early2[j][w] |= f2[j][w] & ~v1[j][w];
     if (!__any_sync(0xffffffffu, (a1 | a2) != 0ull)) break;
   }
-  // Distances that give the same comparison: d2 keeps -1 but 1 at seed 2 (kb_split_seed),
-  // so d1 := 2 on the pixels with d1 > d2 and d1 := -1 at seed 1 when it has not.
+  const int pitch = (W + 31) >> 5;
 #pragma unroll
   for (int j = 0; j < R; j++)
 #pragma unroll
     for (int w = 0; w < C; w++) {
       const u64 second = v1[j][w] & (~v2[j][w] | early2[j][w]);
-      if (second) {
-        int* row = d1 + (size_t)(y0 + lane * R + j) * W + x0 + 64 * w;
-        for (u64 b = second; b; b &= b - 1) row[__ffsll((long long)b) - 1] = 2;
-      }
+      if (second) set_half(half + (size_t)(y0 + lane * R + j) * pitch, x0 + 64 * w, second);
     }
-  if (seed1 >= 0) {
-    // the seed's word selected by masks (an indexed read would put the arrays in local
-    // memory)
-    const int r1 = seed1 / W - y0 - lane * R, c1 = seed1 % W - x0;
-    u64 word = 0;
-#pragma unroll
-    for (int j = 0; j < R; j++)
-#pragma unroll
-      for (int w = 0; w < C; w++)
-        word |= (v1[j][w] & (~v2[j][w] | early2[j][w])) &
-                (0ull - (u64)(r1 == j && (c1 >> 6) == w));
-    if (r1 >= 0 && r1 < R && !((word >> (c1 & 63)) & 1ull)) d1[seed1] = -1;
-  }
 }
 
 __global__ void __launch_bounds__(128, 4) kb_split_bfs(const Slot* __restrict__ slots, int dir_bass,
@@ -363,6 +351,7 @@ __global__ void __launch_bounds__(128, 4) kb_split_bfs(const Slot* __restrict__ 
   if (!S.sc->tmp0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int direction = S.mode ? dir_prop : dir_bass;
+  unsigned* half = half_bits(S);
   const int n = min(S.cap, S.sc->max_spix + 1);
   for (int k = blockIdx.x * 4 + warp; k < n; k += gridDim.x * 4) {
     if (!S.sp.valid[k]) continue;
@@ -379,24 +368,25 @@ __global__ void __launch_bounds__(128, 4) kb_split_bfs(const Slot* __restrict__ 
     const int R = (bh + 31) >> 5;
     if (bw <= 64) {
       switch (R) {
-        case 1: bfs_reg<1, 1>(k, x0, y0, bw, bh, S.W, S.seg, S.d1, S.d2, s1, s2); break;
-        case 2: bfs_reg<2, 1>(k, x0, y0, bw, bh, S.W, S.seg, S.d1, S.d2, s1, s2); break;
-        case 3: bfs_reg<3, 1>(k, x0, y0, bw, bh, S.W, S.seg, S.d1, S.d2, s1, s2); break;
-        default: bfs_reg<4, 1>(k, x0, y0, bw, bh, S.W, S.seg, S.d1, S.d2, s1, s2); break;
+        case 1: bfs_reg<1, 1>(k, x0, y0, bw, bh, S.W, S.seg, half, s1, s2); break;
+        case 2: bfs_reg<2, 1>(k, x0, y0, bw, bh, S.W, S.seg, half, s1, s2); break;
+        case 3: bfs_reg<3, 1>(k, x0, y0, bw, bh, S.W, S.seg, half, s1, s2); break;
+        default: bfs_reg<4, 1>(k, x0, y0, bw, bh, S.W, S.seg, half, s1, s2); break;
       }
     } else {
       switch (R) {
-        case 1: bfs_reg<1, 2>(k, x0, y0, bw, bh, S.W, S.seg, S.d1, S.d2, s1, s2); break;
-        case 2: bfs_reg<2, 2>(k, x0, y0, bw, bh, S.W, S.seg, S.d1, S.d2, s1, s2); break;
-        case 3: bfs_reg<3, 2>(k, x0, y0, bw, bh, S.W, S.seg, S.d1, S.d2, s1, s2); break;
-        default: bfs_reg<4, 2>(k, x0, y0, bw, bh, S.W, S.seg, S.d1, S.d2, s1, s2); break;
+        case 1: bfs_reg<1, 2>(k, x0, y0, bw, bh, S.W, S.seg, half, s1, s2); break;
+        case 2: bfs_reg<2, 2>(k, x0, y0, bw, bh, S.W, S.seg, half, s1, s2); break;
+        case 3: bfs_reg<3, 2>(k, x0, y0, bw, bh, S.W, S.seg, half, s1, s2); break;
+        default: bfs_reg<4, 2>(k, x0, y0, bw, bh, S.W, S.seg, half, s1, s2); break;
       }
     }
   }
 }
 
 // Block per large box; dynamic shared memory of 5 * kBigRows * kBigWpr words.
-__global__ void __launch_bounds__(256) kb_split_bfs_big(const Slot* __restrict__ slots) {
+__global__ void __launch_bounds__(256) kb_split_bfs_big(const Slot* __restrict__ slots, int dir_bass,
+                                                        int dir_prop) {
   pdl_enter();
   SLOT_Y;
   if (!S.sc->tmp0) return;
@@ -412,6 +402,15 @@ __global__ void __launch_bounds__(256) kb_split_bfs_big(const Slot* __restrict__
     const int* bb = S.bbox + 4 * (size_t)k;
     const int x0 = bb[0], y0 = bb[2];
     const int bw = bb[1] - x0 + 1, bh = bb[3] - y0 + 1, area = bw * bh;
+    const int direction = S.mode ? dir_prop : dir_bass;
+    const int s1 = split_seed_index(S, k, 0, direction), s2 = split_seed_index(S, k, 1, direction);
+    for (int i = threadIdx.x; i < area; i += blockDim.x) {
+      const int g = (y0 + i / bw) * W + x0 + i % bw;
+      if (seg[g] != k) continue;
+      __stcg(d1 + g, g == s1 ? 1 : -1);
+      __stcg(d2 + g, g == s2 ? 1 : -1);
+    }
+    __syncthreads();
     if (bw <= 64 * kBigWpr && bh <= kBigRows) {
       bfs_bits<256, kA / 256>(threadIdx.x, k, x0, y0, bw, bh, W, seg, d1, d2, big, big + kA,
                               big + 2 * kA, big + 3 * kA, big + 4 * kA);
@@ -441,18 +440,12 @@ __global__ void __launch_bounds__(256) kb_split_bfs_big(const Slot* __restrict__
       }
     }
     __syncthreads();
-  }
-}
-
-// calc_seg_split (split_merge.cu:847-859): second half when d1 > d2.
-__global__ void kb_split_partition(const Slot* __restrict__ slots) {
-  pdl_enter();
-  SLOT_Y;
-  const int off = S.sc->tmp1;
-  FOR_PIX(t, S.npix) {
-    int v = S.seg[t];
-    if (S.d1[t] > S.d2[t]) v += off;
-    S.smseg[t] = v;
+    for (int i = threadIdx.x; i < area; i += blockDim.x) {
+      const int x = x0 + i % bw, y = y0 + i / bw, g = y * W + x;
+      if (seg[g] == k && __ldcg(d1 + g) > __ldcg(d2 + g))
+        atomicOr(half_bits(S) + (size_t)y * half_pitch(S) + (x >> 5), 1u << (x & 31));
+    }
+    __syncthreads();
   }
 }
 
@@ -480,7 +473,10 @@ __device__ __forceinline__ void sm_accumulate(const Slot& S, float (*cs)[8][3][3
   int gx, by;
   if (!warp_block(W, H, gx, by)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int* __restrict__ labp = split ? S.smseg : S.seg;
+  const int* __restrict__ labp = S.seg;
+  const int second = split ? S.sc->tmp1 : 0;   // offset of the second halves' labels
+  const unsigned* half = half_bits(S) + (gx >> 5);
+  const int pitch = half_pitch(S);
   const int* __restrict__ shifted = (split && S.mode) ? S.shifted : nullptr;
   const float* __restrict__ img = S.img;
   const int cap = split ? S.cap + 2 : S.cap;
@@ -495,6 +491,7 @@ __device__ __forceinline__ void sm_accumulate(const Slot& S, float (*cs)[8][3][3
     const bool in = gx < W && gy < H;
     const size_t g = (size_t)gy * W + gx;
     lab[i] = in ? labp[g] : -1;
+    if (split && in && ((half[(size_t)gy * pitch] >> (gx & 31)) & 1u)) lab[i] += second;
 #pragma unroll
     for (int ch = 0; ch < 3; ch++) {
       c[i][ch] = in ? img[3 * g + ch] : 0.f;
@@ -762,10 +759,10 @@ __global__ void kb_split_apply(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
   int* __restrict__ seg = S.seg;
-  const int* __restrict__ smseg = S.smseg;
+  const unsigned* __restrict__ half = half_bits(S);
+  const int W = S.W, pitch = half_pitch(S);
   const SpDev& sp = S.sp;
   const SmDev& sm = S.sm;
-  const Scalars* __restrict__ sc = S.sc;
   const uint8_t* __restrict__ accept = S.accept;
   const int prop_mode = S.mode;
   FOR_PIX(t, S.npix) {
@@ -775,12 +772,9 @@ __global__ void kb_split_apply(const Slot* __restrict__ slots) {
     if (!fl) continue;
     const int s = sm.newid[k];
     if (s < 0) continue;
-    const int k2 = k + sc->tmp1;
-    if (!prop_mode || (fl & 8)) {
-      if (smseg[t] == k2) seg[t] = s;
-    } else {
-      if (smseg[t] == k) seg[t] = s;
-    }
+    const int y = t / W, x = t - y * W;
+    const bool second = (half[(size_t)y * pitch + (x >> 5)] >> (x & 31)) & 1u;
+    if (second == (!prop_mode || (fl & 8))) seg[t] = s;
   }
 }
 

@@ -72,11 +72,9 @@ __global__ void kb_save_prev(const Slot* slots);
 // k_splitmerge.cu
 __global__ void kb_split_begin(const Slot* slots, int B);
 __global__ void kb_split_clear(const Slot* slots);
-__global__ void kb_split_seed(const Slot* slots, int dir_bass, int dir_prop);
 __global__ void kb_bbox(const Slot* slots);
 __global__ void kb_split_bfs(const Slot* slots, int dir_bass, int dir_prop);
-__global__ void kb_split_bfs_big(const Slot* slots);
-__global__ void kb_split_partition(const Slot* slots);
+__global__ void kb_split_bfs_big(const Slot* slots, int dir_bass, int dir_prop);
 __global__ void kb_sm_accumulate(const Slot* slots);
 __global__ void kb_sq_accumulate(const Slot* slots);
 __global__ void kb_split_decide(const Slot* slots, SmConsts K, float split_alpha);
