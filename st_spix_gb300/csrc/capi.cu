@@ -471,7 +471,6 @@ void preload_kernels() {
       (const void*)kb_copy_labels,
       (const void*)kb_read_params,
       (const void*)kb_save_prev,
-      (const void*)kb_split_begin,
       (const void*)kb_split_clear,
       (const void*)kb_bbox,
       (const void*)kb_split_bfs,
@@ -480,7 +479,6 @@ void preload_kernels() {
       (const void*)kb_split_decide,
       (const void*)kb_split_commit,
       (const void*)kb_split_apply,
-      (const void*)kb_split_end,
       (const void*)kb_merge_clear,
       (const void*)kb_merge_candidates,
       (const void*)kb_merge_single,
@@ -512,7 +510,6 @@ void preload_kernels() {
       (const void*)kb_relabel_ids,
       (const void*)kb_relabel_params,
       (const void*)kb_relabel_apply,
-      (const void*)kb_relabel_end,
 
       (const void*)kb_accumulate_fp, (const void*)kb_accumulate_fp_store,
       (const void*)kb_accumulate_fp_clear, (const void*)k_label_stats,
@@ -802,7 +799,6 @@ int update_seg(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
 int run_split(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmConsts& K,
               const stspix_config& cfg, int dir_b, int dir_p) {
   ctx->cur_fam = STSPIX_FAM_SPLIT;
-  LAUNCHS(kb_split_begin, L, nb);
   LAUNCHI(kb_split_clear, std::max<long long>(L.max_cap, L.max_npix / 32), L, nb);
   LAUNCHG(kb_bbox, dim3(tiles64(L), (unsigned)nb), kThreads, L.d);
   // a warp per superpixel, the blocks of every SM filled (4 each by the registers): with 1024
@@ -822,7 +818,6 @@ int run_split(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmC
   LAUNCHG(kb_scan, (unsigned)nb, 1024, L.d, 1);
   LAUNCHI(kb_split_commit, L.max_cap, L, nb);
   LAUNCHB(kb_split_apply, pix_units(L.max_npix), L, nb);
-  LAUNCHS(kb_split_end, L, nb);
   return STSPIX_OK;
 }
 
@@ -840,7 +835,6 @@ int run_relabel(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
   LAUNCHI(kb_relabel_ids, L.max_cap, L, nb);
   LAUNCHI(kb_relabel_params, L.max_cap, L, nb);
   LAUNCHB(kb_relabel_apply, pix_units(L.max_npix), L, nb);
-  LAUNCHS(kb_relabel_end, L, nb);
   return STSPIX_OK;
 }
 
@@ -954,13 +948,11 @@ int split_only(stspix_ctx* ctx, cudaStream_t st, const List& L, const stspix_con
 int compact(stspix_ctx* ctx, cudaStream_t st, const List& L) {
   ctx->cur_fam = STSPIX_FAM_OTHER;
   LAUNCHI(kb_clear_flags, L.max_cap + 2, L, L.B);
-  LAUNCHS(kb_scalars, L, L.B, (int)kOpCompactN);
   LAUNCHB(kb_mark_present, pix_units(L.max_npix), L, L.B, 1);
   LAUNCHG(kb_scan, (unsigned)L.B, 1024, L.d, 3);
   LAUNCHI(kb_compact_gather, L.max_cap, L, L.B);
   LAUNCHI(kb_compact_scatter, L.max_cap, L, L.B);
   LAUNCHB(kb_remap, pix_units(L.max_npix), L, L.B, 1);
-  LAUNCHS(kb_scalars, L, L.B, (int)kOpCompactEnd);
   return STSPIX_OK;
 }
 
@@ -974,7 +966,6 @@ int bass_init(stspix_ctx* ctx, cudaStream_t st, const List& L, const stspix_conf
   LAUNCHB(kb_mark_present, pix_units(L.max_npix), L, L.B, 0);
   LAUNCHG(kb_scan, (unsigned)L.B, 1024, L.d, 0);
   LAUNCHB(kb_remap, pix_units(L.max_npix), L, L.B, 0);
-  LAUNCHS(kb_scalars, L, L.B, (int)kOpAfterHex);
   LAUNCHI(kb_init_bass_params, L.max_cap, L, L.B);
   LAUNCHI(kb_clear_stats, 4LL * L.max_cap, L, L.B, 1);
   LAUNCHG(kb_accumulate, acc_blocks(ctx, L, L.B), 256, L.d, L.B);
@@ -1218,7 +1209,7 @@ int batch_head(stspix_ctx* ctx, cudaStream_t st, int stages, const List& La, con
   if ((r = upload(ctx, st, La, 0)) || (r = upload(ctx, st, Lb, 1)) || (r = upload(ctx, st, Lp, 2)))
     return r;
   ctx->cur_fam = STSPIX_FAM_OTHER;
-  LAUNCHS(kb_scalars, La, La.B, (int)kOpBegin);
+  LAUNCHS(kb_scalars, La, La.B);
   if (ctx->lab_ingest) LAUNCHB(kb_lab_ingest, La.max_npix, La, La.B);
   if ((stages & kStageShift) && (r = shift_fill(ctx, st, Lp))) return r;
   return bass_init(ctx, st, Lb, cfg);
@@ -1413,7 +1404,7 @@ int run_batch(stspix_ctx* ctx, cudaStream_t st, std::vector<FrameDesc>& fr,
   if ((r = upload(ctx, st, La, 0)) || (r = upload(ctx, st, Lb, 1)) || (r = upload(ctx, st, Lp, 2)))
     return r;
   ctx->cur_fam = STSPIX_FAM_OTHER;
-  LAUNCHS(kb_scalars, La, B, (int)kOpBegin);
+  LAUNCHS(kb_scalars, La, B);
   if ((stages & kStageShift) && (r = shift_fill(ctx, st, Lp))) return r;
   if (!(stages & kStageSeg)) {
     if ((r = read_scalars(ctx, st, B))) return r;

@@ -183,9 +183,6 @@ struct Slot {
   int tile_base[kSweepGeoms];  // first sweep tile of this slot in the batch, per tile size
 };
 
-// kb_scalars operations.
-enum { kOpBegin = 0, kOpAfterHex = 1, kOpCompactN = 2, kOpCompactEnd = 3 };
-
 #define SLOT_Y const Slot& S = slots[blockIdx.y]
 // The slot as the fast grid dimension, for kernels whose few busy blocks of each slot come
 // first and are long: they then start first and spread over the SMs (with the slot as the

@@ -142,7 +142,8 @@ __global__ void __launch_bounds__(1024) kb_scan(const Slot* __restrict__ slots, 
   if (mode == 2 && !S.mode) return;  // mint flags exist on propagated slots only
   __shared__ int part[32];
   const uint8_t* flags = (mode == 1) ? S.accept : (mode == 2) ? S.mint : S.flags;
-  const int n = (mode == 0) ? S.nraw : (mode == 3) ? S.sc->tmp2 : live_ids(S);
+  const int n = (mode == 0) ? S.nraw : (mode == 3) ? min(S.sc->max_spix + 1, S.cap) - S.lo
+                                              : live_ids(S);
   int* excl = S.excl;
   int* total = (mode == 0) ? &S.sc->nspix : (mode == 3) ? &S.sc->tmp1 : &S.sc->tmp2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -180,7 +181,11 @@ __global__ void __launch_bounds__(1024) kb_scan(const Slot* __restrict__ slots, 
     run += __shfl_sync(0xffffffffu, pi, 31);
     __syncthreads();                             // part is free for the next tile
   }
-  if (threadIdx.x == 0) *total = run;
+  if (threadIdx.x == 0) {
+    *total = run;
+    if (mode == 0 && !S.mode) S.sc->max_spix = run - 1;     // the hex ids in use
+    if (mode == 3) S.sc->nspix = S.lo + run;                // the compacted ids
+  }
 }
 
 __global__ void kb_remap(const Slot* __restrict__ slots, int mode) {
@@ -1743,34 +1748,22 @@ __global__ void kb_read_params(const Slot* __restrict__ slots) {
   }
 }
 
-// Per-slot scalar steps, one thread per slot.
-__global__ void kb_scalars(const Slot* __restrict__ slots, int B, int op) {
+// Frame start: counters, buffer sizes of the reference.  One thread per slot (the later steps
+// of these scalars are done by the kernels beside them: a launch of its own took 2.3 us).
+__global__ void kb_scalars(const Slot* __restrict__ slots, int B) {
   pdl_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B) return;
   const Slot& S = slots[i];
   Scalars* sc = S.sc;
-  switch (op) {
-    case kOpBegin:  // frame start: counters, buffer sizes of the reference
-      sc->status = STSPIX_OK;
-      sc->nsplits = sc->nmerges = sc->nrevived = sc->nminted = sc->near_ties = 0;
-      sc->fill_iters = 0;
-      sc->ninvalid = 0;
-      sc->tmp0 = sc->tmp1 = sc->tmp2 = 0;
-      sc->nspix = 0;
-      if (S.mode) { sc->max_spix = S.n_prev - 1; sc->nbuf_logical = 10 * S.n_prev; }
-      else { sc->max_spix = 0; sc->nbuf_logical = 30 * S.nraw; }
-      break;
-    case kOpAfterHex:  // max_spix after compacting the hex ids
-      if (!S.mode) sc->max_spix = sc->nspix - 1;
-      break;
-    case kOpCompactN:  // ids beyond cap were never created
-      sc->tmp2 = min(sc->max_spix + 1, S.cap) - S.lo;
-      break;
-    case kOpCompactEnd:
-      sc->nspix = S.lo + sc->tmp1;
-      break;
-  }
+  sc->status = STSPIX_OK;
+  sc->nsplits = sc->nmerges = sc->nrevived = sc->nminted = sc->near_ties = 0;
+  sc->fill_iters = 0;
+  sc->ninvalid = 0;
+  sc->tmp0 = sc->tmp1 = sc->tmp2 = 0;
+  sc->nspix = 0;
+  if (S.mode) { sc->max_spix = S.n_prev - 1; sc->nbuf_logical = 10 * S.n_prev; }
+  else { sc->max_spix = 0; sc->nbuf_logical = 30 * S.nraw; }
 }
 
 // flags := 0 (cap + 2 entries) before a presence scan.

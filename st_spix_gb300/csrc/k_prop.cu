@@ -1030,6 +1030,11 @@ __global__ void kb_relabel_apply(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
   if (!S.mode) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {     // the minted ids (nothing else here reads these)
+    Scalars* sc = S.sc;
+    sc->nminted += sc->tmp2;
+    sc->max_spix += sc->tmp2;
+  }
   int* __restrict__ seg = S.seg;
   const int cap = S.cap;
   const int* __restrict__ rid = S.rid;
@@ -1040,17 +1045,5 @@ __global__ void kb_relabel_apply(const Slot* __restrict__ slots) {
     if (n >= 0 && n < cap) seg[t] = n;
   }
 }
-
-__global__ void kb_relabel_end(const Slot* __restrict__ slots, int B) {
-  pdl_enter();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B || !slots[i].mode) return;
-  Scalars* sc = slots[i].sc;
-  // bump max_spix by the minted ids
-  int m = sc->tmp2;
-  sc->nminted += m;
-  sc->max_spix += m;
-}
-
 
 }  // namespace stspix

@@ -57,10 +57,17 @@ __device__ __forceinline__ void set_half(unsigned* row, int x, unsigned long lon
     if (v[i]) atomicOr(row + w + i, v[i]);
 }
 
-// Clears a split's sums and bits, and the boxes.
+// Begins a split: its scalars, and the sums, bits and boxes cleared.
 __global__ void kb_split_clear(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    Scalars* sc = S.sc;
+    // split runs unless max_spix > nspix_buffer / 2 (split_merge_orig.cu:215)
+    sc->tmp0 = sc->max_spix > sc->nbuf_logical / 2 ? 0 : 1;
+    sc->tmp1 = sc->max_spix + 1;  // offset of the second half
+    sc->tmp2 = 0;                 // superpixels whose box is too large for one warp
+  }
   const int n_ids = live_ids(S);
   FOR_ID(k, sm_ids(S)) {
     sm_clear(S.sm, k);
@@ -70,17 +77,6 @@ __global__ void kb_split_clear(const Slot* __restrict__ slots) {
   }
   unsigned* half = half_bits(S);
   FOR_ID(q, S.H * half_pitch(S)) half[q] = 0;
-}
-
-__global__ void kb_split_begin(const Slot* __restrict__ slots, int B) {
-  pdl_enter();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B) return;
-  Scalars* sc = slots[i].sc;
-  // split runs unless max_spix > nspix_buffer / 2 (split_merge_orig.cu:215)
-  sc->tmp0 = sc->max_spix > sc->nbuf_logical / 2 ? 0 : 1;
-  sc->tmp1 = sc->max_spix + 1;  // offset of the second half
-  sc->tmp2 = 0;                 // superpixels whose box is too large for one warp
 }
 
 // ---------------------------------------------------------------------------
@@ -758,6 +754,11 @@ __global__ void kb_split_commit(const Slot* __restrict__ slots) {
 __global__ void kb_split_apply(const Slot* __restrict__ slots) {
   pdl_enter();
   SLOT_Y;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {     // (nothing else here reads these)
+    Scalars* sc = S.sc;
+    sc->nsplits += sc->tmp2;
+    sc->max_spix += sc->tmp2;
+  }
   int* __restrict__ seg = S.seg;
   const unsigned* __restrict__ half = half_bits(S);
   const int W = S.W, pitch = half_pitch(S);
@@ -776,16 +777,6 @@ __global__ void kb_split_apply(const Slot* __restrict__ slots) {
     const bool second = (half[(size_t)y * pitch + (x >> 5)] >> (x & 31)) & 1u;
     if (second == (!prop_mode || (fl & 8))) seg[t] = s;
   }
-}
-
-__global__ void kb_split_end(const Slot* __restrict__ slots, int B) {
-  pdl_enter();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B) return;
-  Scalars* sc = slots[i].sc;
-  int n = sc->tmp2;
-  sc->nsplits += n;
-  sc->max_spix += n;
 }
 
 // ---------------------------------------------------------------------------

@@ -18,7 +18,7 @@ __global__ void k_marked(float* out, const float* vid, const int* spix, const fl
                          int W, long long n);
 __global__ void k_dump_state(SpDev sp, stspix_state_dump d);
 
-__global__ void kb_scalars(const Slot* slots, int B, int op);
+__global__ void kb_scalars(const Slot* slots, int B);
 __global__ void kb_init_hex(const Slot* slots);
 __global__ void kb_clear_flags(const Slot* slots);
 __global__ void kb_mark_present(const Slot* slots, int mode);
@@ -70,7 +70,6 @@ __global__ void kb_read_params(const Slot* slots);
 __global__ void kb_save_prev(const Slot* slots);
 
 // k_splitmerge.cu
-__global__ void kb_split_begin(const Slot* slots, int B);
 __global__ void kb_split_clear(const Slot* slots);
 __global__ void kb_bbox(const Slot* slots);
 __global__ void kb_split_bfs(const Slot* slots, int dir_bass, int dir_prop);
@@ -80,7 +79,6 @@ __global__ void kb_sq_accumulate(const Slot* slots);
 __global__ void kb_split_decide(const Slot* slots, SmConsts K, float split_alpha);
 __global__ void kb_split_commit(const Slot* slots);
 __global__ void kb_split_apply(const Slot* slots);
-__global__ void kb_split_end(const Slot* slots, int B);
 __global__ void kb_merge_clear(const Slot* slots);
 __global__ void kb_merge_candidates(const Slot* slots, int dir_bass, int dir_prop, int use_border);
 __global__ void kb_merge_single(const Slot* slots, SmConsts K);
@@ -115,7 +113,6 @@ __global__ void kb_relabel_mark(const Slot* slots, float thresh_replace, float t
 __global__ void kb_relabel_ids(const Slot* slots);
 __global__ void kb_relabel_params(const Slot* slots);
 __global__ void kb_relabel_apply(const Slot* slots);
-__global__ void kb_relabel_end(const Slot* slots, int B);
 
 // k_color.cu
 __global__ void k_rgb2lab(const float* rgb, float* lab, long long npix, int first_blue,
