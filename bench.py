@@ -33,19 +33,18 @@ sys.path.insert(0, ROOT)
 WORKLOAD = dict(name="bist_stream_480x854_T30", H=480, W=854, T=30, nseeds=400, sigma=0.03,
                 sp_size=20, niters=20, prop_niters=20, sm_period=10, potts=0.5,
                 sigma2_app=0.009 ** 2, alpha=math.log(0.5), split_alpha=0.0)
-# Algorithmic bytes of one BASS pass (the scope's measurement rules): 4 sweeps x (label
-# read 4 + image read 12 + label write 4) + the statistics of the new labels 16 = 96 B/px.
-# The sweeps of an update do the whole pass: they keep the statistics current by moving
-# those of every relabelled pixel (incremental statistics), so no separate statistics pass
-# runs between two updates: 24 B/px per sweep, and a launch runs all 4 sweeps of an update
-# (one or two with --sweep-schedule / --sweep-tile / --sweep-queue).
-SWEEP_BYTES_PER_PX = 24
+# Algorithmic bytes of one sweep launch, which runs the 4 sweeps of an update (one or two
+# with --sweep-schedule / --sweep-tile / --sweep-queue): label read 4 + image read 12 + label
+# write 4 per pixel, once however many sweeps it holds, and its share of the update's
+# statistics of the new labels, 16 per 4 sweeps (the sweeps keep them current by moving those
+# of every relabelled pixel, so no statistics pass runs between two updates).
+SWEEP_LAUNCH_BYTES_PER_PX = {1: 24, 2: 28, 4: 36}
 # DRAM bytes (read + write) per sweep launch from one ncu capture of the same workload
-# (a batch of 8 frames, mean of a full and an active-set sweep); a constant of that
+# (a batch of 8 frames, mean over the updates of a frame); a constant of that
 # capture, re-taken whenever the sweep kernel changes, not a live measurement.
-SWEEP_TRAFFIC_NCU = dict(bytes_per_launch=35589120,
+SWEEP_TRAFFIC_NCU = dict(bytes_per_launch=34340000,
                          source="ncu dram__bytes_read.sum + dram__bytes_write.sum, "
-                                "profiles/kb_sweep_bist_stream_480x854_T30.md")
+                                "profiles/kernels_streams8_480x854.md")
 METRIC = "streamed frames/sec"
 SERVE_LANES = 3          # host lanes of the serving legs in the default run
 
@@ -1128,7 +1127,7 @@ def main():
                   1 if args.sweep_schedule or args.sweep_tile or args.sweep_queue else 4)
     sweep_ms = prof["sweep"][1]
     peak, peak_kind = read_peaks()
-    per_launch = SWEEP_BYTES_PER_PX * per_sweeps * npix * B0
+    per_launch = SWEEP_LAUNCH_BYTES_PER_PX[per_sweeps] * npix * B0
     achieved = per_launch * nsweep / (sweep_ms / 1000.0) / 1e9 if sweep_ms else 0
     passes_per_video = w["niters"] + (T - 1) * w["prop_niters"]
     mpix_pass = world * S * args.steps * passes_per_video * npix / elapsed / 1e6
