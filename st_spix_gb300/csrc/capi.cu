@@ -463,6 +463,7 @@ void preload_kernels() {
       (const void*)kb_sweep2_t16,
       (const void*)kb_sweep2_t64,
       (const void*)kb_sweep4_s,
+      (const void*)kb_sweep4_t,
       (const void*)kb_sweep4_m,
       (const void*)kb_sweep4_l,
       (const void*)kb_sweepq_t32,
@@ -698,14 +699,14 @@ struct SweepKernel {
   int geom, threads, smem;
 };
 #define SWEEP_KERNEL(k, geom, threads) SweepKernel{k, #k, geom, threads, k##_smem()}
-const SweepKernel (*sweep_kernels())[3] {
-  static const SweepKernel t[3][3] = {
+const SweepKernel (*sweep_kernels())[4] {
+  static const SweepKernel t[3][4] = {
       {SWEEP_KERNEL(kb_sweep_t32, 0, 256), SWEEP_KERNEL(kb_sweep_t64, 1, 256),
        SWEEP_KERNEL(kb_sweep_t16, 2, 256)},
       {SWEEP_KERNEL(kb_sweep2_t32, 0, 256), SWEEP_KERNEL(kb_sweep2_t64, 1, 256),
        SWEEP_KERNEL(kb_sweep2_t16, 2, 256)},
       {SWEEP_KERNEL(kb_sweep4_s, 0, 512), SWEEP_KERNEL(kb_sweep4_m, 1, 256),
-       SWEEP_KERNEL(kb_sweep4_l, 3, 256)}};
+       SWEEP_KERNEL(kb_sweep4_l, 3, 256), SWEEP_KERNEL(kb_sweep4_t, 0, 256)}};
   return t;
 }
 #undef SWEEP_KERNEL
@@ -760,16 +761,21 @@ int update_seg(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
   };
   // The tile of the four-sweep launches, by the number of 32x32 tiles of the sweeping slots.
   // Up to two per SM the launch is one tile's chain of phases: small tiles of 512 threads
-  // (a phase's pixels in one round).  Above eight per SM the total work decides: the tallest
-  // tile (the least halo); in between 64x32.  Measured, us for 3 frames of one video (20
-  // iterations; 2 frames in the batches), 32x32 / 64x32 / 64x48:
-  //   240x320 (80 tiles)     4204 / 4358 / 4569      360x640 (240)      4471 / 4479 / 4673
-  //   480x854 (405)          5546 / 5002 / 5129      720x1280 (920)     7358 / 5667 / 5729
-  //   4 x 480x854 (1620)     7472 / 5188 / 4771      1080x1920 (2040)  12165 / 8273 / 8089
+  // (a phase's pixels in one round).  Up to four per SM the small tiles still run at once, with
+  // 256 threads.  Above eight per SM the total work decides: the tallest tile (the least
+  // halo); in between 64x32.  Measured, us for 3 frames of one video (20 iterations), 32x32
+  // with 512 threads / with 256 / 64x32:
+  //   240x320  (0.5 tiles per SM) 2825 / 2900 / -      480x640  (2.0) 3230 / 3235 / -
+  //   480x854  (2.7)              3783 / 3415 / 3583   600x1000 (4.0) 4299 / 3781 / 3858
+  //   640x1100 (4.6)              4680 / 4189 / 4002   720x1280 (6.1) 5317 / 4565 / 4227
+  // and, with an earlier form, 64x32 / 64x48 tiles: 720x1280 5667 / 5729, 4 frames of 480x854
+  // (10.7) 5188 / 4771, 1080x1920 (13.4) 8273 / 8089.
   const int tl = std::max(1, L.tiles_upto[0][nb]);
   int v;
   if (per == 4) {
-    v = tl <= kSmallTilesPerSm * ctx->num_sms ? 0 : tl <= kMidTilesPerSm * ctx->num_sms ? 1 : 2;
+    const int sms = ctx->num_sms;
+    v = tl <= kSmallTilesPerSm * sms ? 0 : tl <= kWaveTilesPerSm * sms ? 3
+        : tl <= kMidTilesPerSm * sms ? 1 : 2;
     // recorded per size class (quarter octaves of the tile count) for stspix_sweep_choice
     ctx->sweep_choice[(int)std::floor(4.0 * std::log2((double)tl))] = v;
   } else {

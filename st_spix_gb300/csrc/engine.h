@@ -32,9 +32,9 @@ constexpr int kFillSolo = 4096, kFillList = 16384, kFillSmem = 2 * kFillList * 4
 constexpr int kFillBreakIter = 1000;      // fill_missing.cu: break_iter
 constexpr int kSweepVariants = 3;         // sweep tile shapes: 32x32, 64x32, 16x32
 constexpr int kMaxBatchGraphs = 64;       // captured batch steps kept per context
-// 32x32 tiles per SM up to which four-sweep launches take 32x32 and 64x32 tiles
-// (64x48 above; measured in update_seg)
-constexpr int kSmallTilesPerSm = 2, kMidTilesPerSm = 8;
+// 32x32 tiles per SM up to which four-sweep launches take 32x32 tiles with 512 threads, with
+// 256, and 64x32 tiles (64x48 above; measured in update_seg)
+constexpr int kSmallTilesPerSm = 2, kWaveTilesPerSm = 4, kMidTilesPerSm = 8;
 constexpr int kSweepTileW[kSweepVariants] = {32, 64, 16};
 constexpr int kSweepGeoms = 4;            // sweep tile sizes: the widths above, 64x48
 constexpr int kGeomW[kSweepGeoms] = {32, 64, 16, 64}, kGeomH[kSweepGeoms] = {32, 32, 32, 48};

@@ -1710,6 +1710,7 @@ STSPIX_SWEEP_KERNEL(kb_sweep2_t32, 32, 32, 2, 256, 4)
 STSPIX_SWEEP_KERNEL(kb_sweep2_t16, 16, 32, 2, 256, 4)
 STSPIX_SWEEP_KERNEL(kb_sweep2_t64, 64, 32, 2, 256, 4)
 STSPIX_SWEEP_KERNEL(kb_sweep4_s, 32, 32, 4, 512, 2)
+STSPIX_SWEEP_KERNEL(kb_sweep4_t, 32, 32, 4, 256, 4)
 STSPIX_SWEEP_KERNEL(kb_sweep4_m, 64, 32, 4, 256, 4)
 STSPIX_SWEEP_KERNEL(kb_sweep4_l, 64, 48, 4, 256, 4)
 #undef STSPIX_SWEEP_KERNEL

@@ -54,6 +54,7 @@ STSPIX_DECL_SWEEP(kb_sweep2_t32)
 STSPIX_DECL_SWEEP(kb_sweep2_t64)
 STSPIX_DECL_SWEEP(kb_sweep2_t16)
 STSPIX_DECL_SWEEP(kb_sweep4_s)
+STSPIX_DECL_SWEEP(kb_sweep4_t)
 STSPIX_DECL_SWEEP(kb_sweep4_m)
 STSPIX_DECL_SWEEP(kb_sweep4_l)
 #undef STSPIX_DECL_SWEEP

@@ -19,7 +19,9 @@ pytestmark = pytest.mark.gpu
     (96, 128, 15, 12, 1, 0.0, 1.0),
     (96, 128, 15, 12, 3, -0.6, 1.4),
     (96, 128, 15, 12, 6, 0.0, 1.0),
-    (331, 1000, 20, 6, 4, 0.0, 1.0),        # 352 tiles: 64x32 tiles, 331 = 10 x 32 + 11
+    (331, 1000, 20, 6, 4, 0.0, 1.0),        # 352 tiles: 32x32 by 256 threads, 331 = 10 x 32 + 11
+    (715, 1281, 24, 5, 4, 0.0, 1.0),        # 943 tiles: 64x32 tiles, 715 = 22 x 32 + 11
+    (715, 1281, 24, 4, 6, -0.6, 1.4),
     (331, 1000, 20, 5, 5, -0.6, 1.4),
     (961, 1361, 25, 5, 4, 0.0, 1.0),        # 1333 tiles: 64x48 tiles, 961 = 20 x 48 + 1
     (961, 1361, 25, 4, 7, 0.0, 1.0),
