@@ -348,8 +348,8 @@ int alloc_params(stspix_ctx* ctx, std::vector<Buf>& L, stspix_params& p, int cap
 constexpr long long kPixBytes = 1 + 5 * 4 + 8 + 4 + 2;        // border, d1 d2 smseg hits shifted, best, seg_alt, chg x2
 constexpr long long kSpDevBytes = 4 + 1 + 1 + 4 + 4 + 4 + 12 + 16 + 24 + 8 + 12 + 16 + 24 + 24 + 24 +
                                   64 + (long long)sizeof(SweepRec);
-constexpr long long kSmBytes = 4 + 24 + 24 + 4 + 4 + 4 + 4 + 4 + 1 + 8;
-constexpr long long kAuxBytes = 5 * 1 + 6 * 4 + 16 + 8 + 4 + 16 + 8 + 8 + 72 + 1 + 24;
+constexpr long long kSmBytes = 4 + 24 + 24 + 40 + 4 + 4 + 4 + 4 + 4 + 1 + 8;
+constexpr long long kAuxBytes = 5 * 1 + 6 * 4 + 16 + 8 + 4 + 16 + 16 + 8 + 8 + 72 + 1 + 24;
 constexpr long long kParamBytes = 12 + 12 + 16 + 24 + 4 + 16 + 24 + 24 + 4 + 4 + 4 + 4 + 4;
 
 // Make sure slot position i holds npix pixels and sp_cap superpixels.  Growing
