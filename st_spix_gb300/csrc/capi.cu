@@ -808,8 +808,10 @@ int run_split(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb, const SmC
   LAUNCHI(kb_split_clear, std::max<long long>(L.max_cap, L.max_npix / 32), L, nb);
   LAUNCHG(kb_bbox, dim3(tiles64(L), (unsigned)nb), kThreads, L.d);
   // a warp per superpixel, the blocks of every SM filled (4 each by the registers): with 1024
-  // warps a frame of 1,100 superpixels took a second round, 27 us instead of 20
-  const unsigned bfs = (unsigned)std::max(64, (4 * ctx->num_sms + nb - 1) / nb);
+  // warps a frame of 1,100 superpixels took a second round, 27 us instead of 20.  At least 256
+  // blocks per slot: 16 frames of 240 to 1080 rows take 93 us, with 64 (the largest frame's
+  // superpixels in rounds) 103
+  const unsigned bfs = (unsigned)std::max(256, (4 * ctx->num_sms + nb - 1) / nb);
   LAUNCHG(kb_split_bfs, dim3(bfs, (unsigned)nb), 128, L.d, dir_b, dir_p);
   {
     cudaEvent_t pe_ = prof_begin(ctx, st);
