@@ -6,7 +6,8 @@
  * int status (STSPIX_OK == 0) and never exits the process.  Work is enqueued on
  * the given stream; entry points that must return a host-side value (a count)
  * synchronise that stream and say so.  A context is NOT safe for concurrent use
- * from several host threads; use one context per thread / per stream.
+ * from several host threads; use one context per thread / per stream.  (The quality
+ * entry points take turns on a context: stspix_evaluate to stspix_sp_pooling.)
  *
  * Reference interfaces replaced (paths inside gauenk/st_spix):
  *   stspix_bist_forward        st_spix/csrc/bist/pyapi.cu:200 bist_forward_cuda (+ :46 main_loop)

@@ -125,9 +125,10 @@ struct stspix_ctx {
   stspix_video* fwd = nullptr;
   // device scratch of the quality entry points, kept between calls up to kScratchMax
   // bytes (an allocation per call gave its memory back to the driver at every
-  // synchronisation: 200 us a call).  ev marks its last use: a call on another stream
-  // waits for it.
-  struct { char* p = nullptr; size_t bytes = 0; cudaEvent_t ev = nullptr; cudaStream_t st = nullptr;
+  // synchronisation: 200 us a call).  ev marks its last use: the next call waits for it.
+  // scratch_mu: one call at a time uses it and the pinned staging (see Scratch).
+  std::mutex scratch_mu;
+  struct { char* p = nullptr; size_t bytes = 0; cudaEvent_t ev = nullptr;
            bool used = false; } scratch;
   // pinned staging of small results (kPinBytes)
   char* pin = nullptr;
@@ -2194,21 +2195,35 @@ constexpr size_t kScratchMax = size_t(256) << 20, kPinBytes = size_t(1) << 20;
 
 // `bytes` of device scratch for work on st: the context's own (grown to the next power of
 // two; growing synchronises the device), or, above kScratchMax, an allocation of this call.
-// Released by the destructor, after which nothing more is launched on it.
+// Every use waits for the one before on its event, whatever the streams: equal handles need
+// not be one stream (the per-thread default stream, a recycled handle), and on one stream the
+// wait is free.
+// Holds the context's scratch_mu until it is destroyed (after the last launch on it, and after
+// the host has read the pinned staging): host threads that share a context, as the Python
+// layer's do on one stream, take turns.
 struct Scratch {
   stspix_ctx* ctx;
   cudaStream_t st;
+  std::lock_guard<std::mutex> turn;
   char* p = nullptr;
   bool own = false;
-  Scratch(stspix_ctx* c, cudaStream_t s) : ctx(c), st(s) {}
+  Scratch(stspix_ctx* c, cudaStream_t s) : ctx(c), st(s), turn(c->scratch_mu) {}
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
   ~Scratch() {
     if (!p) return;
     if (own) { cudaFreeAsync(p, st); return; }
-    ctx->scratch.used = cudaEventRecord(ctx->scratch.ev, st) == cudaSuccess;
-    ctx->scratch.st = st;
+    auto& k = ctx->scratch;
+    k.used = cudaEventRecord(k.ev, st) == cudaSuccess;
+    if (!k.used) cudaStreamSynchronize(st);
   }
   int get(size_t bytes) {
     auto& k = ctx->scratch;
+    // (an event recorded in a capture could not be waited for after it)
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone)
+      return fail(ctx, STSPIX_ERR_CUDA, "the call waits for its results: it cannot be captured");
     if (bytes > kScratchMax) {
       CK(cudaMallocAsync((void**)&p, bytes, st));
       own = true;
@@ -2227,14 +2242,16 @@ struct Scratch {
       k.bytes = n;
       if (!k.ev) CK(cudaEventCreateWithFlags(&k.ev, cudaEventDisableTiming));
     }
-    if (k.used && k.st != st) CK(cudaStreamWaitEvent(st, k.ev, 0));
+    if (k.used) CK(cudaStreamWaitEvent(st, k.ev, 0));
     p = k.p;
     return STSPIX_OK;
   }
 };
 
 int ensure_pin(stspix_ctx* ctx) {
-  if (!ctx->pin) CK(cudaMallocHost((void**)&ctx->pin, kPinBytes));
+  if (ctx->pin) return STSPIX_OK;
+  std::lock_guard<std::mutex> lk(g_device_mu);
+  CK(cudaMallocHost((void**)&ctx->pin, kPinBytes));
   return STSPIX_OK;
 }
 
