@@ -2753,9 +2753,9 @@ int stspix_evaluate(stspix_ctx* ctx, void* stream, const float* vid, const int32
   LAUNCHG(k_q_id_time, q_blocks(S), kThreads, q.cnt, q.fsum, T, (int)S, q.ntot, q.stdv, q.vsum);
   LAUNCHG(k_q_frame_ids, dim3(q_blocks(S), T), kThreads, q.cnt, q.fsum, q.mean, q.vsum, q.ntot,
           q.msum, (int)S, (int)npix, q.live, q.pool2, q.cross, q.pool3);
-  if (gt)
-    LAUNCHG(k_q_uesa, dim3((unsigned)((S + kQUesaIds - 1) / kQUesaIds), q_blocks(G1)), kThreads,
-            q.cnt, q.J, q.ntot, T, (int)S, (int)G1, q.ue, q.sa, q.gsize, q.ue3, q.sa3);
+  if (gt)     // (T S G1 <= 2e9: at most 2^29 blocks)
+    LAUNCHG(k_q_uesa, (unsigned)((S + kQUesaIds - 1) / kQUesaIds * q_blocks(G1)), kThreads, q.cnt,
+            q.J, q.ntot, T, (int)S, (int)G1, q.ue, q.sa, q.gsize, q.ue3, q.sa3);
   // per-frame / per-id results to the host
   std::vector<char> buf;
   const char* out_h;

@@ -356,9 +356,10 @@ __global__ void __launch_bounds__(256) k_q_frame_ids(
   if (threadIdx.x == 0) atomicAdd(&pool3[t], b);
 }
 
-// Overlap scores (evaluate.py:436-468), grid (ids / kQUesaIds, ground-truth ids / 256): a
-// thread takes one ground-truth id g and kQUesaIds ids, and reads their overlaps of every
-// frame (neighbouring threads neighbouring words).  Per frame: the corrected
+// Overlap scores (evaluate.py:436-468), one block per kQUesaIds ids and 256 ground-truth ids,
+// in one grid dimension (either count may exceed the 65,535 of the others): a thread takes
+// one ground-truth id g and kQUesaIds ids, and reads their overlaps of every frame
+// (neighbouring threads neighbouring words).  Per frame: the corrected
 // under-segmentation sum (min(out, in) over ids overlapping g), the accuracy sum (in over
 // ids at least half inside g) and g's size; over the video: the same with in and out summed
 // over the frames (out only where the id overlaps g in that frame).  Few pairs overlap, so
@@ -369,9 +370,10 @@ __global__ void __launch_bounds__(256) k_q_uesa(
     int T, int S, int G1, unsigned long long* ue, unsigned long long* sa, unsigned long long* size,
     unsigned long long* ue3, unsigned long long* sa3) {
   pdl_enter();
-  const int g = blockIdx.y * blockDim.x + threadIdx.x;
+  const unsigned ns = ((unsigned)S + kQUesaIds - 1) / kQUesaIds;   // blocks over the ids
+  const int g = (int)(blockIdx.x / ns * blockDim.x + threadIdx.x);
   if (g >= G1) return;
-  const int s0 = blockIdx.x * kQUesaIds;
+  const int s0 = (int)(blockIdx.x % ns) * kQUesaIds;
   long long in[kQUesaIds], out[kQUesaIds];
 #pragma unroll
   for (int i = 0; i < kQUesaIds; i++) in[i] = out[i] = 0;
