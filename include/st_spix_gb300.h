@@ -334,7 +334,7 @@ int stspix_size_variation(stspix_ctx* ctx, void* stream, const int32_t* counts, 
                           double* tex, double* szv, double* ave_nsp);
 
 /* sp_pooling (st_spix/sp_pooling.py:10) for 3-channel frames: with ids 0..nids-1
- * (every id of spix must be in range, else STSPIX_ERR_ARG and unspecified outputs; the
+ * (every id of spix must be in range, else STSPIX_ERR_ARG and untouched outputs; the
  * host waits for that check only), down f32 [T, nids, 3] =
  * per-frame id mean colour (sum / (count + 1e-8); 0 for absent ids) and, when pooled
  * is not NULL, pooled f32 [T,H,W,3] = the mean colour of each pixel's id.            */

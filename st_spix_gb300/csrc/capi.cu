@@ -2455,7 +2455,8 @@ int stspix_sp_pooling(stspix_ctx* ctx, void* stream, const float* vid, const int
   cudaStream_t st = (cudaStream_t)stream;
   const long long npix = (long long)H * W, n = T * npix, TS = (long long)T * nids;
   // the range check's words, counts and per-frame id sums.  The kernels skip ids out of
-  // range, so all of them are launched before the host waits for the range alone.
+  // range, and write no output where there are any, so all of them are launched before the
+  // host waits for the range alone.
   const size_t cbytes = (4 * (size_t)TS + 255) & ~size_t(255);
   const size_t bytes = 256 + cbytes + 24 * (size_t)TS;
   Scratch mem(ctx, st);
@@ -2467,10 +2468,11 @@ int stspix_sp_pooling(stspix_ctx* ctx, void* stream, const float* vid, const int
   double* fsum = (double*)(mem.p + 256 + cbytes);
   LAUNCHG(k_q_accum, dim3(q_tiles(H, W), (unsigned)T), kThreads, vid, spix, nullptr, npix, H, W, 0,
           nids, 1, cnt, fsum, nullptr);
-  LAUNCHG(k_q_down, q_blocks(TS), kThreads, cnt, fsum, TS, down);
+  const int* range = (const int*)mem.p;
+  LAUNCHG(k_q_down, q_blocks(TS), kThreads, range, nids, cnt, fsum, TS, down);
   if (pooled)
-    LAUNCHG(k_q_pool_write, (unsigned)((n + kMarkPix - 1) / kMarkPix), kThreads, spix, (int)npix,
-            nids, n, down, pooled);
+    LAUNCHG(k_q_pool_write, (unsigned)((n + kMarkPix - 1) / kMarkPix), kThreads, range, spix,
+            (int)npix, nids, n, down, pooled);
   CK(cudaGetLastError());
   int mm[4];
   if ((r = range_get(ctx, mm))) return r;

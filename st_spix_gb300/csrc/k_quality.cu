@@ -411,9 +411,15 @@ __global__ void __launch_bounds__(256) k_q_uesa(
 
 // sp_pooling (st_spix/sp_pooling.py:10-47) outputs: down[t][s] = colour sum / (count
 // + 1e-8) for every id 0..S-1 of every frame, pooled[p] = down of the pixel's id.
-__global__ void k_q_down(const int* __restrict__ cnt, const double* __restrict__ fsum,
-                         long long TS, float* __restrict__ down) {
+// mm: the smallest and largest id; with ids outside [0, S) nothing is written (the caller
+// refuses them, after these kernels are launched).
+__device__ __forceinline__ bool q_in_range(const int* __restrict__ mm, int S) {
+  return mm[0] >= 0 && mm[1] < S;
+}
+__global__ void k_q_down(const int* __restrict__ mm, int S, const int* __restrict__ cnt,
+                         const double* __restrict__ fsum, long long TS, float* __restrict__ down) {
   pdl_enter();
+  if (!q_in_range(mm, S)) return;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= TS) return;
   const double n = (double)cnt[i] + 1e-8;
@@ -422,12 +428,14 @@ __global__ void k_q_down(const int* __restrict__ cnt, const double* __restrict__
 
 // A block writes the colours of kMarkPix consecutive pixels: gathered per pixel into shared
 // memory, stored as consecutive 16-byte words (single values where `pooled` is not 16-byte
-// aligned, and in the last block).  Ids outside [0, S) write 0 (the caller refuses them).
-__global__ void __launch_bounds__(256) k_q_pool_write(const int32_t* __restrict__ spix, int npix,
+// aligned, and in the last block).
+__global__ void __launch_bounds__(256) k_q_pool_write(const int* __restrict__ mm,
+                                                      const int32_t* __restrict__ spix, int npix,
                                                       int S, long long n,
                                                       const float* __restrict__ down,
                                                       float* __restrict__ pooled) {
   pdl_enter();
+  if (!q_in_range(mm, S)) return;
   __shared__ __align__(16) float v[3 * kMarkPix];
   const long long p0 = (long long)blockIdx.x * kMarkPix;
   const long long t0 = p0 / npix;
@@ -437,12 +445,9 @@ __global__ void __launch_bounds__(256) k_q_pool_write(const int32_t* __restrict_
     const unsigned k = threadIdx.x + 256 * j;
     float c[3] = {0.f, 0.f, 0.f};
     if (p0 + k < n) {
-      const int s = spix[p0 + k];
-      if (s >= 0 && s < S) {
-        const size_t ts = (size_t)(t0 + (r0 + k) / (unsigned)npix) * S + s;
+      const size_t ts = (size_t)(t0 + (r0 + k) / (unsigned)npix) * S + spix[p0 + k];
 #pragma unroll
-        for (int q = 0; q < 3; q++) c[q] = down[3 * ts + q];
-      }
+      for (int q = 0; q < 3; q++) c[q] = down[3 * ts + q];
     }
 #pragma unroll
     for (int q = 0; q < 3; q++) v[3 * k + q] = c[q];

@@ -142,7 +142,8 @@ __global__ void k_q_frame_ids(const int* cnt, const double* fsum, const double* 
 __global__ void k_q_uesa(const int* cnt, const int* J, const long long* ntot, int T, int S, int G1,
                          unsigned long long* ue, unsigned long long* sa, unsigned long long* size,
                          unsigned long long* ue3, unsigned long long* sa3);
-__global__ void k_q_down(const int* cnt, const double* fsum, long long TS, float* down);
+__global__ void k_q_down(const int* mm, int S, const int* cnt, const double* fsum, long long TS,
+                         float* down);
 
 // k_legacy.cu
 __global__ void k_fill_i32(int32_t* p, long long n, int32_t v);
@@ -159,7 +160,7 @@ __global__ void k_vpool_mean(const double* sum, const unsigned long long* cnt, l
                              int F, float* down, float* counts);
 __global__ void k_vpool_write(const float* down, const int32_t* seg, int T, long long npix, int F,
                               int nspix, float* pooled);
-__global__ void k_q_pool_write(const int32_t* spix, int npix, int S, long long n,
+__global__ void k_q_pool_write(const int* mm, const int32_t* spix, int npix, int S, long long n,
                                const float* down, float* pooled);
 __global__ void k_lmark_ids(const int32_t* spix, long long n, int nids, uint8_t* present);
 __global__ void k_lupdate_prior(const uint8_t* present, int nids, int prev_nspix, int invert,
