@@ -2207,6 +2207,7 @@ struct Scratch {
   std::lock_guard<std::mutex> turn;
   char* p = nullptr;
   bool own = false;
+  bool idle = false;         // the host has waited for the last work on it
   Scratch(stspix_ctx* c, cudaStream_t s) : ctx(c), st(s), turn(c->scratch_mu) {}
   Scratch(const Scratch&) = delete;
   Scratch& operator=(const Scratch&) = delete;
@@ -2214,8 +2215,8 @@ struct Scratch {
     if (!p) return;
     if (own) { cudaFreeAsync(p, st); return; }
     auto& k = ctx->scratch;
-    k.used = cudaEventRecord(k.ev, st) == cudaSuccess;
-    if (!k.used) cudaStreamSynchronize(st);
+    k.used = !idle && cudaEventRecord(k.ev, st) == cudaSuccess;
+    if (!idle && !k.used) cudaStreamSynchronize(st);
   }
   int get(size_t bytes) {
     auto& k = ctx->scratch;
@@ -2359,8 +2360,9 @@ int label_range(stspix_ctx* ctx, cudaStream_t st, const int32_t* a, const int32_
   Scratch mm(ctx, st);
   int r;
   if ((r = mm.get(4 * sizeof(int)))) return r;
-  if ((r = range_launch(ctx, st, (int*)mm.p, a, b, n))) return r;
-  return range_get(ctx, out);
+  if ((r = range_launch(ctx, st, (int*)mm.p, a, b, n)) || (r = range_get(ctx, out))) return r;
+  mm.idle = true;
+  return STSPIX_OK;
 }
 
 // tex / szv from the per-frame live counts and per-id stds (evaluate.py:287-327).
@@ -2435,6 +2437,7 @@ int stspix_size_variation(stspix_ctx* ctx, void* stream, const int32_t* counts, 
   std::vector<char> buf;
   const char* res;
   if ((r = quality_results(ctx, st, mem.p, q, buf, &res))) return r;
+  mem.idle = true;
   const auto* live = (const unsigned long long*)res;
   const auto* stdv = (const double*)(res + ((char*)q.stdv - (char*)q.live));
   size_scores(live, stdv, T, S, tex, szv);
@@ -2762,6 +2765,7 @@ int stspix_evaluate(stspix_ctx* ctx, void* stream, const float* vid, const int32
   std::vector<char> buf;
   const char* out_h;
   if ((r = quality_results(ctx, st, mem.p, q, buf, &out_h))) return r;
+  mem.idle = true;
   auto on_host = [&](const auto* d) {
     return (decltype(d))(out_h + ((const char*)d - (mem.p + q.results)));
   };
