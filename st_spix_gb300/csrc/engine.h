@@ -266,23 +266,29 @@ __device__ __forceinline__ unsigned fx_unit(float v, int shift) {
 // lane's rows of label k, src = the lane that adds the warp's totals to the global sums.
 // pend = the rows to take (labels in range).  A block holds a few labels, so a few warp
 // reductions and one set of atomics per label serve its 256 pixels.
+// One round: label k, the lane's rows of it in m, and the lane src that it was taken from; its
+// pixels leave pend.  False when no pixel was left.
+__device__ __forceinline__ bool label_round(const int (&lab)[8], unsigned& pend, int& k,
+                                            unsigned& m, int& src) {
+  const unsigned any = __ballot_sync(0xffffffffu, pend != 0);
+  if (!any) return false;
+  src = __ffs(any) - 1;
+  const int r = __ffs(__shfl_sync(0xffffffffu, pend, src)) - 1;   // its first pending row
+  const bool b0 = r & 1, b1 = r & 2, b2 = r & 4;
+  const int v0 = b1 ? (b0 ? lab[3] : lab[2]) : (b0 ? lab[1] : lab[0]);
+  const int v1 = b1 ? (b0 ? lab[7] : lab[6]) : (b0 ? lab[5] : lab[4]);
+  k = __shfl_sync(0xffffffffu, b2 ? v1 : v0, src);
+  m = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) m |= (unsigned)(lab[i] == k) << i;
+  pend &= ~m;
+  return true;
+}
 template <typename Body>
 __device__ __forceinline__ void label_rounds(const int (&lab)[8], unsigned pend, Body body) {
-  for (;;) {
-    const unsigned any = __ballot_sync(0xffffffffu, pend != 0);
-    if (!any) break;
-    const int src = __ffs(any) - 1;
-    const int r = __ffs(__shfl_sync(0xffffffffu, pend, src)) - 1;   // its first pending row
-    const bool b0 = r & 1, b1 = r & 2, b2 = r & 4;
-    const int v0 = b1 ? (b0 ? lab[3] : lab[2]) : (b0 ? lab[1] : lab[0]);
-    const int v1 = b1 ? (b0 ? lab[7] : lab[6]) : (b0 ? lab[5] : lab[4]);
-    const int k = __shfl_sync(0xffffffffu, b2 ? v1 : v0, src);
-    unsigned m = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) m |= (unsigned)(lab[i] == k) << i;
-    pend &= ~m;
-    body(k, m, src);
-  }
+  int k, src;
+  unsigned m;
+  while (label_round(lab, pend, k, m, src)) body(k, m, src);
 }
 
 // Sums over the rows of a mask (8 bits) of their numbers, and of the squares << 8.
