@@ -168,7 +168,7 @@ namespace {
 std::mutex g_device_mu;
 
 const int kThreads = 256;
-const int kBfsBigSmem = 5 * 512 * 8 * 8;  // kb_split_bfs_big: 5 arrays of 512 rows x 8 words
+const int kBfsBigSmem = 6 * 512 * 8 * 8;  // kb_split_bfs_big: 6 arrays of 512 rows x 8 words
 inline unsigned blocks_for(long long n) { return (unsigned)std::max(1LL, (n + kThreads - 1) / kThreads); }
 // Threads of a FOR_PIX kernel over n pixels.
 inline long long pix_units(long long n) { return (n + kPixPerThread - 1) / kPixPerThread; }

@@ -119,78 +119,68 @@ __global__ void __launch_bounds__(256) kb_bbox(const Slot* __restrict__ slots) {
 // bit-parallel BFS: the box is held as rows of 64-bit words (label mask M, frontier
 // F and visited V of each field), and one layer is
 //     N = (F << 1 | F >> 1 | F[row-1] | F[row+1]) & M & ~V
-// per word, so a layer costs O(rows x words) however the superpixel is shaped;
-// each newly reached pixel gets distance L + 1 written once.
+// per word, so a layer costs O(rows x words) however the superpixel is shaped.
+// The split's only use of the distances is d1 > d2 (calc_seg_split, split_merge.cu:847-859):
+// true where seed 1 reaches a pixel and seed 2 reaches it strictly later or never.  So beside
+// F and V a search keeps E, the pixels seed 2 reached in a layer where seed 1 had not (yet)
+// reached them, seed 2 itself included, and V1 & (~V2 | E) are the bits of the second half.
 // kb_split_bfs runs one warp per superpixel with the box in registers (boxes up to
 // 128 x 128 pixels, bfs_reg) and lists larger boxes for kb_split_bfs_big (one block
-// each, the box in shared memory up to 512 x 512 pixels, bfs_bits; beyond that the same
-// layers run on the global distances).
+// each, the box in shared memory up to 512 x 512 pixels, bfs_bits; beyond that the
+// layers run on distances in global memory).
 constexpr int kBigRows = 512, kBigWpr = 8;      // block: 512 rows x 8 words
 
-template <int NT>
-__device__ __forceinline__ void group_sync() {
-  if (NT == 32) __syncwarp(); else __syncthreads();
-}
-template <int NT>
-__device__ __forceinline__ int group_any(int v) {
-  if (NT == 32) { __syncwarp(); return __any_sync(0xffffffffu, v); }
-  return __syncthreads_or(v);
-}
-
-// t: thread index in the group of NT threads (NT a multiple of 32; whole warps).
-// Arrays hold bh * wpr words each.
-template <int NT, int ITEMS>
-__device__ void bfs_bits(int t, int k, int x0, int y0, int bw, int bh, int W,
-                         const int* __restrict__ seg, int* d1, int* d2,
-                         unsigned long long* M, unsigned long long* F1, unsigned long long* V1,
-                         unsigned long long* F2, unsigned long long* V2) {
+// A block of 256 threads; six arrays of bh x wpr <= kBigRows x kBigWpr words in shared memory
+// (mem, kBigRows kBigWpr words apart).  The seeds come as pixel indices (split_seed_index), so
+// nothing of the frame but the labels of the box is read, once.  (With distances in global
+// memory, cleared, written per pixel and compared by the one block, 3 frames of 1080x1920 with
+// superpixels of 200 pixels took 26.6 ms; now 18.0; 25.2 with the clears and the comparison as
+// passes over the frame.)
+__device__ void bfs_bits(int k, int x0, int y0, int bw, int bh, int W,
+                         const int* __restrict__ seg, unsigned* half, int seed1, int seed2,
+                         unsigned long long* mem) {
+  using u64 = unsigned long long;
+  constexpr int kA = kBigRows * kBigWpr, NT = 256, kItems = kA / NT;
+  u64 *M = mem, *F1 = mem + kA, *V1 = mem + 2 * kA, *F2 = mem + 3 * kA, *V2 = mem + 4 * kA,
+      *E2 = mem + 5 * kA;
+  const int t = threadIdx.x, lane = t & 31;
   const int wpr = (bw + 63) >> 6;
   const int nwords = bh * wpr;
-  const int lane = t & 31;
-  // masks and seeds: one warp-wide ballot per 32-pixel chunk of a row
-  const int cpr = (bw + 31) >> 5;
+  // the label mask: one warp-wide ballot per 32-pixel half of a word (the halves past the box
+  // are empty)
   unsigned* M32 = (unsigned*)M;
-  unsigned* F132 = (unsigned*)F1;
-  unsigned* F232 = (unsigned*)F2;
+  const int cpr = 2 * wpr;
   for (int c = t >> 5; c < bh * cpr; c += NT >> 5) {
-    const int r = c / cpr, cx = c % cpr;
-    const int xi = cx * 32 + lane;
-    bool m = false, s1 = false, s2 = false;
-    if (xi < bw) {
-      const int g = (y0 + r) * W + x0 + xi;
-      m = seg[g] == k;
-      if (m) { s1 = d1[g] == 1; s2 = d2[g] == 1; }
-    }
-    const unsigned bm = __ballot_sync(0xffffffffu, m);
-    const unsigned b1 = __ballot_sync(0xffffffffu, s1);
-    const unsigned b2 = __ballot_sync(0xffffffffu, s2);
-    if (lane == 0) {
-      const int w32 = r * wpr * 2 + cx;   // 32-bit half-word index (little endian)
-      M32[w32] = bm; F132[w32] = b1; F232[w32] = b2;
-    }
+    const int r = c / cpr, xi = (c - r * cpr) * 32 + lane;
+    const unsigned b =
+        __ballot_sync(0xffffffffu, xi < bw && seg[(size_t)(y0 + r) * W + x0 + xi] == k);
+    if (lane == 0) M32[c] = b;
   }
-  // zero the upper half of a row's last word when the row has an odd chunk count
-  if (cpr & 1)
-    for (int r = t; r < bh; r += NT) {
-      const int w32 = r * wpr * 2 + cpr;
-      M32[w32] = 0; F132[w32] = 0; F232[w32] = 0;
-    }
-  group_sync<NT>();
-  for (int i = t; i < nwords; i += NT) { V1[i] = F1[i]; V2[i] = F2[i]; }
-  group_sync<NT>();
+  auto seed = [&](int g, int i) -> u64 {
+    if (g < 0) return 0;
+    const int c = g % W - x0;
+    return (g / W - y0) * wpr + (c >> 6) == i ? 1ull << (c & 63) : 0;
+  };
+  for (int i = t; i < nwords; i += NT) {
+    const u64 f1 = seed(seed1, i), f2 = seed(seed2, i);
+    F1[i] = V1[i] = f1;
+    F2[i] = V2[i] = f2;
+    E2[i] = f2 & ~f1;
+  }
+  __syncthreads();
   const int area = bw * bh;
   for (int L = 1; L <= area + 1; L++) {
-    unsigned long long n1[ITEMS], n2[ITEMS];
+    u64 n1[kItems], n2[kItems];
 #pragma unroll
-    for (int j = 0; j < ITEMS; j++) {
+    for (int j = 0; j < kItems; j++) {
       const int i = t + j * NT;
       n1[j] = n2[j] = 0;
       if (i < nwords) {
         const int r = i / wpr, w = i - r * wpr;
-        const unsigned long long m = M[i];
+        const u64 m = M[i];
         if (m) {
-          unsigned long long f = F1[i];
-          unsigned long long a = (f << 1) | (f >> 1);
+          u64 f = F1[i];
+          u64 a = (f << 1) | (f >> 1);
           if (w > 0) a |= F1[i - 1] >> 63;
           if (w < wpr - 1) a |= F1[i + 1] << 63;
           if (r > 0) a |= F1[i - wpr];
@@ -206,26 +196,30 @@ __device__ void bfs_bits(int t, int k, int x0, int y0, int bw, int bh, int W,
         }
       }
     }
-    group_sync<NT>();
+    __syncthreads();
     int any = 0;
 #pragma unroll
-    for (int j = 0; j < ITEMS; j++) {
+    for (int j = 0; j < kItems; j++) {
       const int i = t + j * NT;
       if (i < nwords) {
         F1[i] = n1[j];
         F2[i] = n2[j];
         if (n1[j] | n2[j]) {
           any = 1;
-          V1[i] |= n1[j];
+          const u64 v1 = V1[i] | n1[j];
+          V1[i] = v1;
           V2[i] |= n2[j];
-          const int r = i / wpr, w = i - r * wpr;
-          const int gb = (y0 + r) * W + x0 + 64 * w;
-          for (unsigned long long b = n1[j]; b; b &= b - 1) d1[gb + __ffsll((long long)b) - 1] = L + 1;
-          for (unsigned long long b = n2[j]; b; b &= b - 1) d2[gb + __ffsll((long long)b) - 1] = L + 1;
+          E2[i] |= n2[j] & ~v1;
         }
       }
     }
-    if (!group_any<NT>(any)) break;
+    if (!__syncthreads_or(any)) break;
+  }
+  const int pitch = (W + 31) >> 5;
+  for (int i = t; i < nwords; i += NT) {
+    const int r = i / wpr, w = i - r * wpr;
+    const u64 second = V1[i] & (~V2[i] | E2[i]);
+    if (second) set_half(half + (size_t)(y0 + r) * pitch, x0 + 64 * w, second);
   }
 }
 
@@ -234,8 +228,6 @@ __device__ void bfs_bits(int t, int k, int x0, int y0, int bw, int bh, int W,
 // as C 64-bit words each (C = 1, 2 by its width) of each field: label mask m, frontiers
 // f1, f2 and visited v1, v2.  A layer is shifts within a row, the rows above and below
 // from the lane's own rows or one shuffle, and the masks: no shared memory, no barrier.
-// The seeds come as pixel indices (split_seed_index), so the box's distances are not
-// read; only the comparison d1 > d2 is written, once, at the end.
 template <int R, int C>
 __device__ __forceinline__ void bfs_reg(int k, int x0, int y0, int bw, int bh, int W,
                                         const int* __restrict__ seg, unsigned* half,
@@ -311,10 +303,6 @@ __device__ __forceinline__ void bfs_reg(int k, int x0, int y0, int bw, int bh, i
       for (int w = 0; w < C; w++) { f[j][w] = n[j][w]; v[j][w] |= n[j][w]; any |= n[j][w]; }
     return any;
   };
-  // The split's only use of the distances is d1 > d2 (calc_seg_split, split_merge.cu:847-859):
-  // true where seed 1 reaches a pixel and seed 2 reaches it strictly later or never.  early2:
-  // pixels seed 2 reached in a layer where seed 1 had not (yet) reached them, seed 2 itself
-  // included.
   u64 early2[R][C];
 #pragma unroll
   for (int j = 0; j < R; j++)
@@ -380,7 +368,7 @@ __global__ void __launch_bounds__(128, 4) kb_split_bfs(const Slot* __restrict__ 
   }
 }
 
-// Block per large box; dynamic shared memory of 5 * kBigRows * kBigWpr words.
+// Block per large box; dynamic shared memory of 6 * kBigRows * kBigWpr words.
 __global__ void __launch_bounds__(256) kb_split_bfs_big(const Slot* __restrict__ slots, int dir_bass,
                                                         int dir_prop) {
   pdl_enter();
@@ -392,7 +380,6 @@ __global__ void __launch_bounds__(256) kb_split_bfs_big(const Slot* __restrict__
   const int* seg = S.seg;
   int* d1 = S.d1;
   int* d2 = S.d2;
-  constexpr int kA = kBigRows * kBigWpr;
   for (int j = blockIdx.x; j < nbig; j += gridDim.x) {
     const int k = S.sm.newid[j];
     const int* bb = S.bbox + 4 * (size_t)k;
@@ -400,6 +387,11 @@ __global__ void __launch_bounds__(256) kb_split_bfs_big(const Slot* __restrict__
     const int bw = bb[1] - x0 + 1, bh = bb[3] - y0 + 1, area = bw * bh;
     const int direction = S.mode ? dir_prop : dir_bass;
     const int s1 = split_seed_index(S, k, 0, direction), s2 = split_seed_index(S, k, 1, direction);
+    if (bw <= 64 * kBigWpr && bh <= kBigRows) {
+      bfs_bits(k, x0, y0, bw, bh, W, seg, half_bits(S), s1, s2, big);
+      __syncthreads();                             // the shared memory is free for the next box
+      continue;
+    }
     for (int i = threadIdx.x; i < area; i += blockDim.x) {
       const int g = (y0 + i / bw) * W + x0 + i % bw;
       if (seg[g] != k) continue;
@@ -407,33 +399,28 @@ __global__ void __launch_bounds__(256) kb_split_bfs_big(const Slot* __restrict__
       __stcg(d2 + g, g == s2 ? 1 : -1);
     }
     __syncthreads();
-    if (bw <= 64 * kBigWpr && bh <= kBigRows) {
-      bfs_bits<256, kA / 256>(threadIdx.x, k, x0, y0, bw, bh, W, seg, d1, d2, big, big + kA,
-                              big + 2 * kA, big + 3 * kA, big + 4 * kA);
-    } else {
-      for (int L = 1; L <= area + 1; L++) {
-        int ch = 0;
-        for (int i = threadIdx.x; i < area; i += blockDim.x) {
-          const int xi = i % bw, yi = i / bw;
-          const int g = (y0 + yi) * W + x0 + xi;
-          if (seg[g] != k) continue;
-          const int a = __ldcg(d1 + g), b = __ldcg(d2 + g);
-          if (a >= 0 && b >= 0) continue;
-          bool h1 = false, h2 = false;
-          auto look = [&](int q) {
-            if (seg[q] != k) return;
-            if (__ldcg(d1 + q) == L) h1 = true;
-            if (__ldcg(d2 + q) == L) h2 = true;
-          };
-          if (xi > 0) look(g - 1);
-          if (xi < bw - 1) look(g + 1);
-          if (yi > 0) look(g - W);
-          if (yi < bh - 1) look(g + W);
-          if (a < 0 && h1) { __stcg(d1 + g, L + 1); ch = 1; }
-          if (b < 0 && h2) { __stcg(d2 + g, L + 1); ch = 1; }
-        }
-        if (!__syncthreads_or(ch)) break;
+    for (int L = 1; L <= area + 1; L++) {
+      int ch = 0;
+      for (int i = threadIdx.x; i < area; i += blockDim.x) {
+        const int xi = i % bw, yi = i / bw;
+        const int g = (y0 + yi) * W + x0 + xi;
+        if (seg[g] != k) continue;
+        const int a = __ldcg(d1 + g), b = __ldcg(d2 + g);
+        if (a >= 0 && b >= 0) continue;
+        bool h1 = false, h2 = false;
+        auto look = [&](int q) {
+          if (seg[q] != k) return;
+          if (__ldcg(d1 + q) == L) h1 = true;
+          if (__ldcg(d2 + q) == L) h2 = true;
+        };
+        if (xi > 0) look(g - 1);
+        if (xi < bw - 1) look(g + 1);
+        if (yi > 0) look(g - W);
+        if (yi < bh - 1) look(g + W);
+        if (a < 0 && h1) { __stcg(d1 + g, L + 1); ch = 1; }
+        if (b < 0 && h2) { __stcg(d2 + g, L + 1); ch = 1; }
       }
+      if (!__syncthreads_or(ch)) break;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < area; i += blockDim.x) {
