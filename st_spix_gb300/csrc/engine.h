@@ -28,7 +28,12 @@ constexpr int kFxFlowShift = 24;
 // The hole fill in one launch (kb_fill): a cluster of blocks per slot, each with two lists of
 // up to kFillList holes in shared memory; one block up to kFillSolo holes (a 720x1280 frame's
 // second fill takes 32 us in one block, 44 in a cluster; limits of 4,096 to 16,384 time alike).
-constexpr int kFillSolo = 4096, kFillList = 16384, kFillSmem = 2 * kFillList * 4;
+// kFillList: above it times the blocks of a cluster (196,608 holes for 16) the loop over all
+// SMs fills.  A strip of 259,000 holes along a 1080x1920 frame takes 6.1 ms in a cluster, 4.7
+// in the loop; of 229,000 5.0 and 4.2; of 180,000 3.37 and 3.32; of 130,000 2.16 and 2.06; of
+// 99,000 1.55 and 1.64.  Holes spread over a 480x854 frame (about 150,000, few iterations)
+// take 0.76 and 0.97, so the line lies where a strip's loss in the cluster is still small.
+constexpr int kFillSolo = 4096, kFillList = 12288, kFillSmem = 2 * kFillList * 4;
 constexpr int kFillBreakIter = 1000;      // fill_missing.cu: break_iter
 constexpr int kSweepVariants = 3;         // sweep tile shapes: 32x32, 64x32, 16x32
 constexpr int kMaxBatchGraphs = 64;       // captured batch steps kept per context
