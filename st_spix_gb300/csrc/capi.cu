@@ -931,9 +931,11 @@ int bass_loop(stspix_ctx* ctx, cudaStream_t st, const List& L, const std::vector
   }
   // final update_params + store_sample; slots that finished earlier were untouched
   // since, so running theirs here is the same as running it right after their loop
-  // (and their statistics are current too: with fuse every sweep moved them)
-  if ((r = params(L, L.B, fuse && maxn > 0 && nit[L.B - 1] > 0, maxn > 0, maxn == 0)))
-    return r;
+  // (and their statistics are current too: with fuse every sweep moved them).  A slot
+  // without iterations has had no posterior on this frame: the snapshot and the prior
+  // shape term that an incremental one reads are another frame's.
+  const bool all_ran = L.B > 0 && nit[L.B - 1] > 0;
+  if ((r = params(L, L.B, fuse && all_ran, all_ran, !all_ran))) return r;
   ctx->cur_fam = STSPIX_FAM_POSTERIOR;
   LAUNCHI(kb_store_sample, L.max_cap, L, L.B);
   return STSPIX_OK;
