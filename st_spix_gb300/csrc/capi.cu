@@ -1416,6 +1416,7 @@ int run_batch(stspix_ctx* ctx, cudaStream_t st, std::vector<FrameDesc>& fr,
     return r;
   ctx->cur_fam = STSPIX_FAM_OTHER;
   LAUNCHS(kb_scalars, La, B);
+  if (ctx->lab_ingest && (stages & kStageSeg)) LAUNCHB(kb_lab_ingest, La.max_npix, La, La.B);
   if ((stages & kStageShift) && (r = shift_fill(ctx, st, Lp))) return r;
   if (!(stages & kStageSeg)) {
     if ((r = read_scalars(ctx, st, B))) return r;
