@@ -39,6 +39,9 @@ WORKLOAD = dict(name="bist_stream_480x854_T30", H=480, W=854, T=30, nseeds=400, 
 # statistics of the new labels, 16 per 4 sweeps (the sweeps keep them current by moving those
 # of every relabelled pixel, so no statistics pass runs between two updates).
 SWEEP_LAUNCH_BYTES_PER_PX = {1: 24, 2: 28, 4: 36}
+# per kernel of the default schedule, for the per-kernel bandwidths of the precision study
+KERNEL_BYTES_PER_PX = dict({"kb_sweep4_" + v: SWEEP_LAUNCH_BYTES_PER_PX[4] for v in "stml"},
+                           kb_accumulate=16)
 # DRAM bytes (read + write) per sweep launch from one ncu capture of the same workload
 # (a batch of 8 frames, mean over the updates of a frame); a constant of that
 # capture, re-taken whenever the sweep kernel changes, not a live measurement.
@@ -753,12 +756,11 @@ def run_precision(args, world, rank):
         res["superpixels"] = int(live.sum())
         per_frame.append(res)
     # per-kernel bandwidth of the int64 run at 4K (CUDA events)
-    bytes_per_px = {"kb_sweep4_m": 80, "kb_sweep4_l": 80, "kb_accumulate": 16}
     gbs = {}
     for k, (nl, ms) in kern.items():
-        if k in bytes_per_px and ms > 0:
+        if k in KERNEL_BYTES_PER_PX and ms > 0:
             gbs[k] = {"launches": nl, "avg_us": 1000 * ms / nl,
-                      "achieved_gbs": bytes_per_px[k] * npix * nl / (ms / 1000) / 1e9}
+                      "achieved_gbs": KERNEL_BYTES_PER_PX[k] * npix * nl / (ms / 1000) / 1e9}
     peak, peak_kind = read_peaks()
     if rank != 0:
         return
