@@ -491,7 +491,11 @@ int stspix_process_batch(stspix_ctx* ctx, void* stream, stspix_frame* frames, in
                          const stspix_config* cfg);
 
 /* Device bytes held per video stream (resident state) and per batch slot (the
- * working buffers of one frame in flight), for admission under a memory budget. */
+ * working buffers of one frame in flight), for admission under a memory budget.
+ * Not among them: 12 bytes a pixel more per slot with stspix_config.lab_ingest (the
+ * converted frame), and the scratch of the quality entry points, which a context that
+ * has used them keeps (the largest call's, rounded up to a power of two; calls that
+ * need more than 256 MiB allocate and free their own).                            */
 int stspix_footprint(int H, int W, int sp_size, long long* video_bytes,
                      long long* slot_bytes);
 /* GPU time (ms) of the last stspix_process_batch call, from CUDA events. */

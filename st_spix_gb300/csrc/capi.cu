@@ -298,10 +298,14 @@ unsigned id_blocks(const stspix_ctx* ctx, long long n, int per, int nb) {
   return (unsigned)std::max(1LL, std::min((n + per - 1) / per, most));
 }
 
+size_t alloc_bytes(size_t size, size_t n) {
+  return (std::max<size_t>(n, 1) * size + 15) & ~size_t(15);
+}
+
 template <typename T>
 int alloc(stspix_ctx* ctx, std::vector<Buf>& list, T** p, size_t n) {
   void* q = nullptr;
-  size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 15) & ~size_t(15);
+  const size_t bytes = alloc_bytes(sizeof(T), n);
   cudaError_t e = cudaMalloc(&q, bytes);
   if (e != cudaSuccess)
     return fail(ctx, STSPIX_ERR_NOMEM, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
@@ -321,37 +325,79 @@ void free_list(std::vector<Buf>& list) {
     if (r_) return r_;                                        \
   } while (0)
 
-int alloc_spdev(stspix_ctx* ctx, std::vector<Buf>& L, SpDev& s, int cap) {
-  s.cap = cap;
-  AL(L, s.count, cap); AL(L, s.valid, cap); AL(L, s.prop, cap);
-  AL(L, s.prior_count, cap); AL(L, s.icount, cap); AL(L, s.sm_count, cap);
-  AL(L, s.mu_app, 3 * (size_t)cap); AL(L, s.mu_shape, 2 * (size_t)cap);
-  AL(L, s.sigma_shape, 3 * (size_t)cap); AL(L, s.logdet, cap);
-  AL(L, s.prior_mu_app, 3 * (size_t)cap); AL(L, s.prior_mu_shape, 2 * (size_t)cap);
-  AL(L, s.prior_sigma_shape, 3 * (size_t)cap); AL(L, s.prior_icov, 3 * (size_t)cap);
-  AL(L, s.sample_sigma_shape, 3 * (size_t)cap); AL(L, s.acc, 8 * (size_t)cap);
-  AL(L, s.rec, cap);
+// The buffers of a frame's pixels, of its superpixels and of a stream's parameters, as calls
+// f(pointer, elements): allocated from these lists, and counted from them for admission under
+// a memory budget (stspix_footprint).
+#define EACH(ptr, n)                                          \
+  do {                                                        \
+    if (int r_ = f(ptr, (size_t)(n))) return r_;              \
+  } while (0)
+
+template <typename F>
+int each_pix(Slot& s, size_t n, F f) {
+  EACH(s.border, n); EACH(s.d1, n); EACH(s.d2, n); EACH(s.smseg, n);
+  EACH(s.hits, n); EACH(s.shifted, n); EACH(s.best, n); EACH(s.seg_alt, n);
+  EACH(s.chg[0], n); EACH(s.chg[1], n);
   return STSPIX_OK;
+}
+
+template <typename F>
+int each_spdev(SpDev& s, size_t cap, F f) {
+  EACH(s.count, cap); EACH(s.valid, cap); EACH(s.prop, cap);
+  EACH(s.prior_count, cap); EACH(s.icount, cap); EACH(s.sm_count, cap);
+  EACH(s.mu_app, 3 * cap); EACH(s.mu_shape, 2 * cap);
+  EACH(s.sigma_shape, 3 * cap); EACH(s.logdet, cap);
+  EACH(s.prior_mu_app, 3 * cap); EACH(s.prior_mu_shape, 2 * cap);
+  EACH(s.prior_sigma_shape, 3 * cap); EACH(s.prior_icov, 3 * cap);
+  EACH(s.sample_sigma_shape, 3 * cap); EACH(s.acc, 8 * cap);
+  EACH(s.rec, cap);
+  return STSPIX_OK;
+}
+
+template <typename F>
+int each_sp(Slot& s, size_t cap, F f) {
+  if (int r = each_spdev(s.sp, cap, f)) return r;
+  if (int r = each_spdev(s.tmp, cap, f)) return r;
+  const size_t c2 = cap + 2;
+  SmDev& sm = s.sm;
+  EACH(sm.count, c2); EACH(sm.s, 3 * c2); EACH(sm.sq, 3 * c2);
+  EACH(sm.pos, 5 * c2);
+  EACH(sm.ninvalid, c2); EACH(sm.pair, c2); EACH(sm.claim, c2);
+  EACH(sm.target, c2); EACH(sm.newid, c2); EACH(sm.flag, c2);
+  EACH(sm.msingle, c2);
+  EACH(s.flags, c2); EACH(s.accept, c2); EACH(s.valid0, c2);
+  EACH(s.living, c2); EACH(s.mint, c2);
+  EACH(s.excl, c2); EACH(s.rid, c2); EACH(s.src_of, c2);
+  EACH(s.cnt_pool, c2); EACH(s.cs, c2); EACH(s.cf, c2);
+  EACH(s.fs, 2 * c2); EACH(s.fds, 2 * c2); EACH(s.ss, c2);
+  EACH(s.centers, 2 * c2); EACH(s.centers_ff, c2); EACH(s.rbest, c2); EACH(s.ccbest, c2);
+  EACH(s.bbox, 4 * c2);
+  EACH(s.snap, 9 * c2); EACH(s.recchg, c2);
+  EACH(s.pscache, 3 * c2);
+  return STSPIX_OK;
+}
+
+template <typename F>
+int each_params(stspix_params& p, size_t cap, F f) {
+  EACH(p.mu_app, 3 * cap); EACH(p.prior_mu_app, 3 * cap);
+  EACH(p.mu_shape, 2 * cap); EACH(p.sigma_shape, 3 * cap);
+  EACH(p.logdet_sigma_shape, cap); EACH(p.prior_mu_shape, 2 * cap);
+  EACH(p.prior_sigma_shape, 3 * cap); EACH(p.sample_sigma_shape, 3 * cap);
+  EACH(p.counts, cap); EACH(p.sm_counts, cap); EACH(p.prior_counts, cap);
+  EACH(p.ids, cap); EACH(p.invalid_counts, cap);
+  return STSPIX_OK;
+}
+#undef EACH
+
+// f of the lists above: allocates into L.
+auto allocate(stspix_ctx* ctx, std::vector<Buf>& L) {
+  return [ctx, &L](auto*& p, size_t n) { return alloc(ctx, L, &p, n); };
 }
 
 int alloc_params(stspix_ctx* ctx, std::vector<Buf>& L, stspix_params& p, int cap) {
   p.capacity = cap;
-  AL(L, p.mu_app, 3 * (size_t)cap); AL(L, p.prior_mu_app, 3 * (size_t)cap);
-  AL(L, p.mu_shape, 2 * (size_t)cap); AL(L, p.sigma_shape, 3 * (size_t)cap);
-  AL(L, p.logdet_sigma_shape, cap); AL(L, p.prior_mu_shape, 2 * (size_t)cap);
-  AL(L, p.prior_sigma_shape, 3 * (size_t)cap); AL(L, p.sample_sigma_shape, 3 * (size_t)cap);
-  AL(L, p.counts, cap); AL(L, p.sm_counts, cap); AL(L, p.prior_counts, cap);
-  AL(L, p.ids, cap); AL(L, p.invalid_counts, cap);
-  return STSPIX_OK;
+  return each_params(p, cap, allocate(ctx, L));
 }
-
-// Bytes of the buffers above (for admission under a memory budget).
-constexpr long long kPixBytes = 1 + 5 * 4 + 8 + 4 + 2;        // border, d1 d2 smseg hits shifted, best, seg_alt, chg x2
-constexpr long long kSpDevBytes = 4 + 1 + 1 + 4 + 4 + 4 + 12 + 16 + 24 + 8 + 12 + 16 + 24 + 24 + 24 +
-                                  64 + (long long)sizeof(SweepRec);
-constexpr long long kSmBytes = 4 + 24 + 24 + 40 + 4 + 4 + 4 + 4 + 4 + 1 + 8;
-constexpr long long kAuxBytes = 5 * 1 + 6 * 4 + 16 + 8 + 4 + 16 + 16 + 8 + 8 + 72 + 1 + 24;
-constexpr long long kParamBytes = 12 + 12 + 16 + 24 + 4 + 16 + 24 + 24 + 4 + 4 + 4 + 4 + 4;
 
 // Make sure slot position i holds npix pixels and sp_cap superpixels.  Growing
 // synchronises the device and does not preserve contents.
@@ -364,38 +410,15 @@ int ensure_slot(stspix_ctx* ctx, int i, int npix, int sp_cap) {
   if (npix > w.npix_cap) {
     CK(cudaDeviceSynchronize());
     free_list(w.pix);
-    auto& L = w.pix;
-    int n = npix;
-    AL(L, s.border, n); AL(L, s.d1, n); AL(L, s.d2, n); AL(L, s.smseg, n);
-    AL(L, s.hits, n); AL(L, s.shifted, n); AL(L, s.best, n); AL(L, s.seg_alt, n);
-    AL(L, s.chg[0], n); AL(L, s.chg[1], n);
+    if (int r = each_pix(s, npix, allocate(ctx, w.pix))) return r;
     w.npix_cap = npix;
   }
   if (sp_cap > w.sp_cap) {
     CK(cudaDeviceSynchronize());
     free_list(w.sp);
-    auto& L = w.sp;
-    int cap = sp_cap;
-    int r;
-    if ((r = alloc_spdev(ctx, L, s.sp, cap))) return r;
-    if ((r = alloc_spdev(ctx, L, s.tmp, cap))) return r;
-    size_t c2 = (size_t)cap + 2;
-    SmDev& sm = s.sm;
-    AL(L, sm.count, c2); AL(L, sm.s, 3 * c2); AL(L, sm.sq, 3 * c2);
-    AL(L, sm.pos, 5 * c2);
-    AL(L, sm.ninvalid, c2); AL(L, sm.pair, c2); AL(L, sm.claim, c2);
-    AL(L, sm.target, c2); AL(L, sm.newid, c2); AL(L, sm.flag, c2);
-    AL(L, sm.msingle, c2);
-    AL(L, s.flags, c2); AL(L, s.accept, c2); AL(L, s.valid0, c2);
-    AL(L, s.living, c2); AL(L, s.mint, c2);
-    AL(L, s.excl, c2); AL(L, s.rid, c2); AL(L, s.src_of, c2);
-    AL(L, s.cnt_pool, c2); AL(L, s.cs, c2); AL(L, s.cf, c2);
-    AL(L, s.fs, 2 * c2); AL(L, s.fds, 2 * c2); AL(L, s.ss, c2);
-    AL(L, s.centers, 2 * c2); AL(L, s.centers_ff, c2); AL(L, s.rbest, c2); AL(L, s.ccbest, c2);
-    AL(L, s.bbox, 4 * c2);
-    AL(L, s.snap, 9 * c2); AL(L, s.recchg, c2);
-    AL(L, s.pscache, 3 * c2);
-    w.sp_cap = cap;
+    s.sp.cap = s.tmp.cap = sp_cap;
+    if (int r = each_sp(s, sp_cap, allocate(ctx, w.sp))) return r;
+    w.sp_cap = sp_cap;
   }
   return STSPIX_OK;
 }
@@ -2090,11 +2113,26 @@ int stspix_footprint(int H, int W, int sp_size, long long* video_bytes, long lon
   double Hh, w;
   int nx, ny;
   hex_geometry(sp_size, W, H, &Hh, &w, &nx, &ny);
-  const long long npix = (long long)H * W;
-  const long long cap = std::max(30LL * nx * ny, 64LL);
-  if (video_bytes) *video_bytes = 4 * npix + 2 * kParamBytes * cap;
-  if (slot_bytes)
-    *slot_bytes = kPixBytes * npix + (2 * kSpDevBytes + kSmBytes + kAuxBytes) * (cap + 2);
+  const size_t npix = (size_t)H * W, cap = (size_t)std::max(30LL * nx * ny, 64LL);
+  long long bytes = 0;
+  auto count = [&](auto*& p, size_t n) {
+    bytes += (long long)alloc_bytes(sizeof(*p), n);
+    return STSPIX_OK;
+  };
+  if (video_bytes) {
+    stspix_params p{};
+    bytes = (long long)alloc_bytes(sizeof(int), npix);
+    each_params(p, cap, count);
+    each_params(p, cap, count);
+    *video_bytes = bytes;
+  }
+  if (slot_bytes) {
+    Slot s{};
+    bytes = 0;
+    each_pix(s, npix, count);
+    each_sp(s, cap, count);
+    *slot_bytes = bytes;
+  }
   return STSPIX_OK;
 }
 

@@ -260,10 +260,15 @@ class Server:
         vb, _ = self._lib.footprint(H, W, req.sp_size or self.sp_default)
         return vb + 4 * H * W * (T if req.keep_labels else 1)
 
+    def slot_bytes(self, req: StreamRequest) -> int:
+        """Working buffers of one of its frames in flight."""
+        H, W = req.vid.shape[1], req.vid.shape[2]
+        b = self._lib.footprint(H, W, req.sp_size or self.sp_default)[1]
+        return b + (12 * H * W if self.cfg.get("lab_ingest") else 0)
+
     def run(self) -> dict:
         """Serve every stream added since the last run; returns its statistics.  The
-        lanes' CUDA streams (and so their engine contexts and tuned tile shapes) are
-        kept for later runs."""
+        lanes' CUDA streams (and so their engine contexts) are kept for later runs."""
         torch = self._torch
         reqs = list(self.requests.values())
         if not reqs:
@@ -272,8 +277,7 @@ class Server:
             self._streams.append(torch.cuda.Stream(self.device))
         self.batch_sizes, self.batch_ms = [], []
         # the largest frame's working buffers for every batch position of every lane
-        slot_b = max(self._lib.footprint(r.vid.shape[1], r.vid.shape[2],
-                                         r.sp_size or self.sp_default)[1] for r in reqs)
+        slot_b = max(self.slot_bytes(r) for r in reqs)
         sched = Scheduler(self.budget, self.lanes * self.max_batch * slot_b, self.max_batch,
                           self.max_pixels, self.group_sizes)
         lock = threading.Lock()
