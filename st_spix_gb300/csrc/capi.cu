@@ -410,12 +410,14 @@ int ensure_slot(stspix_ctx* ctx, int i, int npix, int sp_cap) {
   if (npix > w.npix_cap) {
     CK(cudaDeviceSynchronize());
     free_list(w.pix);
+    w.npix_cap = 0;                                // (a failure below leaves nothing to use)
     if (int r = each_pix(s, npix, allocate(ctx, w.pix))) return r;
     w.npix_cap = npix;
   }
   if (sp_cap > w.sp_cap) {
     CK(cudaDeviceSynchronize());
     free_list(w.sp);
+    w.sp_cap = 0;
     s.sp.cap = s.tmp.cap = sp_cap;
     if (int r = each_sp(s, sp_cap, allocate(ctx, w.sp))) return r;
     w.sp_cap = sp_cap;
@@ -430,6 +432,7 @@ int ensure_lab(stspix_ctx* ctx, int i, int npix) {
   std::lock_guard<std::mutex> lk(g_device_mu);
   CK(cudaDeviceSynchronize());
   free_list(w.lab);
+  w.lab_cap = 0;
   AL(w.lab, w.lab_img, 3 * (size_t)npix);
   w.lab_cap = npix;
   return STSPIX_OK;
@@ -558,7 +561,8 @@ int ensure_bcap(stspix_ctx* ctx, int B) {
   free_list(ctx->ctl_bufs);
   if (ctx->sc_host) { cudaFreeHost(ctx->sc_host); ctx->sc_host = nullptr; }
   if (ctx->h_slots) { cudaFreeHost(ctx->h_slots); ctx->h_slots = nullptr; }
-  int nb = std::max(B, 2 * ctx->bcap);
+  const int nb = std::max(B, 2 * ctx->bcap);
+  ctx->bcap = 0;                                   // (a failure below leaves nothing to use)
   auto& L = ctx->ctl_bufs;
   AL(L, ctx->sc, nb);
   AL(L, ctx->d_slots, 4 * (size_t)nb);
