@@ -332,7 +332,7 @@ def serve_leg(args, dev, rank, streams, frames, fps, lanes=None, max_batch=None,
                        lanes=lanes or args.lanes, device=dev, seed=rank,
                        max_pixels=max_pixels, group_sizes=group_sizes, **cfg)
     # warm-up run (untimed): two short streams per resolution, so that the lanes'
-    # engine contexts exist and the sweep tile classes are tuned
+    # engine contexts exist
     for j, hw in enumerate(sorted(pool) * 2):
         v, f = pool[hw][0]
         srv.add(serve.StreamRequest(-1 - j, v[:4], f[:3], fps=1000.0))

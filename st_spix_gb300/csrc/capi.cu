@@ -76,7 +76,6 @@ struct List {
   int max_words = 0;               // 16-pixel change words
   bool any_prop = false;
   std::vector<int> tiles_upto[kSweepGeoms];  // sweep tiles of the first i slots, per tile size
-  std::vector<long long> segs_upto;  // 32-pixel row segments of the first i slots
 };
 
 }  // namespace stspix
@@ -649,7 +648,6 @@ List make_list(stspix_ctx* ctx, int off, const std::vector<Slot>& slots) {
   List L;
   L.d = ctx->d_slots + (size_t)off * ctx->bcap;
   for (int v = 0; v < kSweepGeoms; v++) L.tiles_upto[v].assign(1, 0);
-  L.segs_upto.assign(1, 0);
   Slot* h = ctx->h_slots + (size_t)off * ctx->bcap;
   L.B = (int)slots.size();
   for (int i = 0; i < L.B; i++) {
@@ -659,8 +657,6 @@ List make_list(stspix_ctx* ctx, int off, const std::vector<Slot>& slots) {
       const int tw = kGeomW[v], th = kGeomH[v];
       L.tiles_upto[v].push_back(s.tile_base[v] + ((s.W + tw - 1) / tw) * ((s.H + th - 1) / th));
     }
-    if (L.segs_upto.empty()) L.segs_upto.push_back(0);
-    L.segs_upto.push_back(L.segs_upto.back() + (long long)s.H * ((s.W + 31) / 32));
     h[i] = s;
     L.max_npix = std::max(L.max_npix, s.npix);
     L.max_cap = std::max(L.max_cap, s.cap);
@@ -796,8 +792,11 @@ int update_seg(stspix_ctx* ctx, cudaStream_t st, const List& L, int nb,
   //   240x320  (0.5 tiles per SM) 2825 / 2900 / -      480x640  (2.0) 3230 / 3235 / -
   //   480x854  (2.7)              3783 / 3415 / 3583   600x1000 (4.0) 4299 / 3781 / 3858
   //   640x1100 (4.6)              4680 / 4189 / 4002   720x1280 (6.1) 5317 / 4565 / 4227
-  // and, with an earlier form, 64x32 / 64x48 tiles: 720x1280 5667 / 5729, 4 frames of 480x854
-  // (10.7) 5188 / 4771, 1080x1920 (13.4) 8273 / 8089.
+  // and 64x32 / 64x48 tiles (single videos of a region per 1,000 pixels, then batches):
+  //   720x1280 (6.1) 4140 / 4120      800x1360  (7.1) 4225 / 4255     900x1400  (8.4) 4650 / 4460
+  //   960x1600 (9.9) 5230 / 4815      1080x1920 (13.4) 5825 / 5600    2160x3840 (54)  15850 / 14270
+  //   480x854 x2 (5.3) 4200 / 4230    x3 (8.0) 4840 / 4620            x4 (10.7) 5600 / 5060
+  //   x6 (16) 6875 / 6510             x8 (21) 8105 / 7410
   const int tl = std::max(1, L.tiles_upto[0][nb]);
   int v;
   if (per == 4) {
@@ -1352,8 +1351,8 @@ std::string batch_signature(const std::vector<FrameDesc>& fr, const std::vector<
 // The batch runner.  stages: kStageShift and/or kStageSeg.  Frames are processed
 // in workspace positions f.slot (distinct).  Returns a call-level error; per-frame
 // statuses land in out.  A batch step whose signature was seen before runs as a
-// CUDA graph: captured on the second occurrence (the first ran eagerly and tuned
-// the sweeps), replayed from then on.
+// CUDA graph: captured on the second occurrence (the first ran eagerly), replayed from
+// then on.
 int run_batch(stspix_ctx* ctx, cudaStream_t st, std::vector<FrameDesc>& fr,
               const stspix_config& cfg, int stages, BatchOut& out, int stop_after = -1,
               int extra_update = 0, int split_dir = 0) {

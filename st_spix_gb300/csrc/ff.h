@@ -94,7 +94,7 @@ __device__ __forceinline__ bool log_ff(double x, float* out) {
   const float wh = zh * u.h, wl = fmaf(zh, u.h, -wh) + (zh * u.l + zl * u.h);
   const float p = q * wh, pe = fmaf(q, wh, -p) + (q * wl + ql * wh);
   const float lh = 2.f * (q + p), ll = 2.f * ((p - ((q + p) - q)) + (pe + ql));
-  // + e log 2, log 2 = 355 / 512 (times e exact) + a pair
+  // + e log 2, log 2 = 355 / 512 (times e exact; the split of Cody and Waite 1980) + a pair
   constexpr FF k2 = FF_CONST(-2.121944400546905827679e-4);
   const float ef = (float)e;
   const float a = ef * 0.693359375f, b = ef * k2.h;

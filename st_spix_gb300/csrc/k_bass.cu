@@ -729,8 +729,10 @@ __global__ void __launch_bounds__(128) kb_posterior(const Slot* __restrict__ slo
 }
 
 // clear_fields + the helper memset (update_params.cu:54-88, :26): zero the counts and
-// the sums of every slot, of all ids (once per frame) or of the ids in use (a step that
-// raises max_spix is followed by such a clear, so an id's sums start at zero).
+// the sums of every slot, of all ids (once per frame) or of the ids in use.  An id that a
+// step adds gets its sums from that step (kb_split_commit; for minted ids the merge's sums,
+// which the posterior takes over), or from such a clear and a pass over the pixels (the
+// FP32 and FP64 accumulators).
 __global__ void kb_clear_stats(const Slot* __restrict__ slots, int all) {
   pdl_enter();
   SLOT_Y;
@@ -977,9 +979,9 @@ constexpr int kReach = 4;             // a sweep's labels depend on labels this 
 // ones plus, for every pixel a launch relabels from C to bl, its contribution moved
 // from C to bl.  A sweep block collects the moves of its tile's own pixels in a small
 // table in shared memory (label -> count and sums, 32-bit fields: colours split into
-// 16-bit parts, positions relative to the tile; at most 2048 pixels move) and adds each
-// touched label's net change to its 64-bit global sums once per launch.  Integer sums, so the result is identical to clearing and
-// summing every pixel again.
+// 16-bit parts, positions relative to the tile; a tile has at most 3072 pixels to move) and
+// adds each touched label's net change to its 64-bit global sums once per launch.  Integer
+// sums, so the result is identical to clearing and summing every pixel again.
 constexpr int kDeltaTab = 64;         // labels a tile's moves can touch (a power of two)
 
 struct DeltaTab {
@@ -1079,6 +1081,7 @@ struct SweepTile {
   static constexpr int kMaxList = kClass > TX * TY ? kClass : TX * TY;
   static_assert(kLX < 256 && kLY < 256, "list entries pack (y << 8) | x");
   static_assert(kLX % 8 == 0 && kLY % 8 == 0, "8-pixel groups, rows in whole warp spans");
+  static_assert((long long)TX * TY * 65535 < (1LL << 31), "statistics moves fit 32 bits");
   static_assert(kSH % 2 == 0 && TX % 16 == 0 && TY % 2 == 0, "region parity = image parity");
   __align__(16) int L[kLX * kLY];
   unsigned short list[kMaxList];      // pixels of the running phase, (y << 8) | x
