@@ -1171,6 +1171,8 @@ def main():
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if peak else None, "traffic": SWEEP_TRAFFIC_NCU["bytes_per_launch"],
                      "traffic_source": SWEEP_TRAFFIC_NCU["source"],
+                     "note": "algorithmic bytes count every colour; the kernel reads those of "
+                             "scored pixels only and is bound by issue and barriers",
                      "peak_source": peak_kind,
                      "algorithmic_bytes_per_launch": per_launch,
                      "dominant_family": fam,
